@@ -19,6 +19,7 @@
 
 #include "../../include/assist.h"
 #include "device_forces.cuh"
+#include "fast_forces.cuh"
 #include "internal.h"
 #include "shared_sim.h"
 
@@ -72,6 +73,8 @@ static ForceCfg make_cfg(int forces, int gr, int geo, double alpha, double nk, d
     c.e_ca = std::cos(rae); c.e_sa = std::sin(rae); c.e_cd = std::cos(dece); c.e_sd = std::sin(dece);
     const double ras = 286.13 * M_PI / 180., decs = 63.87 * M_PI / 180.;
     c.s_ca = std::cos(ras); c.s_sa = std::sin(ras); c.s_cd = std::cos(decs); c.s_sd = std::sin(decs);
+    const double pole[8] = {c.e_sa, c.e_ca, c.e_sd, c.e_cd, c.s_sa, c.s_ca, c.s_sd, c.s_cd};
+    for (int k = 0; k < 8; k++) c.f_pole[k] = (float)pole[k];
     return c;
 }
 
@@ -607,7 +610,8 @@ struct BatchScratch {
     float2* d_sunv = nullptr;
     double* h_in = nullptr;         /* pinned: t0, t_end, states, parameters read back for grouping */
     size_t h_in_cap = 0;
-    float* h_ratio = nullptr;       /* pinned: the pilot's ratios */
+    float* h_ratio = nullptr;       /* pinned: the pilot's ratios, then its deep-pass flags */
+    unsigned char* d_deep = nullptr;
     int h_ratio_cap = 0;
 };
 #define AG_PILOT_G 1024
@@ -918,6 +922,8 @@ struct AgLaunchPlan {
     std::vector<int> order, gstart, gsize;
     bool grouped = false, coop = false;
     bool learned = false;           /* the warm-start build of the block-cooperative kernel */
+    bool fast = false;              /* the kernel on fast_forces.cuh, but for the first n_deep groups */
+    int n_deep = 0, deep_slots = 0;
     int occ = 2, stage = 0, tpb = 128, nslots = 0;
 };
 
@@ -980,6 +986,8 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
      * device while the host sorts the batch; its ratios are read before the
      * group costs are formed */
     const float* enc = nullptr;
+    unsigned char* deep = nullptr;      /* particles that pass deep inside a planet's sphere of influence */
+    const bool may_fast = o->group_steps == 2 && n_var == 0 && ag_fast_covers(c);
     if (grouped) {
         double tmin = t0[0], tmax = t0[0];
         for (int i = 0; i < n; i++) {
@@ -988,12 +996,15 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
         }
         if (g_batch.ratio_cap < n) {
             if (g_batch.d_ratio) cudaFree(g_batch.d_ratio);
+            if (g_batch.d_deep) cudaFree(g_batch.d_deep);
             if (g_batch.h_ratio) cudaFreeHost(g_batch.h_ratio);
             g_batch.d_ratio = nullptr;
+            g_batch.d_deep = nullptr;
             g_batch.h_ratio = nullptr;
             g_batch.ratio_cap = 0;
             if (ag_cuda_check(cudaMalloc(&g_batch.d_ratio, sizeof(float) * (size_t)n), "cudaMalloc(pilot)") ||
-                ag_cuda_check(cudaMallocHost(&g_batch.h_ratio, sizeof(float) * (size_t)n), "cudaMallocHost(pilot)"))
+                ag_cuda_check(cudaMalloc(&g_batch.d_deep, (size_t)n), "cudaMalloc(pilot)") ||
+                ag_cuda_check(cudaMallocHost(&g_batch.h_ratio, (sizeof(float) + 1) * (size_t)n), "cudaMallocHost(pilot)"))
                 return ASSIST_ERROR_EPHEM_FILE;
             g_batch.ratio_cap = n;
         }
@@ -1002,12 +1013,18 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
              ag_cuda_check(cudaMalloc(&g_batch.d_sunv, sizeof(float2) * AG_PILOT_G), "cudaMalloc(pilot grid)")))
             return ASSIST_ERROR_EPHEM_FILE;
         if (ag_cuda_check((cudaError_t)ag_pilot_encounters(D, n, d_t0, d_t_end, d_state, tmin, tmax, g_batch.d_ratio,
-                                                           g_batch.d_grid, g_batch.d_sunv, AG_PILOT_G, s),
+                                                           may_fast ? g_batch.d_deep : nullptr, g_batch.d_grid,
+                                                           g_batch.d_sunv, AG_PILOT_G, s),
                           "pilot kernels") ||
             ag_cuda_check(cudaMemcpyAsync(g_batch.h_ratio, g_batch.d_ratio, sizeof(float) * n, cudaMemcpyDeviceToHost, s),
                           "read pilot"))
             return ASSIST_ERROR_EPHEM_FILE;
         enc = g_batch.h_ratio;
+        if (may_fast) {
+            deep = reinterpret_cast<unsigned char*>(g_batch.h_ratio + g_batch.ratio_cap);
+            if (ag_cuda_check(cudaMemcpyAsync(deep, g_batch.d_deep, (size_t)n, cudaMemcpyDeviceToHost, s), "read pilot"))
+                return ASSIST_ERROR_EPHEM_FILE;
+        }
     }
     std::vector<int> order((size_t)n), gstart, gsize;
     for (int i = 0; i < n; i++) order[(size_t)i] = i;
@@ -1063,8 +1080,28 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
                 occ = (int)gstart.size() >= 8 * 3 * sms ? 3 : 2;
             }
         }
-        nslots = ag_coop_max_slots(n_var, occ, stage, P.learned ? 1 : 0);
-        const int need = 32 * (int)gstart.size();
+        P.fast = may_fast;
+        if (P.fast && !P.learned) {
+            /* groups with a deep pass first in the list: the kernel with all
+             * terms in FP64 takes them */
+            std::vector<int> s2, z2;
+            for (int pass = 0; pass < 2; pass++) {
+                for (size_t k = 0; k < gstart.size(); k++) {
+                    bool d = false;
+                    for (int i = 0; i < gsize[k] && !d; i++) d = deep[order[(size_t)(gstart[k] + i)]] != 0;
+                    if (d == (pass == 0)) { s2.push_back(gstart[k]); z2.push_back(gsize[k]); }
+                }
+                if (pass == 0) P.n_deep = (int)s2.size();
+            }
+            gstart.swap(s2);
+            gsize.swap(z2);
+            const int need = 32 * P.n_deep;
+            P.deep_slots = ag_coop_max_slots(0, 2, 0, 0);
+            if (P.deep_slots > need) P.deep_slots = need;
+        }
+        nslots = P.fast ? ag_fast_max_slots(occ, stage, P.learned ? 1 : 0, D.n_ast)
+                        : ag_coop_max_slots(n_var, occ, stage, P.learned ? 1 : 0);
+        const int need = 32 * ((int)gstart.size() - P.n_deep);
         if (nslots > need) nslots = need;
     } else if (grouped) {
         nslots = ag_group_max_slots(n_var);
@@ -1088,6 +1125,43 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
     return ASSIST_SUCCESS;
 }
 
+/* The batched kernels of a launch plan on stream s.  With groups on both
+ * kernels the pair-term one runs on a stream forked from s and joined again;
+ * a.queue holds two counters then. */
+static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var, cudaStream_t s) {
+    if (!P.fast)
+        return P.coop ? ag_launch_coop(P.D, P.c, a, n_var, P.occ, P.stage, s)
+                      : (P.grouped ? ag_launch_group(P.D, P.c, a, n_var, s) : ag_launch_batch(P.D, P.c, a, n_var, P.tpb, s));
+    AgBatchArgs f = a;
+    f.grp_start += P.n_deep;
+    f.grp_size += P.n_deep;
+    f.n_groups -= P.n_deep;
+    if (!P.n_deep) return ag_launch_fast(P.D, P.c, f, P.occ, P.stage, s);
+    AgBatchArgs d = a;
+    d.n_groups = P.n_deep;
+    d.nslots = P.deep_slots;
+    d.queue = a.queue + 1;
+    if (!f.n_groups) return ag_launch_coop(P.D, P.c, d, 0, 2, 0, s);
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int e = (int)cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+    if (!e) e = (int)cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    if (!e) e = (int)cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+    if (!e) e = (int)cudaEventRecord(fork, s);
+    if (!e) e = (int)cudaStreamWaitEvent(side, fork, 0);
+    if (!e) {
+        /* the longest groups start first: the other kernel's blocks fill the device */
+        e = ag_launch_coop(P.D, P.c, d, 0, 2, 0, s);
+        if (!e) e = ag_launch_fast(P.D, P.c, f, P.occ, P.stage, side);
+        const int j = (int)cudaEventRecord(join, side), w = (int)cudaStreamWaitEvent(s, join, 0);
+        if (!e) e = j ? j : w;
+    }
+    if (fork) cudaEventDestroy(fork);
+    if (join) cudaEventDestroy(join);
+    if (side) cudaStreamDestroy(side);
+    return e;
+}
+
 static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_gb300_options* o, int n,
                               const double* d_t0, const double* d_t_end, double* d_state, const double* d_params,
                               int n_var, double* d_var_state, int* d_status, void* stream,
@@ -1100,13 +1174,11 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
     std::lock_guard<std::mutex> lk(g_batch_mu);
     AgLaunchPlan P;
     if ((rc = ag_batch_prepare(e, o, n, d_t0, d_t_end, d_state, d_params, n_var, s, P))) return rc;
-    const DevEphem& D = P.D;
-    const ForceCfg& c = P.c;
     const std::vector<int>& order = P.order;
     const std::vector<int>& gstart = P.gstart;
     const std::vector<int>& gsize = P.gsize;
     const bool grouped = P.grouped, coop = P.coop;
-    const int occ = P.occ, stage = P.stage, tpb = P.tpb, nslots = P.nslots;
+    const int nslots = P.nslots;
     if (g_batch.order_cap < n) {
         if (g_batch.d_order) cudaFree(g_batch.d_order);
         if (ag_cuda_check(cudaMalloc(&g_batch.d_order, sizeof(int) * (size_t)n), "cudaMalloc(order)")) return ASSIST_ERROR_EPHEM_FILE;
@@ -1121,7 +1193,7 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
     /* counters: 8 words, then the per-SM block counters of the role rotation */
     const size_t cnt_bytes = 8 * sizeof(unsigned long long) + AG_SM_SLOTS * sizeof(int);
     if (!g_batch.d_queue) {
-        if (ag_cuda_check(cudaMalloc(&g_batch.d_queue, sizeof(int)), "cudaMalloc") ||
+        if (ag_cuda_check(cudaMalloc(&g_batch.d_queue, 2 * sizeof(int)), "cudaMalloc") ||
             ag_cuda_check(cudaMalloc(&g_batch.d_counters, cnt_bytes), "cudaMalloc"))
             return ASSIST_ERROR_EPHEM_FILE;
     }
@@ -1140,7 +1212,7 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
         cudaMemcpyAsync(g_batch.d_grp, gstart.data(), sizeof(int) * (size_t)ng, cudaMemcpyHostToDevice, s);
         cudaMemcpyAsync(g_batch.d_grp + ng, gsize.data(), sizeof(int) * (size_t)ng, cudaMemcpyHostToDevice, s);
     }
-    cudaMemsetAsync(g_batch.d_queue, 0, sizeof(int), s);
+    cudaMemsetAsync(g_batch.d_queue, 0, 2 * sizeof(int), s);
     cudaMemsetAsync(g_batch.d_counters, 0, cnt_bytes, s);
     AgBatchArgs a;
     std::memset(&a, 0, sizeof(a));
@@ -1169,8 +1241,7 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0); cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    int le = coop ? ag_launch_coop(D, c, a, n_var, occ, stage, s)
-                  : (grouped ? ag_launch_group(D, c, a, n_var, s) : ag_launch_batch(D, c, a, n_var, tpb, s));
+    const int le = ag_launch_plan(P, a, n_var, s);
     cudaEventRecord(e1, s);
     if (le) { cudaEventDestroy(e0); cudaEventDestroy(e1); ag_cuda_check((cudaError_t)le, "batch kernel launch"); return ASSIST_ERROR_EPHEM_FILE; }
     if (stats) {
@@ -1257,7 +1328,7 @@ extern "C" int assist_gb300_plan_create(const struct assist_ephem* e, const stru
     const size_t wsn = ag_batch_ws_doubles(P.nslots, n_var);
     bool ok = !ag_cuda_check(cudaMalloc(&p->d_order, sizeof(int) * (size_t)n), "cudaMalloc(plan order)") &&
               (!P.grouped || !ag_cuda_check(cudaMalloc(&p->d_grp, sizeof(int) * 2 * (size_t)ng), "cudaMalloc(plan groups)")) &&
-              !ag_cuda_check(cudaMalloc(&p->d_queue, sizeof(int)), "cudaMalloc(plan queue)") &&
+              !ag_cuda_check(cudaMalloc(&p->d_queue, 2 * sizeof(int)), "cudaMalloc(plan queue)") &&
               !ag_cuda_check(cudaMalloc(&p->d_counters, 8 * sizeof(unsigned long long) + AG_SM_SLOTS * sizeof(int)),
                              "cudaMalloc(plan counters)") &&
               !ag_cuda_check(cudaMalloc(&p->d_ws, sizeof(double) * wsn), "cudaMalloc(plan IAS15 slots)") &&
@@ -1267,7 +1338,8 @@ extern "C" int assist_gb300_plan_create(const struct assist_ephem* e, const stru
                (!ag_cuda_check(cudaMemcpy(p->d_grp, P.gstart.data(), sizeof(int) * (size_t)ng, cudaMemcpyHostToDevice), "plan groups") &&
                 !ag_cuda_check(cudaMemcpy(p->d_grp + ng, P.gsize.data(), sizeof(int) * (size_t)ng, cudaMemcpyHostToDevice), "plan groups"))) &&
               !ag_cuda_check((cudaError_t)ag_batch_ready(), "batched kernel set-up") &&
-              !ag_cuda_check((cudaError_t)ag_coop_ready(), "batched kernel set-up");
+              !ag_cuda_check((cudaError_t)ag_coop_ready(), "batched kernel set-up") &&
+              !ag_cuda_check((cudaError_t)ag_fast_ready(), "batched kernel set-up");
     if (!ok) { assist_gb300_plan_free(p); return ASSIST_ERROR_EPHEM_FILE; }
     AgBatchArgs& a = p->a;
     std::memset(&a, 0, sizeof(a));
@@ -1292,10 +1364,9 @@ extern "C" int assist_gb300_plan_create(const struct assist_ephem* e, const stru
     int le = 0;
     ok = !ag_cuda_check(cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed), "plan capture");
     if (ok) {
-        cudaMemsetAsync(p->d_queue, 0, sizeof(int), cs);
+        cudaMemsetAsync(p->d_queue, 0, 2 * sizeof(int), cs);
         cudaMemsetAsync(p->d_counters, 0, 8 * sizeof(unsigned long long) + AG_SM_SLOTS * sizeof(int), cs);
-        le = P.coop ? ag_launch_coop(P.D, P.c, a, n_var, P.occ, P.stage, cs)
-                    : (P.grouped ? ag_launch_group(P.D, P.c, a, n_var, cs) : ag_launch_batch(P.D, P.c, a, n_var, P.tpb, cs));
+        le = ag_launch_plan(P, a, n_var, cs);
         cudaMemcpyAsync(p->h_counters, p->d_counters, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, cs);
         const cudaError_t ce = cudaStreamEndCapture(cs, &p->graph);
         ok = !le && !ag_cuda_check(ce, "plan capture") &&
@@ -1407,7 +1478,7 @@ extern "C" int assist_gb300_encounter_ratio_device(const struct assist_ephem* e,
         (ag_cuda_check(cudaMalloc(&g_batch.d_grid, sizeof(float4) * AG_PILOT_G * 10), "cudaMalloc(pilot grid)") ||
          ag_cuda_check(cudaMalloc(&g_batch.d_sunv, sizeof(float2) * AG_PILOT_G), "cudaMalloc(pilot grid)")))
         return ASSIST_ERROR_EPHEM_FILE;
-    if (ag_cuda_check((cudaError_t)ag_pilot_encounters(D, n, d_t0, d_t_end, d_state, tmin, tmax, d_ratio,
+    if (ag_cuda_check((cudaError_t)ag_pilot_encounters(D, n, d_t0, d_t_end, d_state, tmin, tmax, d_ratio, nullptr,
                                                        g_batch.d_grid, g_batch.d_sunv, AG_PILOT_G, s),
                       "pilot kernels") ||
         ag_cuda_check(cudaStreamSynchronize(s), "pilot kernels"))

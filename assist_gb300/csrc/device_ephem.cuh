@@ -18,11 +18,16 @@
 
 #include <cstdint>
 
+#include "pair_terms.cuh"
+
 #define AG_NPL 11
 #define AG_MAX_AST 32
 #define AG_MAX_BODIES (AG_NPL + AG_MAX_AST)
 #define AG_MAX_NCF 24
 #define AG_MAX_SPK_P 32
+/* bodies of the pair terms: every planet but Jupiter, then the asteroids */
+#define AG_PAIR_PL 9
+#define AG_MAX_PACKS ((AG_PAIR_PL + AG_MAX_AST + 1) / 2)
 
 enum { AG_OK = 0, AG_ERR_EPHEM_FILE = 1, AG_ERR_AST_FILE = 2, AG_ERR_NAST = 3, AG_ERR_NEPHEM = 4, AG_ERR_COVERAGE = 5 };
 enum { AG_SUN = 0, AG_MER, AG_VEN, AG_EAR, AG_MOO, AG_MAR, AG_JUP, AG_SAT, AG_URA, AG_NEP, AG_PLU };
@@ -44,6 +49,18 @@ struct AgSpkSeg {
  * z = 86400/RADIUS, w unused (32-byte aligned for one vector load). */
 struct __align__(32) AgRecMeta {
     double x, y, z, w;
+};
+
+/* What the pair terms read of the masses and constants (host_ephem.cpp fills
+ * it): per two bodies GM and threshold, the Sun's GM and 1/c^2 as float
+ * pairs, FP32 coefficients of the harmonics, and the .440 columns 0..9 by
+ * falling coefficient count. */
+struct AgPairView {
+    AgPkGm gm[AG_MAX_PACKS];
+    float gm_sun_h, gm_sun_l, oc2_h, oc2_l;
+    float gm_jup, ek2, ek3, ek4, sk2;
+    int n_packs;
+    int col_sorted[10];
 };
 
 /* Everything a kernel needs to evaluate bodies; passed by value. */
@@ -85,11 +102,18 @@ struct DevEphem {
     double au_km;                /* the file's AU (km) */
     /* constants (ASSIST src/assist.c:296-309) */
     double J2E, J3E, J4E, J2SUN, Re_eq, Rs_eq, c_squared, over_c_squared;
+    AgPairView pv;
     /* device copy of this view: kernels read the ephemeris through it (a
      * by-value kernel parameter indexed with run-time indices would be
      * copied into every thread's local memory) */
     const struct DevEphem* self_dev;
 };
+
+/* Body k of the pair terms' list as a planet index (k < AG_PAIR_PL). */
+__host__ __device__ __forceinline__ int ag_pair_planet(int k) {
+    /* Mercury, Venus, Earth, Moon, Mars, Saturn, Uranus, Neptune, Pluto */
+    return k < 5 ? k + 1 : k + 2;
+}
 
 /* isnormal() for a non-negative argument (the IAS15 error measures take
  * maxima of |a| and |b|): at least the smallest normal double and finite;

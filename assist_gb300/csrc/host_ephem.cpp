@@ -19,6 +19,7 @@
  * The parsed files are copied to device memory once; the kernels read the
  * same words ASSIST reads through its mmap.
  */
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -449,6 +450,37 @@ static void ag_ascii_view(const ascii_s* a, DevEphem& D) {
     D.pl_inv_inc = 1.0 / a->inc;
 }
 
+/* The pair terms' view of the masses and constants (pair_terms.cuh). */
+static void ag_pair_view(DevEphem& D) {
+    AgPairView& V = D.pv;
+    const int n = AG_PAIR_PL + D.n_ast;
+    std::memset(&V, 0, sizeof(V));
+    V.n_packs = (n + 1) / 2;
+    for (int k = 0; k < n; k++) {
+        const bool planet = k < AG_PAIR_PL;
+        const double gm = planet ? D.gm[ag_pair_planet(k)] : D.ast_gm[k - AG_PAIR_PL];
+        const float hi = (float)gm, lo = (float)(gm - (double)hi), thr = ag_pair_thr2(gm / D.gm[AG_SUN]);
+        AgPkGm& G = V.gm[k / 2];
+        std::memcpy((char*)&G.h + 4 * (k & 1), &hi, 4);
+        std::memcpy((char*)&G.l + 4 * (k & 1), &lo, 4);
+        ((k & 1) ? G.tb : G.ta) = thr;
+        ((k & 1) ? G.gb : G.ga) = planet ? hi : 0.0f;
+    }
+    const double gms = D.gm[AG_SUN], gme = D.gm[AG_EAR], Re2 = D.Re_eq * D.Re_eq;
+    V.gm_sun_h = (float)gms;
+    V.gm_sun_l = (float)(gms - (double)V.gm_sun_h);
+    V.oc2_h = (float)D.over_c_squared;
+    V.oc2_l = (float)(D.over_c_squared - (double)V.oc2_h);
+    V.gm_jup = (float)D.gm[AG_JUP];
+    V.ek2 = (float)(gme * 1.5 * D.J2E * Re2);
+    V.ek3 = (float)(gme * 2.5 * D.J3E * Re2 * D.Re_eq);
+    V.ek4 = (float)(gme * 0.625 * D.J4E * Re2 * Re2);
+    V.sk2 = (float)(gms * 1.5 * D.J2SUN * D.Rs_eq * D.Rs_eq);
+    for (int k = 0; k < 10; k++) V.col_sorted[k] = k;
+    if (!D.pl_spk)
+        std::stable_sort(V.col_sorted, V.col_sorted + 10, [&](int a, int b) { return D.col_ncf[a] > D.col_ncf[b]; });
+}
+
 /* Asteroids and constants, then the device copy of the view. */
 static int ag_finish_view(const struct assist_ephem* e, DevEphem& D, DevEphem* out, bool may_upload) {
     const spk_s* s = e->spk_asteroids;
@@ -474,6 +506,8 @@ static int ag_finish_view(const struct assist_ephem* e, DevEphem& D, DevEphem* o
     /* the view is owned by the planets object (one view per ephemeris) */
     DevEphem** d_view = e->spk_planets ? &e->spk_planets->d_view : &e->ascii_planets->d_view;
     DevEphem* h_view = e->spk_planets ? &e->spk_planets->h_view : &e->ascii_planets->h_view;
+    /* the pair terms' view follows from the rest: formed only when that changed */
+    std::memcpy(&D.pv, &h_view->pv, sizeof(D.pv));
     if (!may_upload) {
         /* the device view must exist and match the ephemeris as it is now */
         if (!*d_view) {
@@ -494,6 +528,7 @@ static int ag_finish_view(const struct assist_ephem* e, DevEphem& D, DevEphem* o
     D.self_dev = *d_view;
     if (std::memcmp(h_view, &D, sizeof(D)) != 0) {
         /* the view changed (first use, jd_ref or constants edited): refresh the device copy */
+        ag_pair_view(D);
         if (ag_cuda_check(cudaMemcpy(*d_view, &D, sizeof(D), cudaMemcpyHostToDevice), "upload ephemeris view"))
             return ASSIST_ERROR_EPHEM_FILE;
         *h_view = D;

@@ -51,6 +51,7 @@
  */
 
 #include "coop_forces.cuh"
+#include "ias15_warm.cuh"
 
 /* b, e of one component from the last accepted step's br, er (the shift of
  * the acceleration polynomial to the new step). */
@@ -120,93 +121,19 @@ struct AgCoopShared {
     int rot;                                        /* role rotation of this block */
 };
 
-/* Shared buffers of the learned warm start (dynamic shared memory, present
- * only when a network is loaded or steps are logged). */
-struct AgWarmSmem {
-    AgMlpSmem M;
-    double corr[7][3][32];          /* (br - er)_kc of each lane */
-    float bpa[7][3][32];            /* |b_pred_kc| */
-    float tgt[7][3][32];            /* logged targets */
-    float xf[32][AG_MLP_IN + 1];    /* features of this step (logged with the target) */
-    double kappa[7][32];
-    int valid[32];
-};
-
 /* Distance from (x, y, z) to the nearest of the eleven planets in the table. */
-__device__ __forceinline__ double ag_nearest_planet(const AgTable& T, double x, double y, double z) {
-    double m = 1e300;
+struct AgTableNearest {
+    const AgTable& T;
+    __device__ __forceinline__ double operator()(double x, double y, double z) const {
+        double m = 1e300;
 #pragma unroll
-    for (int k = 0; k < AG_NPL; k++) {
-        const double dx = x - T.P.x[k], dy = y - T.P.y[k], dz = z - T.P.z[k];
-        m = fmin(m, fma(dx, dx, fma(dy, dy, dz * dz)));
-    }
-    return sqrt(m);
-}
-
-/* Node-0 part of the learned warm start for one group (all threads of the
- * block call it): owners publish (br - er) and |b_pred| of the particle's
- * x, y, z (variational particles keep the plain prediction), warp 0 forms
- * the features, the block runs the network, owners add kappa_k y_kc to b.
- * Every 8th step of a group is a plain probe (no inference).  Returns whether
- * the network ran (block-uniform).  Kept out of line so the plain kernel's
- * register allocation is not shaped by it. */
-template <int NV>
-__device__ __noinline__ bool ag_coop_warm_start(const AgBatchArgs& A, double* ws, int nslots, int slot, AgWarmSmem& WS,
-                                               const AgTable& Tab, int lane, int wid, bool live, bool warm, bool wl_on,
-                                               double hstep, double dtls, long long steps, bool& w_applied,
-                                               bool& w_probe, unsigned long long& n_wused,
-                                               unsigned long long& n_wfall) {
-    const Ws<3 * (1 + NV)> W{ws, nslots, slot};
-    const int pc = ag_coop_pcomp<NV>(wid);
-    if (live && pc >= 0)
-        for (int k = 0; k < 7; k++) {
-            WS.corr[k][pc][lane] = W(W_BR + k, pc) - W(W_ER + k, pc);
-            WS.bpa[k][pc][lane] = (float)fabs(W(W_B + k, pc));
+        for (int k = 0; k < AG_NPL; k++) {
+            const double dx = x - T.P.x[k], dy = y - T.P.y[k], dz = z - T.P.z[k];
+            m = fmin(m, fma(dx, dx, fma(dy, dy, dz * dz)));
         }
-    __syncthreads();
-    if (wid == 0) {
-        bool ok = false;
-        if (live) {
-            double corr[7][3], kap[7];
-            float bpa[7][3], x[AG_MLP_IN];
-            for (int k = 0; k < 7; k++)
-                for (int c = 0; c < 3; c++) { corr[k][c] = WS.corr[k][c][lane]; bpa[k][c] = WS.bpa[k][c][lane]; }
-            const double x0 = W(W_X0, 0), y0 = W(W_X0, 1), z0 = W(W_X0, 2);
-            const double rx = sqrt(fma(x0, x0, fma(y0, y0, z0 * z0)));
-            ok = ag_warm_features(corr, bpa, hstep, dtls, rx, ag_nearest_planet(Tab, x0, y0, z0), x, kap);
-            for (int k = 0; k < 7; k++) WS.kappa[k][lane] = kap[k];
-            for (int i = 0; i < AG_MLP_IN; i++) { WS.xf[lane][i] = x[i]; WS.M.X[lane][i] = __float2bfloat16_rn(x[i]); }
-        } else {
-            for (int i = 0; i < AG_MLP_IN; i++) WS.M.X[lane][i] = __float2bfloat16_rn(0.0f);
-        }
-        WS.valid[lane] = ok ? 1 : 0;
+        return sqrt(m);
     }
-    __syncthreads();
-    const bool valid = live && WS.valid[lane];
-    w_probe = warm && valid && wl_on && (steps & 7) == 7;
-    const bool want = warm && valid && wl_on && !w_probe;
-    const bool ran = __syncthreads_or(want);
-    if (ran) {
-        ag_mlp_infer_block(*A.mlp, WS.M, wid, lane);
-        if (want) {
-            bool ok_y = true;
-            for (int o = 0; o < AG_MLP_OUT; o++) {
-                const float y = WS.M.Y[lane][o];
-                ok_y = ok_y && isfinite(y) && fabsf(y) <= AG_MLP_YCLIP;
-            }
-            if (ok_y) {
-                w_applied = true;
-                if (pc >= 0)
-                    for (int k = 0; k < 7; k++)
-                        W(W_B + k, pc) = fma(WS.kappa[k][lane], (double)WS.M.Y[lane][3 * k + pc], W(W_B + k, pc));
-                if (wid == 0) n_wused++;
-            } else if (wid == 0) {
-                n_wfall++;
-            }
-        }
-    }
-    return ran;
-}
+};
 
 /* Dynamic shared memory of a block: the warm-start buffers (when present)
  * or, in the plain kernel without variational particles, the group's IAS15
@@ -490,9 +417,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             bool w_applied = false, w_probe = false, w_ran = false;
             if constexpr (WARM) {
                 if (warm || logp)
-                    w_ran = ag_coop_warm_start<NV>(A, W.w, W.ns, W.slot, WS, Tab.T, lane, wid, live, warm,
-                                                   wl_on && S.wg_off == 0, hstep, dtls, steps, w_applied, w_probe,
-                                                   n_wused, n_wfall);
+                    w_ran = ag_warm_start<C>(A, W.w, W.ns, W.slot, ag_coop_pcomp<NV>(wid), WS, AgTableNearest{Tab.T}, lane,
+                                             wid, live, warm, wl_on && S.wg_off == 0, hstep, dtls, steps, w_applied,
+                                             w_probe, n_wused, n_wfall);
             }
             if (live) {
                 for (int comp = 0; comp < C; comp++) {
@@ -723,29 +650,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             }
             /* ---- log (features, target) pairs of accepted steps: target =
              * (b_conv - b_pred) / kappa with b_pred = e + (br - er), the plain prediction */
-            if (logp) {
-                const bool lg = live && WS.valid[lane] && (steps % A.log_every) == 0;
-                if (lg && ag_coop_pcomp<NV>(wid) >= 0)
-                    for (int k = 0; k < 7; k++) {
-                        const int c = ag_coop_pcomp<NV>(wid);
-                        const double bp = W(W_E + k, c) + (W(W_BR + k, c) - W(W_ER + k, c));
-                        WS.tgt[k][c][lane] = (float)((W(W_B + k, c) - bp) / WS.kappa[k][lane]);
-                    }
-                __syncthreads();
-                if (lg && wid == 0) {
-                    bool fin = true;
-                    for (int k = 0; k < 7; k++)
-                        for (int c = 0; c < 3; c++) fin = fin && isfinite(WS.tgt[k][c][lane]) && fabsf(WS.tgt[k][c][lane]) < 1e6f;
-                    if (fin) {
-                        const int row = atomicAdd(A.log_count, 1);
-                        if (row < A.log_cap) {
-                            for (int i = 0; i < AG_MLP_IN; i++) A.log_x[(size_t)row * AG_MLP_IN + i] = WS.xf[lane][i];
-                            for (int k = 0; k < 7; k++)
-                                for (int c = 0; c < 3; c++) A.log_t[(size_t)row * AG_MLP_OUT + 3 * k + c] = WS.tgt[k][c][lane];
-                        }
-                    }
-                }
-            }
+            if (logp)
+                ag_warm_log<C>(A, W.w, W.ns, W.slot, ag_coop_pcomp<NV>(wid), WS, lane, wid,
+                               live && WS.valid[lane] && (steps % A.log_every) == 0);
             /* ---- dense output: states at the output times this step covers,
              * from the step's polynomial (the interpolation of ASSIST's
              * assist_interpolate, src/assist.c:556-597: s- and sv-coefficients

@@ -1,0 +1,197 @@
+/*
+ * ias15_fast.cuh -- device pieces of IAS15 shared by the two integrators that
+ * use the evaluation of fast_forces.cuh: the batched kernel (kernels_fast.cu)
+ * and the shared-step kernel (kernels_shared.cu).  A 128-thread block holds
+ * up to 32 particles, lane l of every warp working on particle l; the
+ * components x, y, z of the IAS15 state belong to warps 0, 2 and 3, and warp 1
+ * (which evaluates the terms kept in FP64) controls the steps.
+ */
+#ifndef ASSIST_GB300_IAS15_FAST_CUH
+#define ASSIST_GB300_IAS15_FAST_CUH
+
+#include "fast_forces.cuh"
+#include "ias15_common.cuh"
+
+/* Position component of warp w (-1: none). */
+__device__ __forceinline__ int ag_fast_comp(int w) { return w == 0 ? 0 : w - (w == 1 ? 2 : 1); }
+
+/* Shared arrays of a block's steps. */
+struct AgFastStep {
+    AgFastShared F;
+    double ra[3][32], rdb[3][32], rb6[3][32];   /* |a|, |delta b6|, |b6| of x, y, z at node 7 */
+    double pcx[8][9], pcv[8][8], ptn[8];        /* predictor coefficients and times of the nodes */
+    double hstep, t, tc;                        /* this step */
+    double ah, aratio;                          /* the accepted (or rejected) step and the next one's size over it */
+    unsigned live, fin, last;                   /* lanes integrating, to be retired, ending with this step */
+    unsigned nf[3];                             /* lanes with a non-finite x, y, z */
+    int cmd;
+};
+
+/* Predictor coefficients and times of the nodes of a step of size h from
+ * t + tc, by lanes 1..7 of a warp (lane 0: the start). */
+__device__ __forceinline__ void ag_fast_nodes(AgFastStep& S, int lane, double t, double tc, double h) {
+    if (lane == 0) S.ptn[0] = t;
+    if (lane < 1 || lane > 7) return;
+    const double s0 = h * ag_ias.h[lane];
+    /* the product rounded on its own, as the oracle forms a node time */
+    S.ptn[lane] = t + (tc + __dmul_rn(h, ag_ias.h[lane]));
+    double x = s0 * s0 * 0.5, v = s0;
+    S.pcx[lane][0] = s0; S.pcx[lane][1] = x; S.pcv[lane][0] = v;
+#pragma unroll
+    for (int k = 2; k < 9; k++) { x = x * ag_ias.fx[lane][k]; S.pcx[lane][k] = x; }
+#pragma unroll
+    for (int k = 1; k < 8; k++) { v = v * ag_ias.fv[lane][k]; S.pcv[lane][k] = v; }
+}
+
+/* The state of component c at node n into the evaluation's arrays. */
+__device__ __forceinline__ void ag_fast_predict(const Ws<3>& W, AgFastStep& S, int c, int lane, int n) {
+    double x, v;
+    if (n == 0) {
+        x = W(W_X0, c);
+        v = W(W_V0, c);
+    } else {
+        const double *sx = S.pcx[n], *sv = S.pcv[n];
+        const double a0 = W(W_A0, c), v0 = W(W_V0, c);
+        double b = W(W_B + 6, c);
+        double px = sx[8] * b, pv = sv[7] * b;
+#pragma unroll
+        for (int j = 5; j >= 0; j--) {
+            b = W(W_B + j, c);
+            px = fma(sx[j + 2], b, px);
+            pv = fma(sv[j + 1], b, pv);
+        }
+        px = fma(sx[1], a0, px);
+        px = fma(sx[0], v0, px);
+        x = W(W_X0, c) + (px + W(W_XC, c));
+        pv = fma(sv[0], a0, pv);
+        v = v0 + (pv + W(W_VC, c));
+    }
+    S.F.xs[c][lane] = x; S.F.vs[c][lane] = v;
+    S.F.xf[c][lane] = ag_f2_of(x); S.F.vf[c][lane] = ag_f2_of(v);
+}
+
+/* Start of a step: g from the predicted b. */
+__device__ __forceinline__ void ag_fast_start(const Ws<3>& W, int c) {
+    double b[7];
+#pragma unroll
+    for (int k = 0; k < 7; k++) b[k] = W(W_B + k, c);
+#pragma unroll
+    for (int j = 0; j < 7; j++) {
+        double s = b[j];
+#pragma unroll
+        for (int k = j + 1; k < 7; k++) s = fma(b[k], ag_ias.d[j][k], s);
+        W(W_G + j, c) = s;
+    }
+}
+
+/* Corrector of component c at node n; node 7 leaves the error measures. */
+__device__ __forceinline__ void ag_fast_correct(const Ws<3>& W, AgFastStep& S, int c, int lane, int n) {
+    const double at = ag_fast_sum(S.F, c, lane);
+    double gn = (at - W(W_A0, c)) * ag_ias.rrinv[n][0];
+    for (int j = 1; j < n; j++) gn = (gn - W(W_G + j - 1, c)) * ag_ias.rrinv[n][j];
+    const double delta = gn - W(W_G + n - 1, c);
+    W(W_G + n - 1, c) = gn;
+    for (int k = 0; k < n - 1; k++) W(W_B + k, c) = fma(delta, ag_ias.c[n - 1][k], W(W_B + k, c));
+    const double bn = W(W_B + n - 1, c) + delta;
+    W(W_B + n - 1, c) = bn;
+    if (n == 7) {
+        const double aa = fabs(at), db = fabs(delta), bb = fabs(bn);
+        S.ra[c][lane] = ag_isnormal_pos(aa) ? aa : 0.0;
+        S.rdb[c][lane] = ag_isnormal_pos(db) ? db : 0.0;
+        S.rb6[c][lane] = ag_isnormal_pos(bb) ? bb : 0.0;
+    }
+}
+
+/* The larger of a lane's three measures. */
+__device__ __forceinline__ double ag_max3(const double (*r)[32], int lane) {
+    return ag_max_nonneg(ag_max_nonneg(r[0][lane], r[1][lane]), r[2][lane]);
+}
+
+/* maxdb / maxa as IAS15's convergence test reads it: compared with 1e-16 and
+ * with the last iteration's, for which FP32 does (FP64 where FP32's range
+ * ends). */
+__device__ __forceinline__ double ag_fast_pc_err(double maxdb, double maxa) {
+    const float a = ag_d2f_int(maxa), d = ag_d2f_int(maxdb);
+    if (a > 1e-18f && a < 1e18f && d < 1e18f) return ag_f2d_int(d / a);
+    return maxdb / maxa;
+}
+
+/* x^(-1/7): an FP32 estimate (1e-6) and two Newton steps
+ * z <- z + z (1 - x z^7) / 7, each squaring the relative error (times 4):
+ * full precision from 14 FP64 instructions, where pow takes about a hundred. */
+__device__ __forceinline__ double ag_inv_root7(double x) {
+    if (!(x > 1e-30 && x < 1e30)) return pow(x, -1.0 / 7.0);
+    double z = ag_f2d_int(exp2f(log2f(ag_d2f_int(x)) * (-1.0f / 7.0f)));
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const double z2 = z * z, z4 = z2 * z2, z7 = z4 * z2 * z;
+        z = fma(z * fma(-x, z7, 1.0), 1.0 / 7.0, z);
+    }
+    return z;
+}
+
+/* b, e of component c for a next step of ratio times the last accepted one
+ * (the shift of the acceleration polynomial). */
+__device__ __forceinline__ void ag_fast_shift(const Ws<3>& W, int c, double ratio) {
+    if (ratio > 20.0) {
+        for (int k = 0; k < 7; k++) { W(W_E + k, c) = 0.0; W(W_B + k, c) = 0.0; }
+        return;
+    }
+    constexpr double binom[8][8] = {
+        {1, 0, 0, 0, 0, 0, 0, 0}, {1, 1, 0, 0, 0, 0, 0, 0}, {1, 2, 1, 0, 0, 0, 0, 0}, {1, 3, 3, 1, 0, 0, 0, 0},
+        {1, 4, 6, 4, 1, 0, 0, 0}, {1, 5, 10, 10, 5, 1, 0, 0}, {1, 6, 15, 20, 15, 6, 1, 0}, {1, 7, 21, 35, 35, 21, 7, 1}};
+    double br[7], q = 1.0;
+#pragma unroll
+    for (int k = 0; k < 7; k++) br[k] = W(W_BR + k, c);
+#pragma unroll
+    for (int j = 0; j < 7; j++) {
+        double s = 0.0;
+#pragma unroll
+        for (int k = 6; k >= j; k--) s = k == j ? s + br[k] : fma(br[k], binom[k + 1][j + 1], s);
+        q *= ratio;
+        const double e = q * s, d = br[j] - W(W_ER + j, c);
+        W(W_E + j, c) = e;
+        W(W_B + j, c) = e + d;
+    }
+}
+
+/* Accepted step of size h: x, v advanced by the step's quadratures with
+ * compensated sums; b and e for the next step of ratio times this one. */
+__device__ __forceinline__ void ag_fast_accept(const Ws<3>& W, int c, double h, double ratio) {
+    double b[7];
+#pragma unroll
+    for (int k = 0; k < 7; k++) b[k] = W(W_B + k, c);
+    const double a0 = W(W_A0, c), x0 = W(W_X0, c), v0 = W(W_V0, c);
+    double ix = b[6] * (1.0 / 72.0), iv = b[6] * (1.0 / 8.0);
+    ix = fma(b[5], 1.0 / 56.0, ix); iv = fma(b[5], 1.0 / 7.0, iv);
+    ix = fma(b[4], 1.0 / 42.0, ix); iv = fma(b[4], 1.0 / 6.0, iv);
+    ix = fma(b[3], 1.0 / 30.0, ix); iv = fma(b[3], 1.0 / 5.0, iv);
+    ix = fma(b[2], 1.0 / 20.0, ix); iv = fma(b[2], 1.0 / 4.0, iv);
+    ix = fma(b[1], 1.0 / 12.0, ix); iv = fma(b[1], 1.0 / 3.0, iv);
+    ix = fma(b[0], 1.0 / 6.0, ix);  iv = fma(b[0], 1.0 / 2.0, iv);
+    ix = fma(a0, 0.5, ix);
+    iv = (iv + a0) * h;
+    ix = fma(ix, h * h, v0 * h);
+    double y = ix + W(W_XC, c), s = x0 + y;
+    W(W_XC, c) = y - (s - x0);
+    W(W_X0, c) = s;
+    y = iv + W(W_VC, c);
+    s = v0 + y;
+    W(W_VC, c) = y - (s - v0);
+    W(W_V0, c) = s;
+#pragma unroll
+    for (int k = 0; k < 7; k++) { W(W_ER + k, c) = W(W_E + k, c); W(W_BR + k, c) = b[k]; }
+    ag_fast_shift(W, c, ratio);
+}
+
+/* The smallest of the warp's non-negative doubles (integer compares). */
+__device__ __forceinline__ double ag_warp_min_nonneg(double v) {
+    long long m = __double_as_longlong(v);
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long u = __shfl_xor_sync(AG_FULL, m, o);
+        m = u < m ? u : m;
+    }
+    return __longlong_as_double(m);
+}
+
+#endif

@@ -92,12 +92,18 @@ int ag_group_max_slots(int nv);
 int ag_launch_group(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, cudaStream_t s);
 int ag_coop_max_slots(int nv, int occ, int stage, int warm);
 /* Per-particle encounter cost ratio (extra steps / base steps) from a
- * two-body pilot on a G-point time grid over [tmin, tmax]. */
+ * two-body pilot on a G-point time grid over [tmin, tmax] and, unless d_deep
+ * is null, whether the particle passes deep inside a planet's sphere of
+ * influence. */
 int ag_pilot_encounters(const DevEphem& E, int n, const double* d_t0, const double* d_te, const double* d_state,
-                        double tmin, double tmax, float* d_ratio, float4* d_grid, float2* d_sunv, int G,
-                        cudaStream_t s);
+                        double tmin, double tmax, float* d_ratio, unsigned char* d_deep, float4* d_grid,
+                        float2* d_sunv, int G, cudaStream_t s);
 int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int occ, int stage,
                    cudaStream_t s);
+/* the batched kernel on fast_forces.cuh (kernels_fast.cu): configurations ag_fast_covers */
+int ag_fast_max_slots(int occ, int stage, int warm, int n_ast);
+int ag_launch_fast(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int occ, int stage, cudaStream_t s);
+int ag_fast_ready(void);
 double ag_fp64_probe_gflops(void);
 /* first-use set-up of the batched kernels (tables, shared-memory opt-ins), ahead of a stream capture */
 int ag_batch_ready(void);

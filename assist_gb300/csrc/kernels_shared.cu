@@ -31,6 +31,7 @@
 #include "shared_sim.h"
 #include "table_forces.cuh"
 #include "coop_forces.cuh"
+#include "fast_forces.cuh"
 
 __constant__ double sh_h[8];
 __constant__ double sh_rrinv[8][8];
@@ -551,12 +552,66 @@ __global__ void __launch_bounds__(128) sh_k_forces_coop(const DevEphem* __restri
     }
 }
 
+/* The same by the evaluation of fast_forces.cuh, for the configurations it
+ * covers: a block builds the table of t once and takes groups of 32
+ * particles in turn (the table's chain of about 100 FP64 instructions a warp
+ * is a group's evaluation twice over). */
+__global__ void __launch_bounds__(128, 3) sh_k_forces_fast(const DevEphem* __restrict__ Ep, ForceCfg c, int n, double t,
+                                                           const double* __restrict__ state,
+                                                           const double* __restrict__ params, double* acc, int* status) {
+    extern __shared__ __align__(16) unsigned char sh_smem[];
+    __shared__ AgFastShared F;
+    __shared__ double tn[8];
+    const DevEphem& E = *Ep;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const AgFastView V(sh_smem, E.n_ast);
+    if (tid == 0) tn[0] = t;
+    ag_fast_masses(E, c, F, tid);
+    __syncthreads();
+    const int bad = ag_fast_tables(E, c, 1, tn, V, F, tid);
+    for (int i0 = 32 * blockIdx.x; i0 < n; i0 += 32 * gridDim.x) {
+        const int i = i0 + lane;
+        const bool live = i < n;
+        if (bad) {
+            if (status && tid < 32 && live) status[i] = AG_ERR_COVERAGE;
+            continue;
+        }
+        const int k = wid == 0 ? 0 : wid - 1;
+        double prm[3] = {0.0, 0.0, 0.0};
+        if (live && wid != 1) {
+            const double x = state[6 * (size_t)i + k], v = state[6 * (size_t)i + 3 + k];
+            F.xs[k][lane] = x; F.vs[k][lane] = v;
+            F.xf[k][lane] = ag_f2_of(x); F.vf[k][lane] = ag_f2_of(v);
+        } else if (live && params) {
+            for (int q = 0; q < 3; q++) prm[q] = params[3 * (size_t)i + q];
+        }
+        __syncthreads();
+        ag_fast_force(wid, lane, live, E, c, V, 0, F, params ? prm : nullptr);
+        __syncthreads();
+        if (live && wid != 1) {
+            acc[3 * (size_t)i + k] = ag_fast_sum(F, k, lane);
+            if (k == 0 && status) status[i] = AG_OK;
+        }
+    }
+}
+
 int ag_launch_forces_coop(const DevEphem& E, const ForceCfg& c, int n, double t, const double* state,
                           const double* params, double* acc, int* status, cudaStream_t s) {
     if (n <= 0) return 0;
     static bool done[64];
+    static int sms[64];
     int dev = 0;
     cudaGetDevice(&dev);
+    if (ag_fast_covers(c)) {
+        int m = dev >= 0 && dev < 64 ? sms[dev] : 0;
+        if (!m) {
+            cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
+            if (dev >= 0 && dev < 64) sms[dev] = m;
+        }
+        const int groups = (n + 31) / 32, blocks = groups < 3 * m ? groups : 3 * m;
+        sh_k_forces_fast<<<blocks, 128, AgFastLayout(E.n_ast).stride, s>>>(E.self_dev, c, n, t, state, params, acc, status);
+        return (int)cudaGetLastError();
+    }
     if (!(dev >= 0 && dev < 64 && done[dev])) {
         const cudaError_t e = cudaFuncSetAttribute(sh_k_forces_coop, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)sizeof(ShStepSmem));

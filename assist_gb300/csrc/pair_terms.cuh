@@ -1,0 +1,184 @@
+/*
+ * pair_terms.cuh -- direct gravity of two bodies at a time in float-pair
+ * arithmetic on packed FP32 instructions.
+ *
+ * A float pair is an unevaluated sum hi + lo of two floats (about 48
+ * significant bits).  sm_103a's packed instructions (fma/add/mul.rn.f32x2)
+ * do two FP32 operations each, so one instruction stream computes the terms
+ * of two bodies: a warp's FP64 instruction holds the SM's FP64 pipe for 64 to
+ * 76 cycles (measured), a packed FP32 one its issue slot for two, and a term
+ * is 20 FP64 instructions or 68 packed ones.  The methods are Knuth's two-sum
+ * and the product error from a fused multiply-add (Dekker 1971); packed
+ * operations are written as PTX with explicit rounding, which is neither
+ * contracted nor reordered.
+ *
+ * The term of a body, -GM d / |d|^3, from y0 (the FP32 estimate of 1/|d|):
+ * with delta = |d|^2 y0^2 - 1 (about 2^-21, formed from the exact products'
+ * errors), 1/|d|^3 = y0^3 (1 - 3/2 delta + 15/8 delta^2).  Relative error
+ * about 2e-14 of the term (tests/test_pair_terms.py), so the error is below
+ * 2e-17 of the acceleration while the term is below 1e-3 of the Sun's pull
+ * (the body's threshold, ag_pair_thr2; nearer bodies take the FP64 term).
+ *
+ * Plain C++ without CUDA (the packed operations are then two scalar ones), for
+ * the test.
+ */
+#ifndef ASSIST_GB300_PAIR_TERMS_CUH
+#define ASSIST_GB300_PAIR_TERMS_CUH
+
+#include <cmath>
+
+#include "ieee_convert.cuh"
+
+/* Two floats in one 64-bit register: a (low half) and b. */
+struct AgPk {
+#ifdef __CUDACC__
+    unsigned long long v;
+#else
+    float a, b;
+#endif
+};
+
+#ifdef __CUDACC__
+__device__ __forceinline__ AgPk ag_pk(float a, float b) {
+    AgPk r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float ag_pk_a(AgPk p) {
+    float a;
+    asm("mov.b64 {%0, _}, %1;" : "=f"(a) : "l"(p.v));
+    return a;
+}
+__device__ __forceinline__ float ag_pk_b(AgPk p) {
+    float b;
+    asm("mov.b64 {_, %0}, %1;" : "=f"(b) : "l"(p.v));
+    return b;
+}
+__device__ __forceinline__ AgPk ag_pk_add(AgPk x, AgPk y) {
+    AgPk r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ AgPk ag_pk_mul(AgPk x, AgPk y) {
+    AgPk r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ AgPk ag_pk_fma(AgPk x, AgPk y, AgPk z) {
+    AgPk r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(x.v), "l"(y.v), "l"(z.v));
+    return r;
+}
+__device__ __forceinline__ float ag_rsqrt_est(float x) { return rsqrtf(x); }
+#define AG_PT __device__ __forceinline__
+#else
+inline AgPk ag_pk(float a, float b) { return {a, b}; }
+inline float ag_pk_a(AgPk p) { return p.a; }
+inline float ag_pk_b(AgPk p) { return p.b; }
+inline AgPk ag_pk_add(AgPk x, AgPk y) { return {x.a + y.a, x.b + y.b}; }
+inline AgPk ag_pk_mul(AgPk x, AgPk y) { return {x.a * y.a, x.b * y.b}; }
+inline AgPk ag_pk_fma(AgPk x, AgPk y, AgPk z) { return {std::fma(x.a, y.a, z.a), std::fma(x.b, y.b, z.b)}; }
+inline float ag_rsqrt_est(float x) { return 1.0f / std::sqrt(x); }
+#define AG_PT inline
+#endif
+
+/* x - y, exactly rounded (a fused multiply-add by -1). */
+AG_PT AgPk ag_pk_sub(AgPk x, AgPk y) { return ag_pk_fma(y, ag_pk(-1.0f, -1.0f), x); }
+AG_PT AgPk ag_pk_neg(AgPk x) { return ag_pk_mul(x, ag_pk(-1.0f, -1.0f)); }
+
+/* s + e = x + y exactly. */
+AG_PT AgPk ag_pk_two_sum(AgPk x, AgPk y, AgPk& e) {
+    const AgPk s = ag_pk_add(x, y), bb = ag_pk_sub(s, x);
+    e = ag_pk_add(ag_pk_sub(x, ag_pk_sub(s, bb)), ag_pk_sub(y, bb));
+    return s;
+}
+
+/* One component of two bodies' positions relative to the origin, hi and lo
+ * parts packed (a 16-byte load). */
+struct alignas(16) AgPkComp {
+    AgPk h, l;
+};
+/* Two bodies: origin minus body, and their GM and threshold (ag_pair_thr2). */
+struct AgPkRel {
+    AgPkComp c[3];
+};
+struct alignas(16) AgPkGm {
+    AgPk h, l;
+    float ta, tb;
+    float ga, gb;          /* GM in FP32 (the potential of the relativistic term) */
+};
+
+/* The smallest squared distance, over the particle's squared heliocentric
+ * distance, at which a body of mass m (in solar masses) takes the pair term.
+ * The pair's relative error of 2e-14 asks for a share m (r/d)^2 of the Sun's
+ * pull below 1e-3; the separation's absolute error, about 3e-15 r with the
+ * term's slope, for m (r/d)^3 below 1/150: either way 2e-17 of the
+ * acceleration, a fifth of the rounding of its FP64 sum. */
+inline float ag_pair_thr2(double m) {
+    const double a = m / 1e-3, b = std::pow(150.0 * m, 2.0 / 3.0);
+    return (float)(a > b ? a : b);
+}
+
+/* Running sum of packed pair terms: hi and lo per component. */
+struct AgPkSum {
+    AgPk h[3], l[3];
+};
+
+/* Adds the terms of the two bodies of R to S at the position xh + xl
+ * (packed: the same value in both halves); rs2: squared heliocentric distance
+ * (FP32).  Returns bit 0 / bit 1 set for a body below its threshold (or not
+ * finite), whose term is left out. */
+AG_PT unsigned ag_pk_term(const AgPkRel& R, const AgPkGm& G, const AgPk* xh, const AgPk* xl, float rs2, AgPkSum& S) {
+    const AgPk m1 = ag_pk(-1.0f, -1.0f);
+    AgPk dh[3], dl[3], p[3], ne[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const AgPkComp c = R.c[k];
+        AgPk e;
+        const AgPk s = ag_pk_two_sum(xh[k], c.h, e);
+        e = ag_pk_add(e, ag_pk_add(xl[k], c.l));
+        dh[k] = ag_pk_add(s, e);
+        dl[k] = ag_pk_sub(e, ag_pk_sub(dh[k], s));
+        /* d^2 = p - ne */
+        const AgPk nd = ag_pk_mul(dh[k], m1);
+        p[k] = ag_pk_mul(dh[k], dh[k]);
+        ne[k] = ag_pk_fma(ag_pk_add(nd, nd), dl[k], ag_pk_fma(dh[k], nd, p[k]));
+    }
+    AgPk t1, t2;
+    const AgPk r2 = ag_pk_two_sum(ag_pk_two_sum(p[0], p[1], t1), p[2], t2);
+    const AgPk r2l = ag_pk_sub(ag_pk_add(t1, t2), ag_pk_add(ag_pk_add(ne[0], ne[1]), ne[2]));
+    const float ra = ag_pk_a(r2), rb = ag_pk_b(r2);
+    const bool na = !(ra >= G.ta * rs2 && ra < 1e30f), nb = !(rb >= G.tb * rs2 && rb < 1e30f);
+    const AgPk y = ag_pk(ag_rsqrt_est(ra), ag_rsqrt_est(rb)), ny = ag_pk_mul(y, m1);
+    /* y^2 = q - nqe, r2 q = th - nte, delta = |d|^2 y^2 - 1 */
+    const AgPk q = ag_pk_mul(y, y), nqe = ag_pk_fma(y, ny, q), nq = ag_pk_mul(q, m1);
+    const AgPk th = ag_pk_mul(r2, q), nte = ag_pk_fma(r2, nq, th);
+    AgPk del = ag_pk_sub(ag_pk_add(th, m1), nte);
+    del = ag_pk_fma(r2, ag_pk_mul(nqe, m1), del);
+    del = ag_pk_fma(r2l, q, del);
+    const AgPk corr = ag_pk_mul(del, ag_pk_fma(del, ag_pk(1.875f, 1.875f), ag_pk(-1.5f, -1.5f)));
+    /* GM y = w - nwe, GM y^3 = g - ne3, both with the correction: G = -GM / |d|^3 = gh + gl */
+    const AgPk w = ag_pk_mul(G.h, y);
+    const AgPk nwe = ag_pk_sub(ag_pk_fma(G.h, ny, w), ag_pk_mul(G.l, y));
+    const AgPk g = ag_pk_mul(w, q);
+    AgPk gl = ag_pk_fma(w, nq, g);
+    gl = ag_pk_fma(w, nqe, gl);
+    gl = ag_pk_fma(nwe, q, gl);
+    AgPk gh = ag_pk_mul(g, m1);
+    gl = ag_pk_fma(gh, corr, gl);
+    gh = ag_pk(na ? 0.0f : ag_pk_a(gh), nb ? 0.0f : ag_pk_b(gh));
+    gl = ag_pk(na ? 0.0f : ag_pk_a(gl), nb ? 0.0f : ag_pk_b(gl));
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const AgPk ph = ag_pk_mul(gh, dh[k]);
+        AgPk pe = ag_pk_fma(gh, dh[k], ag_pk_mul(ph, m1));
+        pe = ag_pk_fma(gh, dl[k], pe);
+        pe = ag_pk_fma(gl, dh[k], pe);
+        AgPk e;
+        S.h[k] = ag_pk_two_sum(S.h[k], ph, e);
+        S.l[k] = ag_pk_add(S.l[k], ag_pk_add(e, pe));
+    }
+    return (na ? 1u : 0u) | (nb ? 2u : 0u);
+}
+
+#endif

@@ -1,0 +1,75 @@
+"""The evaluation with pair terms (assist_gb300/csrc/fast_forces.cuh) at its
+edges, against the oracle: group remainders, several groups a block, particles
+on either side of every body's threshold and beyond FP32's range, no
+asteroids; and a batch whose groups are split between the two kernels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-14          # the acceleration bar of tests/test_gpu_forces.py
+MASS = {0: 1.66e-7, 1: 2.45e-6, 2: 3.0e-6, 3: 3.7e-8, 4: 3.2e-7, 5: 2.86e-4, 6: 4.4e-5, 7: 5.2e-5, 8: 7.4e-9}
+
+
+@pytest.fixture(scope="module")
+def files(tmp_path_factory):
+    from assist_gb300 import synth
+    return synth.write_ephemeris(str(tmp_path_factory.mktemp("fast")), seed=5, t_beg=7950.0, t_end=8450.0)
+
+
+@pytest.mark.parametrize("n,asteroids", [(1, True), (31, True), (33, True), (33, False), (15000, True)])
+def test_shared_time_forces_at_thresholds(files, n, asteroids):
+    import torch
+    from assist_gb300 import Ephem, batch, synth
+    from tests.oracle_py import Oracle
+    pl, ast, system = files
+    eph = Ephem(pl, ast if asteroids else "/nonexistent")
+    t = 8100.25
+    pop = synth.population(system, "mix", n, seed=n, t0=t, nongrav_frac=0.3)
+    rng = np.random.default_rng(n)
+    extra = []
+    for k in range(9):                      # on either side of each pair body's threshold
+        body = system.body(k + 1 if k < 5 else k + 2, np.array(t))
+        thr = max(MASS[k] / 1e-3, (150 * MASS[k]) ** (2 / 3)) ** 0.5
+        for f in (0.7, 0.95, 1.05):
+            u = rng.normal(size=3); u /= np.linalg.norm(u)
+            extra.append(np.concatenate([body[0] + f * thr * np.linalg.norm(body[0]) * u, body[1]]))
+    for far in (2e6, 1e9, 1e13):            # beyond the range of the FP32 products
+        u = rng.normal(size=3); u /= np.linalg.norm(u)
+        extra.append(np.concatenate([far * u, 1e-2 * u[::-1]]))
+    state = np.concatenate([pop.state, np.array(extra)])
+    params = np.concatenate([pop.params, np.zeros((len(extra), 3))])
+    st, prm = torch.tensor(state, device="cuda"), torch.tensor(params, device="cuda")
+    status = torch.full((len(state),), -1, dtype=torch.int32, device="cuda")
+    acc = batch.forces_shared_time_device(eph, t, st, params=prm, status=status).cpu().numpy()
+    assert (status.cpu().numpy() == 0).all()
+    idx = np.arange(len(state)) if n < 1000 else np.concatenate([np.arange(0, n, 97), np.arange(n - 40, len(state))])
+    ref = Oracle(pl, ast if asteroids else "/nonexistent").forces(t, state[idx], params=params[idx])
+    e = np.linalg.norm(acc[idx] - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert e.max() < TOL, (e.max(), idx[e.argmax()])
+
+
+def test_batch_split_between_kernels(files):
+    """Particles that pass Jupiter well inside its sphere of influence share a
+    batch with ordinary ones: every particle ends where the oracle puts it."""
+    import torch
+    from assist_gb300 import Ephem, batch, synth
+    from tests.oracle_py import Oracle
+    pl, ast, system = files
+    eph = Ephem(pl, ast)
+    pop = synth.population(system, "mba", 100, seed=9, t0=8000.0, length=100.0)
+    jp, jv = system.body(6, np.array(8000.0))
+    fly = []
+    for k in range(5):                      # unbound flybys of Jupiter at about 0.02 AU
+        u, w = np.eye(3)[k % 3], np.eye(3)[(k + 1) % 3]
+        fly.append(np.concatenate([jp + 0.3 * u + 0.02 * w, jv - 0.02 * u]))
+    state = np.concatenate([pop.state, np.array(fly)])
+    n = len(state)
+    t0, te = np.full(n, 8000.0), np.full(n, 8100.0)
+    dev = lambda a: torch.tensor(a, device="cuda")  # noqa: E731
+    st, status = dev(state), torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    batch.integrate_batch_device(eph, dev(t0), dev(te), st, status=status)
+    assert (status.cpu().numpy() == 0).all()
+    ref = Oracle(pl, ast).integrate_batch(t0, te, state)
+    d = np.abs(st.cpu().numpy()[:, :3] - ref[:, :3]).max(axis=1)
+    assert d[:100].max() < 1e-12 and d.max() < 1e-9, (d[:100].max(), d.max())
