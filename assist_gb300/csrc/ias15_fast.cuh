@@ -184,14 +184,18 @@ __device__ __forceinline__ void ag_fast_accept(const Ws<3>& W, int c, double h, 
     ag_fast_shift(W, c, ratio);
 }
 
-/* The smallest of the warp's non-negative doubles (integer compares). */
+/* The smallest and the largest of the warp's non-negative doubles, whose bit
+ * patterns order as integers do: the high words' extreme, then the low words'
+ * among the lanes that have it. */
 __device__ __forceinline__ double ag_warp_min_nonneg(double v) {
-    long long m = __double_as_longlong(v);
-    for (int o = 16; o > 0; o >>= 1) {
-        const long long u = __shfl_xor_sync(AG_FULL, m, o);
-        m = u < m ? u : m;
-    }
-    return __longlong_as_double(m);
+    const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_min_sync(AG_FULL, h), ml = __reduce_min_sync(AG_FULL, h == mh ? l : ~0u);
+    return __hiloint2double((int)mh, (int)ml);
+}
+__device__ __forceinline__ double ag_warp_max_nonneg(double v) {
+    const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v);
+    const unsigned mh = __reduce_max_sync(AG_FULL, h), ml = __reduce_max_sync(AG_FULL, h == mh ? l : 0u);
+    return __hiloint2double((int)mh, (int)ml);
 }
 
 #endif

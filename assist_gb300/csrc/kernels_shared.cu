@@ -31,7 +31,7 @@
 #include "shared_sim.h"
 #include "table_forces.cuh"
 #include "coop_forces.cuh"
-#include "fast_forces.cuh"
+#include "ias15_fast.cuh"
 
 __constant__ double sh_h[8];
 __constant__ double sh_rrinv[8][8];
@@ -423,6 +423,236 @@ __global__ void __launch_bounds__(128) sh_k_step(const DevEphem* __restrict__ Ep
     }
 }
 
+/* ------------------------------------------------------------------ run kernel
+ *
+ * Whole steps of a simulation without variational particles, in the force
+ * configurations of fast_forces.cuh: a launch integrates up to `limit` steps,
+ * step control included, with the block's IAS15 state in shared memory and
+ * the device pieces of the batched kernel (ias15_fast.cuh).  Several blocks
+ * (32 particles each) run in a cooperative launch: the maxima of an iteration
+ * meet in global memory across a bounded grid barrier, and every block takes
+ * the same decisions from them.  What it replaces: a launch, two copies and a
+ * host decision for each step, state in global memory, and the evaluation
+ * with every term in FP64 (a step of three particles 262 us).  The rules are
+ * the host loop's below. */
+struct ShCtl {
+    double t, tc, dt, dtls, dt_done;
+    long long accepted, rejected, iterations;
+    int status, gave_up;
+};
+
+struct ShRunArgs {
+    ShView W;
+    int n;
+    const double* params;        /* 3 n, or null */
+    double tmax, epsilon, min_dt;
+    long long max_steps;         /* accepted steps after which to stop short of tmax (0: none) */
+    int limit;                   /* steps of this launch */
+    const ShCtl* in;
+    ShCtl* out;
+    unsigned long long* red;     /* nine words: three rotating buffers of the maxima, zero at launch */
+    unsigned* bar;               /* grid barrier: arrivals, generation */
+};
+
+/* Device memory of a simulation's run kernel. */
+struct ShRunMem {
+    ShCtl ctl[2];                /* a launch reads one and writes the other */
+    unsigned long long red[9];
+    unsigned bar[2];
+};
+/* Steps of one launch (a year of 1,024 main-belt particles is 65): the device
+ * is not held for longer than some tens of milliseconds at a time. */
+#define SH_RUN_STEPS 256
+
+#define SH_RUN_POLLS (1 << 22)
+/* Grid barrier of one thread a block; false when its polls run out (the block
+ * then leaves, and the others at their own limits). */
+__device__ __forceinline__ bool sh_run_barrier(unsigned* bar) {
+    volatile unsigned* vgen = bar + 1;
+    const unsigned gen = *vgen;
+    __threadfence();
+    if (atomicAdd(&bar[0], 1u) == gridDim.x - 1) {
+        atomicExch(&bar[0], 0u);
+        __threadfence();
+        atomicAdd(&bar[1], 1u);
+        return true;
+    }
+    for (int k = 0; k < SH_RUN_POLLS; k++)
+        if (*vgen != gen) {
+            __threadfence();
+            return true;
+        }
+    return false;
+}
+
+enum { SH_ACCEPT = 0, SH_REJECT, SH_ITERATE, SH_LEAVE };
+
+__global__ void __launch_bounds__(128, 2) sh_k_run(const DevEphem* __restrict__ Ep, ForceCfg c, ShRunArgs A) {
+    extern __shared__ __align__(16) unsigned char sh_smem[];
+    __shared__ AgFastStep S;
+    const DevEphem& E = *Ep;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, pc = ag_fast_comp(wid), i = 32 * blockIdx.x + lane;
+    const bool ctl = wid == 1, live = i < A.n;
+    const Ws<3> W{reinterpret_cast<double*>(sh_smem), 32, lane};
+    const AgFastView V(sh_smem + sizeof(double) * W_NF * 3 * 32, E.n_ast);
+    ag_fast_masses(E, c, S.F, tid);
+    /* fields of the batched layout and of the simulation's */
+    const int mine[8] = {W_X0, W_V0, W_XC, W_VC, W_B, W_E, W_BR, W_ER};
+    const int theirs[8] = {S_X0, S_V0, S_XC, S_VC, S_B, S_E, S_BR, S_ER};
+    if (live && pc >= 0)
+        for (int f = 0; f < 8; f++)
+            for (int k = 0; k < (f < 4 ? 1 : 7); k++) W(mine[f] + k, pc) = A.W(theirs[f] + k, pc, i);
+    double prm[3] = {0.0, 0.0, 0.0};
+    if (ctl && live && A.params)
+        for (int k = 0; k < 3; k++) prm[k] = A.params[3 * (size_t)i + k];
+    const double* Ap = A.params ? prm : nullptr;
+    /* the control warp's state, the same in every block */
+    ShCtl K = *A.in;
+    double hstep = 0.0;
+    bool last = false;
+    int round = 0;                      /* iterations of this launch: the rotating buffers */
+    for (int step = 0; step < A.limit; step++) {
+        if (ctl) {
+            const double rem = (A.tmax - K.t) - K.tc;
+            last = fabs(K.dt) >= fabs(rem);
+            hstep = last ? rem : K.dt;
+            ag_fast_nodes(S, lane, K.t, K.tc, hstep);
+        }
+        __syncthreads();
+        if (live && pc >= 0) ag_fast_predict(W, S, pc, lane, 0);
+        if (ag_fast_tables(E, c, 8, S.ptn, V, S.F, tid)) {
+            K.status = AG_ERR_COVERAGE;          /* every block builds the same tables */
+            break;
+        }
+        ag_fast_force(wid, lane, live, E, c, V, 0, S.F, Ap);
+        __syncthreads();
+        if (live && pc >= 0) {
+            W(W_A0, pc) = ag_fast_sum(S.F, pc, lane);
+            ag_fast_start(W, pc);
+        }
+        double pc_last = 1e300;
+        int iters = 1, cmd;
+        while (true) {
+            for (int n = 1; n < 8; n++) {
+                if (live && pc >= 0) ag_fast_predict(W, S, pc, lane, n);
+                __syncthreads();
+                ag_fast_force(wid, lane, live, E, c, V, n, S.F, Ap);
+                __syncthreads();
+                if (live && pc >= 0) ag_fast_correct(W, S, pc, lane, n);
+            }
+            __syncthreads();
+            if (ctl) {
+                double ma = ag_warp_max_nonneg(live ? ag_max3(S.ra, lane) : 0.0);
+                double mdb = ag_warp_max_nonneg(live ? ag_max3(S.rdb, lane) : 0.0);
+                double mb = ag_warp_max_nonneg(live ? ag_max3(S.rb6, lane) : 0.0);
+                bool ok = true;
+                if (gridDim.x > 1) {
+                    /* buffer round % 3 collects this iteration's maxima, block 0
+                     * clears the next one (last read two barriers ago) */
+                    unsigned long long* rb = A.red + 3 * (round % 3);
+                    if (lane < 3) atomicMax(&rb[lane], (unsigned long long)__double_as_longlong(lane == 0 ? mdb : (lane == 1 ? ma : mb)));
+                    if (blockIdx.x == 0 && lane < 3) A.red[3 * ((round + 1) % 3) + lane] = 0ull;
+                    __threadfence();
+                    __syncwarp();
+                    if (lane == 0) ok = sh_run_barrier(A.bar);
+                    ok = __shfl_sync(AG_FULL, ok ? 1 : 0, 0) != 0;
+                    const double r = lane < 3 ? __longlong_as_double((long long)atomicOr(&rb[lane], 0ull)) : 0.0;
+                    mdb = __shfl_sync(AG_FULL, r, 0);
+                    ma = __shfl_sync(AG_FULL, r, 1);
+                    mb = __shfl_sync(AG_FULL, r, 2);
+                    round++;
+                }
+                const double pc_err = ag_fast_pc_err(mdb, ma);
+                const bool conv = (pc_err < 1e-16) || (iters > 2 && pc_last <= pc_err) || (iters >= 12);
+                pc_last = pc_err;
+                cmd = SH_ITERATE;
+                if (!ok) {
+                    cmd = SH_LEAVE;
+                    K.gave_up = 1;
+                } else if (conv) {
+                    double dt_new = hstep;
+                    cmd = SH_ACCEPT;
+                    if (A.epsilon > 0.0) {
+                        const double err = mb / ma, safety = 0.25, ahs = fabs(hstep);
+                        if (ag_isnormal_pos(err)) dt_new = ag_inv_root7(err / A.epsilon) * hstep;
+                        else dt_new = hstep / safety;
+                        if (fabs(dt_new) < A.min_dt) dt_new = copysign(A.min_dt, dt_new);
+                        if (fabs(dt_new) < safety * ahs) cmd = SH_REJECT;
+                        else if (fabs(dt_new) > ahs / safety) dt_new = hstep / safety;
+                    }
+                    K.iterations += iters;
+                    if (lane == 0) {
+                        S.ah = hstep;
+                        S.aratio = cmd == SH_REJECT ? (K.dtls != 0.0 ? dt_new / K.dtls : 0.0) : dt_new / hstep;
+                    }
+                    K.dt = dt_new;
+                    if (cmd == SH_REJECT) {
+                        K.rejected++;
+                    } else {
+                        const double y = hstep + K.tc, s = K.t + y;
+                        K.tc = y - (s - K.t);
+                        K.t = s;
+                        K.dtls = hstep;
+                        K.dt_done = hstep;
+                        K.accepted++;
+                        if (last) { K.t = A.tmax; K.tc = 0.0; }
+                    }
+                }
+                if (lane == 0) {
+                    S.cmd = cmd;
+                    /* the launch ends: tmax, the steps asked for, or a barrier given up */
+                    S.fin = cmd == SH_LEAVE ||
+                            (cmd == SH_ACCEPT && (K.t == A.tmax || (A.max_steps > 0 && K.accepted >= A.max_steps)));
+                }
+            }
+            __syncthreads();
+            cmd = S.cmd;
+            if (cmd != SH_ITERATE) break;
+            iters++;
+        }
+        const bool leave = S.fin != 0;
+        if (live && pc >= 0) {
+            if (cmd == SH_ACCEPT) {
+                /* the step's start, for dense output */
+                A.W(S_PX, pc, i) = W(W_X0, pc) + W(W_XC, pc);
+                A.W(S_PV, pc, i) = W(W_V0, pc) + W(W_VC, pc);
+                A.W(S_PA, pc, i) = W(W_A0, pc);
+                ag_fast_accept(W, pc, S.ah, S.aratio);
+            } else if (cmd == SH_REJECT) {
+                if (S.aratio != 0.0) ag_fast_shift(W, pc, S.aratio);
+                else
+                    for (int k = 0; k < 7; k++) { W(W_B + k, pc) = 0.0; W(W_E + k, pc) = 0.0; }
+            }
+        }
+        if (leave) break;
+    }
+    if (live && pc >= 0)
+        for (int f = 0; f < 8; f++)
+            for (int k = 0; k < (f < 4 ? 1 : 7); k++) A.W(theirs[f] + k, pc, i) = W(mine[f] + k, pc);
+    if (ctl && lane == 0 && (blockIdx.x == 0 || K.gave_up)) {
+        if (blockIdx.x == 0) *A.out = K;
+        else atomicExch(&A.out->gave_up, 1);
+    }
+}
+
+static size_t sh_run_bytes(int n_ast) { return sizeof(double) * W_NF * 3 * 32 + 8 * (size_t)AgFastLayout(n_ast).stride; }
+
+/* Blocks a cooperative launch of the run kernel can hold on the current
+ * device (0: none). */
+static int sh_run_capacity(int n_ast) {
+    int dev = 0, sms = 0, bps = 0, can = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&can, cudaDevAttrCooperativeLaunch, dev);
+    if (const char* ev = getenv("ASSIST_GB300_SHARED_COOP"))
+        if (atoi(ev) == 0) can = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (cudaFuncSetAttribute(sh_k_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh_run_bytes(AG_MAX_AST)) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, sh_k_run, 128, sh_run_bytes(n_ast)) != cudaSuccess)
+        return 0;
+    return can ? bps * sms : 1;
+}
+
 static int sh_step_attr(void) {
     static bool done[64];
     int dev = 0;
@@ -641,6 +871,9 @@ struct AgSharedSim {
     AgCoopTab* d_tab = nullptr;   /* the step's node tables (several blocks) */
     unsigned long long* d_red = nullptr;  /* 16 words: maxima, iterations, rotating buffers */
     unsigned* d_bar = nullptr;    /* grid barrier of the cooperative step launch */
+    ShRunMem* d_run = nullptr;    /* control state of the run kernel */
+    ShCtl* h_ctl = nullptr;       /* pinned */
+    int run_blocks = -1;          /* blocks a launch of the run kernel can hold (-1: not yet asked) */
     int coop_blocks = -1;         /* blocks a cooperative step launch can hold (-1: not yet asked) */
     int* d_status = nullptr;
     cudaStream_t stream = nullptr;
@@ -664,6 +897,8 @@ void ag_shared_free(AgSharedSim* s) {
     if (s->d_tab) cudaFree(s->d_tab);
     if (s->d_red) cudaFree(s->d_red);
     if (s->d_bar) cudaFree(s->d_bar);
+    if (s->d_run) cudaFree(s->d_run);
+    if (s->h_ctl) cudaFreeHost(s->h_ctl);
     if (s->d_status) cudaFree(s->d_status);
     if (s->h_pin) cudaFreeHost(s->h_pin);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -822,6 +1057,116 @@ int ag_shared_forces(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struc
     return 0;
 }
 
+/* The host particles (authoritative) into the device's state, with the
+ * predictor's state kept when this call continues the previous one. */
+static void sh_upload_state(AgSharedSim* s, struct reb_simulation* r, double dir) {
+    const int n = r->N;
+    const size_t cap = (size_t)s->cap, F = 3 * cap;
+    const bool cont = s->state_on_device && s->t == r->t && s->n == n && s->dir == dir;
+    double* h = s->h_pin;
+    for (int i = 0; i < n; i++) {
+        const reb_particle& p = r->particles[i];
+        h[0 * cap + i] = p.x; h[1 * cap + i] = p.y; h[2 * cap + i] = p.z;
+        h[3 * cap + i] = p.vx; h[4 * cap + i] = p.vy; h[5 * cap + i] = p.vz;
+    }
+    static_assert(S_V0 == S_X0 + 1 && S_VC == S_XC + 1, "x, v and their compensations are neighbours");
+    cudaMemcpyAsync(s->d_ws + (size_t)S_X0 * F, h, sizeof(double) * 2 * F, cudaMemcpyHostToDevice, s->stream);
+    cudaMemsetAsync(s->d_ws + (size_t)S_XC * F, 0, sizeof(double) * 2 * F, s->stream);
+    if (!cont) {
+        cudaMemsetAsync(s->d_ws + (size_t)S_B * F, 0, sizeof(double) * 35 * F, s->stream);
+        s->dt_last_success = 0.0;
+    }
+    s->t = r->t;
+    s->tc = 0.0;
+    s->n = n;
+    s->dir = dir;
+}
+
+/* The integration by the run kernel.  Returns 0, 1 (CUDA error), or -1 when
+ * its blocks do not fit on the device at once (nothing done). */
+static int sh_run(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct reb_simulation* r, const double* params,
+                  double tmax, ShIntegrateOut* out) {
+    const int n = r->N, nb = (n + 31) / 32;
+    if (s->run_blocks < 0) s->run_blocks = sh_run_capacity(E.n_ast);
+    if (nb > s->run_blocks) return -1;
+    cudaStream_t st = s->stream;
+    if (!s->d_run) {
+        if (ag_cuda_check(cudaMalloc(&s->d_run, sizeof(ShRunMem)), "cudaMalloc(run state)")) return 1;
+        if (ag_cuda_check(cudaMallocHost(&s->h_ctl, sizeof(ShCtl)), "cudaMallocHost(run state)")) return 1;
+    }
+    if (params) {
+        const size_t np = 3 * (size_t)n;
+        if (np > s->params_cap) {
+            if (s->d_params) cudaFree(s->d_params);
+            s->params_cap = np + 64;
+            if (ag_cuda_check(cudaMalloc(&s->d_params, sizeof(double) * s->params_cap), "cudaMalloc(params)")) return 1;
+        }
+        cudaMemcpyAsync(s->d_params, params, sizeof(double) * np, cudaMemcpyHostToDevice, st);
+    }
+    const double dir = tmax >= r->t ? 1.0 : -1.0;
+    sh_upload_state(s, r, dir);
+    double dt = r->dt;
+    if (dt * dir <= 0) dt = dir * std::fabs(dt != 0 ? dt : 0.001);
+    ShRunArgs A;
+    A.W = ShView{s->d_ws, s->cap};
+    A.n = n;
+    A.params = params ? s->d_params : nullptr;
+    A.tmax = tmax;
+    A.epsilon = r->ri_ias15.epsilon;
+    A.min_dt = r->ri_ias15.min_dt;
+    A.max_steps = out->max_steps;
+    A.limit = SH_RUN_STEPS;
+    A.red = s->d_run->red;
+    A.bar = s->d_run->bar;
+    ShRunMem m;
+    std::memset(&m, 0, sizeof(m));
+    m.ctl[0].t = s->t; m.ctl[0].dt = dt; m.ctl[0].dtls = s->dt_last_success;
+    const size_t F = 3 * (size_t)s->cap, bytes = sh_run_bytes(E.n_ast);
+    cudaMemcpyAsync(s->d_run, &m, sizeof(m), cudaMemcpyHostToDevice, st);
+    ShCtl& K = *s->h_ctl;
+    for (int launch = 0;; launch++) {
+        A.in = &s->d_run->ctl[launch & 1];
+        A.out = &s->d_run->ctl[1 - (launch & 1)];
+        if (launch) cudaMemsetAsync(A.red, 0, sizeof(m.red) + sizeof(m.bar), st);
+        if (nb == 1) {
+            sh_k_run<<<1, 128, bytes, st>>>(E.self_dev, c, A);
+            if (ag_cuda_check(cudaGetLastError(), "IAS15 run kernel")) return 1;
+        } else {
+            const DevEphem* ep = E.self_dev;
+            ForceCfg cc = c;
+            void* args[] = {(void*)&ep, (void*)&cc, (void*)&A};
+            const cudaError_t le = cudaLaunchCooperativeKernel((const void*)sh_k_run, nb, 128, args, bytes, st);
+            if (le == cudaErrorCooperativeLaunchTooLarge && launch == 0) {
+                cudaGetLastError();
+                s->run_blocks = 1;
+                s->state_on_device = false;
+                return -1;
+            }
+            if (ag_cuda_check(le, "IAS15 run kernel (cooperative)")) return 1;
+        }
+        cudaMemcpyAsync(&K, A.out, sizeof(ShCtl), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(s->h_pin, A.W.w + (size_t)S_X0 * F, sizeof(double) * 5 * F, cudaMemcpyDeviceToHost, st);
+        if (ag_cuda_check(cudaStreamSynchronize(st), "IAS15 run")) return 1;
+        if (K.gave_up) {
+            ag_set_error("IAS15 run kernel: a block stopped waiting at the grid barrier");
+            return 1;
+        }
+        if (K.status || K.t == tmax || (A.max_steps > 0 && K.accepted >= A.max_steps)) break;
+    }
+    s->t = K.t; s->tc = K.tc; s->dt_last_success = K.dtls; s->n_real = n;
+    out->accepted += K.accepted;
+    out->rejected += K.rejected;
+    out->iterations += K.iterations;
+    out->evals += K.accepted + K.rejected + 7 * K.iterations;
+    if (K.dt_done != 0.0) out->dt_last_done = K.dt_done;
+    if (K.status) out->status = K.status;
+    else if (K.t != tmax) out->status = -1;
+    r->dt = K.dt;
+    return 0;
+}
+
+static int sh_copy_back(AgSharedSim* s, struct reb_simulation* r, ShIntegrateOut* out);
+
 /* Integrate r to tmax with IAS15 on the device.  Returns 0 or 1 (CUDA error);
  * *status_out receives an ASSIST status of the force model. */
 int ag_shared_integrate(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct reb_simulation* r,
@@ -832,6 +1177,11 @@ int ag_shared_integrate(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, st
     if (sh_tables_init()) return ag_cuda_check(cudaErrorInvalidValue, "IAS15 tables");
     if (ag_cuda_check((cudaError_t)sh_step_attr(), "IAS15 step kernel shared memory")) return 1;
     if (sh_reserve(s, n)) return 1;
+    if (n == n_real && ag_fast_covers(c)) {
+        if (ag_ias_tables_init()) return ag_cuda_check(cudaErrorInvalidValue, "IAS15 tables");
+        const int rc = sh_run(s, E, c, r, params, tmax, out);
+        if (rc >= 0) return rc ? rc : sh_copy_back(s, r, out);
+    }
     AgForceIO io;
     std::memset(&io, 0, sizeof(io));
     if (sh_upload_vars(s, r, params, &io)) return 1;
@@ -840,28 +1190,7 @@ int ag_shared_integrate(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, st
     const int tpb = 128, blocks3 = (3 * n + tpb - 1) / tpb, nb = s->nblocks;
     cudaStream_t st = s->stream;
     double dir = tmax >= r->t ? 1.0 : -1.0;
-    /* the host particles are authoritative: upload them every call; keep the
-     * predictor state only when this call continues the previous one */
-    const bool cont = s->state_on_device && s->t == r->t && s->n == n && s->dir == dir;
-    {
-        double* h = s->h_pin;
-        for (int i = 0; i < n; i++) {
-            const reb_particle& p = r->particles[i];
-            h[0 * (size_t)s->cap + i] = p.x; h[1 * (size_t)s->cap + i] = p.y; h[2 * (size_t)s->cap + i] = p.z;
-            h[3 * (size_t)s->cap + i] = p.vx; h[4 * (size_t)s->cap + i] = p.vy; h[5 * (size_t)s->cap + i] = p.vz;
-        }
-        cudaMemcpyAsync(W.w + (size_t)S_X0 * F, h, sizeof(double) * F, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(W.w + (size_t)S_V0 * F, h + F, sizeof(double) * F, cudaMemcpyHostToDevice, st);
-        cudaMemsetAsync(W.w + (size_t)S_XC * F, 0, sizeof(double) * 2 * F, st);
-        if (!cont) {
-            cudaMemsetAsync(W.w + (size_t)S_B * F, 0, sizeof(double) * 35 * F, st);
-            s->dt_last_success = 0.0;
-        }
-        s->t = r->t;
-        s->tc = 0.0;
-        s->n = n;
-        s->dir = dir;
-    }
+    sh_upload_state(s, r, dir);
     s->n_real = n_real;
     io.n_real = n_real; io.stride = s->cap;
     io.x = W.w + (size_t)S_XP * F; io.v = W.w + (size_t)S_VP * F; io.a = W.w + (size_t)S_AT * F;
@@ -1002,10 +1331,19 @@ int ag_shared_integrate(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, st
         if (last) { s->t = tmax; s->tc = 0.0; }
         if (out->max_steps > 0 && steps >= out->max_steps && s->t != tmax) { out->status = -1; break; }
     }
-    /* copy back: current state and the last step's start state / b for dense output */
-    double* h = s->h_pin;
-    cudaMemcpyAsync(h, W.w + (size_t)S_X0 * F, sizeof(double) * 5 * F, cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(s->h_pin, W.w + (size_t)S_X0 * F, sizeof(double) * 5 * F, cudaMemcpyDeviceToHost, st);
     if (ag_cuda_check(cudaStreamSynchronize(st), "copy back")) return 1;
+    r->dt = dt;
+    return sh_copy_back(s, r, out);
+}
+
+/* The simulation's particles and time from the device: the current state (in
+ * h_pin) and, for dense output, the last step's start state and b. */
+static int sh_copy_back(AgSharedSim* s, struct reb_simulation* r, ShIntegrateOut* out) {
+    const int n = r->N;
+    const size_t F = 3 * (size_t)s->cap;
+    const ShView W{s->d_ws, s->cap};
+    double* h = s->h_pin;
     const double* X0 = h; const double* V0 = h + F; const double* XC = h + 3 * F; const double* VC = h + 4 * F;
     for (int i = 0; i < n; i++) {
         reb_particle& p = r->particles[i];
@@ -1015,7 +1353,8 @@ int ag_shared_integrate(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, st
     if (out->dense) {
         /* start-of-last-step positions, velocities, accelerations and b */
         std::vector<double> tmp(3 * F);
-        cudaMemcpy(tmp.data(), W.w + (size_t)S_PX * F, sizeof(double) * 3 * F, cudaMemcpyDeviceToHost);
+        if (ag_cuda_check(cudaMemcpy(tmp.data(), W.w + (size_t)S_PX * F, sizeof(double) * 3 * F, cudaMemcpyDeviceToHost), "dense output copy"))
+            return 1;
         for (int i = 0; i < n; i++)
             for (int k = 0; k < 3; k++) {
                 out->dense_x0[3 * i + k] = tmp[(size_t)k * s->cap + i];
@@ -1029,7 +1368,6 @@ int ag_shared_integrate(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, st
                 for (int k = 0; k < 3; k++) out->dense_b[q][3 * i + k] = br[(size_t)q * F + (size_t)k * s->cap + i];
     }
     r->t = s->t;
-    r->dt = dt;
     s->state_on_device = true;
     return 0;
 }

@@ -73,3 +73,36 @@ def test_batch_split_between_kernels(files):
     ref = Oracle(pl, ast).integrate_batch(t0, te, state)
     d = np.abs(st.cpu().numpy()[:, :3] - ref[:, :3]).max(axis=1)
     assert d[:100].max() < 1e-12 and d.max() < 1e-9, (d[:100].max(), d.max())
+
+
+@pytest.mark.parametrize("n,t1", [(1, 8100.0), (32, 7960.0), (33, 8100.0), (300, 8060.0)])
+def test_dropin_run_kernel(files, n, t1):
+    """Shared-step simulations of one block and several, forward and backward,
+    against the oracle; one integration in two calls ends where one call does
+    to rounding, and a step past the ephemeris stops with the coverage error."""
+    from assist_gb300 import Ephem, Extras, Simulation, synth
+    from tests.oracle_py import Oracle
+    pl, ast, system = files
+    eph = Ephem(pl, ast)
+    pop = synth.population(system, "mba", n, seed=n, t0=8000.0)
+
+    def run(stops):
+        sim = Simulation.create(); ex = Extras(sim, eph)
+        for s in pop.state:
+            sim.add(*s)
+        sim.t = 8000.0
+        for t in stops:
+            sim.integrate(t)
+        g = np.array([[p.x, p.y, p.z] for p in sim.particles])
+        out = sim.status, sim.t, sim.steps_done, g
+        ex.detach(sim); sim.free()
+        return out
+
+    st, t, steps, g = run([t1])
+    ref, _, info = Oracle(pl, ast).integrate(8000.0, t1, pop.state)
+    assert st == 0 and t == t1 and abs(steps - info["accepted"]) <= 1
+    assert np.abs(g - ref[:, :3]).max() < 1e-13
+    st, t, _, g2 = run([0.5 * (8000.0 + t1), t1])
+    assert st == 0 and t == t1 and np.abs(g2 - g).max() < 1e-13
+    st, t, _, _ = run([t1, 20000.0])
+    assert st == 1 and t < 8500.0 or t1 < 8000.0
