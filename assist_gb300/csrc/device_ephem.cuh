@@ -76,6 +76,8 @@ struct DevEphem {
     double gm[AG_NPL];
     double inv_cau;              /* 1/AU[km] */
     double cau_per_day;          /* AU[km]/86400 (velocity divisor of the exact path) */
+    double inv_cau_per_day;      /* its reciprocal */
+    double col_rate[13];         /* 2*niv/inc/86400, the derivative factor of a column (two divisions, as the reference's) */
     double f_earth, f_moon;      /* -1/(1+EMRAT), EMRAT/(1+EMRAT) */
     double col_vscale[13];       /* (2*niv/inc/86400) * 86400/AU: d/dtau -> AU/day */
     int pl_inc_pow2;             /* record length is a power of two: divide by multiplying */

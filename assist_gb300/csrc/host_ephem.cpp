@@ -438,11 +438,13 @@ static void ag_ascii_view(const ascii_s* a, DevEphem& D) {
     D.pl_beg = a->beg; D.pl_end = a->end; D.pl_inc = a->inc; D.pl_cau = a->cau; D.pl_cem = a->cem;
     for (int p = 0; p < 13; p++) {
         D.col_off[p] = a->off[p]; D.col_ncf[p] = a->ncf[p]; D.col_niv[p] = a->niv[p];
+        D.col_rate[p] = (double)(a->niv[p] * 2) / a->inc / 86400.0;
         D.col_vscale[p] = ((double)(a->niv[p] * 2) / a->inc / 86400.0) * (86400.0 / a->cau);
     }
     for (int k = 0; k < ASSIST_BODY_NPLANETS; k++) D.gm[k] = a->mass[k];
     D.inv_cau = 1.0 / a->cau;
     D.cau_per_day = a->cau / 86400.;
+    D.inv_cau_per_day = 1.0 / D.cau_per_day;
     D.f_earth = -1.0 / (1.0 + a->cem);
     D.f_moon = a->cem / (1.0 + a->cem);
     const double l2 = std::log2(a->inc);

@@ -106,3 +106,24 @@ def test_dropin_run_kernel(files, n, t1):
     assert st == 0 and t == t1 and np.abs(g2 - g).max() < 1e-13
     st, t, _, _ = run([t1, 20000.0])
     assert st == 1 and t < 8500.0 or t1 < 8000.0
+
+
+@pytest.mark.parametrize("n", [1, 33, 1024, 1025, 1100])
+def test_bodies_bit_identical(files, n):
+    """Both body kernels (few times, many times; remainders of a tile) give the
+    oracle's bits, which are the reference's."""
+    import torch
+    from assist_gb300 import Ephem, batch
+    from tests.oracle_py import Oracle
+    pl, ast, _ = files
+    t = np.random.default_rng(n).uniform(7960.0, 8440.0, n)
+    status = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    B = batch.bodies_device(Ephem(pl, ast), torch.tensor(t, device="cuda"), status=status).cpu().numpy()
+    assert (status.cpu().numpy() == 0).all()
+    O = Oracle(pl, ast)
+    for k in range(0, n, max(1, n // 40)):
+        for i in range(27):
+            _, ref = O.body(i, t[k])
+            m = 10 if i < 11 else 4
+            assert np.array_equal(B[k, i, :m], ref[:m]), (k, i, B[k, i, :m] - ref[:m])
+            assert i < 11 or np.isnan(B[k, i, 4:]).all()
