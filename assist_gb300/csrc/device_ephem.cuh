@@ -61,6 +61,7 @@ struct AgPairView {
     float gm_jup, ek2, ek3, ek4, sk2;
     int n_packs;
     int col_sorted[10];
+    float inv_cau_h, inv_cau_l, f_earth_h, f_earth_l, f_moon_h, f_moon_l;
 };
 
 /* Everything a kernel needs to evaluate bodies; passed by value. */
@@ -86,6 +87,9 @@ struct DevEphem {
     int n_ast;
     const double* spk;           /* the whole SPK file as doubles */
     long long spk_ndbl;
+    const float2* pl_pair;       /* pl_data and spk as float pairs (hi, lo) */
+    const float2* spk_pair;
+    double ast_beg_max, ast_end_min;             /* the span every asteroid covers */
     double ast_beg[AG_MAX_AST], ast_end[AG_MAX_AST], ast_res[AG_MAX_AST], ast_gm[AG_MAX_AST];
     float ast_gm_hi[AG_MAX_AST], ast_gm_lo[AG_MAX_AST];   /* ast_gm as a float pair hi + lo */
     int ast_nseg[AG_MAX_AST], ast_seg0[AG_MAX_AST];

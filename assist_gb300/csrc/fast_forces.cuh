@@ -457,19 +457,20 @@ static __device__ __noinline__ void ag_fast_close(const DevEphem& E, const Force
 
 /* EIH relativity with the Sun as its source (src/forces.c:1288-1983): the
  * Sun's part in float pairs, the planets' and the Sun's motion (1e-3 of it)
- * in FP32.  d: pair separation from the Sun; up: sum of GM/r of the planets. */
-__device__ __forceinline__ void ag_fast_eih(const AgPairView& PV, const AgFastNode& H, const AgF2* d, const AgF2* v,
-                                            float up, AgF2* out) {
+ * in FP32.  w: the Sun's velocity; af, ut: the planets' pull on the Sun and
+ * their potential there; d: pair separation from the Sun; up: the planets'
+ * potential at the particle. */
+__device__ __forceinline__ void ag_fast_eih(const AgPairView& PV, const float* w, const float* af, float ut,
+                                            const AgF2* d, const AgF2* v, float up, AgF2* out) {
     const AgF2 r2 = ag_f2_add(ag_f2_mul(d[0], d[0]), ag_f2_add(ag_f2_mul(d[1], d[1]), ag_f2_mul(d[2], d[2])));
     const AgF2 ri = ag_f2_rsqrt(r2), ri2 = ag_f2_mul(ri, ri);
     const AgF2 gr = ag_f2_mul({PV.gm_sun_h, PV.gm_sun_l}, ri);
     const AgF2 v2 = ag_f2_add(ag_f2_mul(v[0], v[0]), ag_f2_add(ag_f2_mul(v[1], v[1]), ag_f2_mul(v[2], v[2])));
-    const float* w = H.vf;
     const float w2 = fmaf(w[0], w[0], fmaf(w[1], w[1], w[2] * w[2]));
     const float vw = fmaf(v[0].h, w[0], fmaf(v[1].h, w[1], v[2].h * w[2]));
     const float dw = fmaf(d[0].h, w[0], fmaf(d[1].h, w[1], d[2].h * w[2])) * ri.h;
-    const float da = fmaf(d[0].h, H.af[0], fmaf(d[1].h, H.af[1], d[2].h * H.af[2]));
-    const float rest = -4.0f * up - H.ut + 2.0f * w2 - 4.0f * vw - 1.5f * dw * dw - 0.5f * da;
+    const float da = fmaf(d[0].h, af[0], fmaf(d[1].h, af[1], d[2].h * af[2]));
+    const float rest = -4.0f * up - ut + 2.0f * w2 - 4.0f * vw - 1.5f * dw * dw - 0.5f * da;
     const AgF2 fac = ag_f2_add(ag_f2_add(v2, {-4.0f * gr.h, -4.0f * gr.l}), {rest, 0.0f});
     AgF2 f = {0.0f, 0.0f}, rel[3];
 #pragma unroll
@@ -482,7 +483,92 @@ __device__ __forceinline__ void ag_fast_eih(const AgPairView& PV, const AgFastNo
     const float ga = 3.5f * PV.oc2_h * gr.h;
 #pragma unroll
     for (int k = 0; k < 3; k++)
-        out[k] = ag_f2_add(ag_f2_add(ag_f2_mul(pd, d[k]), ag_f2_mul(pf, rel[k])), {ga * H.af[k], 0.0f});
+        out[k] = ag_f2_add(ag_f2_add(ag_f2_mul(pd, d[k]), ag_f2_mul(pf, rel[k])), {ga * af[k], 0.0f});
+}
+
+/* The Earth's J2, J3, J4 in FP32 at separation q (r2 = |q|^2), added to the
+ * low parts of the pair sums. */
+__device__ __forceinline__ void ag_fast_earth_h(const AgPairView& PV, const ForceCfg& c, const float* q, float r2, AgF2* acc) {
+    const float sa = c.f_pole[0], ca = c.f_pole[1], sd = c.f_pole[2], cd = c.f_pole[3];
+    const float p0 = -q[0] * sa + q[1] * ca, p1 = -q[0] * ca * sd - q[1] * sa * sd + q[2] * cd,
+                p2 = q[0] * ca * cd + q[1] * sa * cd + q[2] * sd;
+    const float ri = rsqrtf(r2), r2i = ri * ri, c2 = p2 * p2 * r2i, r5 = r2i * r2i * ri;
+    const float k2 = PV.ek2 * r5, k3 = PV.ek3 * r5, k4 = PV.ek4 * r5 * r2i;
+    const float f2 = 5.0f * c2 - 1.0f, f3 = 3.0f - 7.0f * c2, f4 = (63.0f * c2 - 42.0f) * c2 + 3.0f;
+    const float xy = k2 * f2 - k3 * r2i * f3 * p2 + k4 * f4;
+    const float o0 = xy * p0, o1 = xy * p1;
+    const float o2 = k2 * (f2 - 2.0f) * p2 - k3 * ((6.0f - 7.0f * c2) * c2 - 0.6f) + k4 * (f4 + 12.0f - 28.0f * c2) * p2;
+    acc[0].l += -o0 * sa - o1 * ca * sd + o2 * ca * cd;
+    acc[1].l += o0 * ca - o1 * sa * sd + o2 * sa * cd;
+    acc[2].l += o1 * cd + o2 * sd;
+}
+
+/* The Sun's J2, likewise. */
+__device__ __forceinline__ void ag_fast_sun_h(const AgPairView& PV, const ForceCfg& c, float qx, float qy, float qz, float r2,
+                                              AgF2* acc) {
+    const float nx = c.f_pole[5] * c.f_pole[7], ny = c.f_pole[4] * c.f_pole[7], nz = c.f_pole[6];
+    const float z = qx * nx + qy * ny + qz * nz;
+    const float ri = rsqrtf(r2), r2i = ri * ri, k2 = PV.sk2 * r2i * r2i * ri;
+    const float f2 = 5.0f * z * z * r2i - 1.0f, zz = -2.0f * z;
+    acc[0].l += k2 * (f2 * qx + zz * nx);
+    acc[1].l += k2 * (f2 * qy + zz * ny);
+    acc[2].l += k2 * (f2 * qz + zz * nz);
+}
+
+/* R^T M R of a symmetric M (pole frame) added to the six elements J. */
+__device__ __forceinline__ void ag_fast_rot_sym(const float* pole, const float M[3][3], float* J) {
+    const float sa = pole[0], ca = pole[1], sd = pole[2], cd = pole[3];
+    const float R[3][3] = {{-sa, ca, 0.0f}, {-ca * sd, -sa * sd, cd}, {ca * cd, sa * cd, sd}};
+    int at = 0;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        float v[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) v[k] = M[0][k] * R[0][a] + M[1][k] * R[1][a] + M[2][k] * R[2][a];
+#pragma unroll
+        for (int b = a; b < 3; b++, at++) J[at] += v[0] * R[0][b] + v[1] * R[1][b] + v[2] * R[2][b];
+    }
+}
+
+/* Jacobians of the harmonics in FP32 (the formulas of ag_term_earth_h and
+ * ag_term_sun_h), added to the six elements J. */
+__device__ __forceinline__ void ag_fast_earth_hj(const AgPairView& PV, const ForceCfg& c, const float* q, float r2, float* J) {
+    const float sa = c.f_pole[0], ca = c.f_pole[1], sd = c.f_pole[2], cd = c.f_pole[3];
+    const float p[3] = {-q[0] * sa + q[1] * ca, -q[0] * ca * sd - q[1] * sa * sd + q[2] * cd,
+                        q[0] * ca * cd + q[1] * sa * cd + q[2] * sd};
+    const float ri = rsqrtf(r2), r2i = ri * ri, c2 = p[2] * p[2] * r2i, r5 = r2i * r2i * ri;
+    const float k2 = PV.ek2 * r5, k3 = PV.ek3 * r5, k4 = PV.ek4 * r5 * r2i;
+    const float f2 = 5.0f * c2 - 1.0f, f3 = 3.0f - 7.0f * c2, f4 = (63.0f * c2 - 42.0f) * c2 + 3.0f;
+    const float g2 = 7.0f * c2 - 1.0f, g3 = (35.0f * c2 - 30.0f) * c2 + 3.0f, ct = p[2] * ri;
+    const float h2 = 21.0f * (1.0f - 3.0f * c2) * r2i, h3 = 3.0f * ((-21.0f * c2 + 14.0f) * c2 - 1.0f) * r2i;
+    const float h4 = ((-63.0f * c2 + 70.0f) * c2 - 15.0f) * ct * ri;
+    const float q2 = (33.0f * c2 - 18.0f) * c2 + 1.0f, q3 = (33.0f * c2 - 30.0f) * c2 + 5.0f;
+    const float q4 = ((231.0f * c2 - 315.0f) * c2 + 105.0f) * c2 - 5.0f;
+    float M[3][3];
+#pragma unroll
+    for (int a = 0; a < 2; a++) {
+        M[a][a] = k2 * (f2 - 5.0f * g2 * p[a] * p[a] * r2i) + k3 * ct * (h2 * p[a] * p[a] - f3) * ri +
+                  k4 * (f4 - 21.0f * q2 * p[a] * p[a] * r2i);
+        M[a][2] = M[2][a] = -5.0f * k2 * (g2 - 2.0f) * p[a] * p[2] * r2i + k3 * h3 * p[a] - 21.0f * k4 * q3 * p[a] * p[2] * r2i;
+    }
+    M[0][1] = M[1][0] = -5.0f * k2 * g2 * p[0] * p[1] * r2i + k3 * h2 * ct * p[0] * p[1] * ri - 21.0f * k4 * q2 * p[0] * p[1] * r2i;
+    M[2][2] = -k2 * g3 + k3 * h4 - 3.0f * k4 * q4;
+    ag_fast_rot_sym(c.f_pole, M, J);
+}
+__device__ __forceinline__ void ag_fast_sun_hj(const AgPairView& PV, const ForceCfg& c, const float* q, float r2, float* J) {
+    const float sa = c.f_pole[4], ca = c.f_pole[5], sd = c.f_pole[6], cd = c.f_pole[7];
+    const float p[3] = {-q[0] * sa + q[1] * ca, -q[0] * ca * sd - q[1] * sa * sd + q[2] * cd,
+                        q[0] * ca * cd + q[1] * sa * cd + q[2] * sd};
+    const float ri = rsqrtf(r2), r2i = ri * ri, c2 = p[2] * p[2] * r2i, k2 = PV.sk2 * r2i * r2i * ri;
+    const float f2 = 5.0f * c2 - 1.0f, g2 = 7.0f * c2 - 1.0f, g3 = (35.0f * c2 - 30.0f) * c2 + 3.0f;
+    float M[3][3];
+    M[0][0] = k2 * (f2 - 5.0f * g2 * p[0] * p[0] * r2i);
+    M[1][1] = k2 * (f2 - 5.0f * g2 * p[1] * p[1] * r2i);
+    M[2][2] = -k2 * g3;
+    M[0][1] = M[1][0] = -5.0f * k2 * g2 * p[0] * p[1] * r2i;
+    M[1][2] = M[2][1] = -5.0f * k2 * (g2 - 2.0f) * p[1] * p[2] * r2i;
+    M[0][2] = M[2][0] = -5.0f * k2 * (g2 - 2.0f) * p[0] * p[2] * r2i;
+    ag_fast_rot_sym(c.f_pole + 4, M, J);
 }
 
 /* The packs [p0, p1) of role w (0, 2 or 3). */
@@ -580,7 +666,7 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
             }
             const AgF2 v[3] = {F.vf[0][lane], F.vf[1][lane], F.vf[2][lane]};
             AgF2 e[3];
-            ag_fast_eih(E.pv, H, d, v, up, e);
+            ag_fast_eih(E.pv, H.vf, H.af, H.ut, d, v, up, e);
 #pragma unroll
             for (int k = 0; k < 3; k++)
                 if (!eih) acc[k] = ag_f2_add(acc[k], e[k]);
@@ -593,35 +679,12 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
             for (int k = 0; k < 3; k++) q[k] = xf[k].h + ag_pk_a(R[1].c[k].h);
             const float r2 = fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2]));
             ce = !(r2 >= 4.0e-4f && r2 < 1e30f);
-            if (!ce) {
-                const float sa = c.f_pole[0], ca = c.f_pole[1], sd = c.f_pole[2], cd = c.f_pole[3];
-                const float p0_ = -q[0] * sa + q[1] * ca, p1_ = -q[0] * ca * sd - q[1] * sa * sd + q[2] * cd,
-                            p2_ = q[0] * ca * cd + q[1] * sa * cd + q[2] * sd;
-                const float ri = rsqrtf(r2), r2i = ri * ri, c2 = p2_ * p2_ * r2i, r5 = r2i * r2i * ri;
-                const float k2 = E.pv.ek2 * r5, k3 = E.pv.ek3 * r5, k4 = E.pv.ek4 * r5 * r2i;
-                const float f2 = 5.0f * c2 - 1.0f, f3 = 3.0f - 7.0f * c2, f4 = (63.0f * c2 - 42.0f) * c2 + 3.0f;
-                const float xy = k2 * f2 - k3 * r2i * f3 * p2_ + k4 * f4;
-                const float o0 = xy * p0_, o1 = xy * p1_;
-                const float o2 = k2 * (f2 - 2.0f) * p2_ - k3 * ((6.0f - 7.0f * c2) * c2 - 0.6f) + k4 * (f4 + 12.0f - 28.0f * c2) * p2_;
-                acc[0].l += -o0 * sa - o1 * ca * sd + o2 * ca * cd;
-                acc[1].l += o0 * ca - o1 * sa * sd + o2 * sa * cd;
-                acc[2].l += o1 * cd + o2 * sd;
-            }
+            if (!ce) ag_fast_earth_h(E.pv, c, q, r2, acc);
         }
         if (c.forces & AG_F_SUN_H) {
             /* the Sun's J2: below 1e-9 of the acceleration beyond 0.1 AU */
             cs = !(rs2 >= 1.0e-2f && rs2 < 1e30f);
-            if (!cs) {
-                const float sa = c.f_pole[4], ca = c.f_pole[5], sd = c.f_pole[6], cd = c.f_pole[7];
-                const float qx = d[0].h, qy = d[1].h, qz = d[2].h;
-                const float nx = ca * cd, ny = sa * cd, nz = sd;
-                const float z = qx * nx + qy * ny + qz * nz;
-                const float ri = rsqrtf(rs2), r2i = ri * ri, k2 = E.pv.sk2 * r2i * r2i * ri;
-                const float f2 = 5.0f * z * z * r2i - 1.0f, zz = -2.0f * z;
-                acc[0].l += k2 * (f2 * qx + zz * nx);
-                acc[1].l += k2 * (f2 * qy + zz * ny);
-                acc[2].l += k2 * (f2 * qz + zz * nz);
-            }
+            if (!cs) ag_fast_sun_h(E.pv, c, d[0].h, d[1].h, d[2].h, rs2, acc);
         }
     }
     if (wild) {

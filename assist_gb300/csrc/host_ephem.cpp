@@ -45,6 +45,7 @@ struct ascii_s {
     double mass[ASSIST_BODY_NPLANETS];
     double J2E, J3E, J4E, J2SUN, AU, RE, CLIGHT, ASUN;
     double* d_data = nullptr;
+    float2* d_pair = nullptr;        /* d_data as float pairs */
     DevEphem* d_view = nullptr;      /* device copy of the last view handed to kernels */
     DevEphem h_view;                 /* host copy of *d_view */
     bool find(const char* name, double* out) const {
@@ -70,6 +71,7 @@ struct spk_s {
     std::vector<int> seg0;
     std::string comments;            /* comment area, NUL -> newline */
     double* d_data = nullptr;
+    float2* d_pair = nullptr;        /* asteroid files: d_data as float pairs */
     AgSpkSeg* d_segs = nullptr;
     AgRecMeta* d_meta = nullptr;
     DevEphem* d_view = nullptr;      /* planets files: device copy of the last view */
@@ -198,6 +200,14 @@ static ascii_s* ascii_load(const char* path) {
     return a;
 }
 
+/* The float-pair image of n doubles on the device (complete on return: the
+ * kernels that read it run on streams of their own). */
+static bool pair_upload(const double* d, float2** out, size_t n) {
+    return !ag_cuda_check(cudaMalloc(out, n * sizeof(float2) + 64), "cudaMalloc(float-pair image)") &&
+           !ag_cuda_check((cudaError_t)ag_launch_pair_image(d, *out, n), "float-pair image") &&
+           !ag_cuda_check(cudaStreamSynchronize(0), "float-pair image");
+}
+
 /* The device copy of the .440 image, made on first device use (loading and
  * validating a file is host work only). */
 static int ascii_upload(ascii_s* a) {
@@ -205,9 +215,12 @@ static int ascii_upload(ascii_s* a) {
     /* 64 bytes of padding: a record staged by a bulk copy is read from its
      * address rounded down to 16 bytes, for its length rounded up */
     if (ag_cuda_check(cudaMalloc(&a->d_data, a->data.size() * 8 + 64), "cudaMalloc(.440 records)") ||
-        ag_cuda_check(cudaMemcpy(a->d_data, a->data.data(), a->data.size() * 8, cudaMemcpyHostToDevice), "upload .440")) {
+        ag_cuda_check(cudaMemcpy(a->d_data, a->data.data(), a->data.size() * 8, cudaMemcpyHostToDevice), "upload .440") ||
+        !pair_upload(a->d_data, &a->d_pair, a->data.size())) {
         if (a->d_data) cudaFree(a->d_data);
+        if (a->d_pair) cudaFree(a->d_pair);
         a->d_data = nullptr;
+        a->d_pair = nullptr;
         return ASSIST_ERROR_EPHEM_FILE;
     }
     return 0;
@@ -216,6 +229,7 @@ static int ascii_upload(ascii_s* a) {
 static void ascii_free(ascii_s* a) {
     if (!a) return;
     if (a->d_data) cudaFree(a->d_data);
+    if (a->d_pair) cudaFree(a->d_pair);
     if (a->d_view) cudaFree(a->d_view);
     delete a;
 }
@@ -304,16 +318,19 @@ static spk_s* spk_load(const char* path) {
 
 /* The device copies of an SPK image, its segment table and record metadata,
  * made on first device use. */
-static int spk_upload(spk_s* s) {
+static int spk_upload(spk_s* s, bool pair) {
     if (s->d_data) return 0;
     bool ok = !ag_cuda_check(cudaMalloc(&s->d_data, s->data.size() * 8), "cudaMalloc(SPK)") &&
               !ag_cuda_check(cudaMemcpy(s->d_data, s->data.data(), s->data.size() * 8, cudaMemcpyHostToDevice), "upload SPK") &&
               !ag_cuda_check(cudaMalloc(&s->d_segs, sizeof(AgSpkSeg) * (s->segs.size() + 1)), "cudaMalloc(SPK segments)") &&
               !ag_cuda_check(cudaMemcpy(s->d_segs, s->segs.data(), sizeof(AgSpkSeg) * s->segs.size(), cudaMemcpyHostToDevice), "upload segments") &&
               !ag_cuda_check(cudaMalloc(&s->d_meta, sizeof(AgRecMeta) * (s->meta.size() + 1)), "cudaMalloc(SPK records)") &&
-              !ag_cuda_check(cudaMemcpy(s->d_meta, s->meta.data(), sizeof(AgRecMeta) * s->meta.size(), cudaMemcpyHostToDevice), "upload records");
+              !ag_cuda_check(cudaMemcpy(s->d_meta, s->meta.data(), sizeof(AgRecMeta) * s->meta.size(), cudaMemcpyHostToDevice), "upload records") &&
+              (!pair || pair_upload(s->d_data, &s->d_pair, s->data.size()));
     if (!ok) {
         if (s->d_data) cudaFree(s->d_data);
+        if (s->d_pair) cudaFree(s->d_pair);
+        s->d_pair = nullptr;
         if (s->d_segs) cudaFree(s->d_segs);
         if (s->d_meta) cudaFree(s->d_meta);
         s->d_data = nullptr; s->d_segs = nullptr; s->d_meta = nullptr;
@@ -325,6 +342,7 @@ static int spk_upload(spk_s* s) {
 static void spk_free(spk_s* s) {
     if (!s) return;
     if (s->d_data) cudaFree(s->d_data);
+    if (s->d_pair) cudaFree(s->d_pair);
     if (s->d_segs) cudaFree(s->d_segs);
     if (s->d_meta) cudaFree(s->d_meta);
     if (s->d_view) cudaFree(s->d_view);
@@ -418,8 +436,8 @@ static void spk_planets_view(const struct assist_ephem* e, DevEphem& D) {
 
 int ag_ephem_device(const struct assist_ephem* e, DevEphem* out) {
     if (!e || (!e->ascii_planets && !e->spk_planets)) return ASSIST_ERROR_EPHEM_FILE;
-    if ((e->spk_planets && spk_upload(e->spk_planets)) || (e->ascii_planets && ascii_upload(e->ascii_planets)) ||
-        (e->spk_asteroids && spk_upload(e->spk_asteroids)))
+    if ((e->spk_planets && spk_upload(e->spk_planets, false)) || (e->ascii_planets && ascii_upload(e->ascii_planets)) ||
+        (e->spk_asteroids && spk_upload(e->spk_asteroids, true)))
         return ASSIST_ERROR_EPHEM_FILE;
     DevEphem D;
     std::memset(&D, 0, sizeof(D));
@@ -432,6 +450,7 @@ int ag_ephem_device(const struct assist_ephem* e, DevEphem* out) {
 /* The planets part of the view for a .440/.441 file. */
 static void ag_ascii_view(const ascii_s* a, DevEphem& D) {
     D.pl_data = a->d_data;
+    D.pl_pair = a->d_pair;
     D.pl_ndbl = (long long)a->data.size();
     D.pl_rec_len = (int)a->rec;
     D.pl_nrec = (int)(a->data.size() / a->rec);
@@ -478,6 +497,10 @@ static void ag_pair_view(DevEphem& D) {
     V.ek3 = (float)(gme * 2.5 * D.J3E * Re2 * D.Re_eq);
     V.ek4 = (float)(gme * 0.625 * D.J4E * Re2 * Re2);
     V.sk2 = (float)(gms * 1.5 * D.J2SUN * D.Rs_eq * D.Rs_eq);
+    auto split = [](double x, float& h, float& l) { h = (float)x; l = (float)(x - (double)h); };
+    split(D.inv_cau, V.inv_cau_h, V.inv_cau_l);
+    split(D.f_earth, V.f_earth_h, V.f_earth_l);
+    split(D.f_moon, V.f_moon_h, V.f_moon_l);
     for (int k = 0; k < 10; k++) V.col_sorted[k] = k;
     if (!D.pl_spk)
         std::stable_sort(V.col_sorted, V.col_sorted + 10, [&](int a, int b) { return D.col_ncf[a] > D.col_ncf[b]; });
@@ -491,11 +514,16 @@ static int ag_finish_view(const struct assist_ephem* e, DevEphem& D, DevEphem* o
         if ((int)s->targets.size() > AG_MAX_AST) return ASSIST_ERROR_NAST;
         D.n_ast = (int)s->targets.size();
         D.spk = s->d_data;
+        D.spk_pair = s->d_pair;
         D.spk_ndbl = (long long)s->data.size();
         D.segs = s->d_segs;
         D.rec_meta = s->d_meta;
+        D.ast_beg_max = -1e300;
+        D.ast_end_min = 1e300;
         for (int m = 0; m < D.n_ast; m++) {
             const spk_target_h& t = s->targets[(size_t)m];
+            D.ast_beg_max = std::max(D.ast_beg_max, t.beg);
+            D.ast_end_min = std::min(D.ast_end_min, t.end);
             D.ast_beg[m] = t.beg; D.ast_end[m] = t.end; D.ast_res[m] = t.res; D.ast_gm[m] = t.mass;
             D.ast_gm_hi[m] = (float)t.mass;
             D.ast_gm_lo[m] = (float)(t.mass - (double)D.ast_gm_hi[m]);

@@ -84,6 +84,12 @@ int ag_launch_forces_coop(const DevEphem& E, const ForceCfg& c, int n, double t,
 int ag_launch_forces_each(const DevEphem& E, const ForceCfg& c, int n, const double* t, const double* state,
                           const double* params, int nv, const double* var_state, double* acc, double* var_acc,
                           int* status, cudaStream_t s);
+/* the same for the configurations ag_forces_own_covers (kernels_own.cu) */
+bool ag_forces_own_covers(const DevEphem& E, const ForceCfg& c, int nv);
+int ag_launch_forces_own(const DevEphem& E, const ForceCfg& c, int n, const double* t, const double* state,
+                         const double* params, int nv, const double* var_state, double* acc, double* var_acc, int* status,
+                         cudaStream_t s);
+int ag_launch_pair_image(const double* x, float2* out, size_t n);
 int ag_launch_bodies(const DevEphem& E, int n, const double* t, double* out, int* status, cudaStream_t s);
 size_t ag_batch_ws_doubles(int nslots, int nv);
 int ag_launch_batch(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int tpb, cudaStream_t s);

@@ -124,11 +124,43 @@ struct AgPkSum {
     AgPk h[3], l[3];
 };
 
+/* Running sum of the terms' Jacobian (src/forces.c: 3 GM d d^T / r^5 - GM I /
+ * r^3): its symmetric part xx, xy, xz, yy, yz, zz, times 2^40 (the low parts of
+ * GM / r^5 far from a light body would leave FP32's normal range), and the sum
+ * of GM / r^3. */
+#define AG_PK_JSCALE 0x1p40f
+struct AgPkJac {
+    AgPk h[7], l[7];
+};
+AG_PT void ag_pk_jac_clear(AgPkJac& J) {
+#pragma unroll
+    for (int k = 0; k < 7; k++) J.h[k] = J.l[k] = ag_pk(0.0f, 0.0f);
+}
+/* Element k of half a (0) or b (1) without the factor. */
+AG_PT void ag_pk_jac_get(const AgPkJac& J, int k, int half, float& h, float& l) {
+    const float s = k < 6 ? 1.0f / AG_PK_JSCALE : 1.0f;
+    h = s * (half ? ag_pk_b(J.h[k]) : ag_pk_a(J.h[k]));
+    l = s * (half ? ag_pk_b(J.l[k]) : ag_pk_a(J.l[k]));
+}
+
+/* (h, l) += x y for the pairs x = xh + xl, y = yh + yl. */
+AG_PT void ag_pk_acc(AgPk xh, AgPk xl, AgPk yh, AgPk yl, AgPk& h, AgPk& l) {
+    const AgPk p = ag_pk_mul(xh, yh);
+    AgPk pe = ag_pk_fma(xh, yh, ag_pk_neg(p));
+    pe = ag_pk_fma(xh, yl, pe);
+    pe = ag_pk_fma(xl, yh, pe);
+    AgPk e;
+    h = ag_pk_two_sum(h, p, e);
+    l = ag_pk_add(l, ag_pk_add(e, pe));
+}
+
 /* Adds the terms of the two bodies of R to S at the position xh + xl
  * (packed: the same value in both halves); rs2: squared heliocentric distance
  * (FP32).  Returns bit 0 / bit 1 set for a body below its threshold (or not
- * finite), whose term is left out. */
-AG_PT unsigned ag_pk_term(const AgPkRel& R, const AgPkGm& G, const AgPk* xh, const AgPk* xl, float rs2, AgPkSum& S) {
+ * finite), whose term is left out.  JAC: their Jacobian into J too. */
+template <bool JAC = false>
+AG_PT unsigned ag_pk_term(const AgPkRel& R, const AgPkGm& G, const AgPk* xh, const AgPk* xl, float rs2, AgPkSum& S,
+                          AgPkJac* J = nullptr) {
     const AgPk m1 = ag_pk(-1.0f, -1.0f);
     AgPk dh[3], dl[3], p[3], ne[3];
 #pragma unroll
@@ -169,14 +201,31 @@ AG_PT unsigned ag_pk_term(const AgPkRel& R, const AgPkGm& G, const AgPk* xh, con
     gh = ag_pk(na ? 0.0f : ag_pk_a(gh), nb ? 0.0f : ag_pk_b(gh));
     gl = ag_pk(na ? 0.0f : ag_pk_a(gl), nb ? 0.0f : ag_pk_b(gl));
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const AgPk ph = ag_pk_mul(gh, dh[k]);
-        AgPk pe = ag_pk_fma(gh, dh[k], ag_pk_mul(ph, m1));
-        pe = ag_pk_fma(gh, dl[k], pe);
-        pe = ag_pk_fma(gl, dh[k], pe);
+    for (int k = 0; k < 3; k++) ag_pk_acc(gh, gl, dh[k], dl[k], S.h[k], S.l[k]);
+    if (JAC) {
+        /* f = -3 G / |d|^2 with 1 / |d|^2 = y^2 (1 - delta + delta^2); e = f d */
+        const AgPk m3 = ag_pk(-3.0f, -3.0f);
+        const AgPk c2 = ag_pk_mul(del, ag_pk_sub(del, ag_pk(1.0f, 1.0f)));
+        const AgPk sc = ag_pk(AG_PK_JSCALE, AG_PK_JSCALE);
+        const AgPk ih = ag_pk_mul(q, sc), il = ag_pk_mul(ag_pk_sub(ag_pk_mul(q, c2), nqe), sc);
+        const AgPk g3h = ag_pk_mul(gh, m3), g3l = ag_pk_fma(gl, m3, ag_pk_fma(gh, m3, ag_pk_neg(g3h)));
+        const AgPk fh = ag_pk_mul(g3h, ih);
+        AgPk fl = ag_pk_fma(g3h, ih, ag_pk_neg(fh));
+        fl = ag_pk_fma(g3h, il, fl);
+        fl = ag_pk_fma(g3l, ih, fl);
+        int at = 0;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const AgPk eh = ag_pk_mul(fh, dh[a]);
+            AgPk el = ag_pk_fma(fh, dh[a], ag_pk_neg(eh));
+            el = ag_pk_fma(fh, dl[a], el);
+            el = ag_pk_fma(fl, dh[a], el);
+#pragma unroll
+            for (int b = a; b < 3; b++, at++) ag_pk_acc(eh, el, dh[b], dl[b], J->h[at], J->l[at]);
+        }
         AgPk e;
-        S.h[k] = ag_pk_two_sum(S.h[k], ph, e);
-        S.l[k] = ag_pk_add(S.l[k], ag_pk_add(e, pe));
+        J->h[6] = ag_pk_two_sum(J->h[6], ag_pk_neg(gh), e);
+        J->l[6] = ag_pk_add(J->l[6], ag_pk_sub(e, gl));
     }
     return (na ? 1u : 0u) | (nb ? 2u : 0u);
 }

@@ -127,3 +127,55 @@ def test_bodies_bit_identical(files, n):
             m = 10 if i < 11 else 4
             assert np.array_equal(B[k, i, :m], ref[:m]), (k, i, B[k, i, :m] - ref[:m])
             assert i < 11 or np.isnan(B[k, i, 4:]).all()
+
+
+@pytest.mark.parametrize("n,var", [(1, False), (31, True), (33, False), (70, True)])
+def test_own_time_forces_at_thresholds(files, n, var):
+    """Each particle at its own time: tile remainders, particles on either side
+    of the pair bodies' thresholds and of the harmonics', and (accelerations)
+    beyond FP32's range; a time outside the ephemeris marks its particle only."""
+    import torch
+    from assist_gb300 import Ephem, batch, synth
+    from tests.oracle_py import Oracle
+    pl, ast, system = files
+    t0 = 8200.0
+    rng = np.random.default_rng(n)
+    pop = synth.population(system, "mix", n, seed=n, t0=t0, nongrav_frac=0.3)
+    extra, te = [], []
+    for k in range(9):
+        for f in (0.7, 1.3, 1.5):
+            t = t0 + rng.uniform(-100, 100)
+            body = system.body(k + 1 if k < 5 else k + 2, np.array(t))
+            thr = max(MASS[k] / 1e-3, (150 * MASS[k]) ** (2 / 3)) ** 0.5
+            u = rng.normal(size=3); u /= np.linalg.norm(u)
+            extra.append(np.concatenate([body[0] + f * thr * np.linalg.norm(body[0]) * u, body[1]])); te.append(t)
+    for b, d in ((3, 0.03), (3, 0.09), (3, 0.11), (0, 0.08), (0, 0.12)):
+        body = system.body(b, np.array(t0))
+        u = rng.normal(size=3); u /= np.linalg.norm(u)
+        extra.append(np.concatenate([body[0] + d * u, body[1] + 1e-2 * u[::-1]])); te.append(t0)
+    if not var:
+        for far in (300.0, 2e6, 1e13):
+            u = rng.normal(size=3); u /= np.linalg.norm(u)
+            extra.append(np.concatenate([far * u, 1e-2 * u[::-1]])); te.append(t0)
+    state = np.concatenate([pop.state, np.array(extra)])
+    tt = np.concatenate([t0 + rng.uniform(-100, 100, n), te])
+    params = np.concatenate([pop.params, np.zeros((len(extra), 3))])
+    vs = rng.normal(size=(len(state), 6, 6)) if var else None
+    dev = lambda a: None if a is None else torch.tensor(a, device="cuda")  # noqa: E731
+    eph, O = Ephem(pl, ast), Oracle(pl, ast)
+    status = torch.full((len(state),), -1, dtype=torch.int32, device="cuda")
+    acc, vacc = batch.forces_device(eph, dev(tt), dev(state), params=dev(params), var_state=dev(vs), status=status)
+    assert (status.cpu().numpy() == 0).all()
+    acc = acc.cpu().numpy()
+    for i in range(len(state)):
+        kw = dict(var_state=vs[i], var_tp=np.zeros(6, np.int32)) if var else {}
+        ref = O.forces(tt[i], state[i:i + 1], params=params[i:i + 1], **kw)
+        assert np.linalg.norm(acc[i] - ref[0]) < TOL * np.linalg.norm(ref[0]), (i, np.linalg.norm(acc[i] - ref[0]) / np.linalg.norm(ref[0]))
+        if var:
+            scale = np.linalg.norm(ref[1:], axis=1).max()
+            d = np.linalg.norm(vacc[i].cpu().numpy() - ref[1:], axis=1).max()
+            assert d <= TOL * scale, (i, d / scale)
+    tt[0] = 20000.0
+    _, _ = batch.forces_device(eph, dev(tt), dev(state), params=dev(params), var_state=dev(vs), status=status)
+    s = status.cpu().numpy()
+    assert s[0] == 5 and (s[1:] == 0).all()

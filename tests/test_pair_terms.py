@@ -45,8 +45,27 @@ int main() {
         h[0] = (float)gm; l[0] = (float)(gm - h[0]);
         G.h = ag_pk(h[0], h[0]); G.l = ag_pk(l[0], l[0]);
         G.ta = G.tb = 0.0f;
-        if (ag_pk_term(A, G, xh, xl, 1.0f, S) != 0) bad++;
+        AgPkJac J;
+        ag_pk_jac_clear(J);
+        if (ag_pk_term<true>(A, G, xh, xl, 1.0f, S, &J) != 0) bad++;
         for (int j = 0; j < 2; j++) {
+            /* Jacobian: the term's bound with its slope of 5 over d, per element over its norm */
+            {
+                long double d[3], r2 = 0, t[7], e2 = 0, t2 = 0;
+                for (int k = 0; k < 3; k++) { d[k] = (long double)x[k] - b[j][k]; r2 += d[k] * d[k]; }
+                const long double g = (long double)gm / (r2 * sqrtl(r2));
+                int at = 0;
+                for (int a = 0; a < 3; a++) for (int c = a; c < 3; c++) t[at++] = 3 * g * d[a] * d[c] / r2;
+                t[6] = g;
+                for (int k = 0; k < 7; k++) {
+                    float jh, jl;
+                    ag_pk_jac_get(J, k, j, jh, jl);
+                    const long double v = (long double)jh + jl;
+                    e2 += (v - t[k]) * (v - t[k]); t2 += t[k] * t[k];
+                }
+                const double far = R + (j ? 3.0 : 1.0) * D;
+                if (!((double)sqrtl(e2 / t2) < 2.5e-13 + 5.0 * 2.0 * 0x1p-48 * far / ((j ? 3.0 : 1.0) * D))) { std::printf("jacobian d %g: %g\n", D, (double)sqrtl(e2 / t2)); bad++; }
+            }
             long double d[3], r2 = 0, e2 = 0, t2 = 0;
             for (int k = 0; k < 3; k++) { d[k] = (long double)x[k] - b[j][k]; r2 += d[k] * d[k]; }
             for (int k = 0; k < 3; k++) {
