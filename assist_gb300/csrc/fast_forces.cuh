@@ -9,19 +9,20 @@
  * harmonics, away from their body, are FP32 (below 1e-9).  Each has an error
  * below 2e-17 of the acceleration; an FP64 sum of the terms rounds by 1e-16.
  *
- * Four warps (roles) share an evaluation, lane l of each working on particle l:
- *   role 1       Sun, Jupiter, non-gravitational and GR terms, all FP64
- *   roles 0, 2   half of the pair terms' bodies each (fewer than 3 packs short)
- *   role 3       the rest of them, relativity, harmonics
+ * Eight warps (roles) share an evaluation, lane l of each working on particle l:
+ *   role 0       Jupiter, FP64           role 1   Sun, non-gravitational, GR, FP64
+ *   roles 2, 3   a few of the pair terms' packs; the Sun's, the Earth's harmonics
+ *   role 4       relativity              roles 5, 6, 7   the other packs
  * An SM does one FP64 warp instruction in 19 cycles over its four
- * sub-partitions (64 to 76 on one warp), so what bounds an evaluation is the
- * FP64 instructions: about 150 a group and evaluation with IAS15's own,
- * against 515 with every term but the asteroids' in FP64.
+ * sub-partitions (64 to 76 on one warp): about 150 a group and evaluation with
+ * IAS15's own, against 515 with every term but the asteroids' in FP64.  Two
+ * warps a sub-partition, because the FP32 streams are chains of dependent
+ * instructions (7 cycles an instruction with one).
  *
  * The tables of up to eight times are built together (ag_fast_tables): a
  * lane forms one body's three components at one time, so a step's eight
- * tables take about 105 FP64 instructions on each warp, where eight separate
- * tables with a lane a component took 1,700 over the four.
+ * tables take about 60 FP64 instructions on each warp, where eight separate
+ * tables with a lane a component took 1,700 over four.
  */
 #ifndef ASSIST_GB300_FAST_FORCES_CUH
 #define ASSIST_GB300_FAST_FORCES_CUH
@@ -69,13 +70,16 @@ struct AgFastView {
 };
 
 /* A block's shared arrays of the evaluation. */
+#define AG_FAST_WARPS 8
+#define AG_FAST_THREADS (32 * AG_FAST_WARPS)
+#define AG_FAST_SLOTS 6             /* roles 2..7 */
 struct AgFastShared {
     double xs[3][32], vs[3][32];    /* particle states at the node */
     AgF2 xf[3][32], vf[3][32];      /* and as float pairs */
-    double pa[3][32];               /* role 1's partial accelerations */
-    AgF2 pf[3][3][32];              /* roles 0, 2, 3: [role 0, 2, 3 -> 0, 1, 2] */
-    double pn[3][3][32];            /* their FP64 parts, where near[] says so */
-    int near[3];
+    double pa[2][3][32];            /* roles 0 and 1: FP64 partial accelerations */
+    AgF2 pf[AG_FAST_SLOTS][3][32];  /* roles 2..7: pair sums */
+    double pn[AG_FAST_SLOTS][3][32];            /* their FP64 parts, where near[] says so */
+    int near[AG_FAST_SLOTS];
     double sun[8][3];               /* the Sun's raw position sums of the tables */
     AgPkGm gm[AG_MAX_PACKS];        /* masses; zero where the configuration leaves the body out */
 };
@@ -218,7 +222,7 @@ __device__ __forceinline__ int ag_fast_tables(const DevEphem& E, const ForceCfg&
      * planets (a lane a column and time, columns by falling length), the Sun
      * (a lane a component and time), asteroids (a lane a body and time) */
     const int n_pl = (10 * nn + 31) / 32, n_as = (E.n_ast * nn + 31) / 32;
-    for (int piece = wid; piece < n_pl + 1 + n_as; piece += 4) {
+    for (int piece = wid; piece < n_pl + 1 + n_as; piece += AG_FAST_WARPS) {
         if (piece < n_pl) {
             const int q = piece * 32 + lane, col = q / nn, n = q - col * nn;
             if (col < 10) {
@@ -310,7 +314,7 @@ __device__ __forceinline__ int ag_fast_tables(const DevEphem& E, const ForceCfg&
     /* origin minus body in AU, and its float pair */
     const double icau = E.pl_spk ? 1.0 / E.au_km : E.inv_cau;
     const int per = 3 * nn;
-    for (int q = tid; q < per * (2 + V.L.bodies); q += 128) {
+    for (int q = tid; q < per * (2 + V.L.bodies); q += AG_FAST_THREADS) {
         const int body = q / per, r = q - body * per, n = r / 3, comp = r - 3 * n;
         AgFastNode& H = V.node(n);
         if (body == 0) {
@@ -356,7 +360,7 @@ __device__ __forceinline__ int ag_fast_tables(const DevEphem& E, const ForceCfg&
         pk[2] = 0.0f;
     }
     __syncthreads();
-    if ((c.forces & AG_F_EIH) && wid == 3) {
+    if ((c.forces & AG_F_EIH) && wid == 4) {
         /* the planets' pull on the Sun and their potential there (1e-3 of the
          * relativistic term's factor: FP32), four lanes a time */
         const int n = lane >> 2;
@@ -455,6 +459,22 @@ static __device__ __noinline__ void ag_fast_close(const DevEphem& E, const Force
     a[0] = ax; a[1] = ay; a[2] = az;
 }
 
+/* Pair operations without the final renormalisation (the low part may grow to
+ * a few units of the high part's last place): enough for the relativistic
+ * term, which needs about 30 bits. */
+__device__ __forceinline__ AgF2 ag_q_mul(AgF2 a, AgF2 b) {
+    const float h = __fmul_rn(a.h, b.h);
+    return {h, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.h, b.h, -h)))};
+}
+__device__ __forceinline__ AgF2 ag_q_add(AgF2 a, AgF2 b) {
+    const float s = __fadd_rn(a.h, b.h), bb = __fsub_rn(s, a.h);
+    const float e = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, bb)), __fsub_rn(b.h, bb));
+    return {s, __fadd_rn(e, __fadd_rn(a.l, b.l))};
+}
+__device__ __forceinline__ AgF2 ag_q_dot(const AgF2* a, const AgF2* b) {
+    return ag_q_add(ag_q_mul(a[0], b[0]), ag_q_add(ag_q_mul(a[1], b[1]), ag_q_mul(a[2], b[2])));
+}
+
 /* EIH relativity with the Sun as its source (src/forces.c:1288-1983): the
  * Sun's part in float pairs, the planets' and the Sun's motion (1e-3 of it)
  * in FP32.  w: the Sun's velocity; af, ut: the planets' pull on the Sun and
@@ -462,57 +482,67 @@ static __device__ __noinline__ void ag_fast_close(const DevEphem& E, const Force
  * potential at the particle. */
 __device__ __forceinline__ void ag_fast_eih(const AgPairView& PV, const float* w, const float* af, float ut,
                                             const AgF2* d, const AgF2* v, float up, AgF2* out) {
-    const AgF2 r2 = ag_f2_add(ag_f2_mul(d[0], d[0]), ag_f2_add(ag_f2_mul(d[1], d[1]), ag_f2_mul(d[2], d[2])));
-    const AgF2 ri = ag_f2_rsqrt(r2), ri2 = ag_f2_mul(ri, ri);
-    const AgF2 gr = ag_f2_mul({PV.gm_sun_h, PV.gm_sun_l}, ri);
-    const AgF2 v2 = ag_f2_add(ag_f2_mul(v[0], v[0]), ag_f2_add(ag_f2_mul(v[1], v[1]), ag_f2_mul(v[2], v[2])));
+    const AgF2 r2 = ag_q_dot(d, d);
+    /* 1/r = y (1 - delta / 2 + 3/8 delta^2), delta = r2 y^2 - 1 */
+    const float y = rsqrtf(r2.h);
+    const AgF2 q = ag_q_mul({y, 0.0f}, {y, 0.0f}), t = ag_q_mul(r2, q);
+    const float del = __fadd_rn(__fsub_rn(t.h, 1.0f), t.l);
+    const AgF2 ri = {y, __fmul_rn(y, __fmul_rn(del, fmaf(0.375f, del, -0.5f)))}, ri2 = ag_q_mul(ri, ri);
+    const AgF2 gr = ag_q_mul({PV.gm_sun_h, PV.gm_sun_l}, ri), v2 = ag_q_dot(v, v);
     const float w2 = fmaf(w[0], w[0], fmaf(w[1], w[1], w[2] * w[2]));
     const float vw = fmaf(v[0].h, w[0], fmaf(v[1].h, w[1], v[2].h * w[2]));
-    const float dw = fmaf(d[0].h, w[0], fmaf(d[1].h, w[1], d[2].h * w[2])) * ri.h;
+    const float dw = __fmul_rn(fmaf(d[0].h, w[0], fmaf(d[1].h, w[1], d[2].h * w[2])), ri.h);
     const float da = fmaf(d[0].h, af[0], fmaf(d[1].h, af[1], d[2].h * af[2]));
-    const float rest = -4.0f * up - ut + 2.0f * w2 - 4.0f * vw - 1.5f * dw * dw - 0.5f * da;
-    const AgF2 fac = ag_f2_add(ag_f2_add(v2, {-4.0f * gr.h, -4.0f * gr.l}), {rest, 0.0f});
-    AgF2 f = {0.0f, 0.0f}, rel[3];
+    const float rest = fmaf(-4.0f, up, fmaf(2.0f, w2, fmaf(-4.0f, vw, fmaf(-1.5f, __fmul_rn(dw, dw), fmaf(-0.5f, da, -ut)))));
+    const AgF2 fac = ag_q_add(ag_q_add(v2, {-4.0f * gr.h, -4.0f * gr.l}), {rest, 0.0f});
+    AgF2 fv[3], rel[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        f = ag_f2_add(f, ag_f2_mul(d[k], ag_f2_add({4.0f * v[k].h, 4.0f * v[k].l}, {-3.0f * w[k], 0.0f})));
-        rel[k] = ag_f2_add(v[k], {-w[k], 0.0f});
+        fv[k] = ag_q_add({4.0f * v[k].h, 4.0f * v[k].l}, {-3.0f * w[k], 0.0f});
+        rel[k] = ag_q_add(v[k], {-w[k], 0.0f});
     }
-    const AgF2 pre = ag_f2_mul({PV.oc2_h, PV.oc2_l}, ag_f2_mul(gr, ri2));
-    const AgF2 pf = ag_f2_mul(pre, f), pd = ag_f2_neg(ag_f2_mul(pre, fac));
+    const AgF2 pre = ag_q_mul({PV.oc2_h, PV.oc2_l}, ag_q_mul(gr, ri2));
+    const AgF2 pf = ag_q_mul(pre, ag_q_dot(d, fv)), pd = ag_f2_neg(ag_q_mul(pre, fac));
     const float ga = 3.5f * PV.oc2_h * gr.h;
 #pragma unroll
-    for (int k = 0; k < 3; k++)
-        out[k] = ag_f2_add(ag_f2_add(ag_f2_mul(pd, d[k]), ag_f2_mul(pf, rel[k])), {ga * af[k], 0.0f});
+    for (int k = 0; k < 3; k++) {
+        const AgF2 o = ag_q_add(ag_q_mul(pd, d[k]), ag_q_mul(pf, rel[k]));
+        out[k] = ag_q_add(o, {ga * af[k], 0.0f});
+    }
 }
 
 /* The Earth's J2, J3, J4 in FP32 at separation q (r2 = |q|^2), added to the
  * low parts of the pair sums. */
 __device__ __forceinline__ void ag_fast_earth_h(const AgPairView& PV, const ForceCfg& c, const float* q, float r2, AgF2* acc) {
+    /* explicit roundings: every build of a kernel computes the same bits */
     const float sa = c.f_pole[0], ca = c.f_pole[1], sd = c.f_pole[2], cd = c.f_pole[3];
-    const float p0 = -q[0] * sa + q[1] * ca, p1 = -q[0] * ca * sd - q[1] * sa * sd + q[2] * cd,
-                p2 = q[0] * ca * cd + q[1] * sa * cd + q[2] * sd;
-    const float ri = rsqrtf(r2), r2i = ri * ri, c2 = p2 * p2 * r2i, r5 = r2i * r2i * ri;
-    const float k2 = PV.ek2 * r5, k3 = PV.ek3 * r5, k4 = PV.ek4 * r5 * r2i;
-    const float f2 = 5.0f * c2 - 1.0f, f3 = 3.0f - 7.0f * c2, f4 = (63.0f * c2 - 42.0f) * c2 + 3.0f;
-    const float xy = k2 * f2 - k3 * r2i * f3 * p2 + k4 * f4;
-    const float o0 = xy * p0, o1 = xy * p1;
-    const float o2 = k2 * (f2 - 2.0f) * p2 - k3 * ((6.0f - 7.0f * c2) * c2 - 0.6f) + k4 * (f4 + 12.0f - 28.0f * c2) * p2;
-    acc[0].l += -o0 * sa - o1 * ca * sd + o2 * ca * cd;
-    acc[1].l += o0 * ca - o1 * sa * sd + o2 * sa * cd;
-    acc[2].l += o1 * cd + o2 * sd;
+    const float cs = __fmul_rn(ca, sd), ss = __fmul_rn(sa, sd), cc = __fmul_rn(ca, cd), sc = __fmul_rn(sa, cd);
+    const float p0 = fmaf(-q[0], sa, __fmul_rn(q[1], ca)), p1 = fmaf(-q[0], cs, fmaf(-q[1], ss, __fmul_rn(q[2], cd))),
+                p2 = fmaf(q[0], cc, fmaf(q[1], sc, __fmul_rn(q[2], sd)));
+    const float ri = rsqrtf(r2), r2i = __fmul_rn(ri, ri), c2 = __fmul_rn(__fmul_rn(p2, p2), r2i),
+                r5 = __fmul_rn(__fmul_rn(r2i, r2i), ri);
+    const float k2 = __fmul_rn(PV.ek2, r5), k3 = __fmul_rn(PV.ek3, r5), k4 = __fmul_rn(__fmul_rn(PV.ek4, r5), r2i);
+    const float f2 = fmaf(5.0f, c2, -1.0f), f3 = fmaf(-7.0f, c2, 3.0f), f4 = fmaf(fmaf(63.0f, c2, -42.0f), c2, 3.0f);
+    const float xy = fmaf(k2, f2, fmaf(k4, f4, -__fmul_rn(__fmul_rn(k3, r2i), __fmul_rn(f3, p2))));
+    const float o0 = __fmul_rn(xy, p0), o1 = __fmul_rn(xy, p1);
+    const float o2 = fmaf(__fmul_rn(k2, f2 - 2.0f), p2,
+                          fmaf(-k3, fmaf(fmaf(-7.0f, c2, 6.0f), c2, -0.6f),
+                               __fmul_rn(__fmul_rn(k4, fmaf(-28.0f, c2, f4 + 12.0f)), p2)));
+    acc[0].l = __fadd_rn(acc[0].l, fmaf(-o0, sa, fmaf(-o1, cs, __fmul_rn(o2, cc))));
+    acc[1].l = __fadd_rn(acc[1].l, fmaf(o0, ca, fmaf(-o1, ss, __fmul_rn(o2, sc))));
+    acc[2].l = __fadd_rn(acc[2].l, fmaf(o1, cd, __fmul_rn(o2, sd)));
 }
 
 /* The Sun's J2, likewise. */
 __device__ __forceinline__ void ag_fast_sun_h(const AgPairView& PV, const ForceCfg& c, float qx, float qy, float qz, float r2,
                                               AgF2* acc) {
-    const float nx = c.f_pole[5] * c.f_pole[7], ny = c.f_pole[4] * c.f_pole[7], nz = c.f_pole[6];
-    const float z = qx * nx + qy * ny + qz * nz;
-    const float ri = rsqrtf(r2), r2i = ri * ri, k2 = PV.sk2 * r2i * r2i * ri;
-    const float f2 = 5.0f * z * z * r2i - 1.0f, zz = -2.0f * z;
-    acc[0].l += k2 * (f2 * qx + zz * nx);
-    acc[1].l += k2 * (f2 * qy + zz * ny);
-    acc[2].l += k2 * (f2 * qz + zz * nz);
+    const float nx = __fmul_rn(c.f_pole[5], c.f_pole[7]), ny = __fmul_rn(c.f_pole[4], c.f_pole[7]), nz = c.f_pole[6];
+    const float z = fmaf(qx, nx, fmaf(qy, ny, __fmul_rn(qz, nz)));
+    const float ri = rsqrtf(r2), r2i = __fmul_rn(ri, ri), k2 = __fmul_rn(__fmul_rn(PV.sk2, __fmul_rn(r2i, r2i)), ri);
+    const float f2 = fmaf(__fmul_rn(5.0f, z), __fmul_rn(z, r2i), -1.0f), zz = -2.0f * z;
+    acc[0].l = fmaf(k2, fmaf(f2, qx, __fmul_rn(zz, nx)), acc[0].l);
+    acc[1].l = fmaf(k2, fmaf(f2, qy, __fmul_rn(zz, ny)), acc[1].l);
+    acc[2].l = fmaf(k2, fmaf(f2, qz, __fmul_rn(zz, nz)), acc[2].l);
 }
 
 /* R^T M R of a symmetric M (pole frame) added to the six elements J. */
@@ -571,84 +601,69 @@ __device__ __forceinline__ void ag_fast_sun_hj(const AgPairView& PV, const Force
     ag_fast_rot_sym(c.f_pole + 4, M, J);
 }
 
-/* The packs [p0, p1) of role w (0, 2 or 3). */
+/* The packs [p0, p1) of role w: dealt to roles 5, 6, 7, 2, 3, the remainder
+ * to the first of them. */
 __device__ __forceinline__ void ag_fast_range(int packs, int w, int& p0, int& p1) {
-    const int n3 = packs > 3 ? (packs - 3) / 3 : 0, h = (packs - n3 + 1) / 2;
-    p0 = w == 0 ? 0 : (w == 2 ? h : packs - n3);
-    p1 = w == 0 ? h : (w == 2 ? packs - n3 : packs);
+    const int at = w >= 5 ? w - 5 : w + 1, q = packs / 5, r = packs % 5;
+    p0 = w == 4 ? 0 : at * q + min(at, r);
+    p1 = w == 4 ? 0 : p0 + q + (at < r ? 1 : 0);
 }
 
 /* Role w's share of the evaluation at table n: FP64 partial sums to F.pa
- * (role 1), float pairs to F.pf and, with near[] set, FP64 sums to F.pn
- * (roles 0, 2, 3).  Every lane of the warp calls it; `on` lanes count.  The
+ * (roles 0, 1), float pairs to F.pf and, with near[] set, FP64 sums to F.pn
+ * (roles 2..7).  Every lane of the warp calls it; `on` lanes count.  The
  * caller synchronises the block before (states) and after (sums). */
 __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const DevEphem& E, const ForceCfg& c,
                                               const AgFastView& V, int n, AgFastShared& F, const double* A) {
     const AgFastNode& H = V.node(n);
-    if (w == 1) {
+    if (w < 2) {
         if (!on) return;
         const double x[3] = {F.xs[0][lane], F.xs[1][lane], F.xs[2][lane]};
-        const double s[3] = {x[0] + H.rs[0], x[1] + H.rs[1], x[2] + H.rs[2]};
+        const double* o = w == 0 ? H.rj : H.rs;
+        const double s[3] = {x[0] + o[0], x[1] + o[1], x[2] + o[2]};
         const double ri = rsqrt(fma(s[0], s[0], fma(s[1], s[1], s[2] * s[2])));
         double ax = 0.0, ay = 0.0, az = 0.0;
-        if ((c.forces & AG_F_NONGRAV) && A != nullptr && (A[0] != 0.0 || A[1] != 0.0 || A[2] != 0.0)) {
-            const double dv[3] = {F.vs[0][lane] - H.sv[0], F.vs[1][lane] - H.sv[1], F.vs[2][lane] - H.sv[2]};
-            double JA[3][3];
-            bool has_ng;
-            ag_term_nongrav<false>(c, s, ri, dv, A, ax, ay, az, nullptr, JA, &has_ng);
+        if (w == 1) {
+            const bool ng = (c.forces & AG_F_NONGRAV) && A != nullptr && (A[0] != 0.0 || A[1] != 0.0 || A[2] != 0.0);
+            if (ng || (c.forces & (AG_F_GR_POT | AG_F_GR_SIMPLE))) {
+                const double dv[3] = {F.vs[0][lane] - H.sv[0], F.vs[1][lane] - H.sv[1], F.vs[2][lane] - H.sv[2]};
+                if (ng) {
+                    double JA[3][3];
+                    bool has_ng;
+                    ag_term_nongrav<false>(c, s, ri, dv, A, ax, ay, az, nullptr, JA, &has_ng);
+                }
+                if (c.forces & (AG_F_GR_POT | AG_F_GR_SIMPLE)) {
+                    double a[3] = {ax, ay, az};
+                    ag_coop_gr_cold(E, c, s, ri, dv, a);
+                    ax = a[0]; ay = a[1]; az = a[2];
+                }
+            }
         }
-        if (c.forces & (AG_F_GR_POT | AG_F_GR_SIMPLE)) {
-            const double dv[3] = {F.vs[0][lane] - H.sv[0], F.vs[1][lane] - H.sv[1], F.vs[2][lane] - H.sv[2]};
-            double a[3] = {ax, ay, az};
-            ag_coop_gr_cold(E, c, s, ri, dv, a);
-            ax = a[0]; ay = a[1]; az = a[2];
-        }
-        if (c.forces & AG_F_PLANETS) {
-            const double j[3] = {x[0] + H.rj[0], x[1] + H.rj[1], x[2] + H.rj[2]};
-            const double rj = rsqrt(fma(j[0], j[0], fma(j[1], j[1], j[2] * j[2]))), g = E.gm[AG_JUP] * rj * rj * rj;
-            ax = fma(-g, j[0], ax); ay = fma(-g, j[1], ay); az = fma(-g, j[2], az);
-        }
-        const double g = E.gm[AG_SUN] * ri * ri * ri;
-        F.pa[0][lane] = fma(-g, s[0], ax); F.pa[1][lane] = fma(-g, s[1], ay); F.pa[2][lane] = fma(-g, s[2], az);
+        const double gm = w == 1 ? E.gm[AG_SUN] : ((c.forces & AG_F_PLANETS) ? E.gm[AG_JUP] : 0.0);
+        const double g = gm * ri * ri * ri;
+        F.pa[w][0][lane] = fma(-g, s[0], ax); F.pa[w][1][lane] = fma(-g, s[1], ay); F.pa[w][2][lane] = fma(-g, s[2], az);
         return;
     }
-    const int out = w == 0 ? 0 : w - 1;
+    const int slot = w - 2;
     const AgF2 xf[3] = {F.xf[0][lane], F.xf[1][lane], F.xf[2][lane]};
     const AgPkRel* R = V.packs(n);
-    float rs2;
-    {
-        const float sx = xf[0].h + H.sp[0].h, sy = xf[1].h + H.sp[1].h, sz = xf[2].h + H.sp[2].h;
-        rs2 = fmaf(sx, sx, fmaf(sy, sy, sz * sz));
-    }
-    AgPkSum S;
-    unsigned near = 0;
-    int p0, p1;
-    ag_fast_range(V.L.packs, w, p0, p1);
-    {
-        AgPk xh[3], xl[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            xh[k] = ag_pk(xf[k].h, xf[k].h);
-            xl[k] = ag_pk(xf[k].l, xf[k].l);
-            S.h[k] = S.l[k] = ag_pk(0.0f, 0.0f);
-        }
-#pragma unroll 1
-        for (int p = p0; p < p1; p++) near |= ag_pk_term(R[p], F.gm[p], xh, xl, rs2, S) << (2 * (p - p0));
-    }
-    AgF2 acc[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-        acc[k] = ag_f2_add({ag_pk_a(S.h[k]), ag_pk_a(S.l[k])}, {ag_pk_b(S.h[k]), ag_pk_b(S.l[k])});
+    const float sx = xf[0].h + H.sp[0].h, sy = xf[1].h + H.sp[1].h, sz = xf[2].h + H.sp[2].h;
+    const float rs2 = fmaf(sx, sx, fmaf(sy, sy, sz * sz));
     /* beyond 200 AU the planets' pull on the Sun, FP32 in the pair form, is no
      * longer a small part of the relativistic term: that is FP64 there; beyond
      * 1e6 AU, where the products' small parts approach FP32's smallest numbers,
      * every term is */
     const float big = fmaxf(fabsf(xf[0].h), fmaxf(fabsf(xf[1].h), fabsf(xf[2].h)));
-    const bool wild = !(big < 1e6f), eih = w == 3 && (c.forces & AG_F_EIH) && !(big < 200.0f);
-    bool ce = false, cs = false;
-    if (w == 3) {
-        const AgF2 d[3] = {ag_f2_add(xf[0], H.sp[0]), ag_f2_add(xf[1], H.sp[1]), ag_f2_add(xf[2], H.sp[2])};
+    const bool wild = !(big < 1e6f);
+    bool eih = false, ce = false, cs = false;
+    unsigned near = 0;
+    int p0, p1;
+    ag_fast_range(V.L.packs, w, p0, p1);
+    AgF2 acc[3];
+    if (w == 4) {
+        acc[0] = acc[1] = acc[2] = {0.0f, 0.0f};
         if (c.forces & AG_F_EIH) {
+            eih = !(big < 200.0f);
             /* the planets' potential at the particle */
             float up;
             {
@@ -664,16 +679,28 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
                 up = fmaf(F.gm[p].ga, rsqrtf(ag_pk_a(r2)), up);
                 if (2 * p + 1 < AG_PAIR_PL) up = fmaf(F.gm[p].gb, rsqrtf(ag_pk_b(r2)), up);
             }
+            const AgF2 d[3] = {ag_f2_add(xf[0], H.sp[0]), ag_f2_add(xf[1], H.sp[1]), ag_f2_add(xf[2], H.sp[2])};
             const AgF2 v[3] = {F.vf[0][lane], F.vf[1][lane], F.vf[2][lane]};
             AgF2 e[3];
             ag_fast_eih(E.pv, H.vf, H.af, H.ut, d, v, up, e);
-#pragma unroll
-            for (int k = 0; k < 3; k++)
-                if (!eih) acc[k] = ag_f2_add(acc[k], e[k]);
+            if (!eih) { acc[0] = e[0]; acc[1] = e[1]; acc[2] = e[2]; }
         }
-        if (c.forces & AG_F_EARTH_H) {
-            /* J2, J3, J4 about the pole frame's z axis: below 3e-11 of the
-             * acceleration beyond 0.02 AU */
+    } else {
+        AgPkSum S;
+        AgPk xh[3], xl[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            xh[k] = ag_pk(xf[k].h, xf[k].h);
+            xl[k] = ag_pk(xf[k].l, xf[k].l);
+            S.h[k] = S.l[k] = ag_pk(0.0f, 0.0f);
+        }
+#pragma unroll 1
+        for (int p = p0; p < p1; p++) near |= ag_pk_term(R[p], F.gm[p], xh, xl, rs2, S) << (2 * (p - p0));
+#pragma unroll
+        for (int k = 0; k < 3; k++)
+            acc[k] = ag_f2_add({ag_pk_a(S.h[k]), ag_pk_a(S.l[k])}, {ag_pk_b(S.h[k]), ag_pk_b(S.l[k])});
+        if (w == 3 && (c.forces & AG_F_EARTH_H)) {
+            /* J2, J3, J4: below 3e-11 of the acceleration beyond 0.02 AU */
             float q[3];
 #pragma unroll
             for (int k = 0; k < 3; k++) q[k] = xf[k].h + ag_pk_a(R[1].c[k].h);
@@ -681,18 +708,18 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
             ce = !(r2 >= 4.0e-4f && r2 < 1e30f);
             if (!ce) ag_fast_earth_h(E.pv, c, q, r2, acc);
         }
-        if (c.forces & AG_F_SUN_H) {
-            /* the Sun's J2: below 1e-9 of the acceleration beyond 0.1 AU */
+        if (w == 2 && (c.forces & AG_F_SUN_H)) {
+            /* J2: below 1e-9 of the acceleration beyond 0.1 AU */
             cs = !(rs2 >= 1.0e-2f && rs2 < 1e30f);
-            if (!cs) ag_fast_sun_h(E.pv, c, d[0].h, d[1].h, d[2].h, rs2, acc);
+            if (!cs) ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, acc);
+        }
+        if (wild) {
+            near = (1u << (2 * (p1 - p0))) - 1u;
+#pragma unroll
+            for (int k = 0; k < 3; k++) acc[k] = {0.0f, 0.0f};
         }
     }
-    if (wild) {
-        near = (1u << (2 * (p1 - p0))) - 1u;
-#pragma unroll
-        for (int k = 0; k < 3; k++) acc[k] = {0.0f, 0.0f};
-    }
-    const bool mine = on && (near != 0 || ce || cs || wild || eih);
+    const bool mine = on && (near != 0 || ce || cs || eih);
     const bool any = __any_sync(AG_FULL, mine);
     if (any) {
         double a[3] = {0.0, 0.0, 0.0};
@@ -707,20 +734,23 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
             const double v[3] = {F.vs[0][lane], F.vs[1][lane], F.vs[2][lane]};
             ag_fast_close(E, c, &V, &H, n, 2 * p0, m, ce, cs, eih, x, v, a);
         }
-        F.pn[out][0][lane] = a[0]; F.pn[out][1][lane] = a[1]; F.pn[out][2][lane] = a[2];
+        F.pn[slot][0][lane] = a[0]; F.pn[slot][1][lane] = a[1]; F.pn[slot][2][lane] = a[2];
     }
-    if (lane == 0) F.near[out] = any ? 1 : 0;
-    if (on) { F.pf[out][0][lane] = acc[0]; F.pf[out][1][lane] = acc[1]; F.pf[out][2][lane] = acc[2]; }
+    if (lane == 0) F.near[slot] = any ? 1 : 0;
+    if (on) { F.pf[slot][0][lane] = acc[0]; F.pf[slot][1][lane] = acc[1]; F.pf[slot][2][lane] = acc[2]; }
 }
 
 /* Component k of the acceleration of lane l's particle, after the block has met. */
 __device__ __forceinline__ double ag_fast_sum(const AgFastShared& F, int k, int lane) {
-    const AgF2 s = ag_f2_add(ag_f2_add(F.pf[2][k][lane], F.pf[1][k][lane]), F.pf[0][k][lane]);
-    double a = ag_f2_to(s) + F.pa[k][lane];
-    if (F.near[0] | F.near[1] | F.near[2]) {
-        for (int w = 0; w < 3; w++)
+    const AgF2 s = ag_f2_add(ag_f2_add(ag_f2_add(F.pf[0][k][lane], F.pf[1][k][lane]), F.pf[2][k][lane]),
+                             ag_f2_add(F.pf[3][k][lane], ag_f2_add(F.pf[4][k][lane], F.pf[5][k][lane])));
+    double a = (ag_f2_to(s) + F.pa[0][k][lane]) + F.pa[1][k][lane];
+    int any = 0;
+#pragma unroll
+    for (int w = 0; w < AG_FAST_SLOTS; w++) any |= F.near[w];
+    if (any)
+        for (int w = 0; w < AG_FAST_SLOTS; w++)
             if (F.near[w]) a += F.pn[w][k][lane];
-    }
     return a;
 }
 

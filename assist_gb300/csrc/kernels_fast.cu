@@ -5,14 +5,13 @@
  * the others and the variational particles).
  *
  * A group of up to 32 particles that share their step times is integrated by
- * one 128-thread block, as in ias15_coop.cuh: the same step rules, the same
- * statuses, the same order of the sums over a group.  What differs is where
- * the work goes: warp 1 evaluates the terms kept in FP64 and controls the
- * steps (sizes, times, convergence, retirement: lane masks the other warps
- * read), warps 0, 2 and 3 own the components x, y, z and evaluate the pair
- * terms; the step's eight tables are built together at its start; the
- * quadratures multiply by reciprocals and the step-size root is a Newton
- * iteration (a warp's FP64 division is 8.5 instructions, its pow 100).
+ * one block, as in ias15_coop.cuh, with the same step rules and statuses.
+ * What differs is where the work goes: eight warps with the shares of
+ * ag_fast_force and ias15_fast.cuh, of which warp 1 controls the steps (sizes,
+ * times, convergence, retirement: lane masks the other warps read); the
+ * step's eight tables are built together at its start; the quadratures
+ * multiply by reciprocals and the step-size root is a Newton iteration (a
+ * warp's FP64 division is 8.5 instructions, its pow 100).
  */
 #include <cuda_runtime.h>
 
@@ -102,7 +101,7 @@ struct AgFastNearest {
  * memory; WARM: the learned warm start and the logging of its pairs.  The
  * arithmetic is the same in all. */
 template <int OCC, bool STAGE, bool WARM>
-__global__ void __launch_bounds__(128, OCC) ag_k_fast(const DevEphem* __restrict__ Ep, ForceCfg cf, AgBatchArgs A) {
+__global__ void __launch_bounds__(AG_FAST_THREADS, OCC) ag_k_fast(const DevEphem* __restrict__ Ep, ForceCfg cf, AgBatchArgs A) {
     const DevEphem& E = *Ep;
     __shared__ AgFastSmem M;
     AgFastStep& S = M.S;
@@ -120,8 +119,8 @@ __global__ void __launch_bounds__(128, OCC) ag_k_fast(const DevEphem* __restrict
         M.stage_fail = 0;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31, wid = ((threadIdx.x >> 5) + M.rot) & 3, tid = (wid << 5) | lane;
-    const int pc = ag_fast_comp(wid);
+    const int lane = threadIdx.x & 31, wid = ((threadIdx.x >> 5) + M.rot) & 7, tid = (wid << 5) | lane;
+    const int pc = ag_fast_comp(wid), hc = ag_fast_help(wid);
     const bool ctl = wid == 1;
     extern __shared__ __align__(16) unsigned char ag_dyn_smem[];
     const Ws<3> W{reinterpret_cast<double*>(ag_dyn_smem), 32, lane};
@@ -277,7 +276,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_fast(const DevEphem* __restrict
                     if (fail) { M.stage_fail = 1; srec = nullptr; }
                 }
             }
-            if (live && pc >= 0) ag_fast_predict(W, S, pc, lane, 0);
+            if (live) ag_fast_predict(W, S, pc, hc, lane, 0);
             n_tab += 8;
             if (WARM && tid == 0) clk_step = clock64();
             if (ag_fast_tables(E, cf, 8, S.ptn, V, S.F, tid, srec, ssrc)) {
@@ -298,22 +297,24 @@ __global__ void __launch_bounds__(128, OCC) ag_k_fast(const DevEphem* __restrict
                     w_ran = ag_warm_start<3>(A, W.w, W.ns, W.slot, pc, WS, AgFastNearest{V}, lane, wid, live, warm,
                                              wl_on && M.wg_off == 0, S.hstep, M.dtls, wsteps, w_applied, w_probe,
                                              n_wused, n_wfall);
+                __syncthreads();        /* the owners' b for the helpers */
             }
-            if (live && pc >= 0) ag_fast_start(W, pc);
+            if (live) ag_fast_start(W, pc, hc);
+            __syncthreads();            /* a0 for the velocity predictor's warps */
             /* ---- predictor-corrector iterations */
             int iters = 1, it_lane = 0;
             double pc_last = 1e300, ma7 = 0.0, mb6 = 0.0;
             bool conv = !live;
             while (true) {
                 for (int n = 1; n < 8; n++) {
-                    if (!conv && pc >= 0) ag_fast_predict(W, S, pc, lane, n);
+                    if (!conv) ag_fast_predict(W, S, pc, hc, lane, n);
                     __syncthreads();
                     ag_fast_force(wid, lane, !conv, E, cf, V, n, S.F, Ap);
                     if (ctl && !conv) n_ev++;
                     __syncthreads();
                     if (!conv && pc >= 0) ag_fast_correct(W, S, pc, lane, n);
+                    __syncthreads();
                 }
-                __syncthreads();
                 if (!conv) {
                     ma7 = ag_max3(S.ra, lane);
                     mb6 = ag_max3(S.rb6, lane);
@@ -393,12 +394,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_fast(const DevEphem* __restrict
             const int cmd = S.cmd;
             if (cmd == 2) continue;
             if (cmd == 1) {
-                if (live && pc >= 0) {
-                    const double ratio = S.aratio;
-                    if (ratio != 0.0) ag_fast_shift(W, pc, ratio);
-                    else
-                        for (int k = 0; k < 7; k++) { W(W_B + k, pc) = 0.0; W(W_E + k, pc) = 0.0; }
-                }
+                if (live) ag_fast_retry(W, pc, hc, S.aratio);
                 if (ctl) {
                     if (live) n_rej++;
                     dt = dt_new;
@@ -412,7 +408,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_fast(const DevEphem* __restrict
             }
             /* ---- accept */
             if (dense && live) on = ag_fast_dense(A, W, pc, on, on_end, dir, S.t, S.tc, S.ah, (S.last & bit) != 0, tend);
-            if (live && pc >= 0) ag_fast_accept(W, pc, S.ah, S.aratio);
+            ag_fast_accept(W, pc, hc, live, S.ah, S.aratio);
             if (ctl) {
                 if (live) n_acc++;
                 const double y = hstep + tc, s = t + y;
@@ -456,7 +452,7 @@ template <int OCC, bool STAGE, bool WARM>
 static int ag_fast_blocks_per_sm(int n_ast) {
     int bps = 0;
     if (ag_fast_attr<OCC, STAGE, WARM>() == 0)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ag_k_fast<OCC, STAGE, WARM>, 128,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ag_k_fast<OCC, STAGE, WARM>, AG_FAST_THREADS,
                                                       AgFastDyn<STAGE, WARM>::bytes(n_ast));
     return bps;
 }
@@ -478,7 +474,7 @@ template <int OCC, bool STAGE, bool WARM>
 static int ag_fast_go(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, cudaStream_t s) {
     const int e = ag_fast_attr<OCC, STAGE, WARM>();
     if (e) return e;
-    ag_k_fast<OCC, STAGE, WARM><<<(a.nslots + 31) / 32, 128, AgFastDyn<STAGE, WARM>::bytes(E.n_ast), s>>>(E.self_dev, c, a);
+    ag_k_fast<OCC, STAGE, WARM><<<(a.nslots + 31) / 32, AG_FAST_THREADS, AgFastDyn<STAGE, WARM>::bytes(E.n_ast), s>>>(E.self_dev, c, a);
     return (int)cudaGetLastError();
 }
 

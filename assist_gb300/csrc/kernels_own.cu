@@ -20,7 +20,8 @@
  *   before the barrier   role 1: the Sun; role 0: Jupiter, Earth and Moon,
  *                        an eighth of the asteroids; role 2: the other
  *                        planets, a quarter; role 3: the rest
- *   after it             the roles of ag_fast_force
+ *   after it             role 1: Sun, Jupiter, FP64 terms; roles 0, 2: pair terms;
+ *                        role 3: the rest of them, relativity, harmonics
  */
 #include <cuda_runtime.h>
 
@@ -81,6 +82,14 @@ struct AgOwnJac {
     AgF2 p[3][7][32];                           /* pair parts: symmetric part and trace sum */
 };
 
+/* The packs [p0, p1) of role w (0, 2 or 3; role 3 has relativity and the
+ * harmonics too). */
+__device__ __forceinline__ void ag_own_range(int packs, int w, int& p0, int& p1) {
+    const int n3 = packs > 3 ? (packs - 3) / 3 : 0, h = (packs - n3 + 1) / 2;
+    p0 = w == 0 ? 0 : (w == 2 ? h : packs - n3);
+    p1 = w == 0 ? h : (w == 2 ? packs - n3 : packs);
+}
+
 /* A .440 column as float pairs (km). */
 __device__ __forceinline__ void ag_own_column(const DevEphem& E, size_t rec, int col, double tf, AgF2* u) {
     const int ncf = E.col_ncf[col], niv = E.col_niv[col];
@@ -105,7 +114,7 @@ static __device__ __noinline__ void ag_own_close(const DevEphem& E, const ForceC
     const int packs = E.pv.n_packs;
     for (int r = 0; r < 3; r++) {
         int p0, p1;
-        ag_fast_range(packs, r == 0 ? 0 : r + 1, p0, p1);
+        ag_own_range(packs, r == 0 ? 0 : r + 1, p0, p1);
         unsigned m = S.near[r][lane];
         while (m) {
             const int k = 2 * p0 + __ffs(m) - 1;
@@ -395,7 +404,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
         if (JAC) ag_pk_jac_clear(PJ);
         unsigned near = 0;
         int p0, p1;
-        ag_fast_range(packs, wid, p0, p1);
+        ag_own_range(packs, wid, p0, p1);
 #pragma unroll 1
         for (int p = p0; p < p1; p++) {
             AgPkRel R;

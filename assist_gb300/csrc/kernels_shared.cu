@@ -487,11 +487,12 @@ __device__ __forceinline__ bool sh_run_barrier(unsigned* bar) {
 
 enum { SH_ACCEPT = 0, SH_REJECT, SH_ITERATE, SH_LEAVE };
 
-__global__ void __launch_bounds__(128, 2) sh_k_run(const DevEphem* __restrict__ Ep, ForceCfg c, ShRunArgs A) {
+__global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* __restrict__ Ep, ForceCfg c, ShRunArgs A) {
     extern __shared__ __align__(16) unsigned char sh_smem[];
     __shared__ AgFastStep S;
     const DevEphem& E = *Ep;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, pc = ag_fast_comp(wid), i = 32 * blockIdx.x + lane;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, pc = ag_fast_comp(wid), hc = ag_fast_help(wid);
+    const int i = 32 * blockIdx.x + lane;
     const bool ctl = wid == 1, live = i < A.n;
     const Ws<3> W{reinterpret_cast<double*>(sh_smem), 32, lane};
     const AgFastView V(sh_smem + sizeof(double) * W_NF * 3 * 32, E.n_ast);
@@ -519,28 +520,27 @@ __global__ void __launch_bounds__(128, 2) sh_k_run(const DevEphem* __restrict__ 
             ag_fast_nodes(S, lane, K.t, K.tc, hstep);
         }
         __syncthreads();
-        if (live && pc >= 0) ag_fast_predict(W, S, pc, lane, 0);
+        if (live) ag_fast_predict(W, S, pc, hc, lane, 0);
         if (ag_fast_tables(E, c, 8, S.ptn, V, S.F, tid)) {
             K.status = AG_ERR_COVERAGE;          /* every block builds the same tables */
             break;
         }
         ag_fast_force(wid, lane, live, E, c, V, 0, S.F, Ap);
         __syncthreads();
-        if (live && pc >= 0) {
-            W(W_A0, pc) = ag_fast_sum(S.F, pc, lane);
-            ag_fast_start(W, pc);
-        }
+        if (live && pc >= 0) W(W_A0, pc) = ag_fast_sum(S.F, pc, lane);
+        if (live) ag_fast_start(W, pc, hc);
+        __syncthreads();            /* a0 for the velocity predictor's warps */
         double pc_last = 1e300;
         int iters = 1, cmd;
         while (true) {
             for (int n = 1; n < 8; n++) {
-                if (live && pc >= 0) ag_fast_predict(W, S, pc, lane, n);
+                if (live) ag_fast_predict(W, S, pc, hc, lane, n);
                 __syncthreads();
                 ag_fast_force(wid, lane, live, E, c, V, n, S.F, Ap);
                 __syncthreads();
                 if (live && pc >= 0) ag_fast_correct(W, S, pc, lane, n);
+                __syncthreads();
             }
-            __syncthreads();
             if (ctl) {
                 double ma = ag_warp_max_nonneg(live ? ag_max3(S.ra, lane) : 0.0);
                 double mdb = ag_warp_max_nonneg(live ? ag_max3(S.rdb, lane) : 0.0);
@@ -611,21 +611,20 @@ __global__ void __launch_bounds__(128, 2) sh_k_run(const DevEphem* __restrict__ 
             iters++;
         }
         const bool leave = S.fin != 0;
-        if (live && pc >= 0) {
-            if (cmd == SH_ACCEPT) {
+        if (cmd == SH_ACCEPT) {
+            if (live && pc >= 0) {
                 /* the step's start, for dense output */
                 A.W(S_PX, pc, i) = W(W_X0, pc) + W(W_XC, pc);
                 A.W(S_PV, pc, i) = W(W_V0, pc) + W(W_VC, pc);
                 A.W(S_PA, pc, i) = W(W_A0, pc);
-                ag_fast_accept(W, pc, S.ah, S.aratio);
-            } else if (cmd == SH_REJECT) {
-                if (S.aratio != 0.0) ag_fast_shift(W, pc, S.aratio);
-                else
-                    for (int k = 0; k < 7; k++) { W(W_B + k, pc) = 0.0; W(W_E + k, pc) = 0.0; }
             }
+            ag_fast_accept(W, pc, hc, live, S.ah, S.aratio);
+        } else if (cmd == SH_REJECT && live) {
+            ag_fast_retry(W, pc, hc, S.aratio);
         }
         if (leave) break;
     }
+    __syncthreads();
     if (live && pc >= 0)
         for (int f = 0; f < 8; f++)
             for (int k = 0; k < (f < 4 ? 1 : 7); k++) A.W(theirs[f] + k, pc, i) = W(mine[f] + k, pc);
@@ -648,7 +647,7 @@ static int sh_run_capacity(int n_ast) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (cudaFuncSetAttribute(sh_k_run, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh_run_bytes(AG_MAX_AST)) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, sh_k_run, 128, sh_run_bytes(n_ast)) != cudaSuccess)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, sh_k_run, AG_FAST_THREADS, sh_run_bytes(n_ast)) != cudaSuccess)
         return 0;
     return can ? bps * sms : 1;
 }
@@ -786,7 +785,7 @@ __global__ void __launch_bounds__(128) sh_k_forces_coop(const DevEphem* __restri
  * covers: a block builds the table of t once and takes groups of 32
  * particles in turn (the table's chain of about 100 FP64 instructions a warp
  * is a group's evaluation twice over). */
-__global__ void __launch_bounds__(128, 3) sh_k_forces_fast(const DevEphem* __restrict__ Ep, ForceCfg c, int n, double t,
+__global__ void __launch_bounds__(AG_FAST_THREADS, 2) sh_k_forces_fast(const DevEphem* __restrict__ Ep, ForceCfg c, int n, double t,
                                                            const double* __restrict__ state,
                                                            const double* __restrict__ params, double* acc, int* status) {
     extern __shared__ __align__(16) unsigned char sh_smem[];
@@ -806,19 +805,23 @@ __global__ void __launch_bounds__(128, 3) sh_k_forces_fast(const DevEphem* __res
             if (status && tid < 32 && live) status[i] = AG_ERR_COVERAGE;
             continue;
         }
-        const int k = wid == 0 ? 0 : wid - 1;
+        const int k = ag_fast_comp(wid), h = ag_fast_help(wid);
         double prm[3] = {0.0, 0.0, 0.0};
-        if (live && wid != 1) {
-            const double x = state[6 * (size_t)i + k], v = state[6 * (size_t)i + 3 + k];
-            F.xs[k][lane] = x; F.vs[k][lane] = v;
-            F.xf[k][lane] = ag_f2_of(x); F.vf[k][lane] = ag_f2_of(v);
-        } else if (live && params) {
+        if (live && k >= 0) {
+            const double x = state[6 * (size_t)i + k];
+            F.xs[k][lane] = x;
+            F.xf[k][lane] = ag_f2_of(x);
+        } else if (live && h >= 0) {
+            const double v = state[6 * (size_t)i + 3 + h];
+            F.vs[h][lane] = v;
+            F.vf[h][lane] = ag_f2_of(v);
+        } else if (live && params && wid == 1) {
             for (int q = 0; q < 3; q++) prm[q] = params[3 * (size_t)i + q];
         }
         __syncthreads();
         ag_fast_force(wid, lane, live, E, c, V, 0, F, params ? prm : nullptr);
         __syncthreads();
-        if (live && wid != 1) {
+        if (live && k >= 0) {
             acc[3 * (size_t)i + k] = ag_fast_sum(F, k, lane);
             if (k == 0 && status) status[i] = AG_OK;
         }
@@ -838,8 +841,8 @@ int ag_launch_forces_coop(const DevEphem& E, const ForceCfg& c, int n, double t,
             cudaDeviceGetAttribute(&m, cudaDevAttrMultiProcessorCount, dev);
             if (dev >= 0 && dev < 64) sms[dev] = m;
         }
-        const int groups = (n + 31) / 32, blocks = groups < 3 * m ? groups : 3 * m;
-        sh_k_forces_fast<<<blocks, 128, AgFastLayout(E.n_ast).stride, s>>>(E.self_dev, c, n, t, state, params, acc, status);
+        const int groups = (n + 31) / 32, blocks = groups < 2 * m ? groups : 2 * m;
+        sh_k_forces_fast<<<blocks, AG_FAST_THREADS, AgFastLayout(E.n_ast).stride, s>>>(E.self_dev, c, n, t, state, params, acc, status);
         return (int)cudaGetLastError();
     }
     if (!(dev >= 0 && dev < 64 && done[dev])) {
@@ -1129,13 +1132,13 @@ static int sh_run(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct r
         A.out = &s->d_run->ctl[1 - (launch & 1)];
         if (launch) cudaMemsetAsync(A.red, 0, sizeof(m.red) + sizeof(m.bar), st);
         if (nb == 1) {
-            sh_k_run<<<1, 128, bytes, st>>>(E.self_dev, c, A);
+            sh_k_run<<<1, AG_FAST_THREADS, bytes, st>>>(E.self_dev, c, A);
             if (ag_cuda_check(cudaGetLastError(), "IAS15 run kernel")) return 1;
         } else {
             const DevEphem* ep = E.self_dev;
             ForceCfg cc = c;
             void* args[] = {(void*)&ep, (void*)&cc, (void*)&A};
-            const cudaError_t le = cudaLaunchCooperativeKernel((const void*)sh_k_run, nb, 128, args, bytes, st);
+            const cudaError_t le = cudaLaunchCooperativeKernel((const void*)sh_k_run, nb, AG_FAST_THREADS, args, bytes, st);
             if (le == cudaErrorCooperativeLaunchTooLarge && launch == 0) {
                 cudaGetLastError();
                 s->run_blocks = 1;

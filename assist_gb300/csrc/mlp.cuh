@@ -119,11 +119,12 @@ __device__ __forceinline__ void ag_mlp_layer(const __nv_bfloat16* in, const __nv
 /* Inference for the 32 rows in M.X by a 128-thread block (all threads call
  * it; it synchronises the block).  Result in M.Y. */
 __device__ __forceinline__ void ag_mlp_infer_block(const AgMlpDev& N, AgMlpSmem& M, int wid, int lane) {
-    for (int half = 0; half < 2; half++)
+    /* four warps work, any further ones of the block keep the barriers */
+    for (int half = 0; half < 2 && wid < 4; half++)
         ag_mlp_layer<AG_MLP_IN, AG_MLP_LDX, 4, true>(&M.X[0][0], N.W1, N.b1, 64 * wid + 32 * half, &M.H1[0][0],
                                                      nullptr, lane);
     __syncthreads();
-    for (int half = 0; half < 2; half++)
+    for (int half = 0; half < 2 && wid < 4; half++)
         ag_mlp_layer<AG_MLP_HID, AG_MLP_LDH, 4, true>(&M.H1[0][0], N.W2, N.b2, 64 * wid + 32 * half, &M.H2[0][0],
                                                       nullptr, lane);
     __syncthreads();

@@ -179,3 +179,21 @@ def test_own_time_forces_at_thresholds(files, n, var):
     _, _ = batch.forces_device(eph, dev(tt), dev(state), params=dev(params), var_state=dev(vs), status=status)
     s = status.cpu().numpy()
     assert s[0] == 5 and (s[1:] == 0).all()
+
+
+def test_batch_repeats_bit_for_bit(files):
+    """The builds of the batched kernel, and one build run again, give the same
+    bits (their warps share the state across barriers)."""
+    import torch
+    from assist_gb300 import Ephem, batch, synth
+    pl, ast, system = files
+    eph = Ephem(pl, ast)
+    pop = synth.population(system, "neo", 6000, seed=4, t0=8000.0, length=200.0, nongrav_frac=0.2)
+    dev = lambda a: torch.tensor(a, device="cuda")  # noqa: E731
+    t0, te, prm = dev(pop.t0), dev(pop.t_end), dev(pop.params)
+    out = []
+    for kw in (dict(blocks_per_sm=2), dict(blocks_per_sm=2), dict(blocks_per_sm=3), dict(ephem_staging=1)):
+        st = dev(pop.state)
+        batch.integrate_batch_device(eph, t0, te, st, params=prm, opts=batch.options(**kw))
+        out.append(st.cpu().numpy())
+    assert all(np.array_equal(out[0], o) for o in out[1:])
