@@ -19,7 +19,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libassist_gb300.so")
-SOURCES = ["kernels_forces.cu", "kernels_ias15.cu", "kernels_coop.cu", "kernels_fast.cu", "kernels_own.cu", "kernels_shared.cu", "static_batch.cu", "kernels_mlp.cu",
+SOURCES = ["kernels_forces.cu", "kernels_ias15.cu", "kernels_coop.cu", "kernels_fast.cu", "kernels_own.cu", "kernels_var.cu", "kernels_shared.cu", "static_batch.cu", "kernels_mlp.cu",
            "kernels_pilot.cu", "host_ephem.cpp", "api.cpp", "autotune.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON = ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off", "-lineinfo",

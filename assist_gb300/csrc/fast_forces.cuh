@@ -511,6 +511,47 @@ __device__ __forceinline__ void ag_fast_eih(const AgPairView& PV, const float* w
     }
 }
 
+/* Relativity with its Jacobian in FP64 (the formulas of ag_term_eih_core for
+ * the Sun as the source): d, ri the separation from the Sun, w the Sun's
+ * velocity, aj the planets' pull on the Sun, ut their potential there, up and
+ * gp their potential and the sum of GM d / r^3 at the particle. */
+__device__ __forceinline__ void ag_fast_eih_jac(const DevEphem& E, const double* d, double ri, const double* v, const double* w,
+                                               const double* aj, double ut, double up, const double* gp, double* acc,
+                                               double (*J)[6]) {
+    const double oc2 = E.over_c_squared, gs = E.gm[AG_SUN], r2i = ri * ri, gr = gs * ri, pre = gr * r2i;
+    const double vi2 = fma(v[0], v[0], fma(v[1], v[1], v[2] * v[2])), vj2 = fma(w[0], w[0], fma(w[1], w[1], w[2] * w[2]));
+    const double vivj = fma(v[0], w[0], fma(v[1], w[1], v[2] * w[2]));
+    const double rdvj = fma(d[0], w[0], fma(d[1], w[1], d[2] * w[2]));
+    const double rdaj = fma(d[0], aj[0], fma(d[1], aj[1], d[2] * aj[2]));
+    const double fac = oc2 * (vi2 - 4.0 * (gr + up) - ut + 2.0 * vj2 - 4.0 * vivj - 1.5 * rdvj * rdvj * r2i - 0.5 * rdaj);
+    double fv[3], rel[3];
+    for (int k = 0; k < 3; k++) {
+        fv[k] = 4.0 * v[k] - 3.0 * w[k];
+        rel[k] = v[k] - w[k];
+    }
+    const double f = fma(d[0], fv[0], fma(d[1], fv[1], d[2] * fv[2]));
+    const double pf = pre * fac, pq = oc2 * pre * f, ga = 3.5 * oc2 * gr;
+    const double dpre = -3.0 * pre * r2i, t5 = 3.0 * oc2 * rdvj * r2i;
+    const double sdu = -dpre * fac, swd = oc2 * dpre * f, swf = oc2 * pre, sy = -ga * r2i, sq = 4.0 * oc2 * pre;
+    double u[3], ww[3], y[3], p[3], q[3];
+    for (int b = 0; b < 3; b++) {
+        acc[b] = fma(-pf, d[b], fma(pq, rel[b], ga * aj[b]));
+        /* the factor's derivatives by position and velocity */
+        const double dx = 4.0 * oc2 * fma(pre, d[b], gp[b]) - t5 * (w[b] - rdvj * d[b] * r2i) - 0.5 * oc2 * aj[b];
+        const double dv = oc2 * (2.0 * v[b] - 4.0 * w[b]);
+        u[b] = fma(sdu, d[b], -pre * dx);
+        ww[b] = fma(swd, d[b], swf * fv[b]);
+        y[b] = sy * d[b];
+        p[b] = -pre * dv;
+        q[b] = sq * d[b];
+    }
+    for (int a = 0; a < 3; a++)
+        for (int b = 0; b < 3; b++) {
+            J[a][b] += fma(d[a], u[b], fma(rel[a], ww[b], aj[a] * y[b])) - (a == b ? pf : 0.0);
+            J[a][3 + b] += fma(d[a], p[b], rel[a] * q[b]) + (a == b ? pq : 0.0);
+        }
+}
+
 /* The Earth's J2, J3, J4 in FP32 at separation q (r2 = |q|^2), added to the
  * low parts of the pair sums. */
 __device__ __forceinline__ void ag_fast_earth_h(const AgPairView& PV, const ForceCfg& c, const float* q, float r2, AgF2* acc) {

@@ -29,6 +29,7 @@
 #include "ias15_constants.h"
 #include "internal.h"
 #include "shared_sim.h"
+#include "shared_run.cuh"
 #include "table_forces.cuh"
 #include "coop_forces.cuh"
 #include "ias15_fast.cuh"
@@ -70,16 +71,6 @@ static int sh_tables_init(void) {
     if (dev >= 0 && dev < 64) sh_ready[dev] = true;
     return (int)cudaGetLastError();
 }
-
-/* field layout: f*(3*stride) + k*stride + i */
-enum { S_X0 = 0, S_V0, S_A0, S_XC, S_VC, S_AT, S_XP, S_VP, S_B, S_G = S_B + 7, S_E = S_G + 7, S_BR = S_E + 7, S_ER = S_BR + 7,
-       S_PX = S_ER + 7, S_PV, S_PA, S_NF };
-
-struct ShView {
-    double* w;
-    int stride;
-    __device__ __forceinline__ double& operator()(int f, int k, int i) const { return w[((size_t)f * 3 + k) * stride + i]; }
-};
 
 /* The predictor's coefficients of node `node` (1..7) of a step of size
  * hstep: sx[q] for x, sv[q] for v. */
@@ -435,58 +426,6 @@ __global__ void __launch_bounds__(128) sh_k_step(const DevEphem* __restrict__ Ep
  * host decision for each step, state in global memory, and the evaluation
  * with every term in FP64 (a step of three particles 262 us).  The rules are
  * the host loop's below. */
-struct ShCtl {
-    double t, tc, dt, dtls, dt_done;
-    long long accepted, rejected, iterations;
-    int status, gave_up;
-};
-
-struct ShRunArgs {
-    ShView W;
-    int n;
-    const double* params;        /* 3 n, or null */
-    double tmax, epsilon, min_dt;
-    long long max_steps;         /* accepted steps after which to stop short of tmax (0: none) */
-    int limit;                   /* steps of this launch */
-    const ShCtl* in;
-    ShCtl* out;
-    unsigned long long* red;     /* nine words: three rotating buffers of the maxima, zero at launch */
-    unsigned* bar;               /* grid barrier: arrivals, generation */
-};
-
-/* Device memory of a simulation's run kernel. */
-struct ShRunMem {
-    ShCtl ctl[2];                /* a launch reads one and writes the other */
-    unsigned long long red[9];
-    unsigned bar[2];
-};
-/* Steps of one launch (a year of 1,024 main-belt particles is 65): the device
- * is not held for longer than some tens of milliseconds at a time. */
-#define SH_RUN_STEPS 256
-
-#define SH_RUN_POLLS (1 << 22)
-/* Grid barrier of one thread a block; false when its polls run out (the block
- * then leaves, and the others at their own limits). */
-__device__ __forceinline__ bool sh_run_barrier(unsigned* bar) {
-    volatile unsigned* vgen = bar + 1;
-    const unsigned gen = *vgen;
-    __threadfence();
-    if (atomicAdd(&bar[0], 1u) == gridDim.x - 1) {
-        atomicExch(&bar[0], 0u);
-        __threadfence();
-        atomicAdd(&bar[1], 1u);
-        return true;
-    }
-    for (int k = 0; k < SH_RUN_POLLS; k++)
-        if (*vgen != gen) {
-            __threadfence();
-            return true;
-        }
-    return false;
-}
-
-enum { SH_ACCEPT = 0, SH_REJECT, SH_ITERATE, SH_LEAVE };
-
 __global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* __restrict__ Ep, ForceCfg c, ShRunArgs A) {
     extern __shared__ __align__(16) unsigned char sh_smem[];
     __shared__ AgFastStep S;
@@ -547,63 +486,10 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* _
                 double mb = ag_warp_max_nonneg(live ? ag_max3(S.rb6, lane) : 0.0);
                 bool ok = true;
                 if (gridDim.x > 1) {
-                    /* buffer round % 3 collects this iteration's maxima, block 0
-                     * clears the next one (last read two barriers ago) */
-                    unsigned long long* rb = A.red + 3 * (round % 3);
-                    if (lane < 3) atomicMax(&rb[lane], (unsigned long long)__double_as_longlong(lane == 0 ? mdb : (lane == 1 ? ma : mb)));
-                    if (blockIdx.x == 0 && lane < 3) A.red[3 * ((round + 1) % 3) + lane] = 0ull;
-                    __threadfence();
-                    __syncwarp();
-                    if (lane == 0) ok = sh_run_barrier(A.bar);
-                    ok = __shfl_sync(AG_FULL, ok ? 1 : 0, 0) != 0;
-                    const double r = lane < 3 ? __longlong_as_double((long long)atomicOr(&rb[lane], 0ull)) : 0.0;
-                    mdb = __shfl_sync(AG_FULL, r, 0);
-                    ma = __shfl_sync(AG_FULL, r, 1);
-                    mb = __shfl_sync(AG_FULL, r, 2);
+                    ok = sh_run_maxima(A, round, lane, mdb, ma, mb);
                     round++;
                 }
-                const double pc_err = ag_fast_pc_err(mdb, ma);
-                const bool conv = (pc_err < 1e-16) || (iters > 2 && pc_last <= pc_err) || (iters >= 12);
-                pc_last = pc_err;
-                cmd = SH_ITERATE;
-                if (!ok) {
-                    cmd = SH_LEAVE;
-                    K.gave_up = 1;
-                } else if (conv) {
-                    double dt_new = hstep;
-                    cmd = SH_ACCEPT;
-                    if (A.epsilon > 0.0) {
-                        const double err = mb / ma, safety = 0.25, ahs = fabs(hstep);
-                        if (ag_isnormal_pos(err)) dt_new = ag_inv_root7(err / A.epsilon) * hstep;
-                        else dt_new = hstep / safety;
-                        if (fabs(dt_new) < A.min_dt) dt_new = copysign(A.min_dt, dt_new);
-                        if (fabs(dt_new) < safety * ahs) cmd = SH_REJECT;
-                        else if (fabs(dt_new) > ahs / safety) dt_new = hstep / safety;
-                    }
-                    K.iterations += iters;
-                    if (lane == 0) {
-                        S.ah = hstep;
-                        S.aratio = cmd == SH_REJECT ? (K.dtls != 0.0 ? dt_new / K.dtls : 0.0) : dt_new / hstep;
-                    }
-                    K.dt = dt_new;
-                    if (cmd == SH_REJECT) {
-                        K.rejected++;
-                    } else {
-                        const double y = hstep + K.tc, s = K.t + y;
-                        K.tc = y - (s - K.t);
-                        K.t = s;
-                        K.dtls = hstep;
-                        K.dt_done = hstep;
-                        K.accepted++;
-                        if (last) { K.t = A.tmax; K.tc = 0.0; }
-                    }
-                }
-                if (lane == 0) {
-                    S.cmd = cmd;
-                    /* the launch ends: tmax, the steps asked for, or a barrier given up */
-                    S.fin = cmd == SH_LEAVE ||
-                            (cmd == SH_ACCEPT && (K.t == A.tmax || (A.max_steps > 0 && K.accepted >= A.max_steps)));
-                }
+                cmd = sh_run_decide(A, K, S, ok, mdb, ma, mb, hstep, last, iters, pc_last, lane);
             }
             __syncthreads();
             cmd = S.cmd;
@@ -877,6 +763,7 @@ struct AgSharedSim {
     ShRunMem* d_run = nullptr;    /* control state of the run kernel */
     ShCtl* h_ctl = nullptr;       /* pinned */
     int run_blocks = -1;          /* blocks a launch of the run kernel can hold (-1: not yet asked) */
+    int var_lanes = -1, var_n = 0;  /* particles a block of the run kernel with variational particles, for var_n */
     int coop_blocks = -1;         /* blocks a cooperative step launch can hold (-1: not yet asked) */
     int* d_status = nullptr;
     cudaStream_t stream = nullptr;
@@ -1085,14 +972,67 @@ static void sh_upload_state(AgSharedSim* s, struct reb_simulation* r, double dir
     s->dir = dir;
 }
 
-/* The integration by the run kernel.  Returns 0, 1 (CUDA error), or -1 when
- * its blocks do not fit on the device at once (nothing done). */
+int ag_var_run_lanes(int n, int n_ast, bool coop);
+cudaError_t ag_launch_var_run(const DevEphem& E, const ForceCfg& c, const ShRunArgs& r, const int* vmap, int lanes, cudaStream_t s);
+
+/* The six variational particles of each real one, when every real particle
+ * has exactly six and every variational particle is one real particle's;
+ * empty otherwise. */
+static std::vector<int> sh_var_map(const struct reb_simulation* r) {
+    const int n = r->N - r->N_var, nvc = r->N_var_config;
+    std::vector<int> map, count((size_t)(n > 0 ? n : 0), 0), seen((size_t)(r->N > 0 ? r->N : 0), 0);
+    if (n <= 0 || nvc != 6 * n || r->N_var != 6 * n) return map;
+    map.assign(6 * (size_t)n, 0);
+    for (int v = 0; v < nvc; v++) {
+        const int tp = r->var_config[v].testparticle, i = r->var_config[v].index;
+        if (tp < 0 || tp >= n || i < n || i >= r->N || count[(size_t)tp] == 6 || seen[(size_t)i]++) return std::vector<int>();
+        map[6 * (size_t)tp + (size_t)count[(size_t)tp]++] = i;
+    }
+    return map;
+}
+
+/* The integration by the run kernel (with variational particles that of
+ * kernels_var.cu).  Returns 0, 1 (CUDA error), or -1 when it does not take the
+ * simulation or its blocks do not fit on the device at once (nothing done). */
 static int sh_run(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct reb_simulation* r, const double* params,
                   double tmax, ShIntegrateOut* out) {
-    const int n = r->N, nb = (n + 31) / 32;
-    if (s->run_blocks < 0) s->run_blocks = sh_run_capacity(E.n_ast);
-    if (nb > s->run_blocks) return -1;
+    const bool var = r->N_var != 0;
+    const int n = r->N - r->N_var, nb = var ? 0 : (n + 31) / 32;
     cudaStream_t st = s->stream;
+    std::vector<int> vmap;
+    int lanes = 0;
+    if (var) {
+        /* the variational equations keep bodies whose force is off, and the
+         * parameters have derivatives of their own: the step kernel's */
+        const int all = AG_F_PLANETS | AG_F_AST;
+        if (params || (c.forces & all) != all) return -1;
+        vmap = sh_var_map(r);
+        if (vmap.empty()) return -1;
+        if (s->var_lanes < 0 || s->var_n != n) {
+            const char* ev = getenv("ASSIST_GB300_SHARED_COOP");
+            s->var_lanes = ag_var_run_lanes(n, E.n_ast, !(ev && atoi(ev) == 0));
+            s->var_n = n;
+        }
+        lanes = s->var_lanes;
+        if (!lanes) return -1;
+        if (vmap.size() > s->vcap) {
+            if (s->d_vstart) cudaFree(s->d_vstart);
+            if (s->d_vindex) cudaFree(s->d_vindex);
+            if (s->d_vcfg) cudaFree(s->d_vcfg);
+            s->d_vstart = s->d_vindex = s->d_vcfg = nullptr;
+            s->vcap = 0;
+            const size_t cap = vmap.size() + (size_t)n + 64;
+            if (ag_cuda_check(cudaMalloc(&s->d_vstart, sizeof(int) * cap), "cudaMalloc(vars)") ||
+                ag_cuda_check(cudaMalloc(&s->d_vindex, sizeof(int) * cap), "cudaMalloc(vars)") ||
+                ag_cuda_check(cudaMalloc(&s->d_vcfg, sizeof(int) * cap), "cudaMalloc(vars)"))
+                return 1;
+            s->vcap = cap;
+        }
+        cudaMemcpyAsync(s->d_vindex, vmap.data(), sizeof(int) * vmap.size(), cudaMemcpyHostToDevice, st);
+    } else {
+        if (s->run_blocks < 0) s->run_blocks = sh_run_capacity(E.n_ast);
+        if (nb > s->run_blocks) return -1;
+    }
     if (!s->d_run) {
         if (ag_cuda_check(cudaMalloc(&s->d_run, sizeof(ShRunMem)), "cudaMalloc(run state)")) return 1;
         if (ag_cuda_check(cudaMallocHost(&s->h_ctl, sizeof(ShCtl)), "cudaMallocHost(run state)")) return 1;
@@ -1131,7 +1071,16 @@ static int sh_run(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct r
         A.in = &s->d_run->ctl[launch & 1];
         A.out = &s->d_run->ctl[1 - (launch & 1)];
         if (launch) cudaMemsetAsync(A.red, 0, sizeof(m.red) + sizeof(m.bar), st);
-        if (nb == 1) {
+        if (var) {
+            const cudaError_t le = ag_launch_var_run(E, c, A, s->d_vindex, lanes, st);
+            if (le == cudaErrorCooperativeLaunchTooLarge && launch == 0) {
+                cudaGetLastError();
+                s->var_lanes = 0;
+                s->state_on_device = false;
+                return -1;
+            }
+            if (ag_cuda_check(le, "IAS15 run kernel (variational)")) return 1;
+        } else if (nb == 1) {
             sh_k_run<<<1, AG_FAST_THREADS, bytes, st>>>(E.self_dev, c, A);
             if (ag_cuda_check(cudaGetLastError(), "IAS15 run kernel")) return 1;
         } else {
@@ -1180,7 +1129,7 @@ int ag_shared_integrate(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, st
     if (sh_tables_init()) return ag_cuda_check(cudaErrorInvalidValue, "IAS15 tables");
     if (ag_cuda_check((cudaError_t)sh_step_attr(), "IAS15 step kernel shared memory")) return 1;
     if (sh_reserve(s, n)) return 1;
-    if (n == n_real && ag_fast_covers(c)) {
+    if (n_real > 0 && ag_fast_covers(c)) {
         if (ag_ias_tables_init()) return ag_cuda_check(cudaErrorInvalidValue, "IAS15 tables");
         const int rc = sh_run(s, E, c, r, params, tmax, out);
         if (rc >= 0) return rc ? rc : sh_copy_back(s, r, out);

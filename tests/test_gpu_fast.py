@@ -197,3 +197,35 @@ def test_batch_repeats_bit_for_bit(files):
         batch.integrate_batch_device(eph, t0, te, st, params=prm, opts=batch.options(**kw))
         out.append(st.cpu().numpy())
     assert all(np.array_equal(out[0], o) for o in out[1:])
+
+
+@pytest.mark.parametrize("n,t1", [(1, 8060.0), (9, 8060.0), (70, 8030.0), (2440, 8003.0)])
+def test_dropin_run_kernel_with_variational(files, n, t1):
+    """Six variational particles a particle, their slots dealt in a shuffled
+    order: one block, two with a remainder of one, nine, and more particles
+    than blocks of eight fit on the device (sixteen a block)."""
+    from assist_gb300 import Ephem, Extras, Simulation, synth
+    from tests.oracle_py import Oracle
+    pl, ast, system = files
+    pop = synth.population(system, "neo", n, seed=31, t0=8000.0)
+    tp = np.repeat(np.arange(n, dtype=np.int32), 6)
+    var0 = np.tile(np.eye(6), (n, 1))
+    mix = np.random.default_rng(n).permutation(6 * n)
+    tp, var0 = np.ascontiguousarray(tp[mix]), np.ascontiguousarray(var0[mix])
+    sim = Simulation.create(); ex = Extras(sim, Ephem(pl, ast))
+    for s in pop.state:
+        sim.add(*s)
+    for k in range(6 * n):
+        p = sim.particle(sim.add_variation(int(tp[k])))
+        p.x, p.y, p.z, p.vx, p.vy, p.vz = var0[k]
+    sim.t = 8000.0
+    sim.integrate(t1)
+    assert sim.status == 0 and sim.t == t1
+    g = np.array([[p.x, p.y, p.z, p.vx, p.vy, p.vz] for p in sim.particles])
+    r, rv, info = Oracle(pl, ast).integrate(8000.0, t1, pop.state, var_state=var0, var_tp=tp)
+    assert info["status"] == 0
+    assert np.abs(g[:n, :3] - r[:, :3]).max() < 1e-9
+    rel = np.abs(g[n:] - rv).max(axis=1) / np.abs(rv).max(axis=1)
+    assert rel.max() < 1e-7
+    assert abs(sim.steps_done - info["accepted"]) <= 1
+    ex.detach(sim); sim.free()
