@@ -1080,6 +1080,14 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
                 occ = (int)gstart.size() >= 8 * 3 * sms ? 3 : 2;
             }
         }
+        if (n_var && !P.learned) {
+            /* a block alone on its multiprocessor, its state in shared memory,
+             * while that leaves no more than a second round.  MEASURED-RULE */
+            int dev = 0, sms = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            occ = (int)gstart.size() <= 2 * sms ? 1 : 2;
+        }
         P.fast = may_fast;
         if (P.fast && !P.learned) {
             /* groups with a deep pass first in the list: the kernel with all

@@ -55,8 +55,8 @@
 
 /* b, e of one component from the last accepted step's br, er (the shift of
  * the acceleration polynomial to the new step). */
-template <int C>
-__device__ __forceinline__ void ag_predict_next_comp(const Ws<C>& W, int comp, double ratio) {
+template <class WsT>
+__device__ __forceinline__ void ag_predict_next_comp(const WsT& W, int comp, double ratio) {
     if (ratio > 20.0) {
         for (int k = 0; k < 7; k++) { W(W_E + k, comp) = 0.0; W(W_B + k, comp) = 0.0; }
         return;
@@ -96,12 +96,25 @@ __device__ __forceinline__ int ag_coop_pcomp(int w) {
     return NV == 0 ? (w == 0 ? 0 : (w == 1 ? -1 : w - 1)) : w - 1;
 }
 
+/* IAS15's fields of a block: the fields below W_E (the state, its
+ * compensations, a0, b and g, used at every node) in shared memory, the others
+ * (used once a step) in the global workspace. */
+template <int C>
+struct WsSplit {
+    double *s, *w;
+    int ns, slot;
+    __device__ __forceinline__ double& operator()(int f, int comp) const {
+        return f < W_E ? s[(f * C + comp) * 32] : w[((size_t)f * C + comp) * ns + slot];
+    }
+};
+
 template <int NV>
 struct AgCoopShared {
     static constexpr int C = 3 * (1 + NV);
-    AgCoopTab tab[NV == 0 ? 8 : 1]; /* body tables; without Jacobians one per node, kept through the
-                                       predictor-corrector iterations of a step (the node times do
-                                       not change while it iterates) */
+    AgCoopTab tab[NV == 0 ? 8 : 1]; /* body tables, one per node, kept through the predictor-corrector
+                                       iterations of a step (the node times do not change while it
+                                       iterates); with variational particles in dynamic shared memory
+                                       (learned start: a single one, built anew) */
     AgCoopScratch scr;
     double xs[C][32], vs[C][32];                    /* state at the current node */
     double pa[4][3][32];                            /* partial accelerations */
@@ -121,6 +134,17 @@ struct AgCoopShared {
     int rot;                                        /* role rotation of this block */
 };
 
+/* The warps' parts of the Jacobian summed once, in S.pj[0] (each of the 18
+ * variational components had summed its row: 324 FP64 instructions a node in
+ * place of 54).  Ends with a block barrier. */
+template <class Sh>
+__device__ __forceinline__ void ag_coop_sum_jac(Sh& S, int wid, int lane, bool on) {
+    if (on)
+        for (int q = wid; q < 18; q += 4)
+            S.pj[0][q][lane] = ((S.pj[3][q][lane] + S.pj[2][q][lane]) + S.pj[1][q][lane]) + S.pj[0][q][lane];
+    __syncthreads();
+}
+
 /* Distance from (x, y, z) to the nearest of the eleven planets in the table. */
 struct AgTableNearest {
     const AgTable& T;
@@ -135,19 +159,24 @@ struct AgTableNearest {
     }
 };
 
-/* Dynamic shared memory of a block: the warm-start buffers (when present)
+/* Dynamic shared memory of a block: the warm-start buffers (when present);
  * or, in the plain kernel without variational particles, the group's IAS15
- * state (40 fields x 3 components x 32 lanes, 30 KB).  Otherwise the state
- * stays in the global workspace, indexed by slot (both would not leave room
- * for two blocks per SM). */
-template <int NV, bool WARM, bool STAGE = false>
+ * state (40 fields x 3 components x 32 lanes, 30 KB); or, with them, the
+ * eight body tables and, in the build for one block a multiprocessor, the
+ * state's fields below W_E (19 x 21 x 32, 102 KB).  What is not there stays in
+ * the global workspace, indexed by slot. */
+template <int NV, bool WARM, bool STAGE = false, int OCC = 2>
 struct AgCoopDyn {
     static constexpr bool ws_shared = NV == 0 && !WARM;
+    static constexpr bool ws_split = NV > 0 && !WARM && OCC == 1;
+    static constexpr bool tabs = NV > 0 && !WARM;
     static constexpr size_t warm = WARM ? (sizeof(AgWarmSmem) + 15) / 16 * 16 : 0;
-    static constexpr size_t ws = ws_shared ? sizeof(double) * W_NF * 3 * 32 : 0;
+    static constexpr size_t ws = ws_shared ? sizeof(double) * W_NF * 3 * 32
+                                           : (ws_split ? sizeof(double) * W_E * 3 * (1 + NV) * 32 : 0);
     static constexpr size_t stage_off = warm + ws;        /* the staged .440 record (STAGE) */
     static constexpr size_t stage = STAGE ? (sizeof(AgRecStage) + 15) / 16 * 16 : 0;
-    static constexpr size_t bytes = warm + ws + stage;
+    static constexpr size_t tab_off = stage_off + stage;
+    static constexpr size_t bytes = tab_off + (tabs ? 8 * sizeof(AgCoopTab) : 0);
 };
 
 /* OCC: resident blocks per SM the kernel is compiled for.  The plain kernel
@@ -155,9 +184,9 @@ struct AgCoopDyn {
  * spills: faster on batches with many groups per block, slower on small
  * batches whose longest groups set the time), and 2 with the active .440
  * record staged in shared memory by bulk copies (STAGE; its 8 KB buffer does
- * not fit beside three blocks); the variational and warm-start
- * instantiations have only 2 (their Jacobians or network buffers would
- * spill or not fit). */
+ * not fit beside three blocks); the warm-start instantiations have only 2
+ * (their network buffers would not fit).  The variational kernel comes in 1
+ * and 2: a block alone keeps the state in shared memory.  MEASURED-NV6 */
 template <int NV, bool WARM, int OCC = 2, bool STAGE = false>
 __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict__ Ep, ForceCfg cf, AgBatchArgs A) {
     constexpr int C = 3 * (1 + NV);
@@ -180,19 +209,25 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = ((threadIdx.x >> 5) + S.rot) & 3, tid = (wid << 5) | lane;
-    AgCoopTab& Tab = S.tab[0];
     const int slot = blockIdx.x * 32 + lane;
     extern __shared__ __align__(16) unsigned char ag_dyn_smem[];
+    using Dyn = AgCoopDyn<NV, WARM, STAGE, OCC>;
+    constexpr bool tab8 = NV == 0 || Dyn::tabs;
+    AgCoopTab* const tabs = Dyn::tabs ? reinterpret_cast<AgCoopTab*>(ag_dyn_smem + Dyn::tab_off) : S.tab;
+    AgCoopTab& Tab = tabs[0];
     AgRecStage* const R =
-        STAGE ? reinterpret_cast<AgRecStage*>(ag_dyn_smem + AgCoopDyn<NV, WARM, STAGE>::stage_off) : nullptr;
+        STAGE ? reinterpret_cast<AgRecStage*>(ag_dyn_smem + Dyn::stage_off) : nullptr;
     AgStageCursor cur;
-    constexpr bool wss = AgCoopDyn<NV, WARM>::ws_shared;
-    const Ws<C> W{wss ? reinterpret_cast<double*>(ag_dyn_smem + AgCoopDyn<NV, WARM>::warm) : A.ws,
-                  wss ? 32 : A.nslots, wss ? lane : slot};
+    constexpr bool wss = Dyn::ws_shared;
+    typename std::conditional<Dyn::ws_split, WsSplit<C>, Ws<C>>::type W;
+    if constexpr (Dyn::ws_split) W.s = reinterpret_cast<double*>(ag_dyn_smem) + lane;
+    W.w = wss ? reinterpret_cast<double*>(ag_dyn_smem + Dyn::warm) : A.ws;
+    W.ns = wss ? 32 : A.nslots;
+    W.slot = wss ? lane : slot;
     const long long clk0 = clock64();
     unsigned long long n_acc = 0, n_rej = 0, n_ev = 0, n_it = 0, n_wused = 0, n_wfall = 0, n_tab = 0;
     if (tid == 0) {
-        for (int k = 0; k < (NV == 0 ? 8 : 1); k++) S.tab[k].T.status = AG_OK;
+        for (int k = 0; k < (tab8 ? 8 : 1); k++) tabs[k].T.status = AG_OK;
         S.stop = 0;
         S.stage_fail = 0;
         if (STAGE) ag_mbar_init(&R->bar);
@@ -391,6 +426,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             }
             bad = __syncthreads_or(fst != AG_OK);
             if (bad) { pstat = AG_ST_COVERAGE; finish_now = live; continue; }
+            if constexpr (NV > 0) ag_coop_sum_jac(S, wid, lane, live);
             if (live) {
                 for (int comp = 0; comp < C; comp++) {
                     if (ag_coop_owner<NV>(comp) != wid) continue;
@@ -400,9 +436,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                     } else {
                         const int q = (comp - 3) / 3, a = (comp - 3) % 3;
                         double Jr[6];
-                        for (int b = 0; b < 6; b++)
-                            Jr[b] = ((S.pj[3][6 * a + b][lane] + S.pj[2][6 * a + b][lane]) + S.pj[1][6 * a + b][lane]) +
-                                    S.pj[0][6 * a + b][lane];
+                        for (int b = 0; b < 6; b++) Jr[b] = S.pj[0][6 * a + b][lane];
                         const double* dxq = &S.xs[3 + 3 * q][0];
                         const double* dvq = &S.vs[3 + 3 * q][0];
                         double s = Jr[0] * dxq[lane];
@@ -444,8 +478,8 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             while (true) {
                 for (int n = 1; n < 8; n++) {
                     const double tn = S.ptn[n];
-                    AgCoopTab& TabN = S.tab[NV == 0 ? n : 0];
-                    const bool build = NV != 0 || iters == 1;     /* block-uniform */
+                    AgCoopTab& TabN = tabs[tab8 ? n : 0];
+                    const bool build = !tab8 || iters == 1;     /* block-uniform */
                     bad = build ? ag_coop_table_pass1<STAGE>(E, cf, tn, S.scr, TabN, tid, R, cur, &S.stage_fail) : 0;
                     n_tab += build ? 1 : 0;
                     if (!conv) {
@@ -506,6 +540,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                         }
                     }
                     __syncthreads();
+                    if constexpr (NV > 0) ag_coop_sum_jac(S, wid, lane, !conv);
                     if (!conv) {
                         for (int comp = 0; comp < C; comp++) {
                     if (ag_coop_owner<NV>(comp) != wid) continue;
@@ -515,9 +550,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                             } else {
                                 const int q = (comp - 3) / 3, a = (comp - 3) % 3;
                                 double Jr[6];
-                                for (int b = 0; b < 6; b++)
-                                    Jr[b] = ((S.pj[3][6 * a + b][lane] + S.pj[2][6 * a + b][lane]) + S.pj[1][6 * a + b][lane]) +
-                                            S.pj[0][6 * a + b][lane];
+                                for (int b = 0; b < 6; b++) Jr[b] = S.pj[0][6 * a + b][lane];
                                 const double* dxq = &S.xs[3 + 3 * q][0];
                                 const double* dvq = &S.vs[3 + 3 * q][0];
                                 double s = Jr[0] * dxq[lane];
@@ -640,7 +673,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                     if (wid == 0) n_rej++;
                     for (int comp = 0; comp < C; comp++) {
                     if (ag_coop_owner<NV>(comp) != wid) continue;
-                        if (dtls != 0.0) ag_predict_next_comp<C>(W, comp, dt_new / dtls);
+                        if (dtls != 0.0) ag_predict_next_comp(W, comp, dt_new / dtls);
                         else
                             for (int k = 0; k < 7; k++) { W(W_B + k, comp) = 0.0; W(W_E + k, comp) = 0.0; }
                     }
@@ -719,7 +752,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                     W(W_V0, comp) = s;
 #pragma unroll
                     for (int k = 0; k < 7; k++) { W(W_ER + k, comp) = W(W_E + k, comp); W(W_BR + k, comp) = b[k]; }
-                    ag_predict_next_comp<C>(W, comp, dt_new / hstep);
+                    ag_predict_next_comp(W, comp, dt_new / hstep);
                 }
             }
             {
@@ -753,9 +786,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
 /* Opt the kernel in to its dynamic shared memory (above the 48 KB default). */
 template <int NV, bool WARM, int OCC, bool STAGE = false>
 static int ag_coop_dyn_attr() {
-    if (AgCoopDyn<NV, WARM, STAGE>::bytes == 0) return 0;
+    if (AgCoopDyn<NV, WARM, STAGE, OCC>::bytes == 0) return 0;
     return (int)cudaFuncSetAttribute(ag_k_coop<NV, WARM, OCC, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)AgCoopDyn<NV, WARM, STAGE>::bytes);
+                                     (int)AgCoopDyn<NV, WARM, STAGE, OCC>::bytes);
 }
 
 template <int NV, bool WARM, int OCC, bool STAGE = false>
@@ -763,18 +796,20 @@ static int ag_coop_blocks_per_sm() {
     int bps = 0;
     if (ag_coop_dyn_attr<NV, WARM, OCC, STAGE>() == 0)
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ag_k_coop<NV, WARM, OCC, STAGE>, 128,
-                                                      AgCoopDyn<NV, WARM, STAGE>::bytes);
+                                                      AgCoopDyn<NV, WARM, STAGE, OCC>::bytes);
     return bps;
 }
 
 /* Slots (32 per resident block) of the plain (nv = 0: occ 2 or 3, stage
- * only with occ 2) or variational (nv = 6) kernel, or of their learned
+ * only with occ 2) or variational (nv = 6: occ 1 or 2) kernel, or of their learned
  * warm-start builds (warm), on the current device. */
 int ag_coop_max_slots(int nv, int occ, int stage, int warm) {
     int dev = 0, sms = 0, bps = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (nv == 6) bps = warm ? ag_coop_blocks_per_sm<6, true, 2>() : ag_coop_blocks_per_sm<6, false, 2>();
+    if (nv == 6)
+        bps = warm ? ag_coop_blocks_per_sm<6, true, 2>()
+                   : (occ == 1 ? ag_coop_blocks_per_sm<6, false, 1>() : ag_coop_blocks_per_sm<6, false, 2>());
     else if (warm) bps = ag_coop_blocks_per_sm<0, true, 2>();
     else if (occ == 3) bps = ag_coop_blocks_per_sm<0, false, 3>();
     else if (stage) bps = ag_coop_blocks_per_sm<0, false, 2, true>();
@@ -791,7 +826,11 @@ int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, i
     if (nv == 6 && (a.mlp || a.log_x)) {
         if ((e = ag_coop_dyn_attr<6, true, 2>())) return e;
         ag_k_coop<6, true, 2><<<blocks, 128, AgCoopDyn<6, true>::bytes, s>>>(E.self_dev, c, a);
+    } else if (nv == 6 && occ == 1) {
+        if ((e = ag_coop_dyn_attr<6, false, 1>())) return e;
+        ag_k_coop<6, false, 1><<<blocks, 128, AgCoopDyn<6, false, false, 1>::bytes, s>>>(E.self_dev, c, a);
     } else if (nv == 6) {
+        if ((e = ag_coop_dyn_attr<6, false, 2>())) return e;
         ag_k_coop<6, false, 2><<<blocks, 128, AgCoopDyn<6, false>::bytes, s>>>(E.self_dev, c, a);
     } else if (a.mlp || a.log_x) {
         if ((e = ag_coop_dyn_attr<0, true, 2>())) return e;
@@ -819,5 +858,7 @@ int ag_coop_ready(void) {
     if (!e) e = ag_coop_dyn_attr<0, false, 2, true>();
     if (!e) e = ag_coop_dyn_attr<0, true, 2>();
     if (!e) e = ag_coop_dyn_attr<6, true, 2>();
+    if (!e) e = ag_coop_dyn_attr<6, false, 1>();
+    if (!e) e = ag_coop_dyn_attr<6, false, 2>();
     return e;
 }
