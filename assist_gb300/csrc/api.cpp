@@ -1158,8 +1158,14 @@ static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var
     if (!e) e = (int)cudaEventRecord(fork, s);
     if (!e) e = (int)cudaStreamWaitEvent(side, fork, 0);
     if (!e) {
-        /* the longest groups start first: the other kernel's blocks fill the device */
-        e = ag_launch_coop(P.D, P.c, d, 0, 2, 0, s);
+        /* the longest groups start first, each with a multiprocessor to itself
+         * while they are few (alone the longest of 7 takes 65 ms, beside the
+         * other kernel's blocks 77, on 7 of 152 multiprocessors those lose 5 %);
+         * the other kernel's blocks fill the rest */
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        e = ag_launch_coop(P.D, P.c, d, 0, 8 * P.n_deep <= sms ? 1 : 2, 0, s);
         if (!e) e = ag_launch_fast(P.D, P.c, f, P.occ, P.stage, side);
         const int j = (int)cudaEventRecord(join, side), w = (int)cudaStreamWaitEvent(s, join, 0);
         if (!e) e = j ? j : w;

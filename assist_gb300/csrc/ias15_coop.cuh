@@ -783,12 +783,17 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
     if (STAGE && tid == 0 && S.stage_fail) ag_mbar_wait(&R->bar, cur.phase ^ 1u);
 }
 
+/* Dynamic shared memory that leaves no room on a multiprocessor (228 KB) for a
+ * block of the pair-term kernel (60 KB and more). */
+#define AG_COOP_ALONE (165 * 1024)
+
 /* Opt the kernel in to its dynamic shared memory (above the 48 KB default). */
 template <int NV, bool WARM, int OCC, bool STAGE = false>
 static int ag_coop_dyn_attr() {
-    if (AgCoopDyn<NV, WARM, STAGE, OCC>::bytes == 0) return 0;
-    return (int)cudaFuncSetAttribute(ag_k_coop<NV, WARM, OCC, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)AgCoopDyn<NV, WARM, STAGE, OCC>::bytes);
+    constexpr size_t own = AgCoopDyn<NV, WARM, STAGE, OCC>::bytes;
+    constexpr size_t bytes = NV == 0 && !WARM && OCC == 2 && !STAGE ? (size_t)AG_COOP_ALONE : own;
+    if (bytes == 0) return 0;
+    return (int)cudaFuncSetAttribute(ag_k_coop<NV, WARM, OCC, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 template <int NV, bool WARM, int OCC, bool STAGE = false>
@@ -835,6 +840,10 @@ int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, i
     } else if (a.mlp || a.log_x) {
         if ((e = ag_coop_dyn_attr<0, true, 2>())) return e;
         ag_k_coop<0, true, 2><<<blocks, 128, AgCoopDyn<0, true>::bytes, s>>>(E.self_dev, c, a);
+    } else if (occ == 1) {
+        /* the plain build for two, each block with a multiprocessor to itself */
+        if ((e = ag_coop_dyn_attr<0, false, 2>())) return e;
+        ag_k_coop<0, false, 2><<<blocks, 128, AG_COOP_ALONE, s>>>(E.self_dev, c, a);
     } else if (occ == 3) {
         if ((e = ag_coop_dyn_attr<0, false, 3>())) return e;
         ag_k_coop<0, false, 3><<<blocks, 128, AgCoopDyn<0, false>::bytes, s>>>(E.self_dev, c, a);
