@@ -229,3 +229,27 @@ def test_dropin_run_kernel_with_variational(files, n, t1):
     assert rel.max() < 1e-7
     assert abs(sim.steps_done - info["accepted"]) <= 1
     ex.detach(sim); sim.free()
+
+
+@pytest.mark.parametrize("n,length,sign", [(1, 60.0, 1.0), (33, 60.0, -1.0), (20500, 2.0, 1.0)])
+def test_batch_with_variational(files, n, length, sign):
+    """Batches with six variational particles each, a third with
+    non-gravitational parameters, of unequal lengths, forward and backward:
+    one group, a group's remainder, and more groups than get a multiprocessor
+    each (a sample of those against the oracle)."""
+    from assist_gb300 import Ephem, batch, synth
+    from tests.oracle_py import Oracle
+    pl, ast, system = files
+    pop = synth.population(system, "mix", n, seed=40 + n, t0=8000.0, nongrav_frac=0.34)
+    rng = np.random.default_rng(n)
+    t0 = np.full(n, 8000.0)
+    te = t0 + sign * length * rng.uniform(0.1, 1.0, n)
+    var = np.tile(np.eye(6)[None], (n, 1, 1)) + 1e-3 * rng.standard_normal((n, 6, 6))
+    out, vout, status, _ = batch.integrate_batch(Ephem(pl, ast), t0, te, pop.state, params=pop.params, var_state=var)
+    i = np.arange(n) if n < 1000 else np.arange(0, n, 83)
+    ref, vref, rstat, _ = Oracle(pl, ast).integrate_batch(t0[i], te[i], pop.state[i], params=pop.params[i], var_state=var[i],
+                                                          return_all=True)
+    assert (status == 0).all() and (rstat == 0).all()
+    assert np.abs(out[i, :3] - ref[:, :3]).max() < 1e-9
+    rel = np.abs(vout[i] - vref).max(axis=(1, 2)) / np.abs(vref).max(axis=(1, 2))
+    assert rel.max() < 1e-7
