@@ -1,11 +1,11 @@
 /*
  * autotune.cpp -- build selection for the block-cooperative batched IAS15.
  *
- * The default batched kernel comes in three builds that run each group's
+ * The default batched kernel (kernels_fast.cu; ias15_coop.cuh for the force
+ * configurations that has not) comes in three builds that run each group's
  * arithmetic identically and differ only in how a block uses the SM: two
- * resident blocks per SM (242 registers), three (168 registers, a few
- * spills), and two with the active .440 record staged in shared memory by
- * bulk copies.  Which is fastest depends on the batch: three blocks win when
+ * resident blocks per SM, three (fewer registers, some spills), and two with
+ * the active .440 record staged in shared memory by bulk copies.  Which is fastest depends on the batch: three blocks win when
  * there are many groups per block, two when a few long groups set the time.
  * assist_gb300_autotune_device times every build on the caller's own batch
  * (the whole batch: a sample would not keep its groups per resident block)

@@ -18,6 +18,9 @@
  * iteration and the host reads the three maxima back to decide convergence.
  * The host then decides acceptance and the next step size, with the same
  * rules as the batched kernel (kernels_ias15.cu).
+ * Simulations without variational particles, or with six of each particle,
+ * take whole steps on the device instead, step-size control included: sh_k_run
+ * here and the kernel of kernels_var.cu.
  */
 #include <cuda_runtime.h>
 #include <cmath>

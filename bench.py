@@ -77,12 +77,12 @@ UNIT = "particle-days/s"
 IAS_PER_EVAL = 3 * (34 + 16)
 IAS_PER_STEP = 3 * (2 * 9 + 2 * 8 + 8 + 7 * 8)
 
-# From one ncu capture of the block-cooperative kernel (three-blocks-per-SM
-# build) on the 32,768-particle case of this workload
-# (profiles/ag_k_coop_32768_mixture_1yr.md: 4.64 MB read + written for 11.97M
+# From one ncu capture of the pair-term kernel (two-blocks-per-SM build) on the
+# 32,768-particle case of this workload
+# (profiles/ag_k_fast_32768_mixture_1yr.md: 10.1 MB read + written for 11.97M
 # particle-days): DRAM bytes per particle-day of a launch, scaled to a full
 # launch by its particle-days.
-DRAM_BYTES_PER_PARTICLE_DAY = 0.388
+DRAM_BYTES_PER_PARTICLE_DAY = 0.845
 
 
 def _synth():
@@ -133,7 +133,8 @@ def roofline(stats, model, kernel_s, peak, pdays):
             "traffic_unit": "DRAM bytes per launch (ncu, 32,768-particle case of this kernel, scaled by particle-days)",
             "peak_source": "measured in this run (FP64 FMA chains; MEASURED_PEAKS.json has no FP64 figure)",
             "work": "per force evaluation %d flop of particle-dependent force terms + %d IAS15; per body table "
-                    "%d flop (ephemeris + particle-independent force-term parts); per accepted step %d"
+                    "%d flop (ephemeris + particle-independent force-term parts); per accepted step %d; all counted "
+                    "as FP64, although most force terms run as float pairs on the FP32 pipes (frac can pass 1)"
                     % (model["per_eval_particle"], IAS_PER_EVAL, model["per_body_table"], IAS_PER_STEP),
             "flops_per_launch": work, "force_evals": ev, "body_tables": tabs,
             "frac_vs_independent": indep / kernel_s / peak,
@@ -698,11 +699,12 @@ def main():
                        "warm_start": "plain predictor (the default; the learned warm start is measured "
                                      "beside it under learned_warm_start)",
                        "l2": "flushed (256 MB write) between steps", "kernel": "block-cooperative groups (group_steps=2)",
-                       "precision": "FP64 throughout, except the asteroids' direct terms beyond 0.02 AU of the "
-                                    "particle: float pairs (about 48 bits) on the FP32 pipes, below 1e-17 of the "
-                                    "acceleration",
+                       "precision": "FP64, except the terms of the planets but Jupiter, the asteroids, relativity "
+                                    "and the harmonics away from their bodies: float pairs (about 48 bits) and, for "
+                                    "small factors, FP32, errors below 1e-16 of the acceleration",
                        "parallelism": "dp%d (independent batches, no collective)" % world},
-            # per step: the encounter pilot's two kernels and the IAS15 kernel
+            # per step at least: the encounter pilot's two kernels and an IAS15 kernel
+            # (a second one where groups pass deep inside a planet's sphere of influence)
             "gpu_launches": 3 * args.steps,
             "e2e": e2e, "roofline": roof, "cpu_baseline": cpu, "parity": par,
             "clocks": clocks.summary(),

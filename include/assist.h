@@ -214,8 +214,8 @@ struct assist_gb300_options {
                                leave SMs idle */
     int group_steps;        /* 1: up to 32 particles with the same start time and similar
                                orbital timescale share each adaptive step (one warp);
-                               2 (default): the same groups, each integrated by a 128-thread
-                               block whose four warps split every force evaluation;
+                               2 (default): the same groups, each integrated by a block
+                               whose warps split every force evaluation;
                                0: every particle takes its own adaptive step */
     double dt_floor;        /* a particle whose adaptive step falls below this |dt| (days)
                                stops with ASSIST_GB300_STEP_UNDERFLOW (an impact: any orbit
