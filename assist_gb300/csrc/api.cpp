@@ -922,7 +922,8 @@ struct AgLaunchPlan {
     std::vector<int> order, gstart, gsize;
     bool grouped = false, coop = false;
     bool learned = false;           /* the warm-start build of the block-cooperative kernel */
-    bool fast = false;              /* the kernel on fast_forces.cuh, but for the first n_deep groups */
+    bool fast = false;              /* pair terms (with variational particles in the block-cooperative
+                                       kernel, else kernels_fast.cu), but for the first n_deep groups */
     int n_deep = 0, deep_slots = 0;
     int occ = 2, stage = 0, tpb = 128, nslots = 0;
 };
@@ -987,7 +988,11 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
      * group costs are formed */
     const float* enc = nullptr;
     unsigned char* deep = nullptr;      /* particles that pass deep inside a planet's sphere of influence */
-    const bool may_fast = o->group_steps == 2 && n_var == 0 && ag_fast_covers(c);
+    /* with variational particles: not the learned start, and all direct terms
+     * (the variational equations keep bodies whose force is off) */
+    const int all_direct = AG_F_PLANETS | AG_F_AST;
+    const bool may_fast = o->group_steps == 2 && ag_fast_covers(c) &&
+                          (n_var == 0 || (!o->warm_start && (c.forces & all_direct) == all_direct));
     if (grouped) {
         double tmin = t0[0], tmax = t0[0];
         for (int i = 0; i < n; i++) {
@@ -1091,7 +1096,7 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             occ = (int)gstart.size() <= 4 * sms ? 1 : 2;
         }
-        P.fast = may_fast;
+        P.fast = may_fast && !(n_var && P.learned);
         if (P.fast && !P.learned) {
             /* groups with a deep pass first in the list: the kernel with all
              * terms in FP64 takes them */
@@ -1107,10 +1112,10 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
             gstart.swap(s2);
             gsize.swap(z2);
             const int need = 32 * P.n_deep;
-            P.deep_slots = ag_coop_max_slots(0, 2, 0, 0);
+            P.deep_slots = ag_coop_max_slots(n_var, n_var ? occ : 2, 0, 0);
             if (P.deep_slots > need) P.deep_slots = need;
         }
-        nslots = P.fast ? ag_fast_max_slots(occ, stage, P.learned ? 1 : 0, D.n_ast)
+        nslots = P.fast && !n_var ? ag_fast_max_slots(occ, stage, P.learned ? 1 : 0, D.n_ast)
                         : ag_coop_max_slots(n_var, occ, stage, P.learned ? 1 : 0);
         const int need = 32 * ((int)gstart.size() - P.n_deep);
         if (nslots > need) nslots = need;
@@ -1136,6 +1141,11 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
     return ASSIST_SUCCESS;
 }
 
+/* Doubles of the global workspace of a launch plan's kernels. */
+static size_t ag_plan_ws_doubles(const AgLaunchPlan& P, int n_var) {
+    return ag_batch_ws_doubles(P.nslots, n_var) + (P.fast && n_var ? ag_batch_ws_doubles(P.deep_slots, n_var) : 0);
+}
+
 /* The batched kernels of a launch plan on stream s.  With groups on both
  * kernels the pair-term one runs on a stream forked from s and joined again;
  * a.queue holds two counters then. */
@@ -1147,12 +1157,16 @@ static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var
     f.grp_start += P.n_deep;
     f.grp_size += P.n_deep;
     f.n_groups -= P.n_deep;
-    if (!P.n_deep) return ag_launch_fast(P.D, P.c, f, P.occ, P.stage, s);
+    auto fast = [&](cudaStream_t st) {
+        return n_var ? ag_launch_coop(P.D, P.c, f, n_var, P.occ, 0, st, true) : ag_launch_fast(P.D, P.c, f, P.occ, P.stage, st);
+    };
+    if (!P.n_deep) return fast(s);
     AgBatchArgs d = a;
     d.n_groups = P.n_deep;
     d.nslots = P.deep_slots;
     d.queue = a.queue + 1;
-    if (!f.n_groups) return ag_launch_coop(P.D, P.c, d, 0, 2, 0, s);
+    if (n_var) d.ws = a.ws + ag_batch_ws_doubles(P.nslots, n_var);
+    if (!f.n_groups) return ag_launch_coop(P.D, P.c, d, n_var, n_var ? P.occ : 2, 0, s);
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     int e = (int)cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
@@ -1168,8 +1182,8 @@ static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        e = ag_launch_coop(P.D, P.c, d, 0, 8 * P.n_deep <= sms ? 1 : 2, 0, s);
-        if (!e) e = ag_launch_fast(P.D, P.c, f, P.occ, P.stage, side);
+        e = ag_launch_coop(P.D, P.c, d, n_var, n_var ? P.occ : (8 * P.n_deep <= sms ? 1 : 2), 0, s);
+        if (!e) e = fast(side);
         const int j = (int)cudaEventRecord(join, side), w = (int)cudaStreamWaitEvent(s, join, 0);
         if (!e) e = j ? j : w;
     }
@@ -1214,7 +1228,7 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
             ag_cuda_check(cudaMalloc(&g_batch.d_counters, cnt_bytes), "cudaMalloc"))
             return ASSIST_ERROR_EPHEM_FILE;
     }
-    const size_t wsn = ag_batch_ws_doubles(nslots, n_var);
+    const size_t wsn = ag_plan_ws_doubles(P, n_var);
     if (wsn > g_batch.ws_cap) {
         if (g_batch.d_ws) cudaFree(g_batch.d_ws);
         g_batch.d_ws = nullptr;
@@ -1342,7 +1356,7 @@ extern "C" int assist_gb300_plan_create(const struct assist_ephem* e, const stru
     }
     const AgLaunchPlan& P = p->P;
     const int ng = (int)P.gstart.size();
-    const size_t wsn = ag_batch_ws_doubles(P.nslots, n_var);
+    const size_t wsn = ag_plan_ws_doubles(P, n_var);
     bool ok = !ag_cuda_check(cudaMalloc(&p->d_order, sizeof(int) * (size_t)n), "cudaMalloc(plan order)") &&
               (!P.grouped || !ag_cuda_check(cudaMalloc(&p->d_grp, sizeof(int) * 2 * (size_t)ng), "cudaMalloc(plan groups)")) &&
               !ag_cuda_check(cudaMalloc(&p->d_queue, 2 * sizeof(int)), "cudaMalloc(plan queue)") &&

@@ -51,6 +51,7 @@
  */
 
 #include "coop_forces.cuh"
+#include "fast_forces.cuh"
 #include "ias15_warm.cuh"
 
 /* b, e of one component from the last accepted step's br, er (the shift of
@@ -145,6 +146,190 @@ __device__ __forceinline__ void ag_coop_sum_jac(Sh& S, int wid, int lane, bool o
     __syncthreads();
 }
 
+/* Float pairs of a table's origin minus body: the pair terms' planets, then
+ * the Sun and Jupiter (the asteroids' are in the table). */
+#define AG_PREL (AG_PAIR_PL + 2)
+typedef AgF2 AgPairRow[3];
+__device__ __forceinline__ void ag_coop_pair_rows(const AgCoopTab& CT, AgPairRow* PR, int tid) {
+    if (tid < 3 * AG_PREL) {
+        const int k = tid / 3, comp = tid - 3 * k;
+        PR[k][comp] = ag_f2_of(CT.rel[k < AG_PAIR_PL ? ag_pair_planet(k) : (k == AG_PAIR_PL ? AG_SUN : AG_JUP)][comp]);
+    }
+}
+
+/* Warp w's share of the evaluation with Jacobian on pair terms (the bodies,
+ * thresholds and precisions of fast_forces.cuh, every direct term on):
+ *
+ *   warp 0      Sun and Jupiter, non-gravitational terms (FP64), a third of the packs
+ *   warp 1      relativity (FP64, with FP32 sums over the planets), GR terms
+ *   warps 2, 3  a third of the packs each, the Earth's and the Sun's harmonics (FP32)
+ *
+ * It replaces ag_coop_force_part<true>, whose busiest warp has some 450 FP64
+ * instructions a node; here 200 (warp 1). */
+__device__ __forceinline__ void ag_coop_force_pairs(int w, const AgCoopTab& CT, const AgPairRow* PR, const DevEphem& E, const ForceCfg& c,
+                                                    const double* x, const double* v, const double* A, double* acc, double (*J)[6]) {
+#pragma unroll
+    for (int q = 0; q < 18; q++) J[q / 6][q % 6] = 0.0;
+    acc[0] = acc[1] = acc[2] = 0.0;
+    const AgF2 xf[3] = {ag_f2_of(x[0]), ag_f2_of(x[1]), ag_f2_of(x[2])};
+    if (w == 1) {
+        double d[3], ri;
+        ag_coop_sep(CT, x, AG_SUN, d[0], d[1], d[2], ri);
+        const PlanetState& P = CT.T.P;
+        const double sv[3] = {P.vx[AG_SUN], P.vy[AG_SUN], P.vz[AG_SUN]};
+        if (c.forces & AG_F_EIH) {
+            float up = 0.0f, gp[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+            for (int k = 0; k < AG_PAIR_PL + 1; k++) {
+                const AgPairRow& o = PR[k < AG_PAIR_PL ? k : AG_PAIR_PL + 1];
+                const float gm = k < AG_PAIR_PL ? ((k & 1) ? E.pv.gm[k >> 1].gb : E.pv.gm[k >> 1].ga) : E.pv.gm_jup;
+                const float q[3] = {o[0].h + xf[0].h, o[1].h + xf[1].h, o[2].h + xf[2].h};
+                const float r = rsqrtf(fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2]))), f = gm * r * r * r;
+                up = fmaf(gm, r, up);
+                for (int m = 0; m < 3; m++) gp[m] = fmaf(f, q[m], gp[m]);
+            }
+            const double g[3] = {ag_f2d_int(gp[0]), ag_f2d_int(gp[1]), ag_f2d_int(gp[2])};
+            ag_fast_eih_jac(E, d, ri, v, sv, CT.T.eih_a[AG_SUN], CT.T.eih_t1[AG_SUN], ag_f2d_int(up), g, acc, J);
+        }
+        if (c.forces & AG_F_GR_POT) ag_term_gr_pot<true>(E, d, ri, acc[0], acc[1], acc[2], J);
+        if (c.forces & AG_F_GR_SIMPLE) {
+            const double pv[3] = {v[0] - sv[0], v[1] - sv[1], v[2] - sv[2]};
+            ag_term_gr_simple<true>(E, d, ri, pv, acc[0], acc[1], acc[2], J);
+        }
+        return;
+    }
+    const AgPairRow& sun = PR[AG_PAIR_PL];
+    const float big = fmaxf(fabsf(xf[0].h), fmaxf(fabsf(xf[1].h), fabsf(xf[2].h)));
+    const bool wild = !(big < 1e6f);
+    const float sx = xf[0].h + sun[0].h, sy = xf[1].h + sun[1].h, sz = xf[2].h + sun[2].h;
+    const float rs2 = fmaf(sx, sx, fmaf(sy, sy, sz * sz));
+    const int bodies = AG_PAIR_PL + E.n_ast, packs = (bodies + 1) / 2, slot = w == 0 ? 0 : w - 1;
+    AgPkSum S;
+    AgPkJac PJ;
+    AgPk xh[3], xl[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        xh[k] = ag_pk(xf[k].h, xf[k].h);
+        xl[k] = ag_pk(xf[k].l, xf[k].l);
+        S.h[k] = S.l[k] = ag_pk(0.0f, 0.0f);
+    }
+    ag_pk_jac_clear(PJ);
+    unsigned long long near = 0;
+#pragma unroll 1
+    for (int p = slot; p < packs; p += 3) {
+        const int ka = 2 * p, kb = 2 * p + 1;
+        const AgF2* a = ka < AG_PAIR_PL ? PR[ka] : CT.arel[ka - AG_PAIR_PL];
+        const bool two = kb < bodies;
+        const AgF2* b = !two ? a : (kb < AG_PAIR_PL ? PR[kb] : CT.arel[kb - AG_PAIR_PL]);
+        AgPkRel R;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            /* the last pack's empty half: massless, far away */
+            R.c[k].h = ag_pk(a[k].h, two ? b[k].h : 1e6f);
+            R.c[k].l = ag_pk(a[k].l, two ? b[k].l : 0.0f);
+        }
+        const unsigned n = ag_pk_term<true>(R, E.pv.gm[p], xh, xl, rs2, S, &PJ);
+        near |= (unsigned long long)(two ? n : n & 1u) << ka;
+    }
+    AgF2 s[3], j[7];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+        s[k] = ag_f2_add({ag_pk_a(S.h[k]), ag_pk_a(S.l[k])}, {ag_pk_b(S.h[k]), ag_pk_b(S.l[k])});
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+        AgF2 a, b;
+        ag_pk_jac_get(PJ, k, 0, a.h, a.l);
+        ag_pk_jac_get(PJ, k, 1, b.h, b.l);
+        j[k] = ag_f2_add(a, b);
+    }
+    bool earth = false, sunh = false;          /* harmonics left to FP64 */
+    if (w == 2 && (c.forces & AG_F_EARTH_H)) {
+        float hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        const float q[3] = {xf[0].h + PR[2][0].h, xf[1].h + PR[2][1].h, xf[2].h + PR[2][2].h};
+        const float r2 = fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2]));
+        earth = wild || !(r2 >= 1.0e-2f && r2 < 1e30f);
+        if (!earth) {
+            ag_fast_earth_h(E.pv, c, q, r2, s);
+            ag_fast_earth_hj(E.pv, c, q, r2, hj);
+#pragma unroll
+            for (int k = 0; k < 6; k++) j[k].l += hj[k];
+        }
+    }
+    if (w == 3 && (c.forces & AG_F_SUN_H)) {
+        float hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        sunh = wild || !(rs2 >= 1.0e-2f && rs2 < 1e30f);
+        if (!sunh) {
+            const float q[3] = {sx, sy, sz};
+            ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, s);
+            ag_fast_sun_hj(E.pv, c, q, rs2, hj);
+#pragma unroll
+            for (int k = 0; k < 6; k++) j[k].l += hj[k];
+        }
+    }
+    AgSymJac Y = {{0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, 0.0};
+    double ax = 0.0, ay = 0.0, az = 0.0;
+    if (wild) {
+        near = 0;
+        for (int p = slot; p < packs; p += 3) near |= (2 * p + 1 < bodies ? 3ull : 1ull) << (2 * p);
+    } else {
+        ax = ag_f2_to(s[0]); ay = ag_f2_to(s[1]); az = ag_f2_to(s[2]);
+#pragma unroll
+        for (int a = 0, e = 0; a < 3; a++)
+#pragma unroll
+            for (int b = a; b < 3; b++, e++) {
+                const double t = ag_f2_to(j[e]);
+                J[a][b] = t;
+                if (b != a) J[b][a] = t;
+            }
+        const double g = ag_f2_to(j[6]);
+        J[0][0] -= g; J[1][1] -= g; J[2][2] -= g;
+    }
+    while (near) {
+        const int k = __ffsll((long long)near) - 1;
+        near &= near - 1;
+        double r[3];
+        if (k < AG_PAIR_PL) {
+            const double* o = CT.rel[ag_pair_planet(k)];
+            r[0] = o[0]; r[1] = o[1]; r[2] = o[2];
+        } else ag_coop_ast_rel(CT, false, k - AG_PAIR_PL, r);
+        const double gm = k < AG_PAIR_PL ? E.gm[ag_pair_planet(k)] : E.ast_gm[k - AG_PAIR_PL];
+        const double dx = x[0] + r[0], dy = x[1] + r[1], dz = x[2] + r[2];
+        const double ri = rsqrt(fma(dx, dx, fma(dy, dy, dz * dz))), g = gm * ri * ri * ri;
+        ax = fma(-g, dx, ax); ay = fma(-g, dy, ay); az = fma(-g, dz, az);
+        ag_symjac_term(Y, g, ri, dx, dy, dz);
+    }
+    if (earth) {
+        double dx, dy, dz, ri;
+        ag_coop_sep(CT, x, AG_EAR, dx, dy, dz, ri);
+        ag_term_earth_h<true>(E, c, dx, dy, dz, ri, ax, ay, az, J);
+    }
+    if (sunh) {
+        double dx, dy, dz, ri;
+        ag_coop_sep(CT, x, AG_SUN, dx, dy, dz, ri);
+        ag_term_sun_h<true>(E, c, dx, dy, dz, ri, ax, ay, az, J);
+    }
+    if (w == 0) {
+        double d[3], ri;
+        ag_coop_sep(CT, x, AG_SUN, d[0], d[1], d[2], ri);
+        if ((c.forces & AG_F_NONGRAV) && A != nullptr && (A[0] != 0.0 || A[1] != 0.0 || A[2] != 0.0)) {
+            const PlanetState& P = CT.T.P;
+            const double dv[3] = {v[0] - P.vx[AG_SUN], v[1] - P.vy[AG_SUN], v[2] - P.vz[AG_SUN]};
+            double JA[3][3];
+            bool has_ng;
+            ag_term_nongrav<true>(c, d, ri, dv, A, ax, ay, az, J, JA, &has_ng);
+        }
+        double jx, jy, jz, rj;
+        ag_coop_sep(CT, x, AG_JUP, jx, jy, jz, rj);
+        const double gj = E.gm[AG_JUP] * rj * rj * rj, gs = E.gm[AG_SUN] * ri * ri * ri;
+        ax = fma(-gj, jx, ax); ay = fma(-gj, jy, ay); az = fma(-gj, jz, az);
+        ag_symjac_term(Y, gj, rj, jx, jy, jz);
+        ax = fma(-gs, d[0], ax); ay = fma(-gs, d[1], ay); az = fma(-gs, d[2], az);
+        ag_symjac_term(Y, gs, ri, d[0], d[1], d[2]);
+    }
+    ag_symjac_add(Y, J);
+    acc[0] = ax; acc[1] = ay; acc[2] = az;
+}
+
 /* Distance from (x, y, z) to the nearest of the eleven planets in the table. */
 struct AgTableNearest {
     const AgTable& T;
@@ -162,7 +347,7 @@ struct AgTableNearest {
 /* Dynamic shared memory of a block: the warm-start buffers (when present);
  * or, in the plain kernel without variational particles, the group's IAS15
  * state (40 fields x 3 components x 32 lanes, 30 KB); or, with them, the
- * eight body tables and, in the build for one block a multiprocessor, the
+ * eight body tables with the planets' float pairs and, in the build for one block a multiprocessor, the
  * state's fields below W_E (19 x 21 x 32, 102 KB).  What is not there stays in
  * the global workspace, indexed by slot. */
 template <int NV, bool WARM, bool STAGE = false, int OCC = 2>
@@ -176,7 +361,8 @@ struct AgCoopDyn {
     static constexpr size_t stage_off = warm + ws;        /* the staged .440 record (STAGE) */
     static constexpr size_t stage = STAGE ? (sizeof(AgRecStage) + 15) / 16 * 16 : 0;
     static constexpr size_t tab_off = stage_off + stage;
-    static constexpr size_t bytes = tab_off + (tabs ? 8 * sizeof(AgCoopTab) : 0);
+    static constexpr size_t prel_off = tab_off + (tabs ? 8 * sizeof(AgCoopTab) : 0);
+    static constexpr size_t bytes = prel_off + (tabs ? 8 * AG_PREL * sizeof(AgPairRow) : 0);
 };
 
 /* OCC: resident blocks per SM the kernel is compiled for.  The plain kernel
@@ -190,7 +376,7 @@ struct AgCoopDyn {
  * FP64 pipes' latency, about 2,500 FP64 warp instructions a block and node
  * (3,200 with a table and the 18 components' Jacobian sums at every node):
  * 2,053 mixed particles over 730 days 268.6 ms before, 218.1 now. */
-template <int NV, bool WARM, int OCC = 2, bool STAGE = false>
+template <int NV, bool WARM, int OCC = 2, bool STAGE = false, bool PAIRS = false>
 __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict__ Ep, ForceCfg cf, AgBatchArgs A) {
     constexpr int C = 3 * (1 + NV);
     const DevEphem& E = *Ep;
@@ -218,6 +404,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
     constexpr bool tab8 = NV == 0 || Dyn::tabs;
     AgCoopTab* const tabs = Dyn::tabs ? reinterpret_cast<AgCoopTab*>(ag_dyn_smem + Dyn::tab_off) : S.tab;
     AgCoopTab& Tab = tabs[0];
+    AgPairRow* const prel = PAIRS ? reinterpret_cast<AgPairRow*>(ag_dyn_smem + Dyn::prel_off) : nullptr;
     AgRecStage* const R =
         STAGE ? reinterpret_cast<AgRecStage*>(ag_dyn_smem + Dyn::stage_off) : nullptr;
     AgStageCursor cur;
@@ -396,6 +583,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             ag_coop_table_pass2(E, cf, t, Tab, S.scr, tid);
             __syncthreads();
             if (cf.geocentric == 1) { ag_coop_rel_geo(E, Tab, tid); __syncthreads(); }
+            if constexpr (PAIRS) { ag_coop_pair_rows(Tab, prel, tid); __syncthreads(); }
             if (wid == 1 && (cf.forces & AG_F_EIH)) ag_coop_eih_sources(E, cf, Tab.T, lane);
             int fst = AG_OK;
             {
@@ -405,7 +593,8 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                 if (NV > 0) {
                     if (live) {
                         double J[3][6];
-                        fst = ag_coop_force_part<true>(wid, Tab, E, cf, xp, vp, has_prm ? prm : nullptr, acc, J);
+                        if constexpr (PAIRS) ag_coop_force_pairs(wid, Tab, prel, E, cf, xp, vp, has_prm ? prm : nullptr, acc, J);
+                        else fst = ag_coop_force_part<true>(wid, Tab, E, cf, xp, vp, has_prm ? prm : nullptr, acc, J);
                         for (int a = 0; a < 3; a++)
                             for (int b = 0; b < 6; b++) S.pj[wid][6 * a + b][lane] = J[a][b];
                     }
@@ -511,6 +700,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                         ag_coop_table_pass2(E, cf, tn, TabN, S.scr, tid);
                         __syncthreads();
                         if (cf.geocentric == 1) { ag_coop_rel_geo(E, TabN, tid); __syncthreads(); }
+                        if constexpr (PAIRS) { ag_coop_pair_rows(TabN, prel + AG_PREL * n, tid); __syncthreads(); }
                         if (wid == 1 && (cf.forces & AG_F_EIH)) ag_coop_eih_sources(E, cf, TabN.T, lane);
                     }
                     {
@@ -520,7 +710,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                         if (NV > 0) {
                             if (!conv) {
                                 double J[3][6];
-                                ag_coop_force_part<true>(wid, TabN, E, cf, xp, vp, has_prm ? prm : nullptr, acc, J);
+                                if constexpr (PAIRS)
+                                    ag_coop_force_pairs(wid, TabN, prel + AG_PREL * n, E, cf, xp, vp, has_prm ? prm : nullptr, acc, J);
+                                else ag_coop_force_part<true>(wid, TabN, E, cf, xp, vp, has_prm ? prm : nullptr, acc, J);
                                 for (int a = 0; a < 3; a++)
                                     for (int b = 0; b < 6; b++) S.pj[wid][6 * a + b][lane] = J[a][b];
                             }
@@ -791,12 +983,12 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
 #define AG_COOP_ALONE (165 * 1024)
 
 /* Opt the kernel in to its dynamic shared memory (above the 48 KB default). */
-template <int NV, bool WARM, int OCC, bool STAGE = false>
+template <int NV, bool WARM, int OCC, bool STAGE = false, bool PAIRS = false>
 static int ag_coop_dyn_attr() {
     constexpr size_t own = AgCoopDyn<NV, WARM, STAGE, OCC>::bytes;
     constexpr size_t bytes = NV == 0 && !WARM && OCC == 2 && !STAGE ? (size_t)AG_COOP_ALONE : own;
     if (bytes == 0) return 0;
-    return (int)cudaFuncSetAttribute(ag_k_coop<NV, WARM, OCC, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return (int)cudaFuncSetAttribute(ag_k_coop<NV, WARM, OCC, STAGE, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 template <int NV, bool WARM, int OCC, bool STAGE = false>
@@ -827,13 +1019,19 @@ int ag_coop_max_slots(int nv, int occ, int stage, int warm) {
 }
 
 int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int occ, int stage,
-                   cudaStream_t s) {
+                   cudaStream_t s, bool pairs) {
     int e = ag_ias_tables_init();
     if (e) return e;
     const int blocks = (a.nslots + 31) / 32;
     if (nv == 6 && (a.mlp || a.log_x)) {
         if ((e = ag_coop_dyn_attr<6, true, 2>())) return e;
         ag_k_coop<6, true, 2><<<blocks, 128, AgCoopDyn<6, true>::bytes, s>>>(E.self_dev, c, a);
+    } else if (nv == 6 && pairs && occ == 1) {
+        if ((e = ag_coop_dyn_attr<6, false, 1, false, true>())) return e;
+        ag_k_coop<6, false, 1, false, true><<<blocks, 128, AgCoopDyn<6, false, false, 1>::bytes, s>>>(E.self_dev, c, a);
+    } else if (nv == 6 && pairs) {
+        if ((e = ag_coop_dyn_attr<6, false, 2, false, true>())) return e;
+        ag_k_coop<6, false, 2, false, true><<<blocks, 128, AgCoopDyn<6, false>::bytes, s>>>(E.self_dev, c, a);
     } else if (nv == 6 && occ == 1) {
         if ((e = ag_coop_dyn_attr<6, false, 1>())) return e;
         ag_k_coop<6, false, 1><<<blocks, 128, AgCoopDyn<6, false, false, 1>::bytes, s>>>(E.self_dev, c, a);
@@ -872,5 +1070,7 @@ int ag_coop_ready(void) {
     if (!e) e = ag_coop_dyn_attr<6, true, 2>();
     if (!e) e = ag_coop_dyn_attr<6, false, 1>();
     if (!e) e = ag_coop_dyn_attr<6, false, 2>();
+    if (!e) e = ag_coop_dyn_attr<6, false, 1, false, true>();
+    if (!e) e = ag_coop_dyn_attr<6, false, 2, false, true>();
     return e;
 }

@@ -104,8 +104,10 @@ int ag_coop_max_slots(int nv, int occ, int stage, int warm);
 int ag_pilot_encounters(const DevEphem& E, int n, const double* d_t0, const double* d_te, const double* d_state,
                         double tmin, double tmax, float* d_ratio, unsigned char* d_deep, float4* d_grid,
                         float2* d_sunv, int G, cudaStream_t s);
+/* pairs: with variational particles, the forces on pair terms (ag_fast_covers
+ * and all direct terms on) */
 int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int occ, int stage,
-                   cudaStream_t s);
+                   cudaStream_t s, bool pairs = false);
 /* the batched kernel on fast_forces.cuh (kernels_fast.cu): configurations ag_fast_covers */
 int ag_fast_max_slots(int occ, int stage, int warm, int n_ast);
 int ag_launch_fast(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int occ, int stage, cudaStream_t s);
