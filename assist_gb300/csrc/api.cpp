@@ -925,6 +925,7 @@ struct AgLaunchPlan {
     bool fast = false;              /* pair terms (with variational particles in the block-cooperative
                                        kernel, else kernels_fast.cu), but for the first n_deep groups */
     int n_deep = 0, deep_slots = 0;
+    int pairs = 0;                  /* ag_launch_coop's, with variational particles */
     int occ = 2, stage = 0, tpb = 128, nslots = 0;
 };
 
@@ -1087,10 +1088,10 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
         }
         if (n_var && !P.learned) {
             /* a block alone on its multiprocessor, its state in shared memory,
-             * while a block is faster for it than two together (100 days of
-             * the mixed population, alone / two: 8,000 particles 45.7 / 56.3
-             * ms, 16,000 in some 560 groups 68.2 / 86.5, 40,000 in 1,300
-             * 142.7 / 111.1) */
+             * while a block is faster for it than two together (FP64 forces,
+             * 100 days of the mixed population, alone / two: 8,000 particles
+             * 45.7 / 56.3 ms, 16,000 in 524 groups 68.2 / 86.5, 40,000 in
+             * 1,276 142.7 / 111.1) */
             int dev = 0, sms = 0;
             cudaGetDevice(&dev);
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1115,8 +1116,39 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
             P.deep_slots = ag_coop_max_slots(n_var, n_var ? occ : 2, 0, 0);
             if (P.deep_slots > need) P.deep_slots = need;
         }
+        if (P.fast && n_var) {
+            /* groups of at most sixteen, a particle's 21 components shared by
+             * two lanes, while there are few: a node's latency falls by a
+             * third, its work by particle rises (100 days of the mixed
+             * population, sixteen / thirty-two a group: 2,053 particles 21.4 /
+             * 31.6 ms, 16,000 in 1,024 groups of sixteen 34.8 / 52.3, 40,000
+             * in 2,523 81.6 / 68.9) */
+            int n16 = 0, dev = 0, sms = 0;
+            cudaGetDevice(&dev);
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            for (size_t k = (size_t)P.n_deep; k < gstart.size(); k++) n16 += (gsize[k] + 15) / 16;
+            P.pairs = n16 <= 10 * sms ? 16 : 1;
+            if (P.pairs == 16) {
+                /* alone on a multiprocessor: the longest groups do not share
+                 * one with a block of the second round (alone / two: 277
+                 * groups 25.8 / 27.6 ms, 527 26.1 / 25.2; a batch of 175 took
+                 * 98 ms alone and 98 to 112 otherwise) */
+                occ = n16 <= 3 * sms ? 1 : 2;
+                std::vector<int> s2(gstart.begin(), gstart.begin() + P.n_deep), z2(gsize.begin(), gsize.begin() + P.n_deep);
+                for (size_t k = (size_t)P.n_deep; k < gstart.size(); k++) {
+                    const int parts = (gsize[k] + 15) / 16;
+                    for (int q = 0; q < parts; q++) {
+                        const int a = gsize[k] * q / parts, b = gsize[k] * (q + 1) / parts;
+                        s2.push_back(gstart[k] + a);
+                        z2.push_back(b - a);
+                    }
+                }
+                gstart.swap(s2);
+                gsize.swap(z2);
+            }
+        }
         nslots = P.fast && !n_var ? ag_fast_max_slots(occ, stage, P.learned ? 1 : 0, D.n_ast)
-                        : ag_coop_max_slots(n_var, occ, stage, P.learned ? 1 : 0);
+                        : ag_coop_max_slots(n_var, occ, stage, P.learned ? 1 : 0, P.pairs);
         const int need = 32 * ((int)gstart.size() - P.n_deep);
         if (nslots > need) nslots = need;
     } else if (grouped) {
@@ -1158,7 +1190,7 @@ static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var
     f.grp_size += P.n_deep;
     f.n_groups -= P.n_deep;
     auto fast = [&](cudaStream_t st) {
-        return n_var ? ag_launch_coop(P.D, P.c, f, n_var, P.occ, 0, st, true) : ag_launch_fast(P.D, P.c, f, P.occ, P.stage, st);
+        return n_var ? ag_launch_coop(P.D, P.c, f, n_var, P.occ, 0, st, P.pairs) : ag_launch_fast(P.D, P.c, f, P.occ, P.stage, st);
     };
     if (!P.n_deep) return fast(s);
     AgBatchArgs d = a;

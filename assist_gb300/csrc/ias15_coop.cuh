@@ -97,22 +97,37 @@ __device__ __forceinline__ int ag_coop_pcomp(int w) {
     return NV == 0 ? (w == 0 ? 0 : (w == 1 ? -1 : w - 1)) : w - 1;
 }
 
+/* Component ci of a warp, or -1.  HALF: a group of up to 16 particles, each
+ * on two lanes that share its components, two of them to an instruction: x, y
+ * and z on warps 1, 1 (other half) and 2, a variational particle's three on one
+ * warp. */
+template <int NV, bool HALF>
+__device__ __forceinline__ int ag_coop_comp(int ci, int wid, int half) {
+    if (!HALF) return ag_coop_owner<NV>(ci) == wid ? ci : -1;
+    const int k = 2 * ci + half;                    /* of warp 0: 3..8, 3: 9..14, 1: 0 1 15 16 17, 2: 2 18 19 20 */
+    if (wid == 0) return 3 + k;
+    if (wid == 3) return 9 + k;
+    if (wid == 1) return k < 2 ? k : (k < 5 ? 13 + k : -1);
+    return k == 0 ? 2 : (k < 4 ? 17 + k : -1);
+}
+
 /* IAS15's fields of a block: the fields below W_E (the state, its
  * compensations, a0, b and g, used at every node) in shared memory, the others
  * (used once a step) in the global workspace. */
-template <int C>
+template <int C, int LANES>
 struct WsSplit {
     double *s, *w;
     int ns, slot;
     __device__ __forceinline__ double& operator()(int f, int comp) const {
-        return f < W_E ? s[(f * C + comp) * 32] : w[((size_t)f * C + comp) * ns + slot];
+        return f < W_E ? s[(f * C + comp) * LANES] : w[((size_t)f * C + comp) * ns + slot];
     }
 };
 
-template <int NV>
+template <int NV, bool DYN_TABS = false>
 struct AgCoopShared {
     static constexpr int C = 3 * (1 + NV);
-    AgCoopTab tab[NV == 0 ? 8 : 1]; /* body tables, one per node, kept through the predictor-corrector
+    typename std::conditional<DYN_TABS, char, AgCoopTab[NV == 0 ? 8 : 1]>::type tab;
+                                    /* body tables, one per node, kept through the predictor-corrector
                                        iterations of a step (the node times do not change while it
                                        iterates); with variational particles in dynamic shared memory
                                        (learned start: a single one, built anew) */
@@ -348,16 +363,17 @@ struct AgTableNearest {
  * or, in the plain kernel without variational particles, the group's IAS15
  * state (40 fields x 3 components x 32 lanes, 30 KB); or, with them, the
  * eight body tables with the planets' float pairs and, in the build for one block a multiprocessor, the
- * state's fields below W_E (19 x 21 x 32, 102 KB).  What is not there stays in
+ * state's fields below W_E (19 x 21 x 32, 102 KB; with HALF, for two blocks,
+ * half of that).  What is not there stays in
  * the global workspace, indexed by slot. */
-template <int NV, bool WARM, bool STAGE = false, int OCC = 2>
+template <int NV, bool WARM, bool STAGE = false, int OCC = 2, bool HALF = false>
 struct AgCoopDyn {
     static constexpr bool ws_shared = NV == 0 && !WARM;
-    static constexpr bool ws_split = NV > 0 && !WARM && OCC == 1;
+    static constexpr bool ws_split = NV > 0 && !WARM && (OCC == 1 || HALF);
     static constexpr bool tabs = NV > 0 && !WARM;
     static constexpr size_t warm = WARM ? (sizeof(AgWarmSmem) + 15) / 16 * 16 : 0;
     static constexpr size_t ws = ws_shared ? sizeof(double) * W_NF * 3 * 32
-                                           : (ws_split ? sizeof(double) * W_E * 3 * (1 + NV) * 32 : 0);
+                                           : (ws_split ? sizeof(double) * W_E * 3 * (1 + NV) * (HALF ? 16 : 32) : 0);
     static constexpr size_t stage_off = warm + ws;        /* the staged .440 record (STAGE) */
     static constexpr size_t stage = STAGE ? (sizeof(AgRecStage) + 15) / 16 * 16 : 0;
     static constexpr size_t tab_off = stage_off + stage;
@@ -375,12 +391,14 @@ struct AgCoopDyn {
  * and 2: a block alone keeps the state in shared memory.  It is bound by the
  * FP64 pipes' latency, about 2,500 FP64 warp instructions a block and node
  * (3,200 with a table and the 18 components' Jacobian sums at every node):
- * 2,053 mixed particles over 730 days 268.6 ms before, 218.1 now. */
-template <int NV, bool WARM, int OCC = 2, bool STAGE = false, bool PAIRS = false>
+ * 2,053 mixed particles over 730 days 268.6 ms before, 218.1 so.  PAIRS: the
+ * forces on pair terms, 1,300 a node, 168.2 ms.  HALF: a particle on two
+ * lanes, 800 a node and 115 KB a block: 98.4 ms. */
+template <int NV, bool WARM, int OCC = 2, bool STAGE = false, bool PAIRS = false, bool HALF = false>
 __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict__ Ep, ForceCfg cf, AgBatchArgs A) {
     constexpr int C = 3 * (1 + NV);
     const DevEphem& E = *Ep;
-    __shared__ AgCoopShared<NV> S;
+    __shared__ AgCoopShared<NV, (NV > 0 && !WARM)> S;
     /* Role rotation: warp w of a block runs on sub-partition w % 4 of its SM,
      * and the four roles (planets / relativity / asteroids / asteroids and
      * Sun J2) do unequal FP64 work.  Blocks sharing an SM take successive
@@ -398,19 +416,24 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = ((threadIdx.x >> 5) + S.rot) & 3, tid = (wid << 5) | lane;
-    const int slot = blockIdx.x * 32 + lane;
+    /* the lane's particle in the group, and which of the particle's lanes it is */
+    const int pl = HALF ? lane & 15 : lane, half = HALF ? lane >> 4 : 0;
+    constexpr int n_ci = HALF ? 3 : C;
+    const int slot = blockIdx.x * 32 + pl;
     extern __shared__ __align__(16) unsigned char ag_dyn_smem[];
-    using Dyn = AgCoopDyn<NV, WARM, STAGE, OCC>;
+    using Dyn = AgCoopDyn<NV, WARM, STAGE, OCC, HALF>;
     constexpr bool tab8 = NV == 0 || Dyn::tabs;
-    AgCoopTab* const tabs = Dyn::tabs ? reinterpret_cast<AgCoopTab*>(ag_dyn_smem + Dyn::tab_off) : S.tab;
+    AgCoopTab* tabs;
+    if constexpr (Dyn::tabs) tabs = reinterpret_cast<AgCoopTab*>(ag_dyn_smem + Dyn::tab_off);
+    else tabs = S.tab;
     AgCoopTab& Tab = tabs[0];
     AgPairRow* const prel = PAIRS ? reinterpret_cast<AgPairRow*>(ag_dyn_smem + Dyn::prel_off) : nullptr;
     AgRecStage* const R =
         STAGE ? reinterpret_cast<AgRecStage*>(ag_dyn_smem + Dyn::stage_off) : nullptr;
     AgStageCursor cur;
     constexpr bool wss = Dyn::ws_shared;
-    typename std::conditional<Dyn::ws_split, WsSplit<C>, Ws<C>>::type W;
-    if constexpr (Dyn::ws_split) W.s = reinterpret_cast<double*>(ag_dyn_smem) + lane;
+    typename std::conditional<Dyn::ws_split, WsSplit<C, HALF ? 16 : 32>, Ws<C>>::type W;
+    if constexpr (Dyn::ws_split) W.s = reinterpret_cast<double*>(ag_dyn_smem) + pl;
     W.w = wss ? reinterpret_cast<double*>(ag_dyn_smem + Dyn::warm) : A.ws;
     W.ns = wss ? 32 : A.nslots;
     W.slot = wss ? lane : slot;
@@ -446,7 +469,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             }
             continue;
         }
-        const int pid = lane < gs ? A.order[g0 + lane] : -1;
+        const int pid = pl < gs ? A.order[g0 + pl] : -1;
         double t = A.t0[A.order[g0]], tc = 0.0, dtls = 0.0;
         const double tend = pid >= 0 ? A.t_end[pid] : t;
         double dir;
@@ -462,8 +485,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
         bool live = pid >= 0;
         if (live) {
             const double* s0 = A.state + 6 * (size_t)pid;
-            for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+            for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                 double x0, v0;
                 if (comp < 3) { x0 = s0[comp]; v0 = s0[3 + comp]; }
                 else {
@@ -502,8 +526,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             /* ---- retire lanes whose particle is complete */
             if (__any_sync(AG_FULL, finish_now)) {
                 if (finish_now) {
-                    for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+                    for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                         const double x1 = W(W_X0, comp) + W(W_XC, comp), v1 = W(W_V0, comp) + W(W_VC, comp);
                         if (dense && comp < 3) {
                             /* times left at a completed particle are its t_end: the end
@@ -519,7 +544,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                         if (comp < 3) {
                             double* s0 = A.state + 6 * (size_t)pid;
                             s0[comp] = x1; s0[3 + comp] = v1;
-                            S.fin[comp][lane] = isfinite(x1) && isfinite(v1);
+                            S.fin[comp][pl] = isfinite(x1) && isfinite(v1);
                         } else {
                             double* vs = A.var_state + ((size_t)pid * NV + (comp - 3) / 3) * 6;
                             vs[(comp - 3) % 3] = x1; vs[3 + (comp - 3) % 3] = v1;
@@ -528,7 +553,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                 }
                 __syncthreads();
                 if (finish_now) {
-                    const bool finite = S.fin[0][lane] && S.fin[1][lane] && S.fin[2][lane];
+                    const bool finite = S.fin[0][pl] && S.fin[1][pl] && S.fin[2][pl];
                     if (pstat == AG_ST_OK && !finite) pstat = AG_ST_NONFINITE;
                     if (wid == 0 && A.status) A.status[pid] = pstat;
                     live = false;
@@ -573,11 +598,12 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             int bad = ag_coop_table_pass1<STAGE>(E, cf, t, S.scr, Tab, tid, R, cur, &S.stage_fail);
             n_tab++;
             if (live)
-                for (int comp = 0; comp < C; comp++)
-                    if (ag_coop_owner<NV>(comp) == wid) {
-                        S.xs[comp][lane] = W(W_X0, comp); S.vs[comp][lane] = W(W_V0, comp);
-                        if constexpr (NV == 0 && !WARM) S.xsf[comp][lane] = ag_f2_of(W(W_X0, comp));
-                    }
+                for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
+                    S.xs[comp][pl] = W(W_X0, comp); S.vs[comp][pl] = W(W_V0, comp);
+                    if constexpr (NV == 0 && !WARM) S.xsf[comp][lane] = ag_f2_of(W(W_X0, comp));
+                }
             bad = __syncthreads_or(bad);
             if (bad) { pstat = S.stage_fail ? AG_ST_TIMEOUT : AG_ST_COVERAGE; finish_now = live; continue; }
             ag_coop_table_pass2(E, cf, t, Tab, S.scr, tid);
@@ -587,8 +613,8 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             if (wid == 1 && (cf.forces & AG_F_EIH)) ag_coop_eih_sources(E, cf, Tab.T, lane);
             int fst = AG_OK;
             {
-                const double xp[3] = {S.xs[0][lane], S.xs[1][lane], S.xs[2][lane]};
-                const double vp[3] = {S.vs[0][lane], S.vs[1][lane], S.vs[2][lane]};
+                const double xp[3] = {S.xs[0][pl], S.xs[1][pl], S.xs[2][pl]};
+                const double vp[3] = {S.vs[0][pl], S.vs[1][pl], S.vs[2][pl]};
                 double acc[3] = {0.0, 0.0, 0.0};
                 if (NV > 0) {
                     if (live) {
@@ -613,15 +639,16 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                 }
                 if (live) {
                     S.pa[wid][0][lane] = acc[0]; S.pa[wid][1][lane] = acc[1]; S.pa[wid][2][lane] = acc[2];
-                    if (wid == 0) n_ev++;
+                    if (wid == 0 && half == 0) n_ev++;
                 }
             }
             bad = __syncthreads_or(fst != AG_OK);
             if (bad) { pstat = AG_ST_COVERAGE; finish_now = live; continue; }
             if constexpr (NV > 0) ag_coop_sum_jac(S, wid, lane, live);
             if (live) {
-                for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+                for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                     double at;
                     if (comp < 3) {
                         at = ((S.pa[3][comp][lane] + S.pa[2][comp][lane]) + S.pa[1][comp][lane]) + S.pa[0][comp][lane];
@@ -631,14 +658,15 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                         for (int b = 0; b < 6; b++) Jr[b] = S.pj[0][6 * a + b][lane];
                         const double* dxq = &S.xs[3 + 3 * q][0];
                         const double* dvq = &S.vs[3 + 3 * q][0];
-                        double s = Jr[0] * dxq[lane];
-                        s = fma(Jr[1], dxq[32 + lane], s); s = fma(Jr[2], dxq[64 + lane], s);
-                        s = fma(Jr[3], dvq[lane], s); s = fma(Jr[4], dvq[32 + lane], s); s = fma(Jr[5], dvq[64 + lane], s);
+                        double s = Jr[0] * dxq[pl];
+                        s = fma(Jr[1], dxq[32 + pl], s); s = fma(Jr[2], dxq[64 + pl], s);
+                        s = fma(Jr[3], dvq[pl], s); s = fma(Jr[4], dvq[32 + pl], s); s = fma(Jr[5], dvq[64 + pl], s);
                         at = s;
                     }
                     W(W_A0, comp) = at;
                 }
             }
+            if (HALF) __syncwarp();
             /* ---- learned warm start: features, BF16 inference, b += kappa y */
             bool w_applied = false, w_probe = false, w_ran = false;
             if constexpr (WARM) {
@@ -648,8 +676,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                                              w_probe, n_wused, n_wfall);
             }
             if (live) {
-                for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+                for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                     double b[7];
 #pragma unroll
                     for (int k = 0; k < 7; k++) b[k] = W(W_B + k, comp);
@@ -677,21 +706,22 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                     if (!conv) {
                         const double* sx = S.pcx[n];
                         const double* sv = S.pcv[n];
-                        for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+                        for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                             double px = sx[8] * W(W_B + 6, comp);
 #pragma unroll
                             for (int j = 5; j >= 0; j--) px = fma(sx[j + 2], W(W_B + j, comp), px);
                             px = fma(sx[1], W(W_A0, comp), px);
                             px = fma(sx[0], W(W_V0, comp), px);
                             const double xn = W(W_X0, comp) + (px + W(W_XC, comp));
-                            S.xs[comp][lane] = xn;
+                            S.xs[comp][pl] = xn;
                             if constexpr (NV == 0 && !WARM) S.xsf[comp][lane] = ag_f2_of(xn);
                             double pv = sv[7] * W(W_B + 6, comp);
 #pragma unroll
                             for (int j = 5; j >= 0; j--) pv = fma(sv[j + 1], W(W_B + j, comp), pv);
                             pv = fma(sv[0], W(W_A0, comp), pv);
-                            S.vs[comp][lane] = W(W_V0, comp) + (pv + W(W_VC, comp));
+                            S.vs[comp][pl] = W(W_V0, comp) + (pv + W(W_VC, comp));
                         }
                     }
                     bad = __syncthreads_or(bad);
@@ -704,8 +734,8 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                         if (wid == 1 && (cf.forces & AG_F_EIH)) ag_coop_eih_sources(E, cf, TabN.T, lane);
                     }
                     {
-                        const double xp[3] = {S.xs[0][lane], S.xs[1][lane], S.xs[2][lane]};
-                        const double vp[3] = {S.vs[0][lane], S.vs[1][lane], S.vs[2][lane]};
+                        const double xp[3] = {S.xs[0][pl], S.xs[1][pl], S.xs[2][pl]};
+                        const double vp[3] = {S.vs[0][pl], S.vs[1][pl], S.vs[2][pl]};
                         double acc[3] = {0.0, 0.0, 0.0};
                         if (NV > 0) {
                             if (!conv) {
@@ -731,14 +761,15 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                         }
                         if (!conv) {
                             S.pa[wid][0][lane] = acc[0]; S.pa[wid][1][lane] = acc[1]; S.pa[wid][2][lane] = acc[2];
-                            if (wid == 0) n_ev++;
+                            if (wid == 0 && half == 0) n_ev++;
                         }
                     }
                     __syncthreads();
                     if constexpr (NV > 0) ag_coop_sum_jac(S, wid, lane, !conv);
                     if (!conv) {
-                        for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+                        for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                             double at;
                             if (comp < 3) {
                                 at = ((S.pa[3][comp][lane] + S.pa[2][comp][lane]) + S.pa[1][comp][lane]) + S.pa[0][comp][lane];
@@ -748,9 +779,9 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                                 for (int b = 0; b < 6; b++) Jr[b] = S.pj[0][6 * a + b][lane];
                                 const double* dxq = &S.xs[3 + 3 * q][0];
                                 const double* dvq = &S.vs[3 + 3 * q][0];
-                                double s = Jr[0] * dxq[lane];
-                                s = fma(Jr[1], dxq[32 + lane], s); s = fma(Jr[2], dxq[64 + lane], s);
-                                s = fma(Jr[3], dvq[lane], s); s = fma(Jr[4], dvq[32 + lane], s); s = fma(Jr[5], dvq[64 + lane], s);
+                                double s = Jr[0] * dxq[pl];
+                                s = fma(Jr[1], dxq[32 + pl], s); s = fma(Jr[2], dxq[64 + pl], s);
+                                s = fma(Jr[3], dvq[pl], s); s = fma(Jr[4], dvq[32 + pl], s); s = fma(Jr[5], dvq[64 + pl], s);
                                 at = s;
                             }
                             double gn = (at - W(W_A0, comp)) * ag_ias.rrinv[n][0];
@@ -761,24 +792,25 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                             W(W_B + n - 1, comp) += delta;
                             if (n == 7 && comp < 3) {
                                 const double aa = fabs(at), db = fabs(delta);
-                                S.ra[comp][lane] = ag_isnormal_pos(aa) ? aa : 0.0;
-                                S.rdb[comp][lane] = ag_isnormal_pos(db) ? db : 0.0;
+                                S.ra[comp][pl] = ag_isnormal_pos(aa) ? aa : 0.0;
+                                S.rdb[comp][pl] = ag_isnormal_pos(db) ? db : 0.0;
                             }
                         }
                     }
+                    if (HALF) __syncwarp();      /* the other half has read this node's states */
                 }
                 if (cov) break;
                 __syncthreads();
                 if (!conv) {
                     double maxa = 0.0, maxdb = 0.0;
                     for (int k = 0; k < 3; k++) {
-                        maxa = ag_max_nonneg(maxa, S.ra[k][lane]);
-                        maxdb = ag_max_nonneg(maxdb, S.rdb[k][lane]);
+                        maxa = ag_max_nonneg(maxa, S.ra[k][pl]);
+                        maxdb = ag_max_nonneg(maxdb, S.rdb[k][pl]);
                     }
                     ma7 = maxa;
                     const double pc_err = maxdb / maxa;
                     conv = (pc_err < 1e-16) || (iters > 2 && pc_last <= pc_err) || (iters >= 12);
-                    if (conv) { it_lane = iters; if (wid == 0) n_it += (unsigned long long)iters; }
+                    if (conv) { it_lane = iters; if (wid == 0 && half == 0) n_it += (unsigned long long)iters; }
                     else pc_last = pc_err;
                 }
                 if (__all_sync(AG_FULL, conv)) break;
@@ -810,9 +842,10 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
                 }
             }
             /* ---- step-size control: each lane's choice, the group takes the smallest */
-            if (live && ag_coop_pcomp<NV>(wid) >= 0) {
-                const double bb = fabs(W(W_B + 6, ag_coop_pcomp<NV>(wid)));
-                S.rb6[ag_coop_pcomp<NV>(wid)][lane] = ag_isnormal_pos(bb) ? bb : 0.0;
+            const int pc = HALF ? (wid == 1 ? half : (wid == 2 && half == 0 ? 2 : -1)) : ag_coop_pcomp<NV>(wid);
+            if (live && pc >= 0) {
+                const double bb = fabs(W(W_B + 6, pc));
+                S.rb6[pc][pl] = ag_isnormal_pos(bb) ? bb : 0.0;
             }
             __syncthreads();
             double dt_new_l = 1e300, dt_nocap_l = 1e300;
@@ -822,7 +855,7 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             if (wid == 0) {
                 if (A.epsilon > 0.0 && live) {
                     double mb = 0.0;
-                    for (int k = 0; k < 3; k++) mb = ag_max_nonneg(mb, S.rb6[k][lane]);
+                    for (int k = 0; k < 3; k++) mb = ag_max_nonneg(mb, S.rb6[k][pl]);
                     const double err = mb / ma7;
                     const double safety = 0.25;
                     double dn;
@@ -865,9 +898,10 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             const bool reject = __any_sync(AG_FULL, rej_l);
             if (reject) {
                 if (live) {
-                    if (wid == 0) n_rej++;
-                    for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+                    if (wid == 0 && half == 0) n_rej++;
+                    for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                         if (dtls != 0.0) ag_predict_next_comp(W, comp, dt_new / dtls);
                         else
                             for (int k = 0; k < 7; k++) { W(W_B + k, comp) = 0.0; W(W_E + k, comp) = 0.0; }
@@ -923,10 +957,11 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
             }
             /* ---- accept */
             if (live) {
-                if (wid == 0) n_acc++;
+                if (wid == 0 && half == 0) n_acc++;
                 const double h2 = hstep * hstep;
-                for (int comp = 0; comp < C; comp++) {
-                    if (ag_coop_owner<NV>(comp) != wid) continue;
+                for (int ci = 0; ci < n_ci; ci++) {
+                    const int comp = ag_coop_comp<NV, HALF>(ci, wid, half);
+                    if (comp < 0) continue;
                     double b[7];
 #pragma unroll
                     for (int k = 0; k < 7; k++) b[k] = W(W_B + k, comp);
@@ -978,36 +1013,37 @@ __global__ void __launch_bounds__(128, OCC) ag_k_coop(const DevEphem* __restrict
     if (STAGE && tid == 0 && S.stage_fail) ag_mbar_wait(&R->bar, cur.phase ^ 1u);
 }
 
-/* Dynamic shared memory that leaves no room on a multiprocessor (228 KB) for a
- * block of the pair-term kernel (60 KB and more). */
+/* Dynamic shared memory that leaves no room on a multiprocessor (228 KB) for
+ * another such block or one of the pair-term kernel (60 KB and more). */
 #define AG_COOP_ALONE (165 * 1024)
 
 /* Opt the kernel in to its dynamic shared memory (above the 48 KB default). */
-template <int NV, bool WARM, int OCC, bool STAGE = false, bool PAIRS = false>
+template <int NV, bool WARM, int OCC, bool STAGE = false, bool PAIRS = false, bool HALF = false>
 static int ag_coop_dyn_attr() {
-    constexpr size_t own = AgCoopDyn<NV, WARM, STAGE, OCC>::bytes;
-    constexpr size_t bytes = NV == 0 && !WARM && OCC == 2 && !STAGE ? (size_t)AG_COOP_ALONE : own;
+    constexpr size_t own = AgCoopDyn<NV, WARM, STAGE, OCC, HALF>::bytes;
+    constexpr size_t bytes = (NV == 0 && !WARM && OCC == 2 && !STAGE) || HALF ? (size_t)AG_COOP_ALONE : own;
     if (bytes == 0) return 0;
-    return (int)cudaFuncSetAttribute(ag_k_coop<NV, WARM, OCC, STAGE, PAIRS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return (int)cudaFuncSetAttribute(ag_k_coop<NV, WARM, OCC, STAGE, PAIRS, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-template <int NV, bool WARM, int OCC, bool STAGE = false>
+template <int NV, bool WARM, int OCC, bool STAGE = false, bool PAIRS = false, bool HALF = false>
 static int ag_coop_blocks_per_sm() {
     int bps = 0;
-    if (ag_coop_dyn_attr<NV, WARM, OCC, STAGE>() == 0)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ag_k_coop<NV, WARM, OCC, STAGE>, 128,
-                                                      AgCoopDyn<NV, WARM, STAGE, OCC>::bytes);
+    if (ag_coop_dyn_attr<NV, WARM, OCC, STAGE, PAIRS, HALF>() == 0)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ag_k_coop<NV, WARM, OCC, STAGE, PAIRS, HALF>, 128,
+                                                      AgCoopDyn<NV, WARM, STAGE, OCC, HALF>::bytes);
     return bps;
 }
 
 /* Slots (32 per resident block) of the plain (nv = 0: occ 2 or 3, stage
  * only with occ 2) or variational (nv = 6: occ 1 or 2) kernel, or of their learned
  * warm-start builds (warm), on the current device. */
-int ag_coop_max_slots(int nv, int occ, int stage, int warm) {
+int ag_coop_max_slots(int nv, int occ, int stage, int warm, int pairs) {
     int dev = 0, sms = 0, bps = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (nv == 6)
+    if (nv == 6 && pairs == 16) bps = occ == 1 ? 1 : ag_coop_blocks_per_sm<6, false, 2, false, true, true>();
+    else if (nv == 6)
         bps = warm ? ag_coop_blocks_per_sm<6, true, 2>()
                    : (occ == 1 ? ag_coop_blocks_per_sm<6, false, 1>() : ag_coop_blocks_per_sm<6, false, 2>());
     else if (warm) bps = ag_coop_blocks_per_sm<0, true, 2>();
@@ -1019,16 +1055,17 @@ int ag_coop_max_slots(int nv, int occ, int stage, int warm) {
 }
 
 int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int occ, int stage,
-                   cudaStream_t s, bool pairs) {
+                   cudaStream_t s, int pairs) {
     int e = ag_ias_tables_init();
     if (e) return e;
     const int blocks = (a.nslots + 31) / 32;
     if (nv == 6 && (a.mlp || a.log_x)) {
         if ((e = ag_coop_dyn_attr<6, true, 2>())) return e;
         ag_k_coop<6, true, 2><<<blocks, 128, AgCoopDyn<6, true>::bytes, s>>>(E.self_dev, c, a);
-    } else if (nv == 6 && pairs && occ == 1) {
-        if ((e = ag_coop_dyn_attr<6, false, 1, false, true>())) return e;
-        ag_k_coop<6, false, 1, false, true><<<blocks, 128, AgCoopDyn<6, false, false, 1>::bytes, s>>>(E.self_dev, c, a);
+    } else if (nv == 6 && pairs == 16) {
+        if ((e = ag_coop_dyn_attr<6, false, 2, false, true, true>())) return e;
+        ag_k_coop<6, false, 2, false, true, true>
+            <<<blocks, 128, occ == 1 ? (size_t)AG_COOP_ALONE : AgCoopDyn<6, false, false, 2, true>::bytes, s>>>(E.self_dev, c, a);
     } else if (nv == 6 && pairs) {
         if ((e = ag_coop_dyn_attr<6, false, 2, false, true>())) return e;
         ag_k_coop<6, false, 2, false, true><<<blocks, 128, AgCoopDyn<6, false>::bytes, s>>>(E.self_dev, c, a);
@@ -1070,7 +1107,7 @@ int ag_coop_ready(void) {
     if (!e) e = ag_coop_dyn_attr<6, true, 2>();
     if (!e) e = ag_coop_dyn_attr<6, false, 1>();
     if (!e) e = ag_coop_dyn_attr<6, false, 2>();
-    if (!e) e = ag_coop_dyn_attr<6, false, 1, false, true>();
+    if (!e) e = ag_coop_dyn_attr<6, false, 2, false, true, true>();
     if (!e) e = ag_coop_dyn_attr<6, false, 2, false, true>();
     return e;
 }

@@ -96,7 +96,7 @@ int ag_launch_batch(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, 
 int ag_batch_max_slots(int nv, int tpb);
 int ag_group_max_slots(int nv);
 int ag_launch_group(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, cudaStream_t s);
-int ag_coop_max_slots(int nv, int occ, int stage, int warm);
+int ag_coop_max_slots(int nv, int occ, int stage, int warm, int pairs = 0);
 /* Per-particle encounter cost ratio (extra steps / base steps) from a
  * two-body pilot on a G-point time grid over [tmin, tmax] and, unless d_deep
  * is null, whether the particle passes deep inside a planet's sphere of
@@ -105,9 +105,9 @@ int ag_pilot_encounters(const DevEphem& E, int n, const double* d_t0, const doub
                         double tmin, double tmax, float* d_ratio, unsigned char* d_deep, float4* d_grid,
                         float2* d_sunv, int G, cudaStream_t s);
 /* pairs: with variational particles, the forces on pair terms (ag_fast_covers
- * and all direct terms on) */
+ * and all direct terms on); 16: groups of at most that many particles */
 int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int occ, int stage,
-                   cudaStream_t s, bool pairs = false);
+                   cudaStream_t s, int pairs = 0);
 /* the batched kernel on fast_forces.cuh (kernels_fast.cu): configurations ag_fast_covers */
 int ag_fast_max_slots(int occ, int stage, int warm, int n_ast);
 int ag_launch_fast(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int occ, int stage, cudaStream_t s);

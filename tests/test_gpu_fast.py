@@ -231,12 +231,13 @@ def test_dropin_run_kernel_with_variational(files, n, t1):
     ex.detach(sim); sim.free()
 
 
-@pytest.mark.parametrize("n,length,sign", [(1, 60.0, 1.0), (33, 60.0, -1.0), (20500, 2.0, 1.0)])
+@pytest.mark.parametrize("n,length,sign", [(1, 60.0, 1.0), (16, 60.0, 1.0), (33, 60.0, -1.0), (20500, 2.0, 1.0),
+                                           (27000, 1.0, 1.0)])
 def test_batch_with_variational(files, n, length, sign):
     """Batches with six variational particles each, a third with
     non-gravitational parameters, of unequal lengths, forward and backward:
-    one group, a group's remainder, and more groups than get a multiprocessor
-    each (a sample of those against the oracle)."""
+    one group, remainders of groups of sixteen, many of those, and more than
+    they are formed for (samples of those against the oracle)."""
     from assist_gb300 import Ephem, batch, synth
     from tests.oracle_py import Oracle
     pl, ast, system = files
