@@ -21,12 +21,16 @@
  * half and they exchange them through shared memory at a named barrier
  * (without Jacobians; with them each warp forms all eleven).
  *
+ * With variational particles the forces are on pair terms where those apply
+ * (PAIRS, ag_coop_force_pairs), and a group of up to sixteen may put each
+ * particle on two lanes that share its components (HALF).
+ *
  * The partial accelerations (and partial Jacobians) meet in shared memory and
  * are summed in a fixed order ((w3 + w2) + w1) + w0, so the planets' terms,
  * the largest, come last as in ASSIST's sum.  The body table of each
- * substep time is built by the whole block: column components of the .440
- * record and asteroid components of the SPK records on different threads, in
- * the reference's exact arithmetic.  Each IAS15 state component has an owner
+ * substep time is built by the whole block, once a step: column components of
+ * the .440 record and asteroid components of the SPK records on different
+ * threads, with fused multiply-adds.  Each IAS15 state component has an owner
  * warp that predicts it, forms its acceleration from the partials and
  * updates its g, b and e: x, y, z belong to warps 0, 2, 3 (warps 1, 2, 3
  * with variational particles); the three
