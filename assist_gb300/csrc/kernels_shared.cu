@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* _
     /* the control warp's state, the same in every block */
     ShCtl K = *A.in;
     double hstep = 0.0;
-    bool last = false;
+    bool last = false, gave_up = false;
     int round = 0;                      /* iterations of this launch: the rotating buffers */
     for (int step = 0; step < A.limit; step++) {
         if (ctl) {
@@ -492,6 +492,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* _
                     ok = sh_run_maxima(A, round, lane, mdb, ma, mb);
                     round++;
                 }
+                gave_up = !ok;
                 cmd = sh_run_decide(A, K, S, ok, mdb, ma, mb, hstep, last, iters, pc_last, lane);
             }
             __syncthreads();
@@ -517,10 +518,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* _
     if (live && pc >= 0)
         for (int f = 0; f < 8; f++)
             for (int k = 0; k < (f < 4 ? 1 : 7); k++) A.W(theirs[f] + k, pc, i) = W(mine[f] + k, pc);
-    if (ctl && lane == 0 && (blockIdx.x == 0 || K.gave_up)) {
-        if (blockIdx.x == 0) *A.out = K;
-        else atomicExch(&A.out->gave_up, 1);
-    }
+    if (ctl && lane == 0) sh_run_report(K, gave_up, blockIdx.x, A.out, A.gave_up);
 }
 
 static size_t sh_run_bytes(int n_ast) { return sizeof(double) * W_NF * 3 * 32 + 8 * (size_t)AgFastLayout(n_ast).stride; }
@@ -764,7 +762,7 @@ struct AgSharedSim {
     unsigned long long* d_red = nullptr;  /* 16 words: maxima, iterations, rotating buffers */
     unsigned* d_bar = nullptr;    /* grid barrier of the cooperative step launch */
     ShRunMem* d_run = nullptr;    /* control state of the run kernel */
-    ShCtl* h_ctl = nullptr;       /* pinned */
+    ShRunMem* h_run = nullptr;    /* its copy, pinned */
     int run_blocks = -1;          /* blocks a launch of the run kernel can hold (-1: not yet asked) */
     int var_lanes = -1, var_n = 0;  /* particles a block of the run kernel with variational particles, for var_n */
     int coop_blocks = -1;         /* blocks a cooperative step launch can hold (-1: not yet asked) */
@@ -791,7 +789,7 @@ void ag_shared_free(AgSharedSim* s) {
     if (s->d_red) cudaFree(s->d_red);
     if (s->d_bar) cudaFree(s->d_bar);
     if (s->d_run) cudaFree(s->d_run);
-    if (s->h_ctl) cudaFreeHost(s->h_ctl);
+    if (s->h_run) cudaFreeHost(s->h_run);
     if (s->d_status) cudaFree(s->d_status);
     if (s->h_pin) cudaFreeHost(s->h_pin);
     if (s->stream) cudaStreamDestroy(s->stream);
@@ -1036,10 +1034,8 @@ static int sh_run(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct r
         if (s->run_blocks < 0) s->run_blocks = sh_run_capacity(E.n_ast);
         if (nb > s->run_blocks) return -1;
     }
-    if (!s->d_run) {
-        if (ag_cuda_check(cudaMalloc(&s->d_run, sizeof(ShRunMem)), "cudaMalloc(run state)")) return 1;
-        if (ag_cuda_check(cudaMallocHost(&s->h_ctl, sizeof(ShCtl)), "cudaMallocHost(run state)")) return 1;
-    }
+    if (!s->d_run && ag_cuda_check(cudaMalloc(&s->d_run, sizeof(ShRunMem)), "cudaMalloc(run state)")) return 1;
+    if (!s->h_run && ag_cuda_check(cudaMallocHost(&s->h_run, sizeof(ShRunMem)), "cudaMallocHost(run state)")) return 1;
     if (params) {
         const size_t np = 3 * (size_t)n;
         if (np > s->params_cap) {
@@ -1064,16 +1060,18 @@ static int sh_run(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct r
     A.limit = SH_RUN_STEPS;
     A.red = s->d_run->red;
     A.bar = s->d_run->bar;
-    ShRunMem m;
+    A.gave_up = &s->d_run->gave_up;
+    ShRunMem& m = *s->h_run;
     std::memset(&m, 0, sizeof(m));
     m.ctl[0].t = s->t; m.ctl[0].dt = dt; m.ctl[0].dtls = s->dt_last_success;
     const size_t F = 3 * (size_t)s->cap, bytes = sh_run_bytes(E.n_ast);
     cudaMemcpyAsync(s->d_run, &m, sizeof(m), cudaMemcpyHostToDevice, st);
-    ShCtl& K = *s->h_ctl;
-    for (int launch = 0;; launch++) {
+    const ShCtl* last = nullptr;
+    for (int launch = 0; !last; launch++) {
+        const ShCtl& K = m.ctl[1 - (launch & 1)];
         A.in = &s->d_run->ctl[launch & 1];
         A.out = &s->d_run->ctl[1 - (launch & 1)];
-        if (launch) cudaMemsetAsync(A.red, 0, sizeof(m.red) + sizeof(m.bar), st);
+        if (launch) cudaMemsetAsync(A.red, 0, sizeof(m) - offsetof(ShRunMem, red), st);
         if (var) {
             const cudaError_t le = ag_launch_var_run(E, c, A, s->d_vindex, lanes, st);
             if (le == cudaErrorCooperativeLaunchTooLarge && launch == 0) {
@@ -1099,15 +1097,16 @@ static int sh_run(AgSharedSim* s, const DevEphem& E, const ForceCfg& c, struct r
             }
             if (ag_cuda_check(le, "IAS15 run kernel (cooperative)")) return 1;
         }
-        cudaMemcpyAsync(&K, A.out, sizeof(ShCtl), cudaMemcpyDeviceToHost, st);
+        cudaMemcpyAsync(&m, s->d_run, sizeof(m), cudaMemcpyDeviceToHost, st);
         cudaMemcpyAsync(s->h_pin, A.W.w + (size_t)S_X0 * F, sizeof(double) * 5 * F, cudaMemcpyDeviceToHost, st);
         if (ag_cuda_check(cudaStreamSynchronize(st), "IAS15 run")) return 1;
-        if (K.gave_up) {
+        if (m.gave_up) {
             ag_set_error("IAS15 run kernel: a block stopped waiting at the grid barrier");
             return 1;
         }
-        if (K.status || K.t == tmax || (A.max_steps > 0 && K.accepted >= A.max_steps)) break;
+        if (K.status || K.t == tmax || (A.max_steps > 0 && K.accepted >= A.max_steps)) last = &K;
     }
+    const ShCtl& K = *last;
     s->t = K.t; s->tc = K.tc; s->dt_last_success = K.dtls; s->n_real = n;
     out->accepted += K.accepted;
     out->rejected += K.rejected;

@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 2) ag_k_var_run(const DevEphe
     };
     int round = 0, run_steps = 0;
     double hstep = 0.0;
-    bool last = false;
+    bool last = false, gave_up = false;
     while (true) {
         if (ctl) {
             const double rem = (R.tmax - K.t) - K.tc;
@@ -480,6 +480,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 2) ag_k_var_run(const DevEphe
                     ok = sh_run_maxima(R, round, lane, mdb, ma, mb);
                     round++;
                 }
+                gave_up = !ok;
                 sh_run_decide(R, K, S, ok, mdb, ma, mb, hstep, last, iters, pc_last, lane);
             }
             __syncthreads();
@@ -558,10 +559,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 2) ag_k_var_run(const DevEphe
         R.W(S_XC, k, p) = w[V_XC * T + q]; R.W(S_VC, k, p) = w[V_VC * T + q];
         for (int f = 0; f < 7; f++) R.W(S_B + f, k, p) = w[(V_B + f) * T + q];
     }
-    if (ctl && lane == 0) {
-        if (blockIdx.x == 0) *R.out = K;
-        else if (K.gave_up) atomicExch(&R.out->gave_up, 1);
-    }
+    if (ctl && lane == 0) sh_run_report(K, gave_up, blockIdx.x, R.out, R.gave_up);
 }
 
 template <int L>

@@ -8,6 +8,7 @@
 #include <cstddef>
 
 #include "ias15_fast.cuh"
+#include "run_ctl.h"
 
 /* field layout: f*(3*stride) + k*stride + i */
 enum { S_X0 = 0, S_V0, S_A0, S_XC, S_VC, S_AT, S_XP, S_VP, S_B, S_G = S_B + 7, S_E = S_G + 7, S_BR = S_E + 7, S_ER = S_BR + 7,
@@ -19,12 +20,6 @@ struct ShView {
     __device__ __forceinline__ double& operator()(int f, int k, int i) const { return w[((size_t)f * 3 + k) * stride + i]; }
 };
 
-struct ShCtl {
-    double t, tc, dt, dtls, dt_done;
-    long long accepted, rejected, iterations;
-    int status, gave_up;
-};
-
 struct ShRunArgs {
     ShView W;
     int n;
@@ -34,16 +29,10 @@ struct ShRunArgs {
     int limit;                   /* steps of this launch */
     const ShCtl* in;
     ShCtl* out;
-    unsigned long long* red;     /* nine words: three rotating buffers of the maxima, zero at launch */
-    unsigned* bar;               /* grid barrier: arrivals, generation */
+    unsigned long long* red;     /* ShRunMem's */
+    unsigned *bar, *gave_up;
 };
 
-/* Device memory of a simulation's run kernel. */
-struct ShRunMem {
-    ShCtl ctl[2];                /* a launch reads one and writes the other */
-    unsigned long long red[9];
-    unsigned bar[2];
-};
 /* Steps of one launch (a year of 1,024 main-belt particles is 65): the device
  * is not held for longer than some tens of milliseconds at a time. */
 #define SH_RUN_STEPS 256
@@ -103,7 +92,6 @@ __device__ __forceinline__ int sh_run_decide(const ShRunArgs& A, ShCtl& K, AgFas
     int cmd = SH_ITERATE;
     if (!ok) {
         cmd = SH_LEAVE;
-        K.gave_up = 1;
     } else if (conv) {
         double dt_new = hstep;
         cmd = SH_ACCEPT;
