@@ -550,14 +550,15 @@ int ag_launch_forces_own(const DevEphem& E, const ForceCfg& c, int n, const doub
                          const double* params, int nv, const double* var_state, double* acc, double* var_acc, int* status,
                          cudaStream_t s) {
     const int blocks = (n + 31) / 32;
-    const size_t bytes = sizeof(AgF2) * 3 * 32 * (AG_PAIR_PL + (size_t)E.n_ast);
+    auto bytes = [](int n_ast) { return sizeof(AgF2) * 3 * 32 * (AG_PAIR_PL + (size_t)n_ast); };
     if (nv) {
-        const size_t all = bytes + sizeof(AgOwnJac);
-        const cudaError_t e = cudaFuncSetAttribute(ag_k_forces_own<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)all);
+        /* the limit is the kernel's, shared by every thread of the process: always the largest */
+        const cudaError_t e = cudaFuncSetAttribute(ag_k_forces_own<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)(bytes(AG_MAX_AST) + sizeof(AgOwnJac)));
         if (e != cudaSuccess) return (int)e;
-        ag_k_forces_own<true><<<blocks, 128, all, s>>>(E.self_dev, c, n, t, state, params, var_state, acc, var_acc, status);
+        ag_k_forces_own<true><<<blocks, 128, bytes(E.n_ast) + sizeof(AgOwnJac), s>>>(E.self_dev, c, n, t, state, params, var_state, acc, var_acc, status);
     } else {
-        ag_k_forces_own<false><<<blocks, 128, bytes, s>>>(E.self_dev, c, n, t, state, params, nullptr, acc, nullptr, status);
+        ag_k_forces_own<false><<<blocks, 128, bytes(E.n_ast), s>>>(E.self_dev, c, n, t, state, params, nullptr, acc, nullptr, status);
     }
     return (int)cudaGetLastError();
 }
