@@ -148,8 +148,8 @@ static __device__ __noinline__ void ag_own_close(const DevEphem& E, const ForceC
     const double ri = rsqrt(fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2])));
     if (f & 2) ag_term_sun_h<JAC>(E, c, d[0], d[1], d[2], ri, ax, ay, az, J);
     if (f & 4) {
-        /* relativity far out (without JAC: the Jacobian form is FP64 everywhere) */
-        double af[3] = {0.0, 0.0, 0.0}, ut = 0.0, up = 0.0, v2 = 0.0, w2 = 0.0, vw = 0.0, dw = 0.0, da = 0.0, g = 0.0;
+        /* relativity far out, where the planets' sums are no small parts of it */
+        double af[3] = {0.0, 0.0, 0.0}, gp[3] = {0.0, 0.0, 0.0}, ut = 0.0, up = 0.0;
         for (int k = 1; k < AG_NPL; k++) {
             double b[3];
             ag_planet_exact<false>(E, rec, tf, k, b, nullptr);
@@ -158,18 +158,30 @@ static __device__ __noinline__ void ag_own_close(const DevEphem& E, const ForceC
             ut += gr;
             af[0] = fma(-q, sx, af[0]); af[1] = fma(-q, sy, af[1]); af[2] = fma(-q, sz, af[2]);
             const double px = x[0] - b[0], py = x[1] - b[1], pz = x[2] - b[2];
-            up = fma(E.gm[k], rsqrt(fma(px, px, fma(py, py, pz * pz))), up);
+            const double pi = rsqrt(fma(px, px, fma(py, py, pz * pz)));
+            up = fma(E.gm[k], pi, up);
+            if (JAC) {
+                const double g = E.gm[k] * pi * pi * pi;
+                gp[0] = fma(g, px, gp[0]); gp[1] = fma(g, py, gp[1]); gp[2] = fma(g, pz, gp[2]);
+            }
         }
-        for (int k = 0; k < 3; k++) {
-            const double w = S.sv[k][lane];
-            v2 = fma(v[k], v[k], v2); w2 = fma(w, w, w2); vw = fma(v[k], w, vw);
-            dw = fma(d[k], w, dw); da = fma(d[k], af[k], da); g = fma(d[k], 4.0 * v[k] - 3.0 * w, g);
+        const double w[3] = {S.sv[0][lane], S.sv[1][lane], S.sv[2][lane]};
+        if (JAC) {
+            double ea[3];
+            ag_fast_eih_jac(E, d, ri, v, w, af, ut, up, gp, ea, J);
+            ax += ea[0]; ay += ea[1]; az += ea[2];
+        } else {
+            double v2 = 0.0, w2 = 0.0, vw = 0.0, dw = 0.0, da = 0.0, g = 0.0;
+            for (int k = 0; k < 3; k++) {
+                v2 = fma(v[k], v[k], v2); w2 = fma(w[k], w[k], w2); vw = fma(v[k], w[k], vw);
+                dw = fma(d[k], w[k], dw); da = fma(d[k], af[k], da); g = fma(d[k], 4.0 * v[k] - 3.0 * w[k], g);
+            }
+            const double gr = E.gm[AG_SUN] * ri, pre = E.over_c_squared * gr * ri * ri, ga = 3.5 * E.over_c_squared * gr;
+            const double fac = v2 - 4.0 * (gr + up) - ut + 2.0 * w2 - 4.0 * vw - 1.5 * (dw * ri) * (dw * ri) - 0.5 * da;
+            ax += -pre * fac * d[0] + pre * g * (v[0] - w[0]) + ga * af[0];
+            ay += -pre * fac * d[1] + pre * g * (v[1] - w[1]) + ga * af[1];
+            az += -pre * fac * d[2] + pre * g * (v[2] - w[2]) + ga * af[2];
         }
-        const double gr = E.gm[AG_SUN] * ri, pre = E.over_c_squared * gr * ri * ri, ga = 3.5 * E.over_c_squared * gr;
-        const double fac = v2 - 4.0 * (gr + up) - ut + 2.0 * w2 - 4.0 * vw - 1.5 * (dw * ri) * (dw * ri) - 0.5 * da;
-        ax += -pre * fac * d[0] + pre * g * (v[0] - S.sv[0][lane]) + ga * af[0];
-        ay += -pre * fac * d[1] + pre * g * (v[1] - S.sv[1][lane]) + ga * af[1];
-        az += -pre * fac * d[2] + pre * g * (v[2] - S.sv[2][lane]) + ga * af[2];
     }
     a[0] += ax; a[1] += ay; a[2] += az;
 }
@@ -413,7 +425,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
                     for (int m = 0; m < 3; m++) { af[m] = fmaf(-fa, a[m], af[m]); gp[m] = fmaf(fb, b[m], gp[m]); }
                 }
                 const bool far = !(big < 200.0f);
-                if (JAC) {
+                if (JAC && !far) {
                     const double x[3] = {S.xs[0][lane], S.xs[1][lane], S.xs[2][lane]};
                     const double v[3] = {S.vs[0][lane], S.vs[1][lane], S.vs[2][lane]};
                     const double w[3] = {S.sv[0][lane], S.sv[1][lane], S.sv[2][lane]};
@@ -422,8 +434,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
                     const double g[3] = {ag_f2d_int(gp[0]), ag_f2d_int(gp[1]), ag_f2d_int(gp[2])};
                     ag_fast_eih_jac(E, d, rsqrt(fma(d[0], d[0], fma(d[1], d[1], d[2] * d[2]))), v, w, aj, ag_f2d_int(ut),
                                    ag_f2d_int(up), g, ea, J);
-                    if (!far)
-                        for (int k = 0; k < 3; k++) s[k] = ag_f2_add(s[k], ag_f2_of(ea[k]));
+                    for (int k = 0; k < 3; k++) s[k] = ag_f2_add(s[k], ag_f2_of(ea[k]));
                 } else if (!far) {
                     const AgF2 d[3] = {ag_f2_add(xf[0], sp[0]), ag_f2_add(xf[1], sp[1]), ag_f2_add(xf[2], sp[2])};
                     const AgF2 v[3] = {S.vf[0][lane], S.vf[1][lane], S.vf[2][lane]};
