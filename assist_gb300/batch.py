@@ -239,6 +239,21 @@ def encounter_ratio_device(ephem: Ephem, t0, t_end, state, out=None, stream=None
     return out
 
 
+def deep_pass_device(ephem: Ephem, t0, t_end, state, out=None, stream=None):
+    """Whether each particle passes a planet deep inside its sphere of
+    influence over [t0, t_end] (torch CUDA uint8): the groups of such particles
+    stay on FP64 terms throughout in the default batched kernels."""
+    import torch
+    n = state.shape[0]
+    if out is None:
+        out = torch.empty(n, dtype=torch.uint8, device=state.device)
+    s = None if stream is None else c_void_p(stream.cuda_stream)
+    rc = clib.assist_gb300_deep_pass_device(byref(ephem), n, _ptr(t0), _ptr(t_end), _ptr(state), _ptr(out), s)
+    if rc != 0:
+        raise RuntimeError("assist_gb300_deep_pass_device failed (%d): %s" % (rc, last_error()))
+    return out
+
+
 def group_plan(t0, t_end, state, params=None, ratio=None, group_order: int = 0,
                gm_sun: float = 2.9591220828411951e-04):
     """The grouped kernels' grouping on host arrays: (order, groups) with

@@ -604,19 +604,57 @@ struct BatchScratch {
     double* d_ws = nullptr;
     size_t ws_cap = 0;
     int order_cap = 0;
-    float* d_ratio = nullptr;       /* pilot: encounter cost ratio per particle */
-    int ratio_cap = 0;
-    float4* d_grid = nullptr;       /* pilot: body positions on the time grid */
-    float2* d_sunv = nullptr;
+    AgPilotBuf pilot = {};          /* ratio_cap particles, dgrid_cap samples */
+    int ratio_cap = 0, dgrid_cap = 0;
     double* h_in = nullptr;         /* pinned: t0, t_end, states, parameters read back for grouping */
     size_t h_in_cap = 0;
     float* h_ratio = nullptr;       /* pinned: the pilot's ratios, then its deep-pass flags */
-    unsigned char* d_deep = nullptr;
-    int h_ratio_cap = 0;
 };
-#define AG_PILOT_G 1024
 static std::mutex g_batch_mu;
 static BatchScratch g_batch;
+
+/* The pilot over a batch of times tmin .. tmax, into g_batch's buffers (grown
+ * as needed) but for a ratio array of the caller's; flags too unless deep is
+ * false.  The caller holds g_batch_mu.  0 or an ASSIST status. */
+static int ag_pilot_run(const DevEphem& D, int n, const double* d_t0, const double* d_te, const double* d_state, double tmin,
+                        double tmax, float* ratio, bool deep, cudaStream_t s) {
+    AgPilotBuf& B = g_batch.pilot;
+    const int gd = deep ? ag_pilot_deep_samples(tmax - tmin) : 0;
+    if (g_batch.ratio_cap < n) {
+        if (B.ratio) cudaFree(B.ratio);
+        if (B.deep) cudaFree(B.deep);
+        if (B.list) cudaFree(B.list);
+        if (g_batch.h_ratio) cudaFreeHost(g_batch.h_ratio);
+        B.ratio = nullptr;
+        B.deep = nullptr;
+        B.list = nullptr;
+        g_batch.h_ratio = nullptr;
+        g_batch.ratio_cap = 0;
+        if (ag_cuda_check(cudaMalloc(&B.ratio, sizeof(float) * (size_t)n), "cudaMalloc(pilot)") ||
+            ag_cuda_check(cudaMalloc(&B.deep, (size_t)n), "cudaMalloc(pilot)") ||
+            ag_cuda_check(cudaMalloc(&B.list, sizeof(int) * ((size_t)n + 1)), "cudaMalloc(pilot)") ||
+            ag_cuda_check(cudaMallocHost(&g_batch.h_ratio, (sizeof(float) + 1) * (size_t)n), "cudaMallocHost(pilot)"))
+            return ASSIST_ERROR_EPHEM_FILE;
+        g_batch.ratio_cap = n;
+    }
+    if (!B.grid && ag_cuda_check(cudaMalloc(&B.grid, sizeof(float4) * AG_PILOT_G * 10), "cudaMalloc(pilot grid)"))
+        return ASSIST_ERROR_EPHEM_FILE;
+    if (!B.sunv && ag_cuda_check(cudaMalloc(&B.sunv, sizeof(float2) * AG_PILOT_G), "cudaMalloc(pilot grid)"))
+        return ASSIST_ERROR_EPHEM_FILE;
+    if (g_batch.dgrid_cap < gd) {
+        if (B.dgrid) cudaFree(B.dgrid);
+        B.dgrid = nullptr;
+        g_batch.dgrid_cap = 0;
+        if (ag_cuda_check(cudaMalloc(&B.dgrid, sizeof(float4) * 20 * (size_t)gd), "cudaMalloc(pilot grid)"))
+            return ASSIST_ERROR_EPHEM_FILE;
+        g_batch.dgrid_cap = gd;
+    }
+    AgPilotBuf C = B;
+    if (ratio) C.ratio = ratio;
+    if (!deep) C.deep = nullptr;
+    return ag_cuda_check((cudaError_t)ag_pilot_encounters(D, n, d_t0, d_te, d_state, tmin, tmax, C, s), "pilot kernels")
+               ? ASSIST_ERROR_EPHEM_FILE : ASSIST_SUCCESS;
+}
 
 static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_gb300_options* o, int n,
                               const double* d_t0, const double* d_t_end, double* d_state, const double* d_params,
@@ -984,9 +1022,9 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
     if (read_prm)
         for (int i = 0; i < n; i++)
             has_ng[(size_t)i] = prm[3 * (size_t)i] != 0.0 || prm[3 * (size_t)i + 1] != 0.0 || prm[3 * (size_t)i + 2] != 0.0;
-    /* close-encounter pilot (queue order of the groups only): it runs on the
-     * device while the host sorts the batch; its ratios are read before the
-     * group costs are formed */
+    /* close-encounter pilot (the groups' queue order, and which of them the
+     * FP64 kernel takes): it runs on the device while the host sorts the batch
+     * and is read before the group costs are formed */
     const float* enc = nullptr;
     unsigned char* deep = nullptr;      /* particles that pass deep inside a planet's sphere of influence */
     /* with variational particles: not the learned start, and all direct terms
@@ -1000,35 +1038,14 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
             tmin = std::min(tmin, std::min(t0[(size_t)i], te[(size_t)i]));
             tmax = std::max(tmax, std::max(t0[(size_t)i], te[(size_t)i]));
         }
-        if (g_batch.ratio_cap < n) {
-            if (g_batch.d_ratio) cudaFree(g_batch.d_ratio);
-            if (g_batch.d_deep) cudaFree(g_batch.d_deep);
-            if (g_batch.h_ratio) cudaFreeHost(g_batch.h_ratio);
-            g_batch.d_ratio = nullptr;
-            g_batch.d_deep = nullptr;
-            g_batch.h_ratio = nullptr;
-            g_batch.ratio_cap = 0;
-            if (ag_cuda_check(cudaMalloc(&g_batch.d_ratio, sizeof(float) * (size_t)n), "cudaMalloc(pilot)") ||
-                ag_cuda_check(cudaMalloc(&g_batch.d_deep, (size_t)n), "cudaMalloc(pilot)") ||
-                ag_cuda_check(cudaMallocHost(&g_batch.h_ratio, (sizeof(float) + 1) * (size_t)n), "cudaMallocHost(pilot)"))
-                return ASSIST_ERROR_EPHEM_FILE;
-            g_batch.ratio_cap = n;
-        }
-        if (!g_batch.d_grid &&
-            (ag_cuda_check(cudaMalloc(&g_batch.d_grid, sizeof(float4) * AG_PILOT_G * 10), "cudaMalloc(pilot grid)") ||
-             ag_cuda_check(cudaMalloc(&g_batch.d_sunv, sizeof(float2) * AG_PILOT_G), "cudaMalloc(pilot grid)")))
-            return ASSIST_ERROR_EPHEM_FILE;
-        if (ag_cuda_check((cudaError_t)ag_pilot_encounters(D, n, d_t0, d_t_end, d_state, tmin, tmax, g_batch.d_ratio,
-                                                           may_fast ? g_batch.d_deep : nullptr, g_batch.d_grid,
-                                                           g_batch.d_sunv, AG_PILOT_G, s),
-                          "pilot kernels") ||
-            ag_cuda_check(cudaMemcpyAsync(g_batch.h_ratio, g_batch.d_ratio, sizeof(float) * n, cudaMemcpyDeviceToHost, s),
+        if ((st = ag_pilot_run(D, n, d_t0, d_t_end, d_state, tmin, tmax, nullptr, may_fast, s))) return st;
+        if (ag_cuda_check(cudaMemcpyAsync(g_batch.h_ratio, g_batch.pilot.ratio, sizeof(float) * n, cudaMemcpyDeviceToHost, s),
                           "read pilot"))
             return ASSIST_ERROR_EPHEM_FILE;
         enc = g_batch.h_ratio;
         if (may_fast) {
             deep = reinterpret_cast<unsigned char*>(g_batch.h_ratio + g_batch.ratio_cap);
-            if (ag_cuda_check(cudaMemcpyAsync(deep, g_batch.d_deep, (size_t)n, cudaMemcpyDeviceToHost, s), "read pilot"))
+            if (ag_cuda_check(cudaMemcpyAsync(deep, g_batch.pilot.deep, (size_t)n, cudaMemcpyDeviceToHost, s), "read pilot"))
                 return ASSIST_ERROR_EPHEM_FILE;
         }
     }
@@ -1514,18 +1531,17 @@ extern "C" int assist_gb300_integrate_batch(const struct assist_ephem* e, const 
 /* FP64 FMA throughput of the current device in GFLOP/s (roofline denominator). */
 extern "C" double assist_gb300_fp64_peak_gflops(void) { return ag_fp64_probe_gflops(); }
 
-extern "C" int assist_gb300_encounter_ratio_device(const struct assist_ephem* e, int n, const double* d_t0,
-                                                   const double* d_t_end, const double* d_state, float* d_ratio,
-                                                   void* stream) {
-    if (n < 0 || (n > 0 && (!d_t0 || !d_t_end || !d_state || !d_ratio))) {
-        ag_set_error("encounter ratio: n must be >= 0 and every array given");
+/* The pilot on a batch of its own: into d_ratio, or (null) the deep-pass flags into d_deep. */
+static int ag_pilot_only(const struct assist_ephem* e, int n, const double* d_t0, const double* d_t_end, const double* d_state,
+                         float* d_ratio, unsigned char* d_deep, cudaStream_t s) {
+    if (n < 0 || (n > 0 && (!d_t0 || !d_t_end || !d_state || (!d_ratio && !d_deep)))) {
+        ag_set_error("encounter pilot: n must be >= 0 and every array given");
         return ASSIST_ERROR_N;
     }
     if (n == 0) return ASSIST_SUCCESS;
     DevEphem D;
     int st = ag_ephem_device(e, &D);
     if (st) return st;
-    cudaStream_t s = (cudaStream_t)stream;
     std::vector<double> t0((size_t)n), te((size_t)n);
     if (ag_cuda_check(cudaMemcpyAsync(t0.data(), d_t0, sizeof(double) * n, cudaMemcpyDeviceToHost, s), "read t0") ||
         ag_cuda_check(cudaMemcpyAsync(te.data(), d_t_end, sizeof(double) * n, cudaMemcpyDeviceToHost, s), "read t_end") ||
@@ -1537,16 +1553,30 @@ extern "C" int assist_gb300_encounter_ratio_device(const struct assist_ephem* e,
         tmax = std::max(tmax, std::max(t0[(size_t)i], te[(size_t)i]));
     }
     std::lock_guard<std::mutex> lk(g_batch_mu);
-    if (!g_batch.d_grid &&
-        (ag_cuda_check(cudaMalloc(&g_batch.d_grid, sizeof(float4) * AG_PILOT_G * 10), "cudaMalloc(pilot grid)") ||
-         ag_cuda_check(cudaMalloc(&g_batch.d_sunv, sizeof(float2) * AG_PILOT_G), "cudaMalloc(pilot grid)")))
-        return ASSIST_ERROR_EPHEM_FILE;
-    if (ag_cuda_check((cudaError_t)ag_pilot_encounters(D, n, d_t0, d_t_end, d_state, tmin, tmax, d_ratio, nullptr,
-                                                       g_batch.d_grid, g_batch.d_sunv, AG_PILOT_G, s),
-                      "pilot kernels") ||
+    if ((st = ag_pilot_run(D, n, d_t0, d_t_end, d_state, tmin, tmax, d_ratio, d_deep != nullptr, s))) return st;
+    if ((d_deep && ag_cuda_check(cudaMemcpyAsync(d_deep, g_batch.pilot.deep, (size_t)n, cudaMemcpyDeviceToDevice, s), "pilot flags")) ||
         ag_cuda_check(cudaStreamSynchronize(s), "pilot kernels"))
         return ASSIST_ERROR_EPHEM_FILE;
     return ASSIST_SUCCESS;
+}
+
+extern "C" int assist_gb300_encounter_ratio_device(const struct assist_ephem* e, int n, const double* d_t0,
+                                                   const double* d_t_end, const double* d_state, float* d_ratio,
+                                                   void* stream) {
+    if (n > 0 && !d_ratio) {
+        ag_set_error("encounter ratio: n must be >= 0 and every array given");
+        return ASSIST_ERROR_N;
+    }
+    return ag_pilot_only(e, n, d_t0, d_t_end, d_state, d_ratio, nullptr, (cudaStream_t)stream);
+}
+
+extern "C" int assist_gb300_deep_pass_device(const struct assist_ephem* e, int n, const double* d_t0, const double* d_t_end,
+                                             const double* d_state, unsigned char* d_deep, void* stream) {
+    if (n > 0 && !d_deep) {
+        ag_set_error("deep pass: n must be >= 0 and every array given");
+        return ASSIST_ERROR_N;
+    }
+    return ag_pilot_only(e, n, d_t0, d_t_end, d_state, nullptr, d_deep, (cudaStream_t)stream);
 }
 
 extern "C" int assist_gb300_group_plan(int n, const double* t0, const double* t_end, const double* state,

@@ -97,13 +97,22 @@ int ag_batch_max_slots(int nv, int tpb);
 int ag_group_max_slots(int nv);
 int ag_launch_group(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, cudaStream_t s);
 int ag_coop_max_slots(int nv, int occ, int stage, int warm, int pairs = 0);
-/* Per-particle encounter cost ratio (extra steps / base steps) from a
- * two-body pilot on a G-point time grid over [tmin, tmax] and, unless d_deep
- * is null, whether the particle passes deep inside a planet's sphere of
- * influence. */
+/* Device buffers of the encounter pilot (kernels_pilot.cu). */
+#define AG_PILOT_G 1024          /* samples of the ratio's two-body path */
+struct AgPilotBuf {
+    float* ratio;                /* [n] */
+    unsigned char* deep;         /* [n], or null: ratios only */
+    int* list;                   /* [n + 1] */
+    float4* grid;                /* [AG_PILOT_G][10] */
+    float2* sunv;                /* [AG_PILOT_G] */
+    float4* dgrid;               /* [ag_pilot_deep_samples][10][2] */
+};
+int ag_pilot_deep_samples(double span);
+/* Per-particle encounter cost ratio (extra steps / base steps) over the
+ * batch's times tmin .. tmax and, with buffers for it, whether the particle
+ * passes deep inside a planet's sphere of influence. */
 int ag_pilot_encounters(const DevEphem& E, int n, const double* d_t0, const double* d_te, const double* d_state,
-                        double tmin, double tmax, float* d_ratio, unsigned char* d_deep, float4* d_grid,
-                        float2* d_sunv, int G, cudaStream_t s);
+                        double tmin, double tmax, const AgPilotBuf& B, cudaStream_t s);
 /* pairs: with variational particles, the forces on pair terms (ag_fast_covers
  * and all direct terms on); 16: groups of at most that many particles */
 int ag_launch_coop(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int occ, int stage,

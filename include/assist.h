@@ -451,6 +451,14 @@ int assist_gb300_encounter_ratio_device(const struct assist_ephem* ephem, int n,
                                         const double* d_t_end, const double* d_state, float* d_ratio,
                                         void* stream);
 
+/* Whether each particle passes a planet deep inside its sphere of influence
+ * over [t0, t_end] (device arrays, d_deep receives n bytes, 0 or 1): the flag
+ * by which the default batched kernels keep a group on FP64 terms throughout.
+ * An FP32 path under the Sun and the planets; no counterpart in the
+ * reference. */
+int assist_gb300_deep_pass_device(const struct assist_ephem* ephem, int n, const double* d_t0, const double* d_t_end,
+                                  const double* d_state, unsigned char* d_deep, void* stream);
+
 /* The grouping of the grouped batched kernels, on host arrays and without
  * device work: order[n] receives the particles in key order, gstart[] and
  * gsize[] (room for n each) the groups of at most 32 consecutive entries of

@@ -1,0 +1,99 @@
+"""Particles that pass a planet deep inside its sphere of influence: the pilot
+flags them whatever the batch's span, and the groups that hold one keep FP64
+terms in every form of the batched call."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+T0 = 8000.0
+BODY = {"Venus": (2, 2.45e-6, 0.006), "Earth": (3, 3.0e-6, 0.006), "Mars": (5, 3.2e-7, 0.005), "Jupiter": (6, 9.55e-4, 0.004)}
+
+
+@pytest.fixture(scope="module")
+def files(tmp_path_factory):
+    from assist_gb300 import synth
+    return synth.write_ephemeris(str(tmp_path_factory.mktemp("deep")), seed=8, t_beg=T0 - 100.0, t_end=T0 + 31 * 365.25)
+
+
+def _path(O, t0, t1, state, tol=1e-11):
+    """A path under the Sun and the planets as points of mass (their places from
+    the oracle), by scipy's eighth-order Runge-Kutta."""
+    from scipy.integrate import solve_ivp
+
+    def f(t, y):
+        a = np.zeros(3)
+        for k in range(11):
+            _, b = O.body(k, t)
+            d = b[1:4] - y[:3]
+            a += b[0] * d / (d @ d) ** 1.5
+        return np.concatenate([y[3:], a])
+
+    return solve_ivp(f, (t0, t1), state, method="DOP853", rtol=tol, atol=1e-13).y[:, -1]
+
+
+def _flybys(files, share, when, seed):
+    """States at T0 of particles that pass each planet at `share` of its radius
+    of influence at the times `when`: from the pass backward.  Those whose path
+    back is no moderate ellipse are drawn again."""
+    from tests.oracle_py import Oracle
+    pl, ast, system = files
+    O = Oracle(pl, ast)
+    rng = np.random.default_rng(seed)
+    gms = 2.9591220828411951e-04
+    out, names = [], []
+    for name, (k, m, vinf) in BODY.items():
+        for t in when:
+            while True:
+                p, v = system.body(k, np.array(t))
+                s, sv = system.sun(np.array(t))
+                d = share * np.linalg.norm(p - s) * m ** (1.0 / 3.0)
+                u = rng.normal(size=3); u[2] *= 0.3; u /= np.linalg.norm(u)
+                w = np.cross(u, rng.normal(size=3)); w /= np.linalg.norm(w)
+                st = np.concatenate([p + d * u, v + np.sqrt(vinf ** 2 + 2.0 * m * gms / d) * w])
+                pre = _path(O, t, t - 60.0, st)
+                h = pre - np.concatenate(system.sun(np.array(t - 60.0)))
+                a = 1.0 / (2.0 / np.linalg.norm(h[:3]) - h[3:] @ h[3:] / gms)
+                e = np.linalg.norm(np.cross(h[3:], np.cross(h[:3], h[3:])) / gms - h[:3] / np.linalg.norm(h[:3]))
+                if 0.0 < a < 20.0 and e < 0.7:
+                    break
+            out.append(_path(O, t - 60.0, T0, pre))
+            names.append((name, t))
+    return np.array(out), names
+
+
+def _flags(eph, t0, te, state):
+    import torch
+    from assist_gb300 import batch
+    dev = lambda a: torch.tensor(a, device="cuda")  # noqa: E731
+    return batch.deep_pass_device(eph, dev(t0), dev(te), dev(state)).cpu().numpy()
+
+
+@pytest.mark.parametrize("years", [1, 8, 30])
+def test_deep_passes_are_flagged_whatever_the_span(files, years):
+    """Passes at 0.02 of the radius of influence are flagged in batches of one
+    to thirty years, early and late in them, in a short span inside a long
+    batch too; a main belt is not, but for its few with such a pass."""
+    from assist_gb300 import Ephem, synth
+    pl, ast, system = files
+    eph = Ephem(pl, ast)
+    span = years * 365.25
+    fly, names = _flybys(files, 0.02, T0 + span * np.array([0.3, 0.62, 0.95]), 10 + years)
+    pop = synth.population(system, "mba", 2000, seed=years, t0=T0)
+    state = np.concatenate([fly, pop.state])
+    t0 = np.full(len(state), T0)
+    flags = _flags(eph, t0, np.full(len(state), T0 + span), state)
+    assert [x for x, f in zip(names, flags) if not f] == []
+    assert flags[len(fly):].mean() < 0.01
+    # the same passes in spans that end a day after them, inside the long batch
+    te = np.full(len(state), T0 + span)
+    te[:len(fly)] = [t + 1.0 for _, t in names]
+    flags = _flags(eph, t0, te, state)
+    assert [x for x, f in zip(names, flags) if not f] == []
+    # and spans of a day around each pass, backward, between the samples of the long one
+    from tests.oracle_py import Oracle
+    O = Oracle(pl, ast)
+    late = np.array([_path(O, T0, t + 0.5, f) for f, (_, t) in zip(fly, names)])
+    t = np.array([t for _, t in names])
+    flags = _flags(eph, np.concatenate([t + 0.5, t0[:5]]), np.concatenate([t - 0.5, te[-5:]]), np.concatenate([late, pop.state[:5]]))
+    assert [x for x, f in zip(names, flags) if not f] == []
