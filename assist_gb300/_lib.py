@@ -121,6 +121,8 @@ clib.assist_gb300_encounter_ratio_device.argtypes = [c_void_p, c_int, c_void_p, 
 clib.assist_gb300_encounter_ratio_device.restype = c_int
 clib.assist_gb300_deep_pass_device.argtypes = [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]
 clib.assist_gb300_deep_pass_device.restype = c_int
+clib.assist_gb300_last_deep_groups.argtypes = []
+clib.assist_gb300_last_deep_groups.restype = c_int
 clib.assist_gb300_group_plan.argtypes = [c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_double,
                                          c_void_p, c_void_p, c_void_p, POINTER(c_int)]
 clib.assist_gb300_group_plan.restype = c_int

@@ -254,6 +254,12 @@ def deep_pass_device(ephem: Ephem, t0, t_end, state, out=None, stream=None):
     return out
 
 
+def last_deep_groups() -> int:
+    """Groups of the last batch formed (a batched call or a plan) that run on
+    FP64 terms throughout because a member passes a planet deep."""
+    return int(clib.assist_gb300_last_deep_groups())
+
+
 def group_plan(t0, t_end, state, params=None, ratio=None, group_order: int = 0,
                gm_sun: float = 2.9591220828411951e-04):
     """The grouped kernels' grouping on host arrays: (order, groups) with

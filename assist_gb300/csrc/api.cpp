@@ -606,6 +606,7 @@ struct BatchScratch {
     int order_cap = 0;
     AgPilotBuf pilot = {};          /* ratio_cap particles, dgrid_cap samples */
     int ratio_cap = 0, dgrid_cap = 0;
+    int last_deep = 0;              /* groups with a deep pass in the last batch formed */
     double* h_in = nullptr;         /* pinned: t0, t_end, states, parameters read back for grouping */
     size_t h_in_cap = 0;
     float* h_ratio = nullptr;       /* pinned: the pilot's ratios, then its deep-pass flags */
@@ -1115,9 +1116,10 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
             occ = (int)gstart.size() <= 4 * sms ? 1 : 2;
         }
         P.fast = may_fast && !(n_var && P.learned);
-        if (P.fast && !P.learned) {
+        if (P.fast) {
             /* groups with a deep pass first in the list: the kernel with all
-             * terms in FP64 takes them */
+             * terms in FP64 takes them (its learned build those of a learned
+             * or logged batch) */
             std::vector<int> s2, z2;
             for (int pass = 0; pass < 2; pass++) {
                 for (size_t k = 0; k < gstart.size(); k++) {
@@ -1130,7 +1132,7 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
             gstart.swap(s2);
             gsize.swap(z2);
             const int need = 32 * P.n_deep;
-            P.deep_slots = ag_coop_max_slots(n_var, n_var ? occ : 2, 0, 0);
+            P.deep_slots = ag_coop_max_slots(n_var, n_var ? occ : 2, 0, P.learned ? 1 : 0);
             if (P.deep_slots > need) P.deep_slots = need;
         }
         if (P.fast && n_var) {
@@ -1176,6 +1178,7 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
         nslots = ag_batch_max_slots(n_var, tpb);
         if (nslots > n) nslots = n;
     }
+    g_batch.last_deep = P.n_deep;
     P.D = D;
     P.c = c;
     P.order.swap(order);
@@ -1577,6 +1580,11 @@ extern "C" int assist_gb300_deep_pass_device(const struct assist_ephem* e, int n
         return ASSIST_ERROR_N;
     }
     return ag_pilot_only(e, n, d_t0, d_t_end, d_state, nullptr, d_deep, (cudaStream_t)stream);
+}
+
+extern "C" int assist_gb300_last_deep_groups(void) {
+    std::lock_guard<std::mutex> lk(g_batch_mu);
+    return g_batch.last_deep;
 }
 
 extern "C" int assist_gb300_group_plan(int n, const double* t0, const double* t_end, const double* state,

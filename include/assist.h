@@ -459,6 +459,10 @@ int assist_gb300_encounter_ratio_device(const struct assist_ephem* ephem, int n,
 int assist_gb300_deep_pass_device(const struct assist_ephem* ephem, int n, const double* d_t0, const double* d_t_end,
                                   const double* d_state, unsigned char* d_deep, void* stream);
 
+/* How many groups of the last batch formed in this process (a batched call or
+ * a plan) hold such a particle and run on FP64 terms throughout. */
+int assist_gb300_last_deep_groups(void);
+
 /* The grouping of the grouped batched kernels, on host arrays and without
  * device work: order[n] receives the particles in key order, gstart[] and
  * gsize[] (room for n each) the groups of at most 32 consecutive entries of

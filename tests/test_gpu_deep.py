@@ -97,3 +97,47 @@ def test_deep_passes_are_flagged_whatever_the_span(files, years):
     t = np.array([t for _, t in names])
     flags = _flags(eph, np.concatenate([t + 0.5, t0[:5]]), np.concatenate([t - 0.5, te[-5:]]), np.concatenate([late, pop.state[:5]]))
     assert [x for x, f in zip(names, flags) if not f] == []
+
+
+def _mixed(files, n, n_fly, days, seed):
+    """n main-belt particles and n_fly unbound flybys of Jupiter at about 0.02
+    AU (0.04 of its radius of influence)."""
+    from assist_gb300 import synth
+    pl, ast, system = files
+    pop = synth.population(system, "mba", max(n, 1), seed=seed, t0=T0)
+    jp, jv = system.body(6, np.array(T0))
+    fly = [np.concatenate([jp + 0.3 * np.eye(3)[k % 3] + 0.02 * np.eye(3)[(k + 1) % 3], jv - 0.02 * np.eye(3)[k % 3]])
+           for k in range(n_fly)]
+    state = np.concatenate([pop.state[:n], np.array(fly).reshape(-1, 6)])
+    return state, np.full(len(state), T0), np.full(len(state), T0 + days)
+
+
+@pytest.mark.parametrize("how", ["log", "warm"])
+def test_learned_and_logged_batches_keep_deep_groups_apart(files, how):
+    """With the learned start or the logging of its pairs, too, groups with a
+    deep pass are the FP64 kernel's, and every particle ends where the oracle
+    puts it."""
+    import torch
+    from assist_gb300 import Ephem, batch, warm
+    from assist_gb300._lib import clib
+    from tests.oracle_py import Oracle
+    pl, ast, _ = files
+    state, t0, te = _mixed(files, 200, 5, 100.0, 4)
+    dev = lambda a: torch.tensor(a, device="cuda")  # noqa: E731
+    st, status = dev(state), torch.full((len(state),), -1, dtype=torch.int32, device="cuda")
+    warm.set_params(np.zeros(warm.n_params()))          # a correction of nothing
+    x, t = torch.zeros((4096, 32), device="cuda"), torch.zeros((4096, 21), device="cuda")
+    try:
+        if how == "log":
+            assert clib.assist_gb300_warm_set_log(x.data_ptr(), t.data_ptr(), 4096, 1) == 0
+        batch.integrate_batch_device(Ephem(pl, ast), dev(t0), dev(te), st, status=status,
+                                     opts=batch.options(warm_start=2 if how == "warm" else 0))
+        torch.cuda.synchronize()
+        assert batch.last_deep_groups() > 0
+        assert how == "warm" or clib.assist_gb300_warm_log_count() > 0
+    finally:
+        clib.assist_gb300_warm_set_log(None, None, 0, 1)
+    assert (status.cpu().numpy() == 0).all()
+    ref = Oracle(pl, ast).integrate_batch(t0, te, state)
+    d = np.abs(st.cpu().numpy()[:, :3] - ref[:, :3]).max(axis=1)
+    assert d[:200].max() < 1e-12 and d.max() < 1e-9, (d[:200].max(), d.max())
