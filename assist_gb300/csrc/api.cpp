@@ -1198,10 +1198,32 @@ static size_t ag_plan_ws_doubles(const AgLaunchPlan& P, int n_var) {
     return ag_batch_ws_doubles(P.nslots, n_var) + (P.fast && n_var ? ag_batch_ws_doubles(P.deep_slots, n_var) : 0);
 }
 
+/* The stream that a launch plan with groups on both kernels forks, and its two
+ * events.  A captured launch's live until the capture has ended. */
+struct AgFork {
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    int make() {
+        int e = (int)cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
+        if (!e) e = (int)cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+        if (!e) e = (int)cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
+        return e;
+    }
+    AgFork() = default;
+    AgFork(const AgFork&) = delete;
+    AgFork& operator=(const AgFork&) = delete;
+    ~AgFork() {
+        if (fork) cudaEventDestroy(fork);
+        if (join) cudaEventDestroy(join);
+        if (side) cudaStreamDestroy(side);
+    }
+};
+
 /* The batched kernels of a launch plan on stream s.  With groups on both
- * kernels the pair-term one runs on a stream forked from s and joined again;
- * a.queue holds two counters then. */
-static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var, cudaStream_t s) {
+ * kernels the pair-term one runs on a stream forked from s and joined again
+ * (F, made by the caller); a.queue holds two counters then. */
+static bool ag_plan_forks(const AgLaunchPlan& P) { return P.fast && P.n_deep && (int)P.gstart.size() > P.n_deep; }
+static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var, cudaStream_t s, const AgFork& F) {
     if (!P.fast)
         return P.coop ? ag_launch_coop(P.D, P.c, a, n_var, P.occ, P.stage, s)
                       : (P.grouped ? ag_launch_group(P.D, P.c, a, n_var, s) : ag_launch_batch(P.D, P.c, a, n_var, P.tpb, s));
@@ -1219,13 +1241,8 @@ static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var
     d.queue = a.queue + 1;
     if (n_var) d.ws = a.ws + ag_batch_ws_doubles(P.nslots, n_var);
     if (!f.n_groups) return ag_launch_coop(P.D, P.c, d, n_var, n_var ? P.occ : 2, 0, s);
-    cudaStream_t side = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    int e = (int)cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking);
-    if (!e) e = (int)cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
-    if (!e) e = (int)cudaEventCreateWithFlags(&join, cudaEventDisableTiming);
-    if (!e) e = (int)cudaEventRecord(fork, s);
-    if (!e) e = (int)cudaStreamWaitEvent(side, fork, 0);
+    int e = (int)cudaEventRecord(F.fork, s);
+    if (!e) e = (int)cudaStreamWaitEvent(F.side, F.fork, 0);
     if (!e) {
         /* the longest groups start first, each with a multiprocessor to itself
          * while they are few (alone the longest of 7 takes 65 ms, beside the
@@ -1235,13 +1252,10 @@ static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         e = ag_launch_coop(P.D, P.c, d, n_var, n_var ? P.occ : (8 * P.n_deep <= sms ? 1 : 2), 0, s);
-        if (!e) e = fast(side);
-        const int j = (int)cudaEventRecord(join, side), w = (int)cudaStreamWaitEvent(s, join, 0);
+        if (!e) e = fast(F.side);
+        const int j = (int)cudaEventRecord(F.join, F.side), w = (int)cudaStreamWaitEvent(s, F.join, 0);
         if (!e) e = j ? j : w;
     }
-    if (fork) cudaEventDestroy(fork);
-    if (join) cudaEventDestroy(join);
-    if (side) cudaStreamDestroy(side);
     return e;
 }
 
@@ -1324,7 +1338,9 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0); cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    const int le = ag_launch_plan(P, a, n_var, s);
+    AgFork fork;
+    int le = ag_plan_forks(P) ? fork.make() : 0;
+    if (!le) le = ag_launch_plan(P, a, n_var, s, fork);
     cudaEventRecord(e1, s);
     if (le) { cudaEventDestroy(e0); cudaEventDestroy(e1); ag_cuda_check((cudaError_t)le, "batch kernel launch"); return ASSIST_ERROR_EPHEM_FILE; }
     if (stats) {
@@ -1350,8 +1366,8 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
  * A batch integrated again and again with the same particles' times and
  * grouping (new initial states written into the same device arrays between
  * launches: clones of an orbit, Monte Carlo samples, restarts): the host
- * work of a call (read-back, encounter pilot, sort, upload) is done once, and
- * each launch replays a CUDA graph of the device work (queue and counter
+ * work of a call (read-back, encounter pilot, sort, upload; so also which
+ * groups are the FP64 kernel's) is done once, and each launch replays a CUDA graph of the device work (queue and counter
  * reset, the persistent kernel, the counters' copy to pinned host memory). */
 struct assist_gb300_plan {
     int n = 0;
@@ -1444,12 +1460,13 @@ extern "C" int assist_gb300_plan_create(const struct assist_ephem* e, const stru
         assist_gb300_plan_free(p);
         return ASSIST_ERROR_EPHEM_FILE;
     }
-    int le = 0;
-    ok = !ag_cuda_check(cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed), "plan capture");
+    AgFork fork;
+    int le = ag_plan_forks(P) ? fork.make() : 0;
+    ok = !le && !ag_cuda_check(cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed), "plan capture");
     if (ok) {
         cudaMemsetAsync(p->d_queue, 0, 2 * sizeof(int), cs);
         cudaMemsetAsync(p->d_counters, 0, 8 * sizeof(unsigned long long) + AG_SM_SLOTS * sizeof(int), cs);
-        le = ag_launch_plan(P, a, n_var, cs);
+        le = ag_launch_plan(P, a, n_var, cs, fork);
         cudaMemcpyAsync(p->h_counters, p->d_counters, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, cs);
         const cudaError_t ce = cudaStreamEndCapture(cs, &p->graph);
         ok = !le && !ag_cuda_check(ce, "plan capture") &&

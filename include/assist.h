@@ -341,7 +341,11 @@ int assist_gb300_integrate_batch_device_static(const struct assist_ephem* ephem,
  * (and times, if they keep the grouping's meaning) into them between
  * launches.  A replay gives the result of a direct call whose grouping is
  * the plan's (bit for bit when the inputs are the ones the plan was made
- * from).  No dense output or pair logging.  assist_gb300_plan_stats waits
+ * from).  The grouping includes which groups run on FP64 terms throughout
+ * (assist_gb300_deep_pass_device): it is that of the states the plan was made
+ * from, and a later state that passes a planet deep in another group is
+ * integrated on the default terms; make a new plan for states whose
+ * encounters differ.  No dense output or pair logging.  assist_gb300_plan_stats waits
  * for the last launch and returns its counters (kernel_ms -1: time launches
  * with events on their stream).  A plan belongs to the device that was
  * current at its creation. */

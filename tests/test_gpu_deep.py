@@ -141,3 +141,63 @@ def test_learned_and_logged_batches_keep_deep_groups_apart(files, how):
     ref = Oracle(pl, ast).integrate_batch(t0, te, state)
     d = np.abs(st.cpu().numpy()[:, :3] - ref[:, :3]).max(axis=1)
     assert d[:200].max() < 1e-12 and d.max() < 1e-9, (d[:200].max(), d.max())
+
+
+@pytest.mark.parametrize("n,n_fly,nv,dense", [(300, 5, 0, False), (0, 5, 0, False), (300, 5, 6, False), (0, 40, 6, False),
+                                              (300, 5, 0, True)])
+def test_split_batches_and_their_plans(files, n, n_fly, nv, dense):
+    """Batches of which some groups or all hold a deep pass, with and without
+    variational particles: against the oracle; a plan's replays have the direct
+    call's bits, and so has a direct call again; dense output ends in the end
+    states."""
+    import torch
+    from assist_gb300 import Ephem, batch
+    from tests.oracle_py import Oracle
+    pl, ast, _ = files
+    eph = Ephem(pl, ast)
+    state, t0, te = _mixed(files, n, n_fly, 100.0, 5)
+    m = len(state)
+    dev = lambda a: torch.tensor(a, device="cuda")  # noqa: E731
+    flags = _flags(eph, t0, te, state)
+    assert flags[n:].all() and not flags[:n].any()
+    _, groups = batch.group_plan(t0, te, state)
+    var = np.tile(np.eye(6)[None], (m, 1, 1)) if nv else None
+    got = []
+    for _ in range(2):
+        st, vs = dev(state), dev(var) if nv else None
+        status = torch.full((m,), -1, dtype=torch.int32, device="cuda")
+        if dense:
+            out = torch.empty((2 * m, 6), dtype=torch.float64, device="cuda")
+            batch.integrate_batch_dense_device(eph, dev(t0), dev(te), st, torch.arange(0, 2 * m + 1, 2, dtype=torch.int32, device="cuda"),
+                                               dev(np.tile([T0 + 50.0, T0 + 100.0], m)), out, status=status)
+            assert torch.equal(out[1::2], st)
+        else:
+            batch.integrate_batch_device(eph, dev(t0), dev(te), st, var_state=vs, status=status)
+        deep = batch.last_deep_groups()
+        assert deep == sum(flags[g].any() for g in groups) and (deep == len(groups)) == (n == 0)
+        assert (status.cpu().numpy() == 0).all()
+        got.append((st, vs))
+    assert torch.equal(got[0][0], got[1][0]) and (not nv or torch.equal(got[0][1], got[1][1]))
+    ref = Oracle(pl, ast).integrate_batch(t0, te, state, var_state=var, return_all=True)
+    d = np.abs(got[0][0].cpu().numpy()[:, :3] - ref[0][:, :3]).max(axis=1)
+    assert d.max() < 1e-9 and (n == 0 or d[:n].max() < 1e-12), d.max()
+    if nv:
+        rel = np.abs(got[0][1].cpu().numpy() - ref[1]).max(axis=(1, 2)) / np.abs(ref[1]).max(axis=(1, 2))
+        assert rel.max() < 1e-6, rel.max()
+    if dense:
+        return
+    # a plan over the same particles
+    a, b = dev(t0), dev(te)
+    st, vs = dev(state), dev(var) if nv else None
+    status = torch.full((m,), -1, dtype=torch.int32, device="cuda")
+    plan = batch.Plan(eph, a, b, st, var_state=vs, status=status)
+    assert batch.last_deep_groups() == deep
+    for _ in range(3):
+        st.copy_(dev(state))
+        if nv:
+            vs.copy_(dev(var))
+        plan.launch()
+        plan.stats()
+        assert (status.cpu().numpy() == 0).all()
+        assert torch.equal(st, got[0][0]) and (not nv or torch.equal(vs, got[0][1]))
+    plan.close()
