@@ -574,8 +574,13 @@ extern "C" int assist_gb300_forces_device(const struct assist_ephem* e, const st
     int st = ag_ephem_device(e, &D);
     if (st) return st;
     const ForceCfg c = make_cfg(o->forces, o->gr_eih_sources, o->geocentric, o->alpha, o->nk, o->nm, o->nn, o->r0);
-    if (ag_cuda_check((cudaError_t)ag_launch_forces_each(D, c, n, d_t, d_state, d_params, n_var, d_var_state, d_acc,
-                                                         d_var_acc, d_status, (cudaStream_t)stream), "force kernel"))
+    cudaStream_t s = (cudaStream_t)stream;
+    const float2 *pl = nullptr, *spk = nullptr;
+    int le;
+    if (n > 0 && ag_forces_own_covers(D, c, n_var) && ag_ephem_pairs(e, s, &pl, &spk))
+        le = ag_launch_forces_own(D, pl, spk, c, n, d_t, d_state, d_params, n_var, d_var_state, d_acc, d_var_acc, d_status, s);
+    else le = ag_launch_forces_each(D, c, n, d_t, d_state, d_params, n_var, d_var_state, d_acc, d_var_acc, d_status, s);
+    if (ag_cuda_check((cudaError_t)le, "force kernel"))
         return ASSIST_ERROR_EPHEM_FILE;
     return ASSIST_SUCCESS;
 }

@@ -87,8 +87,6 @@ struct DevEphem {
     int n_ast;
     const double* spk;           /* the whole SPK file as doubles */
     long long spk_ndbl;
-    const float2* pl_pair;       /* pl_data and spk as float pairs (hi, lo) */
-    const float2* spk_pair;
     double ast_beg_max, ast_end_min;             /* the span every asteroid covers */
     double ast_beg[AG_MAX_AST], ast_end[AG_MAX_AST], ast_res[AG_MAX_AST], ast_gm[AG_MAX_AST];
     float ast_gm_hi[AG_MAX_AST], ast_gm_lo[AG_MAX_AST];   /* ast_gm as a float pair hi + lo */

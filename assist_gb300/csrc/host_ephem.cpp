@@ -25,6 +25,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <fcntl.h>
+#include <mutex>
 #include <string>
 #include <unistd.h>
 #include <vector>
@@ -45,7 +46,7 @@ struct ascii_s {
     double mass[ASSIST_BODY_NPLANETS];
     double J2E, J3E, J4E, J2SUN, AU, RE, CLIGHT, ASUN;
     double* d_data = nullptr;
-    float2* d_pair = nullptr;        /* d_data as float pairs */
+    float2* d_pair = nullptr;        /* d_data as float pairs (ag_ephem_pairs) */
     DevEphem* d_view = nullptr;      /* device copy of the last view handed to kernels */
     DevEphem h_view;                 /* host copy of *d_view */
     bool find(const char* name, double* out) const {
@@ -71,7 +72,7 @@ struct spk_s {
     std::vector<int> seg0;
     std::string comments;            /* comment area, NUL -> newline */
     double* d_data = nullptr;
-    float2* d_pair = nullptr;        /* asteroid files: d_data as float pairs */
+    float2* d_pair = nullptr;        /* asteroid files: d_data as float pairs (ag_ephem_pairs) */
     AgSpkSeg* d_segs = nullptr;
     AgRecMeta* d_meta = nullptr;
     DevEphem* d_view = nullptr;      /* planets files: device copy of the last view */
@@ -200,14 +201,6 @@ static ascii_s* ascii_load(const char* path) {
     return a;
 }
 
-/* The float-pair image of n doubles on the device (complete on return: the
- * kernels that read it run on streams of their own). */
-static bool pair_upload(const double* d, float2** out, size_t n) {
-    return !ag_cuda_check(cudaMalloc(out, n * sizeof(float2) + 64), "cudaMalloc(float-pair image)") &&
-           !ag_cuda_check((cudaError_t)ag_launch_pair_image(d, *out, n), "float-pair image") &&
-           !ag_cuda_check(cudaStreamSynchronize(0), "float-pair image");
-}
-
 /* The device copy of the .440 image, made on first device use (loading and
  * validating a file is host work only). */
 static int ascii_upload(ascii_s* a) {
@@ -215,12 +208,9 @@ static int ascii_upload(ascii_s* a) {
     /* 64 bytes of padding: a record staged by a bulk copy is read from its
      * address rounded down to 16 bytes, for its length rounded up */
     if (ag_cuda_check(cudaMalloc(&a->d_data, a->data.size() * 8 + 64), "cudaMalloc(.440 records)") ||
-        ag_cuda_check(cudaMemcpy(a->d_data, a->data.data(), a->data.size() * 8, cudaMemcpyHostToDevice), "upload .440") ||
-        !pair_upload(a->d_data, &a->d_pair, a->data.size())) {
+        ag_cuda_check(cudaMemcpy(a->d_data, a->data.data(), a->data.size() * 8, cudaMemcpyHostToDevice), "upload .440")) {
         if (a->d_data) cudaFree(a->d_data);
-        if (a->d_pair) cudaFree(a->d_pair);
         a->d_data = nullptr;
-        a->d_pair = nullptr;
         return ASSIST_ERROR_EPHEM_FILE;
     }
     return 0;
@@ -318,19 +308,16 @@ static spk_s* spk_load(const char* path) {
 
 /* The device copies of an SPK image, its segment table and record metadata,
  * made on first device use. */
-static int spk_upload(spk_s* s, bool pair) {
+static int spk_upload(spk_s* s) {
     if (s->d_data) return 0;
     bool ok = !ag_cuda_check(cudaMalloc(&s->d_data, s->data.size() * 8), "cudaMalloc(SPK)") &&
               !ag_cuda_check(cudaMemcpy(s->d_data, s->data.data(), s->data.size() * 8, cudaMemcpyHostToDevice), "upload SPK") &&
               !ag_cuda_check(cudaMalloc(&s->d_segs, sizeof(AgSpkSeg) * (s->segs.size() + 1)), "cudaMalloc(SPK segments)") &&
               !ag_cuda_check(cudaMemcpy(s->d_segs, s->segs.data(), sizeof(AgSpkSeg) * s->segs.size(), cudaMemcpyHostToDevice), "upload segments") &&
               !ag_cuda_check(cudaMalloc(&s->d_meta, sizeof(AgRecMeta) * (s->meta.size() + 1)), "cudaMalloc(SPK records)") &&
-              !ag_cuda_check(cudaMemcpy(s->d_meta, s->meta.data(), sizeof(AgRecMeta) * s->meta.size(), cudaMemcpyHostToDevice), "upload records") &&
-              (!pair || pair_upload(s->d_data, &s->d_pair, s->data.size()));
+              !ag_cuda_check(cudaMemcpy(s->d_meta, s->meta.data(), sizeof(AgRecMeta) * s->meta.size(), cudaMemcpyHostToDevice), "upload records");
     if (!ok) {
         if (s->d_data) cudaFree(s->d_data);
-        if (s->d_pair) cudaFree(s->d_pair);
-        s->d_pair = nullptr;
         if (s->d_segs) cudaFree(s->d_segs);
         if (s->d_meta) cudaFree(s->d_meta);
         s->d_data = nullptr; s->d_segs = nullptr; s->d_meta = nullptr;
@@ -436,8 +423,8 @@ static void spk_planets_view(const struct assist_ephem* e, DevEphem& D) {
 
 int ag_ephem_device(const struct assist_ephem* e, DevEphem* out) {
     if (!e || (!e->ascii_planets && !e->spk_planets)) return ASSIST_ERROR_EPHEM_FILE;
-    if ((e->spk_planets && spk_upload(e->spk_planets, false)) || (e->ascii_planets && ascii_upload(e->ascii_planets)) ||
-        (e->spk_asteroids && spk_upload(e->spk_asteroids, true)))
+    if ((e->spk_planets && spk_upload(e->spk_planets)) || (e->ascii_planets && ascii_upload(e->ascii_planets)) ||
+        (e->spk_asteroids && spk_upload(e->spk_asteroids)))
         return ASSIST_ERROR_EPHEM_FILE;
     DevEphem D;
     std::memset(&D, 0, sizeof(D));
@@ -450,7 +437,6 @@ int ag_ephem_device(const struct assist_ephem* e, DevEphem* out) {
 /* The planets part of the view for a .440/.441 file. */
 static void ag_ascii_view(const ascii_s* a, DevEphem& D) {
     D.pl_data = a->d_data;
-    D.pl_pair = a->d_pair;
     D.pl_ndbl = (long long)a->data.size();
     D.pl_rec_len = (int)a->rec;
     D.pl_nrec = (int)(a->data.size() / a->rec);
@@ -514,7 +500,6 @@ static int ag_finish_view(const struct assist_ephem* e, DevEphem& D, DevEphem* o
         if ((int)s->targets.size() > AG_MAX_AST) return ASSIST_ERROR_NAST;
         D.n_ast = (int)s->targets.size();
         D.spk = s->d_data;
-        D.spk_pair = s->d_pair;
         D.spk_ndbl = (long long)s->data.size();
         D.segs = s->d_segs;
         D.rec_meta = s->d_meta;
@@ -565,6 +550,45 @@ static int ag_finish_view(const struct assist_ephem* e, DevEphem& D, DevEphem* o
     }
     *out = D;
     return ASSIST_SUCCESS;
+}
+
+/* The float-pair image of n doubles on the device, complete on return (the
+ * kernels that read it run on streams of their own), or null. */
+static float2* pair_image(const double* d, size_t n) {
+    float2* p = nullptr;
+    cudaStream_t st = nullptr;
+    bool ok = cudaMalloc(&p, n * sizeof(float2) + 64) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) == cudaSuccess && ag_launch_pair_image(d, p, n, st) == 0 &&
+              cudaStreamSynchronize(st) == cudaSuccess;
+    if (st) cudaStreamDestroy(st);
+    if (!ok) {
+        cudaGetLastError();
+        if (p) cudaFree(p);
+        p = nullptr;
+    }
+    return p;
+}
+
+bool ag_ephem_pairs(const struct assist_ephem* e, cudaStream_t s, const float2** pl, const float2** spk) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    ascii_s* a = e->ascii_planets;
+    spk_s* k = e->spk_asteroids;
+    if (!a || !a->d_data || (k && !k->d_data)) return false;
+    if (!a->d_pair || (k && !k->d_pair)) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+        if (cap != cudaStreamCaptureStatusNone) return false;
+        /* another thread's or stream's capture is left alone */
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (!a->d_pair) a->d_pair = pair_image(a->d_data, a->data.size());
+        if (k && !k->d_pair) k->d_pair = pair_image(k->d_data, k->data.size());
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    *pl = a->d_pair;
+    *spk = k ? k->d_pair : nullptr;
+    return a->d_pair && (!k || k->d_pair);
 }
 
 int ag_ephem_device_current(const struct assist_ephem* e, DevEphem* out) {

@@ -84,12 +84,13 @@ int ag_launch_forces_coop(const DevEphem& E, const ForceCfg& c, int n, double t,
 int ag_launch_forces_each(const DevEphem& E, const ForceCfg& c, int n, const double* t, const double* state,
                           const double* params, int nv, const double* var_state, double* acc, double* var_acc,
                           int* status, cudaStream_t s);
-/* the same for the configurations ag_forces_own_covers (kernels_own.cu) */
+/* the same for the configurations ag_forces_own_covers, with the float-pair
+ * images of the files (kernels_own.cu) */
 bool ag_forces_own_covers(const DevEphem& E, const ForceCfg& c, int nv);
-int ag_launch_forces_own(const DevEphem& E, const ForceCfg& c, int n, const double* t, const double* state,
-                         const double* params, int nv, const double* var_state, double* acc, double* var_acc, int* status,
-                         cudaStream_t s);
-int ag_launch_pair_image(const double* x, float2* out, size_t n);
+int ag_launch_forces_own(const DevEphem& E, const float2* pl_pair, const float2* spk_pair, const ForceCfg& c, int n,
+                         const double* t, const double* state, const double* params, int nv, const double* var_state,
+                         double* acc, double* var_acc, int* status, cudaStream_t s);
+int ag_launch_pair_image(const double* x, float2* out, size_t n, cudaStream_t s);
 int ag_launch_bodies(const DevEphem& E, int n, const double* t, double* out, int* status, cudaStream_t s);
 size_t ag_batch_ws_doubles(int nslots, int nv);
 int ag_launch_batch(const DevEphem& E, const ForceCfg& c, const AgBatchArgs& a, int nv, int tpb, cudaStream_t s);
@@ -141,6 +142,12 @@ int ag_ephem_device(const struct assist_ephem* e, DevEphem* out);
 /* The device view of an ephemeris that already has one matching its current
  * contents, without allocating or uploading anything (an error otherwise). */
 int ag_ephem_device_current(const struct assist_ephem* e, DevEphem* out);
+
+/* The float-pair images of an ephemeris's .440 and asteroid files (after
+ * ag_ephem_device), as large as the files again: made by the first own-time
+ * force call, which alone reads them.  False when they are not there and
+ * cannot be made now: s is being captured, or no memory is left. */
+bool ag_ephem_pairs(const struct assist_ephem* e, cudaStream_t s, const float2** pl, const float2** spk);
 
 /* 1 when the ephemeris's device view exists (ag_ephem_device will not allocate) */
 int ag_ephem_view_ready(const struct assist_ephem* e);

@@ -412,8 +412,6 @@ int ag_launch_forces_each(const DevEphem& E, const ForceCfg& c, int n, const dou
                           const double* params, int nv, const double* var_state, double* acc, double* var_acc,
                           int* status, cudaStream_t s) {
     if (n <= 0) return 0;
-    if (ag_forces_own_covers(E, c, nv))
-        return ag_launch_forces_own(E, c, n, t, state, params, nv, var_state, acc, var_acc, status, s);
     const int tpb = 128;
     const int blocks = (n + tpb - 1) / tpb;
     if (nv == 6) ag_k_forces_each<6><<<blocks, tpb, 0, s>>>(E.self_dev, c, n, t, state, params, var_state, acc, var_acc, status);

@@ -37,10 +37,10 @@ __global__ void ag_k_pair_image(const double* __restrict__ x, float2* __restrict
 }
 
 /* out[i] = x[i] as a float pair (hi, lo). */
-int ag_launch_pair_image(const double* x, float2* out, size_t n) {
+int ag_launch_pair_image(const double* x, float2* out, size_t n, cudaStream_t s) {
     if (n == 0) return 0;
     const size_t blocks = (n + 255) / 256;
-    ag_k_pair_image<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256>>>(x, out, n);
+    ag_k_pair_image<<<(unsigned)(blocks < 4096 ? blocks : 4096), 256, 0, s>>>(x, out, n);
     return (int)cudaGetLastError();
 }
 
@@ -91,12 +91,13 @@ __device__ __forceinline__ void ag_own_range(int packs, int w, int& p0, int& p1)
 }
 
 /* A .440 column as float pairs (km). */
-__device__ __forceinline__ void ag_own_column(const DevEphem& E, size_t rec, int col, double tf, AgF2* u) {
+__device__ __forceinline__ void ag_own_column(const DevEphem& E, const float2* __restrict__ pl_pair, size_t rec, int col, double tf,
+                                              AgF2* u) {
     const int ncf = E.col_ncf[col], niv = E.col_niv[col];
     const double tt = tf * (double)niv;
     double fl;
     const int b = ag_subinterval(tt, niv, &fl);
-    ag_cheb_pair(E.pl_pair + rec + E.col_off[col] + ncf * 3 * b, ncf, ag_f2_of(fma(2.0, tt - fl, -1.0)), u);
+    ag_cheb_pair(pl_pair + rec + E.col_off[col] + ncf * 3 * b, ncf, ag_f2_of(fma(2.0, tt - fl, -1.0)), u);
 }
 
 /* Bodies close to the particle, or all of them far out, in FP64 from the
@@ -187,7 +188,8 @@ static __device__ __noinline__ void ag_own_close(const DevEphem& E, const ForceC
 }
 
 template <bool JAC>
-__global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEphem* __restrict__ Ep, ForceCfg c, int n,
+__global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEphem* __restrict__ Ep, const float2* __restrict__ pl_pair,
+                                                                    const float2* __restrict__ spk_pair, ForceCfg c, int n,
                                                                     const double* __restrict__ t, const double* __restrict__ state,
                                                                     const double* __restrict__ params,
                                                                     const double* __restrict__ var_state, double* __restrict__ acc,
@@ -246,8 +248,8 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
             ag_planet_exact<false>(E, rec, tf, AG_JUP, b, nullptr);
             for (int m = 0; m < 3; m++) S.rj[m][lane] = 0.0 - b[m];
             AgF2 e[3], l[3], u[3];
-            ag_own_column(E, ro, AG_C_EMB, tf, e);
-            ag_own_column(E, ro, AG_C_LUN, tf, l);
+            ag_own_column(E, pl_pair, ro, AG_C_EMB, tf, e);
+            ag_own_column(E, pl_pair, ro, AG_C_LUN, tf, l);
             for (int m = 0; m < 3; m++) u[m] = ag_f2_add(e[m], ag_f2_mul(l[m], {E.pv.f_earth_h, E.pv.f_earth_l}));
             put(2, u);
             for (int m = 0; m < 3; m++) u[m] = ag_f2_add(e[m], ag_f2_mul(l[m], {E.pv.f_moon_h, E.pv.f_moon_l}));
@@ -258,7 +260,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
             for (int q = 0; q < 7; q++) {
                 AgF2 u[3];
                 const int k = q < 2 ? q : q + 2;
-                ag_own_column(E, ro, k < 2 ? k : (k == 4 ? AG_C_MAR : k), tf, u);
+                ag_own_column(E, pl_pair, ro, k < 2 ? k : (k == 4 ? AG_C_MAR : k), tf, u);
                 put(k, u);
             }
         }
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
                     mid = meta.x;
                     rad = meta.z;
                 }
-                ag_cheb_pair(E.spk_pair + sg.data_off + (size_t)bb * sg.R + 2, sg.P, z, u);
+                ag_cheb_pair(spk_pair + sg.data_off + (size_t)bb * sg.R + 2, sg.P, z, u);
             } else if (need) {
                 S.bad[lane] = AG_ERR_COVERAGE;
             }
@@ -557,9 +559,9 @@ bool ag_forces_own_covers(const DevEphem& E, const ForceCfg& c, int nv) {
     return !E.pl_spk && ag_fast_covers(c) && (nv == 0 || (c.forces & all) == all);
 }
 
-int ag_launch_forces_own(const DevEphem& E, const ForceCfg& c, int n, const double* t, const double* state,
-                         const double* params, int nv, const double* var_state, double* acc, double* var_acc, int* status,
-                         cudaStream_t s) {
+int ag_launch_forces_own(const DevEphem& E, const float2* pl_pair, const float2* spk_pair, const ForceCfg& c, int n,
+                         const double* t, const double* state, const double* params, int nv, const double* var_state,
+                         double* acc, double* var_acc, int* status, cudaStream_t s) {
     const int blocks = (n + 31) / 32;
     auto bytes = [](int n_ast) { return sizeof(AgF2) * 3 * 32 * (AG_PAIR_PL + (size_t)n_ast); };
     if (nv) {
@@ -567,9 +569,9 @@ int ag_launch_forces_own(const DevEphem& E, const ForceCfg& c, int n, const doub
         const cudaError_t e = cudaFuncSetAttribute(ag_k_forces_own<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)(bytes(AG_MAX_AST) + sizeof(AgOwnJac)));
         if (e != cudaSuccess) return (int)e;
-        ag_k_forces_own<true><<<blocks, 128, bytes(E.n_ast) + sizeof(AgOwnJac), s>>>(E.self_dev, c, n, t, state, params, var_state, acc, var_acc, status);
+        ag_k_forces_own<true><<<blocks, 128, bytes(E.n_ast) + sizeof(AgOwnJac), s>>>(E.self_dev, pl_pair, spk_pair, c, n, t, state, params, var_state, acc, var_acc, status);
     } else {
-        ag_k_forces_own<false><<<blocks, 128, bytes(E.n_ast), s>>>(E.self_dev, c, n, t, state, params, nullptr, acc, nullptr, status);
+        ag_k_forces_own<false><<<blocks, 128, bytes(E.n_ast), s>>>(E.self_dev, pl_pair, spk_pair, c, n, t, state, params, nullptr, acc, nullptr, status);
     }
     return (int)cudaGetLastError();
 }
