@@ -27,6 +27,7 @@ struct AgFastStep {
     double ah, aratio;                          /* the accepted (or rejected) step and the next one's size over it */
     unsigned live, fin, last;                   /* lanes integrating, to be retired, ending with this step */
     unsigned nf[3];                             /* lanes with a non-finite x, y, z */
+    unsigned conv;                              /* lanes whose corrector has converged (or that do not integrate) */
     int cmd;
 };
 
@@ -115,13 +116,26 @@ __device__ __forceinline__ double ag_max3(const double (*r)[32], int lane) {
     return ag_max_nonneg(ag_max_nonneg(r[0][lane], r[1][lane]), r[2][lane]);
 }
 
-/* maxdb / maxa as IAS15's convergence test reads it: compared with 1e-16 and
- * with the last iteration's, for which FP32 does (FP64 where FP32's range
- * ends). */
-__device__ __forceinline__ double ag_fast_pc_err(double maxdb, double maxa) {
-    const float a = ag_d2f_int(maxa), d = ag_d2f_int(maxdb);
-    if (a > 1e-18f && a < 1e18f && d < 1e18f) return ag_f2d_int(d / a);
-    return maxdb / maxa;
+/* IAS15's convergence test on the error e = maxdb / maxa (non-negative): below
+ * 1e-16, or no smaller than the last iteration's.  As products in FP64, one
+ * rounding like the quotients' (a division is 600 cycles of the one warp that
+ * judges, three products 200); the quotients where a product could leave the
+ * range.  db, a: the last iteration's measures, updated. */
+__device__ __forceinline__ bool ag_fast_converged(double maxdb, double maxa, int iters, double& db, double& a) {
+    /* in 2^-300 .. 2^300 */
+    auto mid = [](double x) { return ag_hi_word(x) - (723u << 20) < (600u << 20); };
+    bool below, stalled = false;
+    if (mid(maxa) && (iters == 1 || mid(a)) && ag_hi_word(maxdb) < (1323u << 20)) {
+        below = __double_as_longlong(maxdb) < __double_as_longlong(1e-16 * maxa);
+        if (iters > 2) stalled = __double_as_longlong(db * maxa) <= __double_as_longlong(maxdb * a);
+    } else {
+        const double e = maxdb / maxa;
+        below = e < 1e-16;
+        if (iters > 2) stalled = db / a <= e;
+    }
+    db = maxdb;
+    a = maxa;
+    return below || stalled || iters >= 12;
 }
 
 /* x^(-1/7): an FP32 estimate (1e-6) and two Newton steps

@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, OCC) ag_k_fast(const DevEphem
             __syncthreads();            /* a0 for the velocity predictor's warps */
             /* ---- predictor-corrector iterations */
             int iters = 1, it_lane = 0;
-            double pc_last = 1e300, ma7 = 0.0, mb6 = 0.0;
+            double last_db = 0.0, last_a = 0.0, ma7 = 0.0, mb6 = 0.0;
             bool conv = !live;
             while (true) {
                 for (int n = 1; n < 8; n++) {
@@ -315,15 +315,22 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, OCC) ag_k_fast(const DevEphem
                     if (!conv && pc >= 0) ag_fast_correct(W, S, pc, lane, n);
                     __syncthreads();
                 }
-                if (!conv) {
-                    ma7 = ag_max3(S.ra, lane);
-                    mb6 = ag_max3(S.rb6, lane);
-                    const double pc_err = ag_fast_pc_err(ag_max3(S.rdb, lane), ma7);
-                    conv = (pc_err < 1e-16) || (iters > 2 && pc_last <= pc_err) || (iters >= 12);
-                    if (conv) { it_lane = iters; if (ctl) n_it += (unsigned long long)iters; }
-                    else pc_last = pc_err;
+                if (ctl) {
+                    /* one warp judges */
+                    bool c = conv;
+                    if (!c) {
+                        ma7 = ag_max3(S.ra, lane);
+                        mb6 = ag_max3(S.rb6, lane);
+                        c = ag_fast_converged(ag_max3(S.rdb, lane), ma7, iters, last_db, last_a);
+                        if (c) n_it += (unsigned long long)iters;
+                    }
+                    const unsigned m = __ballot_sync(AG_FULL, c);
+                    if (lane == 0) S.conv = m;
                 }
-                if (__all_sync(AG_FULL, conv)) break;
+                __syncthreads();
+                const unsigned done = S.conv;
+                if (!conv && (done & bit)) { conv = true; it_lane = iters; }
+                if (done == 0xffffffffu) break;
                 iters++;
             }
             if (WARM && warm && live) {

@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* _
         if (live && pc >= 0) W(W_A0, pc) = ag_fast_sum(S.F, pc, lane);
         if (live) ag_fast_start(W, pc, hc);
         __syncthreads();            /* a0 for the velocity predictor's warps */
-        double pc_last = 1e300;
+        ShMeasure before = {0.0, 0.0};
         int iters = 1, cmd;
         while (true) {
             for (int n = 1; n < 8; n++) {
@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 1) sh_k_run(const DevEphem* _
                     round++;
                 }
                 gave_up = !ok;
-                cmd = sh_run_decide(A, K, S, ok, mdb, ma, mb, hstep, last, iters, pc_last, lane);
+                cmd = sh_run_decide(A, K, S, ok, mdb, ma, mb, hstep, last, iters, before, lane);
             }
             __syncthreads();
             cmd = S.cmd;

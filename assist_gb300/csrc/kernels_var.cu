@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 2) ag_k_var_run(const DevEphe
         __syncthreads();         /* the variational states at node 0 have been read */
         /* ---- predictor-corrector iterations */
         int iters = 1, cmd;
-        double pc_last = 1e300;
+        ShMeasure before = {0.0, 0.0};
         while (true) {
             for (int n = 1; n < 8; n++) {
                 predict(n);
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 2) ag_k_var_run(const DevEphe
                     round++;
                 }
                 gave_up = !ok;
-                sh_run_decide(R, K, S, ok, mdb, ma, mb, hstep, last, iters, pc_last, lane);
+                sh_run_decide(R, K, S, ok, mdb, ma, mb, hstep, last, iters, before, lane);
             }
             __syncthreads();
             cmd = S.cmd;

@@ -58,6 +58,11 @@ __device__ __forceinline__ bool sh_run_barrier(unsigned* bar) {
     return false;
 }
 
+/* The last iteration's measures. */
+struct ShMeasure {
+    double db, a;
+};
+
 /* What the control warp decides at the end of an iteration. */
 enum { SH_ACCEPT = 0, SH_REJECT, SH_ITERATE, SH_LEAVE };
 
@@ -85,10 +90,8 @@ __device__ __forceinline__ bool sh_run_maxima(const ShRunArgs& A, int round, int
  * every block): K advanced; the decision, the step and the next one's ratio in
  * S, with S.fin set when the launch ends here. */
 __device__ __forceinline__ int sh_run_decide(const ShRunArgs& A, ShCtl& K, AgFastStep& S, bool ok, double mdb, double ma, double mb,
-                                             double hstep, bool last, int iters, double& pc_last, int lane) {
-    const double pc_err = ag_fast_pc_err(mdb, ma);
-    const bool conv = (pc_err < 1e-16) || (iters > 2 && pc_last <= pc_err) || (iters >= 12);
-    pc_last = pc_err;
+                                             double hstep, bool last, int iters, ShMeasure& before, int lane) {
+    const bool conv = ag_fast_converged(mdb, ma, iters, before.db, before.a);
     int cmd = SH_ITERATE;
     if (!ok) {
         cmd = SH_LEAVE;
