@@ -264,7 +264,9 @@ __device__ __forceinline__ void ag_coop_force_pairs(int w, const AgCoopTab& CT, 
     bool earth = false, sunh = false;          /* harmonics left to FP64 */
     if (w == 2 && (c.forces & AG_F_EARTH_H)) {
         float hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-        const float q[3] = {xf[0].h + PR[2][0].h, xf[1].h + PR[2][1].h, xf[2].h + PR[2][2].h};
+        float q[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) q[k] = ag_f2_sep(xf[k], PR[2][k].h, PR[2][k].l);
         const float r2 = fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2]));
         earth = wild || !(r2 >= 1.0e-2f && r2 < 1e30f);
         if (!earth) {

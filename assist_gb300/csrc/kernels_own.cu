@@ -449,7 +449,10 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
             }
             if (c.forces & AG_F_EARTH_H) {
                 float q[3];
-                for (int m = 0; m < 3; m++) q[m] = xf[m].h - pos[(3 * 2 + m) * 32 + lane].h;
+                for (int m = 0; m < 3; m++) {
+                    const AgF2 p = pos[(3 * 2 + m) * 32 + lane];
+                    q[m] = ag_f2_sep(xf[m], -p.h, -p.l);
+                }
                 const float r2 = fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2]));
                 /* the Jacobian's share is larger by r / d: FP64 within 0.1 AU */
                 if (!(r2 >= (JAC ? 1.0e-2f : 4.0e-4f) && r2 < 1e30f)) flag |= 1;

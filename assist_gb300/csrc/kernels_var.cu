@@ -223,7 +223,7 @@ __device__ __forceinline__ void ag_var_force(int w, int lane, bool on, const Dev
         /* the Jacobian's share is larger than the term's by r / d: FP64 within 0.1 AU */
         float q[3], hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-        for (int k = 0; k < 3; k++) q[k] = xf[k].h + ag_pk_a(R[1].c[k].h);
+        for (int k = 0; k < 3; k++) q[k] = ag_f2_sep(xf[k], ag_pk_a(R[1].c[k].h), ag_pk_a(R[1].c[k].l));
         const float r2 = fmaf(q[0], q[0], fmaf(q[1], q[1], q[2] * q[2]));
         if (!(r2 >= 1.0e-2f && r2 < 1e30f)) near |= 1ull << 62;
         else {

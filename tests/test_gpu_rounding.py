@@ -1,0 +1,72 @@
+"""The small terms' own rounding: what a term adds to an evaluation, and an
+evaluation's whole error, against the oracle in double-double."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+EARTH_H, SUN_H, ALL = 0x10, 0x20, 0x7F
+T = 8200.0
+N = 1000
+# Two evaluations that differ in one small term share every other operation
+# but the roundings of the sums that it enters: at most two FP64 additions
+# each, so four roundings of up to half an ulp, 2^-53 of the component,
+# uniformly distributed.
+DIFF_RMS = 2.0 * 2.0 ** -53 / 3.0 ** 0.5
+
+
+@pytest.fixture(scope="module")
+def world(tmp_path_factory):
+    from assist_gb300 import Ephem, synth
+    from tests.oracle_py import Oracle
+    pl, ast, system = synth.write_ephemeris(str(tmp_path_factory.mktemp("round")), seed=6, t_beg=7950.0, t_end=8450.0)
+    return Ephem(pl, ast), Oracle(pl, ast), system
+
+
+def _around(system, body, lo, hi, seed):
+    """N states at lo..hi AU from a body at T, moving with it on the whole."""
+    rng = np.random.default_rng(seed)
+    x, v = system.body(body, np.array(T))
+    u = rng.normal(size=(N, 3))
+    u *= rng.uniform(lo, hi, (N, 1)) / np.linalg.norm(u, axis=1, keepdims=True)
+    return np.concatenate([x + u, v + 1e-3 * rng.normal(size=(N, 3))], axis=1)
+
+
+def _gpu(eph, state, forces, kind):
+    """acc (N, 3), or with kind "var" the derivatives by state too (N, 7, 3)."""
+    import torch
+    from assist_gb300 import batch
+    dev = lambda a: torch.tensor(a, device="cuda")  # noqa: E731
+    o = batch.options(forces=forces)
+    if kind == "shared":
+        return batch.forces_shared_time_device(eph, T, dev(state), opts=o).cpu().numpy()
+    var = dev(np.tile(np.eye(6), (len(state), 1, 1))) if kind == "var" else None
+    acc, vacc = batch.forces_device(eph, dev(np.full(len(state), T)), dev(state), var_state=var, opts=o)
+    if var is None:
+        return acc.cpu().numpy()
+    return np.concatenate([acc.cpu().numpy()[:, None], vacc.cpu().numpy()], axis=1)
+
+
+def _oracle(O, state, forces, kind, dd=True):
+    if kind != "var":
+        return O.forces(T, state, forces=forces, dd=dd)
+    n = len(state)
+    got = O.forces(T, state, var_state=np.tile(np.eye(6), (n, 1)), var_tp=np.repeat(np.arange(n), 6).astype(np.int32),
+                   forces=forces, dd=dd)
+    lay = lambda a: np.concatenate([a[:n, None], a[n:].reshape(n, 6, 3)], axis=1)  # noqa: E731
+    return lay(got) if not dd else (lay(got[0]), lay(got[1]))
+
+
+@pytest.mark.parametrize("kind", ["shared", "own"])
+@pytest.mark.parametrize("term,lo,hi", [(EARTH_H, 0.0205, 0.023)])
+def test_harmonics_add_no_more_than_rounding(world, kind, term, lo, hi):
+    """The harmonics just beyond the distance within which they are FP64: what
+    switching them on adds, against the double-double oracle."""
+    eph, O, system = world
+    state = _around(system, 3 if term == EARTH_H else 0, lo, hi, 1)
+    got = _gpu(eph, state, ALL, kind) - _gpu(eph, state, ALL & ~term, kind)
+    (ah, al), (bh, bl) = _oracle(O, state, ALL, kind), _oracle(O, state, ALL & ~term, kind)
+    e = np.linalg.norm(got - ((ah - bh) + (al - bl)), axis=1) / np.linalg.norm(ah, axis=1)
+    rms = np.sqrt((e ** 2).mean())
+    print("%s: rms %.2e of the acceleration, bound %.2e" % (kind, rms, DIFF_RMS))
+    assert rms < DIFF_RMS
