@@ -75,6 +75,11 @@ static ForceCfg make_cfg(int forces, int gr, int geo, double alpha, double nk, d
     c.s_ca = std::cos(ras); c.s_sa = std::sin(ras); c.s_cd = std::cos(decs); c.s_sd = std::sin(decs);
     const double pole[8] = {c.e_sa, c.e_ca, c.e_sd, c.e_cd, c.s_sa, c.s_ca, c.s_sd, c.s_cd};
     for (int k = 0; k < 8; k++) c.f_pole[k] = (float)pole[k];
+    const double sun[3] = {c.s_ca * c.s_cd, c.s_sa * c.s_cd, c.s_sd};
+    for (int k = 0; k < 3; k++) {
+        c.f_sun[k] = (float)sun[k];
+        c.f_sun[3 + k] = (float)(sun[k] - (double)c.f_sun[k]);
+    }
     return c;
 }
 

@@ -46,6 +46,7 @@ struct ForceCfg {
     double e_sa, e_ca, e_sd, e_cd;     /* Earth pole: RA 0 deg, Dec 90 deg */
     double s_sa, s_ca, s_sd, s_cd;     /* Sun pole: RA 286.13 deg, Dec 63.87 deg */
     float f_pole[8];                   /* the eight in FP32 */
+    float f_sun[6];                    /* the Sun's pole as a vector, high parts then low parts */
 };
 
 

@@ -482,8 +482,8 @@ static void ag_pair_view(DevEphem& D) {
     V.ek2 = (float)(gme * 1.5 * D.J2E * Re2);
     V.ek3 = (float)(gme * 2.5 * D.J3E * Re2 * D.Re_eq);
     V.ek4 = (float)(gme * 0.625 * D.J4E * Re2 * Re2);
-    V.sk2 = (float)(gms * 1.5 * D.J2SUN * D.Rs_eq * D.Rs_eq);
     auto split = [](double x, float& h, float& l) { h = (float)x; l = (float)(x - (double)h); };
+    split(gms * 1.5 * D.J2SUN * D.Rs_eq * D.Rs_eq, V.sk2, V.sk2_l);
     split(D.inv_cau, V.inv_cau_h, V.inv_cau_l);
     split(D.f_earth, V.f_earth_h, V.f_earth_l);
     split(D.f_moon, V.f_moon_h, V.f_moon_l);

@@ -279,7 +279,10 @@ __device__ __forceinline__ void ag_coop_force_pairs(int w, const AgCoopTab& CT, 
     if (w == 3 && (c.forces & AG_F_SUN_H)) {
         float hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         sunh = wild || !(rs2 >= 1.0e-2f && rs2 < 1e30f);
-        if (!sunh) {
+        if (!sunh && rs2 < AG_SUN_H_FAR2) {
+            const AgF2 d[3] = {ag_q_add(xf[0], sun[0]), ag_q_add(xf[1], sun[1]), ag_q_add(xf[2], sun[2])};
+            ag_fast_sun_near<true>(E.pv, c, d, s, j);
+        } else if (!sunh) {
             const float q[3] = {sx, sy, sz};
             ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, s);
             ag_fast_sun_hj(E.pv, c, q, rs2, hj);

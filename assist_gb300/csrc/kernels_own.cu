@@ -398,7 +398,9 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
         unsigned flag = 0;
         double J[3][6];
         double ea[3];
-        float hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};    /* harmonics' Jacobian, xx xy xz yy yz zz */
+        /* harmonics' Jacobian, xx xy xz yy yz zz: FP32 and, of a Sun nearer than 0.5 AU, float pairs */
+        float hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        AgF2 nj[6] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
         if (wid == 3) {
             if (JAC)
                 for (int a = 0; a < 3; a++)
@@ -463,7 +465,10 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
             }
             if (c.forces & AG_F_SUN_H) {
                 if (!(rs2 >= 1.0e-2f && rs2 < 1e30f)) flag |= 2;
-                else {
+                else if (rs2 < AG_SUN_H_FAR2) {
+                    const AgF2 d[3] = {ag_q_add(xf[0], sp[0]), ag_q_add(xf[1], sp[1]), ag_q_add(xf[2], sp[2])};
+                    ag_fast_sun_near<JAC>(E.pv, c, d, s, nj);
+                } else {
                     ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, s);
                     const float q[3] = {sx, sy, sz};
                     if (JAC) ag_fast_sun_hj(E.pv, c, q, rs2, hj);
@@ -486,7 +491,9 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
                 ag_pk_jac_get(PJ, k, 0, ah, al);
                 ag_pk_jac_get(PJ, k, 1, bh, bl);
                 if (k < 6) bl += hj[k];
-                JS.p[out][k][lane] = wild ? AgF2{0.0f, 0.0f} : ag_f2_add({ah, al}, {bh, bl});
+                AgF2 p = ag_f2_add({ah, al}, {bh, bl});
+                if (wid == 3 && k < 6) p = ag_f2_add(p, nj[k]);
+                JS.p[out][k][lane] = wild ? AgF2{0.0f, 0.0f} : p;
             }
             if (wid == 3) {
 #pragma unroll

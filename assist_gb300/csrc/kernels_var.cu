@@ -236,7 +236,10 @@ __device__ __forceinline__ void ag_var_force(int w, int lane, bool on, const Dev
     if (sub == 0 && w == 2 && (c.forces & AG_F_SUN_H)) {
         float hj[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         if (!(rs2 >= 1.0e-2f && rs2 < 1e30f)) near |= 1ull << 63;
-        else {
+        else if (rs2 < AG_SUN_H_FAR2) {
+            const AgF2 d[3] = {ag_q_add(xf[0], H.sp[0]), ag_q_add(xf[1], H.sp[1]), ag_q_add(xf[2], H.sp[2])};
+            ag_fast_sun_near<true>(E.pv, c, d, s, j);
+        } else {
             const float q[3] = {sx, sy, sz};
             ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, s);
             ag_fast_sun_hj(E.pv, c, q, rs2, hj);
