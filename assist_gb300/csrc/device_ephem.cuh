@@ -52,11 +52,12 @@ struct __align__(32) AgRecMeta {
 };
 
 /* What the pair terms read of the masses and constants (host_ephem.cpp fills
- * it): per two bodies GM and threshold, the Sun's GM and 1/c^2 as float
+ * it): per two bodies GM and threshold (and with Jacobian), the Sun's GM and 1/c^2 as float
  * pairs, FP32 coefficients of the harmonics (the Sun's as a float pair), and the .440 columns 0..9 by
  * falling coefficient count. */
 struct AgPairView {
     AgPkGm gm[AG_MAX_PACKS];
+    float jac_thr[2 * AG_MAX_PACKS];
     float gm_sun_h, gm_sun_l, oc2_h, oc2_l;
     float gm_jup, ek2, ek3, ek4, sk2, sk2_l;
     int n_packs;

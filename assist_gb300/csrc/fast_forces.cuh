@@ -84,12 +84,14 @@ struct AgFastShared {
     AgPkGm gm[AG_MAX_PACKS];        /* masses; zero where the configuration leaves the body out */
 };
 
-/* Masses of the pair terms for configuration c (whole block; the caller
- * synchronises). */
+/* Masses and thresholds (JAC: for terms with Jacobian) of the pair terms for
+ * configuration c (whole block; the caller synchronises). */
+template <bool JAC = false>
 __device__ __forceinline__ void ag_fast_masses(const DevEphem& E, const ForceCfg& c, AgFastShared& F, int tid) {
     const bool pl = (c.forces & AG_F_PLANETS) != 0, as = (c.forces & AG_F_AST) != 0;
     if (tid < E.pv.n_packs) {
         AgPkGm g = E.pv.gm[tid];
+        if (JAC) { g.ta = E.pv.jac_thr[2 * tid]; g.tb = E.pv.jac_thr[2 * tid + 1]; }
         const bool a = 2 * tid < AG_PAIR_PL ? pl : as, b = 2 * tid + 1 < AG_PAIR_PL ? pl : as;
         g.h = ag_pk(a ? ag_pk_a(g.h) : 0.0f, b ? ag_pk_b(g.h) : 0.0f);
         g.l = ag_pk(a ? ag_pk_a(g.l) : 0.0f, b ? ag_pk_b(g.l) : 0.0f);

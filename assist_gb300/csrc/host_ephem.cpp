@@ -471,6 +471,7 @@ static void ag_pair_view(DevEphem& D) {
         std::memcpy((char*)&G.h + 4 * (k & 1), &hi, 4);
         std::memcpy((char*)&G.l + 4 * (k & 1), &lo, 4);
         ((k & 1) ? G.tb : G.ta) = thr;
+        V.jac_thr[k] = ag_pair_thr2_jac(gm / D.gm[AG_SUN]);
         ((k & 1) ? G.gb : G.ga) = planet ? hi : 0.0f;
     }
     const double gms = D.gm[AG_SUN], gme = D.gm[AG_EAR], Re2 = D.Re_eq * D.Re_eq;

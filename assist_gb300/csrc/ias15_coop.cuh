@@ -247,7 +247,10 @@ __device__ __forceinline__ void ag_coop_force_pairs(int w, const AgCoopTab& CT, 
             R.c[k].h = ag_pk(a[k].h, two ? b[k].h : 1e6f);
             R.c[k].l = ag_pk(a[k].l, two ? b[k].l : 0.0f);
         }
-        const unsigned n = ag_pk_term<true>(R, E.pv.gm[p], xh, xl, rs2, S, &PJ);
+        AgPkGm G = E.pv.gm[p];
+        G.ta = E.pv.jac_thr[ka];
+        G.tb = E.pv.jac_thr[kb];
+        const unsigned n = ag_pk_term<true>(R, G, xh, xl, rs2, S, &PJ);
         near |= (unsigned long long)(two ? n : n & 1u) << ka;
     }
     AgF2 s[3], j[7];

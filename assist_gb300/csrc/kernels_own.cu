@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
             const bool a = 2 * tid < AG_PAIR_PL ? pl : as, b = 2 * tid + 1 < AG_PAIR_PL ? pl : as;
             g.h = ag_pk(a ? ag_pk_a(g.h) : 0.0f, b ? ag_pk_b(g.h) : 0.0f);
             g.l = ag_pk(a ? ag_pk_a(g.l) : 0.0f, b ? ag_pk_b(g.l) : 0.0f);
-            g.ta = a ? 2.0f * g.ta : 0.0f;
-            g.tb = b ? 2.0f * g.tb : 0.0f;
+            g.ta = a ? fmaxf(2.0f * g.ta, JAC ? E.pv.jac_thr[2 * tid] : 0.0f) : 0.0f;
+            g.tb = b ? fmaxf(2.0f * g.tb, JAC ? E.pv.jac_thr[2 * tid + 1] : 0.0f) : 0.0f;
             S.gm[tid] = g;
         }
     }

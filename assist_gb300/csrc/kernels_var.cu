@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(AG_FAST_THREADS, 2) ag_k_var_run(const DevEphe
     };
     if (tid == 0) M.any = 0;
     if (tid < L) M.close[tid] = 0ull;
-    ag_fast_masses(E, cf, S.F, tid);
+    ag_fast_masses<true>(E, cf, S.F, tid);
     ShCtl K = *R.in;
     const int gs = min(L, R.n - L * (int)blockIdx.x);
     for (int q = tid; q < 7 * L; q += AG_FAST_THREADS) {

@@ -81,3 +81,21 @@ def test_harmonics_add_no_more_than_rounding(world, kind, term, lo, hi):
         rms = np.sqrt((e ** 2).mean())
         print("%s: rms %.2e, bound %.2e" % (kind, rms, DIFF_RMS))
         assert rms < DIFF_RMS
+
+
+@pytest.mark.parametrize("body,lo,hi", [(10, 0.45, 0.8), (5, 0.05, 0.2), (3, 0.08, 0.3), (11, 0.004, 0.05)])
+def test_derivatives_near_light_bodies(world, body, lo, hi):
+    """The Jacobian by position about bodies whose pull is small beside the
+    Sun's when their tidal field is not: its error is no more than twice the
+    FP64 oracle's (whose square root and division round to half an ulp each
+    where the kernels' reciprocal root has one)."""
+    eph, O, system = world
+    state = _around(system, body, lo, hi, 2)
+    ref = _oracle(O, state, ALL, "var")
+
+    def rms(x):
+        e = ((x - ref[0]) - ref[1])[:, 1:4].reshape(N, 9)
+        return np.sqrt(((np.linalg.norm(e, axis=1) / np.linalg.norm(ref[0][:, 1:4].reshape(N, 9), axis=1)) ** 2).mean())
+    g, o = rms(_gpu(eph, state, ALL, "var")), rms(_oracle(O, state, ALL, "var", dd=False))
+    print("body %d: rms %.2e, oracle %.2e" % (body, g, o))
+    assert g < 2.0 * o
