@@ -128,7 +128,7 @@ static __device__ __noinline__ void ag_own_close(const DevEphem& E, const ForceC
                 ag_planet_exact<false>(E, rec, tf, ag_pair_planet(k), b, nullptr);
             } else {
                 gm = E.ast_gm[k - AG_PAIR_PL];
-                ag_asteroid_pos(E, k - AG_PAIR_PL, t, b);
+                ag_asteroid_exact(E, k - AG_PAIR_PL, t, b);
                 b[0] -= rs[0]; b[1] -= rs[1]; b[2] -= rs[2];
             }
             const double dx = x[0] + (0.0 - b[0]), dy = x[1] + (0.0 - b[1]), dz = x[2] + (0.0 - b[2]);
