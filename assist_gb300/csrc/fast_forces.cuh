@@ -76,7 +76,8 @@ struct AgFastView {
 struct AgFastShared {
     double xs[3][32], vs[3][32];    /* particle states at the node */
     AgF2 xf[3][32], vf[3][32];      /* and as float pairs */
-    double pa[2][3][32];            /* roles 0 and 1: FP64 partial accelerations */
+    double pa[2][3][32];            /* roles 0 and 1: FP64 partial accelerations without the Sun's */
+    double ss[3][32], gs[32];       /* separation from the Sun and -GM / r^3 there */
     AgF2 pf[AG_FAST_SLOTS][3][32];  /* roles 2..7: pair sums */
     double pn[AG_FAST_SLOTS][3][32];            /* their FP64 parts, where near[] says so */
     int near[AG_FAST_SLOTS];
@@ -730,7 +731,14 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
         }
         const double gm = w == 1 ? E.gm[AG_SUN] : ((c.forces & AG_F_PLANETS) ? E.gm[AG_JUP] : 0.0);
         const double g = gm * ri * ri * ri;
-        F.pa[w][0][lane] = fma(-g, s[0], ax); F.pa[w][1][lane] = fma(-g, s[1], ay); F.pa[w][2][lane] = fma(-g, s[2], az);
+        if (w == 0) {
+            F.pa[0][0][lane] = -g * s[0]; F.pa[0][1][lane] = -g * s[1]; F.pa[0][2][lane] = -g * s[2];
+        } else {
+            /* the Sun's term goes into the last sum unrounded */
+            F.gs[lane] = -g;
+            F.ss[0][lane] = s[0]; F.ss[1][lane] = s[1]; F.ss[2][lane] = s[2];
+            F.pa[1][0][lane] = ax; F.pa[1][1][lane] = ay; F.pa[1][2][lane] = az;
+        }
         return;
     }
     const int slot = w - 2;
@@ -845,7 +853,7 @@ __device__ __forceinline__ double ag_fast_sum(const AgFastShared& F, int k, int 
     if (any)
         for (int w = 0; w < AG_FAST_SLOTS; w++)
             if (F.near[w]) a += F.pn[w][k][lane];
-    return a;
+    return fma(F.gs[lane], F.ss[k][lane], a);
 }
 
 #endif

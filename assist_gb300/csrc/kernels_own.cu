@@ -69,7 +69,8 @@ struct AgOwnSmem {
     AgF2 xf[3][32], vf[3][32];
     double rs[3][32], rj[3][32], sv[3][32];     /* origin minus Sun, minus Jupiter; the Sun's velocity */
     AgF2 sp[3][32];                             /* rs as float pairs */
-    double pa[3][32];                           /* role 1's FP64 sums, then the total */
+    double pa[3][32];                           /* role 1's FP64 sums without the Sun */
+    double ss[3][32], gs[32];                   /* separation from the Sun and -GM / r^3 there */
     AgF2 pf[3][3][32];                          /* pair sums of roles 0, 2, 3 */
     unsigned near[3][32];                       /* bodies left to FP64 */
     unsigned char flag[32];                     /* role 3: harmonics and relativity left to FP64 */
@@ -344,8 +345,12 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
             const double rj = rsqrt(fma(j[0], j[0], fma(j[1], j[1], j[2] * j[2])));
             ag_term_planet<JAC>(E, true, AG_JUP, j[0], j[1], j[2], rj, ax, ay, az, &Y);
         }
-        ag_term_planet<JAC>(E, true, AG_SUN, s[0], s[1], s[2], ri, ax, ay, az, &Y);
+        /* the Sun's term goes into the last sum unrounded */
+        const double gs = E.gm[AG_SUN] * ri * ri * ri;
+        S.gs[lane] = -gs;
+        S.ss[0][lane] = s[0]; S.ss[1][lane] = s[1]; S.ss[2][lane] = s[2];
         if (JAC) {
+            ag_symjac_term(Y, gs, ri, s[0], s[1], s[2]);
             ag_symjac_add(Y, J);
 #pragma unroll
             for (int a = 0; a < 3; a++)
@@ -519,7 +524,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
     if (on && wid != 1) {
         const int k = wid == 0 ? 0 : wid - 1;
         const AgF2 s = ag_f2_add(ag_f2_add(S.pf[2][k][lane], S.pf[1][k][lane]), S.pf[0][k][lane]);
-        if (S.bad[lane] == AG_OK) acc[3 * (size_t)i + k] = ag_f2_to(s) + S.pa[k][lane];
+        if (S.bad[lane] == AG_OK) acc[3 * (size_t)i + k] = fma(S.gs[lane], S.ss[k][lane], ag_f2_to(s) + S.pa[k][lane]);
         if (k == 0 && status) status[i] = S.bad[lane];
     }
     if constexpr (JAC) {
@@ -529,7 +534,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
         for (int q = 0; q < 18; q++) {
             const int a = q / 6, b = q % 6;
             if ((q & 3) != wid) continue;
-            double s = JS.j[q][lane] + JS.e[q][lane];
+            double s = JS.e[q][lane];
             if (b < 3) {
                 AgF2 p = ag_f2_add(ag_f2_add(JS.p[0][sym[a][b % 3]][lane], JS.p[1][sym[a][b % 3]][lane]),
                                    JS.p[2][sym[a][b % 3]][lane]);
@@ -537,7 +542,7 @@ __global__ void __launch_bounds__(128, JAC ? 2 : 4) ag_k_forces_own(const DevEph
                     p = ag_f2_add(p, ag_f2_neg(ag_f2_add(ag_f2_add(JS.p[0][6][lane], JS.p[1][6][lane]), JS.p[2][6][lane])));
                 s += ag_f2_to(p);
             }
-            JS.j[q][lane] = s;
+            JS.j[q][lane] += s;
         }
         __syncthreads();
         if (on && S.bad[lane] == AG_OK) {

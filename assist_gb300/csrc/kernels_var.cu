@@ -43,7 +43,8 @@ struct AgVarSmem {
     double J[18][L], Je[18][L];                     /* FP64 parts of the Jacobian (roles 1 and 4); J then the whole */
     AgF2 pj[AG_VAR_SLOTS][7][L];                    /* pair parts: symmetric part and trace sum */
     AgF2 pf[AG_VAR_SLOTS + 1][3][L];                /* pair accelerations; the last: relativity */
-    double pa[3][L], acc[3][L];                     /* role 1's acceleration; the sum */
+    double pa[3][L], acc[3][L];                     /* role 1's acceleration without the Sun's; the sum */
+    double ss[3][L], gs[L];                         /* separation from the Sun and -GM / r^3 there */
     unsigned long long close[L];                    /* pair bodies left to FP64; bit 62 Earth's, 63 the Sun's harmonics */
     int any;
     int pidx[7][L];                                 /* particle of each (variational, lane) */
@@ -127,7 +128,13 @@ __device__ __forceinline__ void ag_var_force(int w, int lane, bool on, const Dev
         }
         AgSymJac Y = {{0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, 0.0};
         const double g = (sub == 1 ? E.gm[AG_JUP] : E.gm[AG_SUN]) * ri * ri * ri;
-        a[0] = fma(-g, s[0], a[0]); a[1] = fma(-g, s[1], a[1]); a[2] = fma(-g, s[2], a[2]);
+        if (sub == 0) {
+            /* the Sun's term goes into the last sum unrounded */
+            M.gs[l] = -g;
+            M.ss[0][l] = s[0]; M.ss[1][l] = s[1]; M.ss[2][l] = s[2];
+        } else {
+            a[0] = -g * s[0]; a[1] = -g * s[1]; a[2] = -g * s[2];
+        }
         ag_symjac_term(Y, g, ri, s[0], s[1], s[2]);
         /* Jupiter's to the Sun's lanes */
 #pragma unroll
@@ -299,7 +306,7 @@ __device__ __forceinline__ void ag_var_assemble(const DevEphem& E, const ForceCf
         const int q = t / L, l = t - q * L;
         if (q < 18) {
             const int a = q / 6, b = q - 6 * a;
-            double s = M.J[q][l] + M.Je[q][l];
+            double s = M.Je[q][l];
             if (b < 3) {
                 const int lo = a < b ? a : b, hi = a < b ? b : a, e = lo == 0 ? hi : lo + hi + 1;
                 AgF2 p = M.pj[0][e][l];
@@ -313,13 +320,13 @@ __device__ __forceinline__ void ag_var_assemble(const DevEphem& E, const ForceCf
                 }
                 s += ag_f2_to(p);
             }
-            M.J[q][l] = s;
+            M.J[q][l] += s;
         } else {
             const int k = q - 18;
             AgF2 p = M.pf[0][k][l];
 #pragma unroll
             for (int m = 1; m <= AG_VAR_SLOTS; m++) p = ag_f2_add(p, M.pf[m][k][l]);
-            M.acc[k][l] = ag_f2_to(p) + M.pa[k][l];
+            M.acc[k][l] = fma(M.gs[l], M.ss[k][l], ag_f2_to(p) + M.pa[k][l]);
         }
     }
     __syncthreads();

@@ -99,3 +99,22 @@ def test_derivatives_near_light_bodies(world, body, lo, hi):
     g, o = rms(_gpu(eph, state, ALL, "var")), rms(_oracle(O, state, ALL, "var", dd=False))
     print("body %d: rms %.2e, oracle %.2e" % (body, g, o))
     assert g < 2.0 * o
+
+
+@pytest.mark.parametrize("kind", ["shared", "own", "var"])
+def test_sums_round_once(world, kind):
+    """The terms beside the Sun's enter the acceleration in one rounding: it
+    differs from the Sun's alone by the double-double difference and two
+    roundings, uniform over an ulp of each component (a tenth more for
+    sampling and for the small terms' own rounding; a third would be 1.22)."""
+    from assist_gb300 import synth
+    eph, O, system = world
+    state = synth.population(system, "mba", N, seed=8, t0=T, length=1.0).state
+    one = 0x1
+    a, b = _gpu(eph, state, ALL, kind), _gpu(eph, state, one, "own" if kind == "var" else kind)
+    (ah, al), (bh, bl) = _oracle(O, state, ALL, "own"), _oracle(O, state, one, "own")
+    e = ((a[:, 0] if kind == "var" else a) - b) - ((ah - bh) + (al - bl))
+    expect = np.sqrt((2.0 * np.spacing(np.abs(ah)) ** 2 / 12.0).mean())
+    rms = np.sqrt((e ** 2).mean())
+    print("%s: rms %.3f of the expected" % (kind, rms / expect))
+    assert rms < 1.1 * expect
