@@ -118,3 +118,31 @@ def test_sums_round_once(world, kind):
     rms = np.sqrt((e ** 2).mean())
     print("%s: rms %.3f of the expected" % (kind, rms / expect))
     assert rms < 1.1 * expect
+
+
+# solar masses by ASSIST's body index: Mercury, Venus, Earth, Mars, Saturn, Uranus, Neptune (the bound has one close
+# body: the Moon's neighbourhood is the Earth's too)
+LIGHT = {1: 1.66e-7, 2: 2.45e-6, 3: 3.0e-6, 5: 3.2e-7, 7: 2.86e-4, 8: 4.37e-5, 9: 5.15e-5}
+
+
+@pytest.mark.parametrize("kind", ["shared", "own"])
+@pytest.mark.parametrize("body", sorted(LIGHT))
+def test_close_bodies_in_fp64(world, kind, body):
+    """Particles 0.02 to 0.7 of the way to a body's threshold, where its term
+    has to be FP64's.  Bound of an error: four ulp of the body's and the
+    particle's place, with the term's slope of 3, and 4e-16 of the whole; a
+    float pair's 1.5e-15 of the place rms is 3.4 times the first."""
+    eph, O, system = world
+    m, (x, _) = LIGHT[body], system.body(body, np.array(T))
+    R = np.linalg.norm(x)
+    thr = max(m / 1e-3, (150 * m) ** (2 / 3)) ** 0.5 * R
+    state = _around(system, body, 0.02 * thr, 0.7 * thr, 3)
+    got = _gpu(eph, state, ALL, kind)
+    h, l = _oracle(O, state, ALL, "own")
+    d = np.linalg.norm(state[:, :3] - x, axis=1)
+    pull = 2.9591220828559115e-4 * m / d ** 2
+    a = np.linalg.norm(h, axis=1)
+    bound = 3.0 * 4.0 * 2.0 ** -53 * R / d * pull + 4e-16 * a
+    e = np.linalg.norm((got - h) - l, axis=1) / bound
+    print("body %d %s: rms %.2f of the bound" % (body, kind, np.sqrt((e ** 2).mean())))
+    assert np.sqrt((e ** 2).mean()) < 1.0
