@@ -1111,6 +1111,13 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
                 int dev = 0, sms = 0;
                 cudaGetDevice(&dev);
                 cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                /* two / three blocks a multiprocessor on ag_k_fast, ms: from 8
+                 * groups for each of three blocks on, three are faster (mixed
+                 * population, 365 days: 116,736 particles 140 / 128, 262,144
+                 * 154 / 143; main belt 58 / 53, 126 / 115) or alike (60 days:
+                 * 28.7 / 27.1, 73.5 / 73.2); below, it depends on the batch
+                 * (30,000 for 60 days 13.1 / 14.2, for 365 days 52.7 / 53.1,
+                 * main belt 19.3 / 18.2): the autotuner's to find */
                 occ = (int)gstart.size() >= 8 * 3 * sms ? 3 : 2;
             }
         }

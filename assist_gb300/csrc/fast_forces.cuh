@@ -6,8 +6,10 @@
  * other planets and the asteroids, whose terms are below 1e-3 of the Sun's,
  * are float pairs two at a time (pair_terms.cuh); the relativistic term (below
  * 1e-6 of the Sun's) is a float pair with its small parts in FP32; the
- * harmonics, away from their body, are FP32 (below 1e-9).  Each has an error
- * below 2e-17 of the acceleration; an FP64 sum of the terms rounds by 1e-16.
+ * harmonics are FP32 where they are below 1.1e-10 (the Earth's beyond 0.02 AU,
+ * the Sun's beyond 0.5 AU), the Sun's float pairs down to 0.1 AU and FP64
+ * nearer.  The evaluation's error is what it is with every term in FP64
+ * (ag_pair_thr2's comment has the figures).
  *
  * Eight warps (roles) share an evaluation, lane l of each working on particle l:
  *   role 0       Jupiter, FP64           role 1   Sun, non-gravitational, GR, FP64

@@ -13,9 +13,9 @@
  * reference's exact operations, the Sun in FP64 with fused multiply-adds (its
  * distance from the particles makes an ulp of its 0.01 AU 1e-18), and a body
  * close to the particle again in the exact operations.  About 300 FP64
- * instructions a block without variational particles.  33 particles 125 -> 31
- * us, 100,003 674 -> 233 us, 20,011 with six variational particles each 312 ->
- * 122 us.
+ * instructions a block without variational particles.  33 particles 125 -> 27
+ * to 29 us, 100,003 674 -> 231 to 239 us, 20,011 with six variational particles
+ * each 312 -> 123 to 132 us (by the population drawn).
  *
  *   before the barrier   role 1: the Sun; role 0: Jupiter, Earth and Moon,
  *                        an eighth of the asteroids; role 2: the other

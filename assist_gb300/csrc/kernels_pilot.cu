@@ -1,6 +1,7 @@
 /*
- * kernels_pilot.cu -- expected close-encounter cost of each particle, used
- * only to order the grouped batched kernels' work queue.
+ * kernels_pilot.cu -- expected close-encounter cost of each particle, which
+ * orders the grouped batched kernels' work queue, and its deep passes, which
+ * choose a group's kernel (below).
  *
  * A group of particles steps at the smallest step any member needs, and a
  * member passing close to a planet needs many small steps: such a group runs
@@ -74,7 +75,8 @@ __global__ void ag_k_pilot_grid(const DevEphem* __restrict__ Ep, double tmin, do
  * within 0.025 (all of them plunging into Jupiter); the rest is for the path's
  * own error: 0.035 of the radius is 5e-4 AU at the Earth, where the path of a
  * near-Earth orbit is off by up to 3e-5 AU after a year and 2e-4 after thirty.
- * 5 in 65,536 of the mixture come within 0.06 in a year. */
+ * 5 to 15 in 65,536 of the mixture come within 0.06 in a year, by the system
+ * drawn. */
 #define AG_DEEP 0.06f
 #define AG_DEEP_DAYS 2.0
 #define AG_DEEP_MAX_G 65536

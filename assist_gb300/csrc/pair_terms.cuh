@@ -14,10 +14,12 @@
  *
  * The term of a body, -GM d / |d|^3, from y0 (the FP32 estimate of 1/|d|):
  * with delta = |d|^2 y0^2 - 1 (about 2^-21, formed from the exact products'
- * errors), 1/|d|^3 = y0^3 (1 - 3/2 delta + 15/8 delta^2).  Relative error
- * about 2e-14 of the term (tests/test_pair_terms.py), so the error is below
- * 2e-17 of the acceleration while the term is below 1e-3 of the Sun's pull
- * (the body's threshold, ag_pair_thr2; nearer bodies take the FP64 term).
+ * errors), 1/|d|^3 = y0^3 (1 - 3/2 delta + 15/8 delta^2).  A term's
+ * relative error is at most 8e-14 where the positions' own pairs play no part
+ * (bound 1.5e-13, tests/test_pair_terms.py), so below 1e-16 of the acceleration,
+ * an FP64 sum's rounding, for a term of 1e-3 of the Sun's pull (the body's
+ * threshold, ag_pair_thr2; nearer bodies take the FP64 term) and less for all
+ * smaller ones.
  *
  * Plain C++ without CUDA (the packed operations are then two scalar ones), for
  * the test.
@@ -110,10 +112,13 @@ struct alignas(16) AgPkGm {
 
 /* The smallest squared distance, over the particle's squared heliocentric
  * distance, at which a body of mass m (in solar masses) takes the pair term.
- * The pair's relative error of 2e-14 asks for a share m (r/d)^2 of the Sun's
- * pull below 1e-3; the separation's absolute error, about 3e-15 r with the
- * term's slope, for m (r/d)^3 below 1/150: either way 2e-17 of the
- * acceleration, a fifth of the rounding of its FP64 sum. */
+ * The pair's relative error (at most 8e-14) asks for a share m (r/d)^2 of the
+ * Sun's pull below 1e-3; the separation's absolute error, about 3e-15 r rms with
+ * the term's slope, for m (r/d)^3 below 1/150: 2e-17 of the acceleration rms.
+ * The whole evaluation's error is no larger than with every term in FP64:
+ * over 16 distances from the Sun and 49 from the planets, each 200 to 300
+ * particles, 0.98 of it for shared times and 1.00 for own times (rms against
+ * double-double; tests/test_gpu_rounding.py holds the single terms). */
 inline float ag_pair_thr2(double m) {
     const double a = m / 1e-3, b = std::pow(150.0 * m, 2.0 / 3.0);
     return (float)(a > b ? a : b);

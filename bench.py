@@ -83,6 +83,8 @@ IAS_PER_STEP = 3 * (2 * 9 + 2 * 8 + 8 + 7 * 8)
 # particle-days): DRAM bytes per particle-day of a launch, scaled to a full
 # launch by its particle-days.
 DRAM_BYTES_PER_PARTICLE_DAY = 0.845
+# Share of the active cycles in which the FP64 pipe is busy (ncu, the same case).
+FP64_PIPE_BUSY = 0.67
 
 
 def _synth():
@@ -134,9 +136,13 @@ def roofline(stats, model, kernel_s, peak, pdays):
             "peak_source": "measured in this run (FP64 FMA chains; MEASURED_PEAKS.json has no FP64 figure)",
             "work": "per force evaluation %d flop of particle-dependent force terms + %d IAS15; per body table "
                     "%d flop (ephemeris + particle-independent force-term parts); per accepted step %d; all counted "
-                    "as FP64, although most force terms run as float pairs on the FP32 pipes (frac can pass 1)"
+                    "as FP64, although most force terms run as float pairs on the FP32 pipes: frac is work over the "
+                    "FP64 rate, not a pipe's occupancy, and can pass 1 (fp64_pipe_busy is that)"
                     % (model["per_eval_particle"], IAS_PER_EVAL, model["per_body_table"], IAS_PER_STEP),
             "flops_per_launch": work, "force_evals": ev, "body_tables": tabs,
+            "fp64_pipe_busy": FP64_PIPE_BUSY,
+            "fp64_pipe_busy_source": "ncu, 32,768-particle case of this kernel "
+                                     "(profiles/ag_k_fast_32768_mixture_1yr.md)",
             "frac_vs_independent": indep / kernel_s / peak,
             "frac_vs_independent_note": "the work of independent steps (every evaluation evaluating all bodies at "
                                         "its own time, %d flop + IAS15) per the kernel's evaluations: a throughput "
