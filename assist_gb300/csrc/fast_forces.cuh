@@ -404,8 +404,65 @@ __device__ __forceinline__ int ag_fast_tables(const DevEphem& E, const ForceCfg&
 
 /* ------------------------------------------------------------------ terms */
 
+/* Pair operations without the final renormalisation (the low part may grow to
+ * a few units of the high part's last place): enough for the relativistic
+ * term, which needs about 30 bits. */
+__device__ __forceinline__ AgF2 ag_q_mul(AgF2 a, AgF2 b) {
+    const float h = __fmul_rn(a.h, b.h);
+    return {h, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.h, b.h, -h)))};
+}
+__device__ __forceinline__ AgF2 ag_q_add(AgF2 a, AgF2 b) {
+    const float s = __fadd_rn(a.h, b.h), bb = __fsub_rn(s, a.h);
+    const float e = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, bb)), __fsub_rn(b.h, bb));
+    return {s, __fadd_rn(e, __fadd_rn(a.l, b.l))};
+}
+__device__ __forceinline__ AgF2 ag_q_dot(const AgF2* a, const AgF2* b) {
+    return ag_q_add(ag_q_mul(a[0], b[0]), ag_q_add(ag_q_mul(a[1], b[1]), ag_q_mul(a[2], b[2])));
+}
+
+/* The Sun's J2 between 0.1 and 0.5 AU, in float pairs: there it is up to 1e-9
+ * of the acceleration, and its FP32 form's error was 2.5e-16 rms of it at 0.11
+ * AU, as much as the whole FP64 sum's (1.2e-17 at 0.5 AU).  With the pole n,
+ * z = d.n, c = z / |d|, k = GM 3/2 J2 R^2 / |d|^5: k ((5 c^2 - 1) d - 2 z n)
+ * added to acc; JAC: its Jacobian, k ((5 c^2 - 1) I + 10 z (d n^T + n d^T) /
+ * |d|^2 - 2 n n^T - 5 (7 c^2 - 1) d d^T / |d|^2), to j.  Out of line: few
+ * particles are there. */
+#define AG_SUN_H_FAR2 0.25f
+template <bool JAC>
+static __device__ __noinline__ void ag_fast_sun_near(const AgPairView& PV, const ForceCfg& c, const AgF2* d, AgF2* acc, AgF2* j) {
+    const AgF2 n[3] = {{c.f_sun[0], c.f_sun[3]}, {c.f_sun[1], c.f_sun[4]}, {c.f_sun[2], c.f_sun[5]}};
+    const AgF2 r2 = ag_q_dot(d, d), z = ag_q_dot(d, n);
+    /* 1/|d|^2 = y^2 (1 - delta), 1/|d|^5 = y^5 (1 - 5/2 delta), delta = r2 y^2 - 1 */
+    const float y = rsqrtf(r2.h);
+    const AgF2 q = ag_q_mul({y, 0.0f}, {y, 0.0f}), t = ag_q_mul(r2, q);
+    const float del = __fadd_rn(__fsub_rn(t.h, 1.0f), t.l);
+    const AgF2 r2i = {q.h, __fmaf_rn(-q.h, del, q.l)};
+    AgF2 k = ag_q_mul({PV.sk2, PV.sk2_l}, ag_q_mul(ag_q_mul(q, q), {y, 0.0f}));
+    k.l = __fmaf_rn(k.h, __fmul_rn(-2.5f, del), k.l);
+    const AgF2 zr = ag_q_mul(z, r2i), c2 = ag_q_mul(z, zr);
+    const AgF2 f = ag_q_add(ag_q_mul({5.0f, 0.0f}, c2), {-1.0f, 0.0f}), z2 = {-2.0f * z.h, -2.0f * z.l};
+    for (int a = 0; a < 3; a++)
+        acc[a] = ag_f2_add(acc[a], ag_q_mul(k, ag_q_add(ag_q_mul(f, d[a]), ag_q_mul(z2, n[a]))));
+    if (JAC) {
+        const AgF2 h = ag_q_mul({10.0f, 0.0f}, zr);
+        const AgF2 g = ag_q_mul(r2i, ag_q_add(ag_q_mul({-35.0f, 0.0f}, c2), {5.0f, 0.0f}));
+        AgF2 A[3], B[3];
+        for (int a = 0; a < 3; a++) {
+            A[a] = ag_q_add(ag_q_mul(g, d[a]), ag_q_mul(h, n[a]));
+            B[a] = ag_q_add(ag_q_mul(h, d[a]), {-2.0f * n[a].h, -2.0f * n[a].l});
+        }
+        int at = 0;
+        for (int a = 0; a < 3; a++)
+            for (int b = a; b < 3; b++, at++) {
+                AgF2 s = ag_q_add(ag_q_mul(d[a], A[b]), ag_q_mul(n[a], B[b]));
+                if (a == b) s = ag_q_add(s, f);
+                j[at] = ag_f2_add(j[at], ag_q_mul(k, s));
+            }
+    }
+}
+
 /* Bodies close to the particle (bit k of near: pair body k0 + k), and the
- * harmonics of a body close by, in FP64.  Out of line: a rare path whose
+ * harmonics of a body close by, in FP64 (the Sun's beyond 0.1 AU in pairs).  Out of line: a rare path whose
  * registers the evaluation should not carry. */
 static __device__ __noinline__ void ag_fast_close(const DevEphem& E, const ForceCfg& c, const AgFastView* V,
                                                   const AgFastNode* H, int n, int k0, unsigned near, bool earth,
@@ -425,8 +482,15 @@ static __device__ __noinline__ void ag_fast_close(const DevEphem& E, const Force
         ag_term_earth_h<false>(E, c, dx, dy, dz, rsqrt(fma(dx, dx, fma(dy, dy, dz * dz))), ax, ay, az, nullptr);
     }
     if (sun) {
-        const double dx = x[0] + H->rs[0], dy = x[1] + H->rs[1], dz = x[2] + H->rs[2];
-        ag_term_sun_h<false>(E, c, dx, dy, dz, rsqrt(fma(dx, dx, fma(dy, dy, dz * dz))), ax, ay, az, nullptr);
+        const double dx = x[0] + H->rs[0], dy = x[1] + H->rs[1], dz = x[2] + H->rs[2], r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+        if (r2 >= 1.0e-2 && r2 < 1e30) {
+            const AgF2 d[3] = {ag_f2_of(dx), ag_f2_of(dy), ag_f2_of(dz)};
+            AgF2 o[3] = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+            ag_fast_sun_near<false>(E.pv, c, d, o, nullptr);
+            ax += ag_f2_to(o[0]); ay += ag_f2_to(o[1]); az += ag_f2_to(o[2]);
+        } else {
+            ag_term_sun_h<false>(E, c, dx, dy, dz, rsqrt(r2), ax, ay, az, nullptr);
+        }
     }
     if (eih) {
         /* relativity far out: ag_fast_eih's formula */
@@ -462,22 +526,6 @@ static __device__ __noinline__ void ag_fast_close(const DevEphem& E, const Force
         az += -pre * fac * d[2] + pre * f * rel_v[2] + ga * af[2];
     }
     a[0] = ax; a[1] = ay; a[2] = az;
-}
-
-/* Pair operations without the final renormalisation (the low part may grow to
- * a few units of the high part's last place): enough for the relativistic
- * term, which needs about 30 bits. */
-__device__ __forceinline__ AgF2 ag_q_mul(AgF2 a, AgF2 b) {
-    const float h = __fmul_rn(a.h, b.h);
-    return {h, __fmaf_rn(a.l, b.h, __fmaf_rn(a.h, b.l, __fmaf_rn(a.h, b.h, -h)))};
-}
-__device__ __forceinline__ AgF2 ag_q_add(AgF2 a, AgF2 b) {
-    const float s = __fadd_rn(a.h, b.h), bb = __fsub_rn(s, a.h);
-    const float e = __fadd_rn(__fsub_rn(a.h, __fsub_rn(s, bb)), __fsub_rn(b.h, bb));
-    return {s, __fadd_rn(e, __fadd_rn(a.l, b.l))};
-}
-__device__ __forceinline__ AgF2 ag_q_dot(const AgF2* a, const AgF2* b) {
-    return ag_q_add(ag_q_mul(a[0], b[0]), ag_q_add(ag_q_mul(a[1], b[1]), ag_q_mul(a[2], b[2])));
 }
 
 /* EIH relativity with the Sun as its source (src/forces.c:1288-1983): the
@@ -594,47 +642,6 @@ __device__ __forceinline__ void ag_fast_sun_h(const AgPairView& PV, const ForceC
     acc[0].l = fmaf(k2, fmaf(f2, qx, __fmul_rn(zz, nx)), acc[0].l);
     acc[1].l = fmaf(k2, fmaf(f2, qy, __fmul_rn(zz, ny)), acc[1].l);
     acc[2].l = fmaf(k2, fmaf(f2, qz, __fmul_rn(zz, nz)), acc[2].l);
-}
-
-/* The Sun's J2 between 0.1 and 0.5 AU, in float pairs: there it is up to 1e-9
- * of the acceleration, and its FP32 form's error was 2.5e-16 rms of it at 0.11
- * AU, as much as the whole FP64 sum's (1.2e-17 at 0.5 AU).  With the pole n,
- * z = d.n, c = z / |d|, k = GM 3/2 J2 R^2 / |d|^5: k ((5 c^2 - 1) d - 2 z n)
- * added to acc; JAC: its Jacobian, k ((5 c^2 - 1) I + 10 z (d n^T + n d^T) /
- * |d|^2 - 2 n n^T - 5 (7 c^2 - 1) d d^T / |d|^2), to j.  Out of line: few
- * particles are there. */
-#define AG_SUN_H_FAR2 0.25f
-template <bool JAC>
-static __device__ __noinline__ void ag_fast_sun_near(const AgPairView& PV, const ForceCfg& c, const AgF2* d, AgF2* acc, AgF2* j) {
-    const AgF2 n[3] = {{c.f_sun[0], c.f_sun[3]}, {c.f_sun[1], c.f_sun[4]}, {c.f_sun[2], c.f_sun[5]}};
-    const AgF2 r2 = ag_q_dot(d, d), z = ag_q_dot(d, n);
-    /* 1/|d|^2 = y^2 (1 - delta), 1/|d|^5 = y^5 (1 - 5/2 delta), delta = r2 y^2 - 1 */
-    const float y = rsqrtf(r2.h);
-    const AgF2 q = ag_q_mul({y, 0.0f}, {y, 0.0f}), t = ag_q_mul(r2, q);
-    const float del = __fadd_rn(__fsub_rn(t.h, 1.0f), t.l);
-    const AgF2 r2i = {q.h, __fmaf_rn(-q.h, del, q.l)};
-    AgF2 k = ag_q_mul({PV.sk2, PV.sk2_l}, ag_q_mul(ag_q_mul(q, q), {y, 0.0f}));
-    k.l = __fmaf_rn(k.h, __fmul_rn(-2.5f, del), k.l);
-    const AgF2 zr = ag_q_mul(z, r2i), c2 = ag_q_mul(z, zr);
-    const AgF2 f = ag_q_add(ag_q_mul({5.0f, 0.0f}, c2), {-1.0f, 0.0f}), z2 = {-2.0f * z.h, -2.0f * z.l};
-    for (int a = 0; a < 3; a++)
-        acc[a] = ag_f2_add(acc[a], ag_q_mul(k, ag_q_add(ag_q_mul(f, d[a]), ag_q_mul(z2, n[a]))));
-    if (JAC) {
-        const AgF2 h = ag_q_mul({10.0f, 0.0f}, zr);
-        const AgF2 g = ag_q_mul(r2i, ag_q_add(ag_q_mul({-35.0f, 0.0f}, c2), {5.0f, 0.0f}));
-        AgF2 A[3], B[3];
-        for (int a = 0; a < 3; a++) {
-            A[a] = ag_q_add(ag_q_mul(g, d[a]), ag_q_mul(h, n[a]));
-            B[a] = ag_q_add(ag_q_mul(h, d[a]), {-2.0f * n[a].h, -2.0f * n[a].l});
-        }
-        int at = 0;
-        for (int a = 0; a < 3; a++)
-            for (int b = a; b < 3; b++, at++) {
-                AgF2 s = ag_q_add(ag_q_mul(d[a], A[b]), ag_q_mul(n[a], B[b]));
-                if (a == b) s = ag_q_add(s, f);
-                j[at] = ag_f2_add(j[at], ag_q_mul(k, s));
-            }
-    }
 }
 
 /* R^T M R of a symmetric M (pole frame) added to the six elements J. */
@@ -809,13 +816,8 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
         }
         if (w == 2 && (c.forces & AG_F_SUN_H)) {
             /* J2: below 4e-11 of the acceleration beyond 0.5 AU */
-            cs = !(rs2 >= 1.0e-2f && rs2 < 1e30f);
-            if (rs2 >= AG_SUN_H_FAR2) {
-                if (!cs) ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, acc);
-            } else if (!cs) {
-                const AgF2 d[3] = {ag_q_add(xf[0], H.sp[0]), ag_q_add(xf[1], H.sp[1]), ag_q_add(xf[2], H.sp[2])};
-                ag_fast_sun_near<false>(E.pv, c, d, acc, nullptr);
-            }
+            cs = !(rs2 >= AG_SUN_H_FAR2 && rs2 < 1e30f);
+            if (!cs) ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, acc);
         }
         if (wild) {
             near = (1u << (2 * (p1 - p0))) - 1u;
