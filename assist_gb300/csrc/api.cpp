@@ -19,6 +19,7 @@
 
 #include "../../include/assist.h"
 #include "device_forces.cuh"
+#include "batch_ws.h"
 #include "fast_forces.cuh"
 #include "internal.h"
 #include "shared_sim.h"
@@ -1210,9 +1211,9 @@ static int ag_batch_prepare(const struct assist_ephem* e, const struct assist_gb
     return ASSIST_SUCCESS;
 }
 
-/* Doubles of the global workspace of a launch plan's kernels. */
-static size_t ag_plan_ws_doubles(const AgLaunchPlan& P, int n_var) {
-    return ag_batch_ws_doubles(P.nslots, n_var) + (P.fast && n_var ? ag_batch_ws_doubles(P.deep_slots, n_var) : 0);
+/* The global workspace of a launch plan's kernels. */
+static AgBatchWs ag_plan_ws(const AgLaunchPlan& P, int n_var) {
+    return ag_batch_ws(ag_batch_ws_doubles(1, n_var), P.nslots, P.fast ? P.deep_slots : 0);
 }
 
 /* The stream that a launch plan with groups on both kernels forks, and its two
@@ -1256,7 +1257,7 @@ static int ag_launch_plan(const AgLaunchPlan& P, const AgBatchArgs& a, int n_var
     d.n_groups = P.n_deep;
     d.nslots = P.deep_slots;
     d.queue = a.queue + 1;
-    if (n_var) d.ws = a.ws + ag_batch_ws_doubles(P.nslots, n_var);
+    d.ws = a.ws + ag_plan_ws(P, n_var).deep_at;
     if (!f.n_groups) return ag_launch_coop(P.D, P.c, d, n_var, n_var ? P.occ : 2, 0, s);
     int e = (int)cudaEventRecord(F.fork, s);
     if (!e) e = (int)cudaStreamWaitEvent(F.side, F.fork, 0);
@@ -1311,7 +1312,7 @@ static int ag_integrate_batch(const struct assist_ephem* e, const struct assist_
             ag_cuda_check(cudaMalloc(&g_batch.d_counters, cnt_bytes), "cudaMalloc"))
             return ASSIST_ERROR_EPHEM_FILE;
     }
-    const size_t wsn = ag_plan_ws_doubles(P, n_var);
+    const size_t wsn = ag_plan_ws(P, n_var).total;
     if (wsn > g_batch.ws_cap) {
         if (g_batch.d_ws) cudaFree(g_batch.d_ws);
         g_batch.d_ws = nullptr;
@@ -1441,7 +1442,7 @@ extern "C" int assist_gb300_plan_create(const struct assist_ephem* e, const stru
     }
     const AgLaunchPlan& P = p->P;
     const int ng = (int)P.gstart.size();
-    const size_t wsn = ag_plan_ws_doubles(P, n_var);
+    const size_t wsn = ag_plan_ws(P, n_var).total;
     bool ok = !ag_cuda_check(cudaMalloc(&p->d_order, sizeof(int) * (size_t)n), "cudaMalloc(plan order)") &&
               (!P.grouped || !ag_cuda_check(cudaMalloc(&p->d_grp, sizeof(int) * 2 * (size_t)ng), "cudaMalloc(plan groups)")) &&
               !ag_cuda_check(cudaMalloc(&p->d_queue, 2 * sizeof(int)), "cudaMalloc(plan queue)") &&

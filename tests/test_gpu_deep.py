@@ -201,3 +201,40 @@ def test_split_batches_and_their_plans(files, n, n_fly, nv, dense):
         assert (status.cpu().numpy() == 0).all()
         assert torch.equal(st, got[0][0]) and (not nv or torch.equal(vs, got[0][1]))
     plan.close()
+
+
+LEARNED = """
+import sys
+import numpy as np, torch
+from assist_gb300 import Ephem, batch
+from tests.test_gpu_deep import _mixed
+from assist_gb300 import warm
+pl, ast, out = sys.argv[1:4]
+warm.set_params(np.zeros(warm.n_params()))          # a correction of nothing
+d = np.load(out)
+dev = lambda a: torch.tensor(a, device="cuda")
+st = dev(d["state"])
+status = torch.full((len(st),), -1, dtype=torch.int32, device="cuda")
+batch.integrate_batch_device(Ephem(pl, ast), dev(d["t0"]), dev(d["te"]), st, status=status, opts=batch.options(warm_start=2))
+torch.cuda.synchronize()
+np.savez(out, state=st.cpu().numpy(), status=status.cpu().numpy(), deep=batch.last_deep_groups())
+"""
+
+
+def test_learned_batch_of_deep_groups_only(files, tmp_path):
+    """The learned start with every group deep, in a process whose first batch
+    this is: the workspace is this batch's alone."""
+    import os
+    import subprocess
+    import sys
+    from tests.oracle_py import Oracle
+    pl, ast, _ = files
+    state, t0, te = _mixed(files, 0, 40, 100.0, 5)
+    f = str(tmp_path / "batch.npz")
+    np.savez(f, state=state, t0=t0, te=te)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", LEARNED, pl, ast, f], check=True, cwd=root, timeout=300)
+    got = np.load(f)
+    assert (got["status"] == 0).all() and got["deep"] >= 2
+    ref = Oracle(pl, ast).integrate_batch(t0, te, state)
+    assert np.abs(got["state"][:, :3] - ref[:, :3]).max() < 1e-9
