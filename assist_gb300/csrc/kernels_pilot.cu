@@ -213,8 +213,9 @@ __global__ void __launch_bounds__(128) ag_k_deep(const DevEphem* __restrict__ Ep
     const int limit = 1000 + (int)fminf(2.0f * span, 60000.0f);
     int found = 0;
     ag_deep_acc<true>(grid, G, idt, gm, mu, sub, x, w, j, u, a, w2, reach, q);
-    for (int s = 0; s < limit; s++) {
-        if (run && q < AG_DEEP) { found = 1; run = false; }
+    /* the warp's lanes leave the loop together (its shuffles are the whole warp's) */
+    for (int s = 0;; s++) {
+        if (run && (s == limit || q < AG_DEEP)) { found = 1; run = false; }
         const float rem = sgn * ((float)(jb - j) + (ub - u)) * (float)dt, h = fminf(fminf(c * rsqrtf(w2), 0.25f * reach), rem);
         if (!(h > 0.0f)) run = false;
         if (!__any_sync(0xffffffffu, run)) break;
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(128) ag_k_deep(const DevEphem* __restrict__ Ep
         u = ue;
         ag_deep_acc<true>(grid, G, idt, gm, mu, sub, x, w, j, u, a, w2, reach, q);
     }
-    if ((run || found) && sub == 0) deep[i] = 1;     /* run: not searched to its end */
+    if (found && sub == 0) deep[i] = 1;
 }
 
 /* The ratios; DEEP: also list[1 .. list[0]] (list[0] zero before), the

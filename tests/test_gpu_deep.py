@@ -203,6 +203,27 @@ def test_split_batches_and_their_plans(files, n, n_fly, nv, dense):
     plan.close()
 
 
+def test_step_limits_of_unequal_spans(files):
+    """Satellites of the Earth, whose search ends at its step limit (1,000 and
+    two a day), with spans from 30 to 440 days beside each other in a warp, and
+    main-belt particles among them."""
+    from assist_gb300 import Ephem, synth
+    pl, ast, system = files
+    ep, ev = system.body(3, np.array(T0))
+    gm = 2.9591220828559115e-4 * 3.003e-6
+    pop = synth.population(system, "mba", 24, seed=3, t0=T0)
+    state, te = pop.state.copy(), np.full(24, T0 + 100.0)
+    sat = np.arange(24) % 3 != 2
+    for i in np.flatnonzero(sat):
+        r = 0.0100 * (0.10 + 0.0007 * i)
+        u, w = np.eye(3)[i % 3], np.eye(3)[(i + 1) % 3]
+        state[i] = np.concatenate([ep + r * u, ev + (gm / r) ** 0.5 * w])
+        te[i] = T0 + 30.0 + 17.8 * i
+    flags = _flags(Ephem(pl, ast), np.full(24, T0), te, state)
+    long = sat & (te - T0 > 200.0)
+    assert flags[long].all() and not flags[~sat].any()
+
+
 LEARNED = """
 import sys
 import numpy as np, torch
