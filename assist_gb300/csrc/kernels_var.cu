@@ -23,7 +23,7 @@
  *
  * What bounds it is the latency of a node (role 4's FP64 Jacobian and the
  * components' two tasks a thread); 70 near-Earth particles over 60 days, 9
- * blocks: 22.0 ms with a launch a step and 32 particles a block in FP64, 6.1
+ * blocks: 22.0 ms with a launch a step and 32 particles a block in FP64, 6.5
  * here.  The step rules are those of kernels_shared.cu's run kernel
  * (variational particles never enter the error measures).
  */

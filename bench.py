@@ -79,12 +79,12 @@ IAS_PER_STEP = 3 * (2 * 9 + 2 * 8 + 8 + 7 * 8)
 
 # From one ncu capture of the pair-term kernel (two-blocks-per-SM build) on the
 # 32,768-particle case of this workload
-# (profiles/ag_k_fast_32768_mixture_1yr.md: 10.1 MB read + written for 11.97M
+# (profiles/ag_k_fast_32768_mixture_1yr.md: 11.3 MB read + written for 11.97M
 # particle-days): DRAM bytes per particle-day of a launch, scaled to a full
 # launch by its particle-days.
-DRAM_BYTES_PER_PARTICLE_DAY = 0.845
+DRAM_BYTES_PER_PARTICLE_DAY = 0.942
 # Share of the active cycles in which the FP64 pipe is busy (ncu, the same case).
-FP64_PIPE_BUSY = 0.67
+FP64_PIPE_BUSY = 0.65
 
 
 def _synth():
