@@ -420,7 +420,7 @@ __device__ __forceinline__ AgF2 ag_q_dot(const AgF2* a, const AgF2* b) {
     return ag_q_add(ag_q_mul(a[0], b[0]), ag_q_add(ag_q_mul(a[1], b[1]), ag_q_mul(a[2], b[2])));
 }
 
-/* The Sun's J2 between 0.1 and 0.5 AU, in float pairs: there it is up to 1e-9
+/* The Sun's J2 between 0.1 and 0.5 AU, in float pairs: there it is up to 1.5e-9
  * of the acceleration, and its FP32 form's error was 2.5e-16 rms of it at 0.11
  * AU, as much as the whole FP64 sum's (1.2e-17 at 0.5 AU).  With the pole n,
  * z = d.n, c = z / |d|, k = GM 3/2 J2 R^2 / |d|^5: k ((5 c^2 - 1) d - 2 z n)
@@ -815,7 +815,7 @@ __device__ __forceinline__ void ag_fast_force(int w, int lane, bool on, const De
             if (!ce) ag_fast_earth_h(E.pv, c, q, r2, acc);
         }
         if (w == 2 && (c.forces & AG_F_SUN_H)) {
-            /* J2: below 4e-11 of the acceleration beyond 0.5 AU */
+            /* J2: below 6e-11 of the acceleration beyond 0.5 AU */
             cs = !(rs2 >= AG_SUN_H_FAR2 && rs2 < 1e30f);
             if (!cs) ag_fast_sun_h(E.pv, c, sx, sy, sz, rs2, acc);
         }
